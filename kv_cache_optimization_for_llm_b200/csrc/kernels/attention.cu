@@ -73,7 +73,7 @@ paged_attention_generic_kernel(const T* __restrict__ q_base, int q_row_stride,
     const float m_new = fmaxf(m, cm);
     const float corr = (m == -CUDART_INF_F) ? 0.f : expf(m - m_new);
     const float p = (off >= 0) ? expf(s - m_new) : 0.f;
-    l = l * corr + warp_sum(p);
+    l = fmaf(l, corr, warp_sum(p));
 #pragma unroll
     for (int r = 0; r < kMaxHeadDim / 32; ++r) acc[r] *= corr;
     const int n_in_chunk = min(32, pos - c * 32 + 1);
@@ -104,12 +104,12 @@ paged_attention_generic_kernel(const T* __restrict__ q_base, int q_row_stride,
     float L = 0.f, f[kWarps];
     for (int w = 0; w < kWarps; ++w) {
       f[w] = (m_s[w] == -CUDART_INF_F) ? 0.f : expf(m_s[w] - M);
-      L += l_s[w] * f[w];
+      L = fmaf(l_s[w], f[w], L);
     }
     T* o = out + ((size_t)t * nq + h) * d;
     for (int i = lane; i < d; i += 32) {
       float a = 0.f;
-      for (int w = 0; w < kWarps; ++w) a += acc_s[w][i] * f[w];
+      for (int w = 0; w < kWarps; ++w) a = fmaf(acc_s[w][i], f[w], a);
       o[i] = from_f32<T>(L > 0.f ? a / L : 0.f);
     }
   }
@@ -131,6 +131,247 @@ KVB_EXPORT int kvb_paged_attention_generic(const void* q, int q_row_stride, cons
                                             (const T*)q, q_row_stride, (const T*)k_pages, (const T*)v_pages,
                                             block_table, max_pages, page_size, num_pages, positions, token_req,
                                             (T*)out, nq, nkv, d, scale, window, status)));
+  return kvb_launch_result();
+}
+
+// ===========================================================================
+// The general attention over tiles of query rows (float32 steps with runs of tokens): the same sums as the kernel above, to
+// the bit, so that a token's result does not depend on which of the two its step was given to.
+//
+// A block takes a tile of consecutive tokens of one request with all query heads of one key/value head, up to 8 RT rows (token,
+// head), and brings every chunk of 32 keys and values into shared memory once for the whole tile.  Its four groups of 64 threads
+// are the four warps of the kernel above: group g takes the chunks c with c % 4 == g, with a maximum, a sum and a weighted
+// sum of values of its own, merged at the end in the same order.  Within a group a thread stands at row 8 r + ty (r < RT) and
+// keys tx, tx + 8, tx + 16, tx + 24 of the chunk: every score is one chain of fmaf over the head's channels; the 32
+// exponentials are added as warp_sum adds them (partners 16, 8, 4, 2, 1 apart); a value channel is one chain over the keys
+// in order.  A key that a row does not see adds nothing to any of the three.
+//
+// What bounds it: the kernel above reads a key's channels one by one, a lane per key (32 rows a warp and load), and every
+// (token, head) reads them again: 575 us for 333 + 5 tokens of 32 heads of 64 over 8 key/value heads.  Here the loads are 16
+// bytes wide and shared by the tile: 95 us.
+constexpr int kTileThreads = 256;
+
+// floats of a group's chunk of keys, in whose place its exponentials are kept
+__host__ __device__ constexpr int tile_key_floats(int dmax, int rt) {
+  return 32 * (dmax + 4) > 8 * rt * 36 ? 32 * (dmax + 4) : 8 * rt * 36;
+}
+
+template <int DMAX, int RT>
+__global__ void __launch_bounds__(kTileThreads)
+paged_attention_tiles_kernel(const float* __restrict__ q_base, int q_row_stride, const float* __restrict__ k_pages,
+                             const float* __restrict__ v_pages, const int* __restrict__ block_table, int max_pages,
+                             int page_size, int num_pages, const int* __restrict__ positions, const int4* __restrict__ tiles,
+                             float* __restrict__ out, int nq, int nkv, int d, float scale, int window, int* status) {
+  constexpr int ROWS = 8 * RT, LD = DMAX + 4, LDP = 36, DT = DMAX / 32;      // DT: groups of four channels a thread owns
+  constexpr int KREG = tile_key_floats(DMAX, RT), PER_GROUP = KREG + 32 * LD;
+  extern __shared__ __align__(16) float tsm[];
+  float* q_s = tsm;                                    // [ROWS][LD]
+  const int tid = threadIdx.x, g = tid >> 6, gt = tid & 63, tx = gt & 7, ty = gt >> 3;
+  float* k_s = q_s + ROWS * LD + g * PER_GROUP;        // [32][LD]
+  float* v_s = k_s + KREG;                             // [32][LD]
+  float* p_s = k_s;                                    // [ROWS][LDP], once the scores are made
+  __shared__ float m_s[kWarps][ROWS], l_s[kWarps][ROWS];
+  pdl_trigger();
+  pdl_wait();
+  const int4 tile = tiles[blockIdx.x];
+  const int hk = blockIdx.y, group = nq / nkv, rows = tile.z * group, nr = (rows + 7) / 8;     // r < nr: rows that exist
+  const int* table = block_table + (size_t)tile.x * max_pages;
+  int pos_lo = 0x7fffffff, pos_hi = -1;                // of the tile's tokens
+  for (int t = 0; t < tile.z; ++t) {
+    const int p = positions[tile.y + t];
+    pos_lo = min(pos_lo, p);
+    pos_hi = max(pos_hi, p);
+  }
+  const int d4 = d >> 2;
+  for (int x = tid; x < ROWS * d4; x += kTileThreads) {
+    const int row = x / d4, i = (x - row * d4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < rows)
+      v = *reinterpret_cast<const float4*>(q_base + (size_t)(tile.y + row / group) * q_row_stride + (size_t)(hk * group + row % group) * d + i);
+    *reinterpret_cast<float4*>(q_s + row * LD + i) = v;
+  }
+  int pos[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) pos[r] = 8 * r + ty < rows ? positions[tile.y + (8 * r + ty) / group] : -1;
+  __syncthreads();
+
+  float m[RT], l[RT], acc[RT][4 * DT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    m[r] = -CUDART_INF_F;
+    l[r] = 0.f;
+#pragma unroll
+    for (int x = 0; x < 4 * DT; ++x) acc[r][x] = 0.f;
+  }
+  const int first = (window > 0 ? max(0, pos_lo - window + 1) : 0) / 32;
+  for (int c = first + ((g - first) % kWarps + kWarps) % kWarps; c * 32 <= pos_hi; c += kWarps) {
+    // bit k of `mapped`: key k of the chunk lies in a page (the same word in every thread of the warp)
+    bool mine = false;
+    {
+      const int j = c * 32 + (tid & 31);
+      const int lp = j / page_size;
+      const int page = j <= pos_hi && lp < max_pages ? table[lp] : -1;
+      mine = page >= 0 && page < num_pages;
+      if (!mine && j <= pos_hi && (window <= 0 || j > pos_lo - window)) atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE);
+    }
+    const unsigned mapped = __ballot_sync(0xffffffffu, mine);
+    for (int x = gt; x < 32 * d4; x += 64) {
+      const int kk = x / d4, i = (x - kk * d4) * 4, j = c * 32 + kk;
+      float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+      if (mapped >> kk & 1) {
+        const long long off = (((long long)table[j / page_size] * nkv + hk) * page_size + (j % page_size)) * d + i;
+        kv = *reinterpret_cast<const float4*>(k_pages + off);
+        vv = *reinterpret_cast<const float4*>(v_pages + off);
+      }
+      *reinterpret_cast<float4*>(k_s + kk * LD + i) = kv;
+      *reinterpret_cast<float4*>(v_s + kk * LD + i) = vv;
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+    float s[RT][4];
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[r][u] = 0.f;
+    for (int i = 0; i < d; i += 4) {
+      float4 kv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) kv[u] = *reinterpret_cast<const float4*>(k_s + (tx + 8 * u) * LD + i);
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        if (r >= nr) break;
+        const float4 qv = *reinterpret_cast<const float4*>(q_s + (8 * r + ty) * LD + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          s[r][u] = fmaf(qv.x, kv[u].x, s[r][u]);
+          s[r][u] = fmaf(qv.y, kv[u].y, s[r][u]);
+          s[r][u] = fmaf(qv.z, kv[u].z, s[r][u]);
+          s[r][u] = fmaf(qv.w, kv[u].w, s[r][u]);
+        }
+      }
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+    bool whole = mapped == 0xffffffffu;                // every row of this thread sees every key of the chunk
+#pragma unroll
+    for (int r = 0; r < RT; ++r) {
+      if (r >= nr) break;
+      unsigned seen = 0;                               // bit u: key tx + 8 u
+      float cm = -CUDART_INF_F;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int kk = tx + 8 * u, j = c * 32 + kk;
+        const bool on = j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> kk & 1);
+        s[r][u] = on ? s[r][u] * scale : -CUDART_INF_F;
+        seen |= (on ? 1u : 0u) << u;
+        cm = fmaxf(cm, s[r][u]);
+      }
+      whole = whole && c * 32 + 31 <= pos[r] && (window <= 0 || c * 32 > pos[r] - window);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+      const float m_new = fmaxf(m[r], cm);
+      const float corr = m[r] == -CUDART_INF_F ? 0.f : expf(m[r] - m_new);
+      float p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        p[u] = seen >> u & 1 ? expf(s[r][u] - m_new) : 0.f;
+        p_s[(8 * r + ty) * LDP + tx + 8 * u] = p[u];
+      }
+      float sum = (p[0] + p[2]) + (p[1] + p[3]);       // keys 16 apart, then 8 apart
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (cm != -CUDART_INF_F) {                       // a row that sees nothing of the chunk stays as it is
+        l[r] = fmaf(l[r], corr, sum);
+#pragma unroll
+        for (int x = 0; x < 4 * DT; ++x) acc[r][x] *= corr;
+        m[r] = m_new;
+      }
+    }
+    __syncwarp();
+    for (int jj = 0; jj < 32; jj += 4) {
+      float4 pv[RT];
+#pragma unroll
+      for (int r = 0; r < RT; ++r) pv[r] = *reinterpret_cast<const float4*>(p_s + (8 * r + ty) * LDP + jj);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float4 vv[DT];
+#pragma unroll
+        for (int x = 0; x < DT; ++x) vv[x] = *reinterpret_cast<const float4*>(v_s + (jj + u) * LD + 32 * x + 4 * tx);
+        const int j = c * 32 + jj + u;
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          if (r >= nr) break;
+          const float pj = u == 0 ? pv[r].x : u == 1 ? pv[r].y : u == 2 ? pv[r].z : pv[r].w;
+          // a value that the row does not see is left out, whatever it holds
+          if (whole || (j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> (jj + u) & 1))) {
+#pragma unroll
+            for (int x = 0; x < DT; ++x) {
+              acc[r][4 * x + 0] = fmaf(pj, vv[x].x, acc[r][4 * x + 0]);
+              acc[r][4 * x + 1] = fmaf(pj, vv[x].y, acc[r][4 * x + 1]);
+              acc[r][4 * x + 2] = fmaf(pj, vv[x].z, acc[r][4 * x + 2]);
+              acc[r][4 * x + 3] = fmaf(pj, vv[x].w, acc[r][4 * x + 3]);
+            }
+          }
+        }
+      }
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+  }
+
+  // merge: every group leaves its weighted sums where its chunks of keys and values lay
+  float* acc_s = k_s;                                  // [ROWS][LD]
+  static_assert(ROWS * LD <= PER_GROUP, "the weighted sums take the room of both chunks");
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    const int row = 8 * r + ty;
+#pragma unroll
+    for (int x = 0; x < DT; ++x)
+      *reinterpret_cast<float4*>(acc_s + row * LD + 32 * x + 4 * tx) =
+          make_float4(acc[r][4 * x], acc[r][4 * x + 1], acc[r][4 * x + 2], acc[r][4 * x + 3]);
+    if (tx == 0) { m_s[g][row] = m[r]; l_s[g][row] = l[r]; }
+  }
+  __syncthreads();
+  const float* acc0 = q_s + ROWS * LD;
+  for (int x = tid; x < rows * d; x += kTileThreads) {
+    const int row = x / d, i = x - row * d;
+    float M = m_s[0][row];
+    for (int w = 1; w < kWarps; ++w) M = fmaxf(M, m_s[w][row]);
+    float L = 0.f, a = 0.f;
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = m_s[w][row] == -CUDART_INF_F ? 0.f : expf(m_s[w][row] - M);
+      L = fmaf(l_s[w][row], f, L);
+      a = fmaf(acc0[(size_t)w * PER_GROUP + row * LD + i], f, a);
+    }
+    out[((size_t)(tile.y + row / group) * nq + hk * group + row % group) * d + i] = L > 0.f ? a / L : 0.f;
+  }
+}
+
+// Tokens in one tile of the kernel above (0: it does not take these sizes): 64 rows at head sizes up to 64, 32 up to 128.
+KVB_EXPORT int kvb_paged_attention_tile_tokens(int d, int group) {
+  if (d < 4 || d > 128 || d % 4 || group < 1) return 0;
+  return (d <= 64 ? 64 : 32) / group;
+}
+
+// tiles [n_tiles, 4]: request row, first token row, tokens (at most kvb_paged_attention_tile_tokens), 0.  float32 only; q, the
+// pages and their rows start on 16-byte boundaries.
+KVB_EXPORT int kvb_paged_attention_tiles(const float* q, int q_row_stride, const float* k_pages, const float* v_pages,
+                                         const int* block_table, int max_pages, int page_size, int num_pages,
+                                         const int* positions, const int* tiles, int n_tiles, float* out, int nq, int nkv,
+                                         int d, float scale, int window, int* status, cudaStream_t stream) {
+  if (n_tiles <= 0) return 0;
+  if (nkv < 1 || nkv > 65535 || nq % nkv || kvb_paged_attention_tile_tokens(d, nq / nkv) < 1) return KVB_ERR_BAD_SIZE;
+  if (q_row_stride % 4 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_pages) |
+                            reinterpret_cast<uintptr_t>(v_pages) | reinterpret_cast<uintptr_t>(tiles)) & 15)) return KVB_ERR_ALIGN;
+#define KVB_TILES(DMAX, RT)                                                                                            \
+  {                                                                                                                    \
+    constexpr int smem = (8 * RT * (DMAX + 4) + kWarps * (tile_key_floats(DMAX, RT) + 32 * (DMAX + 4))) * (int)sizeof(float); \
+    cudaError_t e = cudaFuncSetAttribute(paged_attention_tiles_kernel<DMAX, RT>,                                       \
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                           \
+    if (e != cudaSuccess) return (int)e;                                                                               \
+    kvb_launch(paged_attention_tiles_kernel<DMAX, RT>, dim3(n_tiles, nkv), dim3(kTileThreads), smem, stream, q,        \
+               q_row_stride, k_pages, v_pages, block_table, max_pages, page_size, num_pages, positions,                \
+               reinterpret_cast<const int4*>(tiles), out, nq, nkv, d, scale, window, status);                          \
+  }
+  if (d <= 64) KVB_TILES(64, 8) else KVB_TILES(128, 4)
+#undef KVB_TILES
   return kvb_launch_result();
 }
 

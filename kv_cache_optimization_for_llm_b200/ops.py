@@ -807,6 +807,38 @@ def paged_attention_generic(qkv, k_pages, v_pages, block_table, positions, token
     return out
 
 
+_attention_tile_tokens: Dict[tuple, int] = {}
+
+
+def paged_attention_tile_tokens(d: int, group: int) -> int:
+    """Query tokens in one tile of :func:`paged_attention_tiles` (0: these sizes are refused)."""
+    key = (int(d), int(group))
+    if key not in _attention_tile_tokens:
+        _attention_tile_tokens[key] = int(lib("attention").kvb_paged_attention_tile_tokens(c_int(key[0]), c_int(key[1])))
+    return _attention_tile_tokens[key]
+
+
+def paged_attention_tiles_supported(qkv, k_pages, v_pages, d: int, group: int) -> bool:
+    """Whether :func:`paged_attention_tiles` takes these sizes and addresses (16-byte accesses)."""
+    return (paged_attention_tile_tokens(d, group) > 0 and qkv.stride(0) % 4 == 0 and qkv.data_ptr() % 16 == 0
+            and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0)
+
+
+def paged_attention_tiles(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window) -> torch.Tensor:
+    """:func:`paged_attention_generic` for float32 steps with runs of tokens, with the same result to the bit: a block takes a
+    tile of tokens with all heads of a group, so that keys and values are read once for all of them."""
+    _need_cuda(qkv, k_pages)
+    tiles = tiles_of_height(batch, paged_attention_tile_tokens(d, nq // nkv))
+    out = new((qkv.shape[0], nq * d), qkv.dtype, qkv.device)
+    rc = lib("attention").kvb_paged_attention_tiles(
+        _p(qkv), c_int(qkv.stride(0)), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]),
+        c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), _p(batch.positions), _p(tiles), c_int(tiles.shape[0]), _p(out),
+        c_int(nq), c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)), _p(batch.status), _stream())
+    _check(rc, "paged_attention_tiles")
+    choices["paged_attention_tiles"] += 1
+    return out
+
+
 def kv_rows_append(src: torch.Tensor, k_off: int, v_off: int, pages: torch.Tensor, block_table, batch,
                    kv_heads: int, dk: int, dv: int) -> None:
     """Writes the step's keys (``src[:, k_off : k_off + kv_heads * dk]``) and values (from ``v_off``) into the
@@ -2120,7 +2152,8 @@ def attention_step(qkv, k_pages, v_pages, write_kv, block_table, batch, nq, nkv,
     encoding, the write of keys and values into their pages, attention over the pages.
     Picks the kernels:
     * float32: rotary/write kernel, then the general kernel, whose sums follow absolute
-      positions in one fixed order whatever the shape of the step;
+      positions in one fixed order whatever the shape of the step; steps with runs of tokens and head sizes up to 128
+      take its form over tiles of queries, which makes the same sums to the bit;
     * bfloat16, single tokens only: one fused launch, on tensor cores where the sizes allow
       (head size 64/128), else the FMA form (head size 32);
     * bfloat16, runs of tokens: rotary/write kernel, then the tensor-core kernel; single tokens
@@ -2152,6 +2185,9 @@ def attention_step(qkv, k_pages, v_pages, write_kv, block_table, batch, nq, nkv,
                   v_pages if write_kv else None, block_table, page_size, nq, nkv, d, rot, batch.status)
     if qkv.dtype == torch.bfloat16 and not batch.decode_only and flash_attention_supported(d, group, page_size):
         return flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window)
+    if (qkv.dtype == torch.float32 and not batch.decode_only
+            and paged_attention_tiles_supported(qkv, k_pages, v_pages, d, group)):
+        return paged_attention_tiles(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window)
     return paged_attention_generic(qkv, k_pages, v_pages, block_table, batch.positions, batch.token_req,
                                    nq, nkv, d, scale, window, batch.status)
 

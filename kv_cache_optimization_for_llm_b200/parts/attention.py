@@ -74,11 +74,13 @@ class GroupedQueryAttention(Part):
         return [(self.nq + 2 * self.nkv) * self.d, self.nq * self.d, 2 * hidden]
 
     def query_tile_heights(self):
-        """Tokens per tile of the tensor-core attention for prompt portions (bfloat16, head sizes
-        it takes): the step's batch lays the tiles out for them."""
-        if self.ctx.dtype != torch.bfloat16 or self.d not in (64, 128):
-            return []
+        """Tokens per tile of the attention for prompt portions (float32, or bfloat16 with the head sizes that the
+        tensor-core kernels take): the step's batch lays the tiles out for them."""
         g = self.nq // self.nkv
+        if self.ctx.dtype == torch.float32:
+            return [ops.paged_attention_tile_tokens(self.d, g)]
+        if self.d not in (64, 128):
+            return []
         return [ops.flash_tokens_per_tile(g, False), ops.flash_tokens_per_tile(g, True)]
 
     def forward(self, x, batch, cache, into=None):

@@ -1,0 +1,76 @@
+"""The float32 path's product over tiles and its attention over tiles of queries: every tile gives the same bits, and the
+attention the bits of the general kernel."""
+
+import ctypes
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from test_kernels_gpu import _attention_case, as64, dev, status
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 63, 17), (16, 64, 16), (33, 65, 40), (95, 129, 100), (129, 127, 260), (257, 320, 64)])
+def test_every_tile_of_the_float32_product_gives_the_same_bits(M, N, K):
+    from kv_cache_optimization_for_llm_b200 import ops
+    rng = np.random.default_rng(M * N + K)
+    a, w = rng.normal(size=(M, K)).astype(np.float32), rng.normal(size=(N, K)).astype(np.float32)
+    # the same values once more with rows that start on odd addresses
+    wide = dev(np.concatenate([a, a[:, :1]], axis=1))[:, :K]
+    A, W = dev(a), dev(w)
+    ref = a.astype(np.float64) @ w.astype(np.float64).T
+    # float32 FMA chains of length K: error ~ K * 2^-24 relative to the sum of magnitudes
+    bound = (np.abs(a).astype(np.float64) @ np.abs(w).astype(np.float64).T) * K * 2.0 ** -24 + 1e-30
+    first = ops.linear(A, W)
+    assert (np.abs(as64(first) - ref) <= bound).all()
+    assert torch.equal(ops.linear(wide, W), first)
+    for tile in range(6):
+        out = torch.full((M, N + 3), 7.0, device="cuda")
+        rc = ops.lib("gemm_f32").kvb_sgemm_nt_tile(ops._p(A), K, ops._p(W), K, ops._p(out), N + 3, M, N, K, tile,
+                                                   ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        assert torch.equal(out[:, :N], first) and bool((out[:, N:] == 7.0).all()), tile
+
+
+class _Batch:
+    def __init__(self, c, tile, st):
+        self.positions, self.status = c["positions"], st
+        qs = c["q_start"].tolist()
+        rows = [[r, t, min(tile, b - t), 0] for r, (a, b) in enumerate(zip(qs, qs[1:])) for t in range(a, b, tile)]
+        self.tiles = {tile: dev(rows, torch.int32)}
+
+
+@pytest.mark.parametrize("nq,nkv,d,page_size,window", [
+    (4, 2, 16, 4, None), (6, 1, 32, 16, None), (5, 5, 48, 16, None), (8, 2, 64, 16, None), (32, 8, 64, 16, None),
+    (3, 1, 128, 32, None), (24, 8, 128, 16, None), (4, 2, 64, 16, 37), (6, 3, 32, 4, 5), (8, 2, 80, 8, 33)])
+def test_attention_over_tiles_gives_the_bits_of_the_general_kernel(nq, nkv, d, page_size, window):
+    from kv_cache_optimization_for_llm_b200 import ops
+    c = _attention_case("float32", nq, nkv, d, ctxs=[1, 33, 130, 64, 257, 300], q_lens=[1, 33, 2, 1, 40, 129],
+                        page_size=page_size, window=window, seed=d + nq)
+    scale, st = 1 / math.sqrt(d), status()
+    # values that later positions of a request hold must not reach earlier ones, whatever they are
+    page, slot = int(c["table"][5, 299 // page_size]), 299 % page_size
+    c["vp"][page, :, slot] = float("inf")
+    ref = ops.paged_attention_generic(c["qkv"], c["kp"], c["vp"], c["table"], c["positions"], c["token_req"], nq, nkv, d, scale,
+                                      window, st)
+    tile = ops.paged_attention_tile_tokens(d, nq // nkv)
+    assert tile > 0
+    out = ops.paged_attention_tiles(c["qkv"], c["kp"], c["vp"], c["table"], _Batch(c, tile, st), nq, nkv, d, scale, window)
+    assert int(st.item()) == 0
+    assert bool(torch.isfinite(out[:-1]).all())
+    assert torch.equal(out[:-1], ref[:-1])
+    assert torch.equal(torch.nan_to_num(out[-1]), torch.nan_to_num(ref[-1]))
+
+
+def test_attention_over_tiles_reports_an_unmapped_page():
+    from kv_cache_optimization_for_llm_b200 import ops
+    c = _attention_case("float32", 4, 2, 16, ctxs=[40], q_lens=[3], page_size=4, window=None, seed=1)
+    c["table"][0, 3] = -1
+    st = status()
+    args = (c["qkv"], c["kp"], c["vp"], c["table"])
+    out = ops.paged_attention_tiles(*args, _Batch(c, ops.paged_attention_tile_tokens(16, 2), st), 4, 2, 16, 0.25, None)
+    assert int(st.item()) == 1
+    assert torch.equal(out, ops.paged_attention_generic(*args, c["positions"], c["token_req"], 4, 2, 16, 0.25, None, st))
