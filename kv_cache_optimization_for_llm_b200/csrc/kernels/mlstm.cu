@@ -28,6 +28,7 @@
 //           (m' = max(F + m, m_c);  C' = exp(F + m - m') C + exp(m_c - m') C_c)
 //   FINAL   every chunk from what it begins with, writing y; the run's last chunk leaves the state in the slot
 // A run of one chunk reads and writes its slot directly.
+#include "chunk_walk.cuh"
 #include "common.cuh"
 
 #include <math_constants.h>
@@ -336,6 +337,25 @@ KVB_EXPORT int kvb_mlstm_scan(const MlstmArgs* args, int R, int max_run, int dty
 #undef KVB_ML_VEC
 #undef KVB_ML_MODE
   return kvb_launch_result();
+}
+
+// The runs of requests first .. first + R - 1 walked in pieces of 64 tokens on tensor cores (chunk_walk.cuh): bfloat16, N 64 or
+// 128, Dv a multiple of 64, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).  The chunk fields are not read.
+KVB_EXPORT int kvb_mlstm_walk(const MlstmArgs* args, int first, int R, cudaStream_t stream) {
+  const MlstmArgs& p = *args;
+  if (R <= 0) return 0;
+  if (!(p.cap > 0.f)) return KVB_ERR_BAD_SIZE;
+  const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(p.qkv);
+  walk::Args a = {};
+  a.q = x + p.q_off; a.k = x + p.k_off; a.v = x + p.v_off;
+  a.ld = p.ld;
+  a.share = 1;
+  if (!walk::takes(p.N, p.Dv, a.q, a.k, a.v, a.ld)) return KVB_ERR_BAD_SIZE;
+  a.gates = p.gates; a.ld_g = p.ld_g; a.bi = p.bi; a.bf = p.bf; a.cap = p.cap; a.q_scale = p.q_scale;
+  a.state = p.state; a.slot_stride = p.slot_stride; a.y = p.y;
+  a.q_start = p.q_start; a.req_start = p.req_start; a.slots = p.slots;
+  a.H = p.H; a.Dv = p.Dv; a.first = first;
+  return walk::launch_any<walk::MLSTM>(a, p.N, R, stream);
 }
 
 // ---------------------------------------------------------------- a norm per head, a weight, a sigmoid gate

@@ -15,6 +15,7 @@
 // precisions.  A request that starts at position 0 starts from a zero state whatever its slot holds.  Sums run
 // in an order fixed by the sizes alone, so a token's result does not depend on how its request was cut into
 // steps or on the rest of the batch.
+#include "chunk_walk.cuh"
 #include "common.cuh"
 
 #include <math_constants.h>
@@ -521,6 +522,28 @@ KVB_EXPORT int kvb_ssd_scan(const SsdArgs* args, int R, int max_run, int dtype, 
 #undef KVB_SSD_VEC
 #undef KVB_SSD_MODE
   return kvb_launch_result();
+}
+
+// The runs of requests first .. first + R - 1 walked in pieces of 64 tokens on tensor cores (chunk_walk.cuh): bfloat16, N 64 or
+// 128, Dv a multiple of 64, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).  The chunk fields are not read.
+KVB_EXPORT int kvb_ssd_walk(const SsdArgs* args, int first, int R, cudaStream_t stream) {
+  const SsdArgs& p = *args;
+  if (R <= 0) return 0;
+  if (p.H < 1 || p.G < 1 || p.H % p.G) return KVB_ERR_BAD_SIZE;
+  walk::Args a = {};
+  a.v = static_cast<const __nv_bfloat16*>(p.xbc);
+  a.k = a.v + (size_t)p.H * p.Dv;
+  a.q = a.k + (size_t)p.G * p.N;
+  a.ld = p.ld_xbc;
+  a.share = p.H / p.G;
+  if (!walk::takes(p.N, p.Dv, a.q, a.k, a.v, a.ld)) return KVB_ERR_BAD_SIZE;
+  a.dt = static_cast<const __nv_bfloat16*>(p.dt);
+  a.ld_g = p.ld_dt;
+  a.dt_bias = p.dt_bias; a.A_log = p.A_log; a.D = p.D;
+  a.state = p.state; a.slot_stride = p.slot_stride; a.y = p.y;
+  a.q_start = p.q_start; a.req_start = p.req_start; a.slots = p.slots;
+  a.H = p.H; a.Dv = p.Dv; a.first = first;
+  return walk::launch_any<walk::SSD>(a, p.N, R, stream);
 }
 
 // ---------------------------------------------------------------- gate, then a norm per group of channels

@@ -1380,6 +1380,19 @@ def _chunk_rows(batch, chunk: int):
     return batch.num_reqs - first + batch.num_tokens // chunk + 1, first
 
 
+# bfloat16 steps with a run of at least this many tokens walk their runs in pieces of 64 tokens on tensor cores where the sizes
+# allow (the matrix states with one decay per head and token).  Measured at 32 heads of 64 x 64: WALK_MIN_MEASURED.
+WALK_MIN_RUN = int(os.environ.get('KVB200_WALK_MIN_RUN', '16'))
+
+
+def _walks(batch, n: int, dv: int, x: torch.Tensor, *columns: int) -> bool:
+    """Whether a step's runs go to the walk on tensor cores: bfloat16, a state of 64 or 128 rows, whole blocks of 64 value columns,
+    every segment of ``x``'s rows (from ``columns``) on a 16-byte boundary."""
+    return (x.dtype == torch.bfloat16 and n in (64, 128) and dv >= 64 and dv % 64 == 0 and x.stride(0) % 8 == 0
+            and all(_at(x, c) % 16 == 0 for c in columns)
+            and 0 < WALK_MIN_RUN <= int(getattr(batch, "max_q_len", 0) or 0))
+
+
 class _DiagArgs(ctypes.Structure):
     _fields_ = [("a", c_void_p), ("b", c_void_p), ("y", c_void_p), ("ld_y", c_int), ("y_bias", c_void_p),
                 ("out_scale", c_float), ("out", c_void_p), ("state", c_void_p), ("slot_stride", c_longlong),
@@ -1432,7 +1445,8 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
     step:  ``dt = softplus(dt_raw + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + dt B x^T``, ``y = S^T C + D x``.
     ``xbc`` [T, heads dv + 2 groups n]: x | B | C (head h reads group ``h // (heads / groups)``); ``dt``: (tensor, first
     column) of the raw step sizes [T, heads].  ``state``: float32 [slots, >= heads * dv * n], zero for a request
-    that starts at position 0.  Returns float32 y [T, heads * dv].  A step with a run of ``SCAN_CHUNK_MIN_RUN``
+    that starts at position 0.  Returns float32 y [T, heads * dv].  bfloat16 steps with runs of ``WALK_MIN_RUN`` tokens go to
+    the walk on tensor cores where the sizes allow (:func:`_walks`); otherwise a step with a run of ``SCAN_CHUNK_MIN_RUN``
     tokens or more walks chunks of its runs side by side (64 tokens a chunk, 128 from runs of 1024 on)."""
     _need_cuda(xbc, state)
     T = xbc.shape[0]
@@ -1444,6 +1458,19 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
     y = new((T, heads * dv), torch.float32, xbc.device)
     max_run = int(getattr(batch, "max_q_len", 0) or 0)
     chunk = first = local = carry = decay = 0
+    if _walks(batch, n, dv, xbc, 0, heads * dv, heads * dv + groups * n):
+        # single tokens beside the runs (the step's first requests) go token by token
+        singles = int(getattr(batch, "num_single", 0) or 0)
+        p = _SsdArgs(xbc.data_ptr(), xbc.stride(0), _at(dtt, dcol), dtt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(),
+                     d_skip.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), batch.q_start.data_ptr(),
+                     batch.req_start.data_ptr(), batch.slots.data_ptr(), heads, groups, n, dv, 0, 0, 0, 0, 0, 0)
+        if singles:
+            _check(lib("recurrence").kvb_ssd_scan(ctypes.byref(p), c_int(singles), c_int(1), c_int(dtype_code(xbc.dtype)), _stream()),
+                   "ssd_scan")
+        rc = lib("recurrence").kvb_ssd_walk(ctypes.byref(p), c_int(singles), c_int(batch.num_reqs - singles), _stream())
+        _check(rc, "ssd_scan")
+        choices["ssd_walk"] += 1
+        return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():
         chunk = 128 if max_run >= 1024 else 64
         rows, first = _chunk_rows(batch, chunk)
@@ -1537,7 +1564,8 @@ def mlstm_scan(p: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch
 
     ``p`` [T, ...] holds q (``heads * n`` from column ``q_off``; multiplied by ``q_scale``), k and v; ``gates`` float32
     [T, 2 heads]: the raw a, then the raw b.  ``state``: float32 [slots, >= mlstm_state_floats], empty (m = 0) for a
-    request that starts at position 0.  Returns float32 y [T, heads * dv].  A step with a run of
+    request that starts at position 0.  Returns float32 y [T, heads * dv].  bfloat16 steps with runs of ``WALK_MIN_RUN``
+    tokens go to the walk on tensor cores where the sizes allow (:func:`_walks`); otherwise a step with a run of
     ``SCAN_CHUNK_MIN_RUN`` tokens or more walks chunks of 64 tokens side by side."""
     _need_cuda(p, gates, state)
     T = p.shape[0]
@@ -1548,6 +1576,20 @@ def mlstm_scan(p: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch
     y = new((T, heads * dv), torch.float32, p.device)
     max_run = int(getattr(batch, "max_q_len", 0) or 0)
     chunk = first = local = carry = fsum = 0
+    if _walks(batch, n, dv, p, q_off, k_off, v_off):
+        # single tokens beside the runs (the step's first requests) go token by token
+        singles = int(getattr(batch, "num_single", 0) or 0)
+        a = _MlstmArgs(p.data_ptr(), p.stride(0), q_off, k_off, v_off, gates.data_ptr(), gates.stride(0),
+                       0 if bi is None else bi.data_ptr(), 0 if bf is None else bf.data_ptr(), float(cap), float(q_scale),
+                       state.data_ptr(), state.stride(0), y.data_ptr(), batch.q_start.data_ptr(), batch.req_start.data_ptr(),
+                       batch.slots.data_ptr(), heads, n, dv, 0, 0, 0, 0, 0)
+        if singles:
+            _check(lib("mlstm").kvb_mlstm_scan(ctypes.byref(a), c_int(singles), c_int(1), c_int(dtype_code(p.dtype)), _stream()),
+                   "mlstm_scan")
+        rc = lib("mlstm").kvb_mlstm_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), _stream())
+        _check(rc, "mlstm_scan")
+        choices["mlstm_walk"] += 1
+        return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():
         chunk = 64
         rows, first = _chunk_rows(batch, chunk)

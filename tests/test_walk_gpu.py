@@ -1,0 +1,141 @@
+"""The walk of long runs on tensor cores (matrix states with one decay per head and token), against the recurrence in float64 and
+beside the token-by-token kernels: pieces of 64 tokens that are full, one short, one over, runs that continue from a slot's
+state, single tokens beside runs, both widths of blocks, two blocks of value columns."""
+
+import numpy as np
+import pytest
+import torch
+
+from part_harness import _Manager
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(steps, slots):
+    """steps: (request, start, tokens) of one step; requests of single tokens come first in the batch."""
+    from kv_cache_optimization_for_llm_b200 import ops
+    from kv_cache_optimization_for_llm_b200.engine.batch import BatchBuilder, StepEntry
+    dev = torch.device("cuda:0")
+    b = BatchBuilder(4096, 64, [512], dev, ops.kernel_status(dev))
+    return b.build([StepEntry(r, [0] * n, s, ()) for r, s, n in steps], _Manager({r: list(range(512)) for r, _, _ in steps}, slots))
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+STEPS = [
+    [(0, 0, 64)], [(0, 0, 16), (1, 7, 63)], [(0, 0, 65), (1, 3, 1), (2, 0, 1), (3, 100, 200)], [(0, 5, 128), (1, 0, 129)],
+    [(0, 0, 700)], [(r, 2 * r, 17 + 30 * r) for r in range(9)],
+]
+
+
+def _ssd_plain(xbc, dt, bias, a_log, d, S, H, G, N, Dv):
+    """In float64 from S [H, N, Dv]: y [T, H Dv] and the last state."""
+    T = xbc.shape[0]
+    x, B, C = xbc.double().split([H * Dv, G * N, G * N], 1)
+    x, B, C = x.view(T, H, Dv), *(m.reshape(T, G, N).repeat_interleave(H // G, 1) for m in (B, C))
+    dt = torch.nn.functional.softplus(dt.double() + bias.double())
+    keep = torch.exp(-a_log.double().exp() * dt)
+    y = torch.empty((T, H, Dv), dtype=torch.float64, device=x.device)
+    for t in range(T):
+        S = S * keep[t, :, None, None] + (dt[t, :, None] * B[t])[:, :, None] * x[t][:, None]
+        y[t] = torch.einsum("hkv,hk->hv", S, C[t]) + d.double()[:, None] * x[t]
+    return y.reshape(T, -1), S
+
+
+@pytest.mark.parametrize("steps", STEPS)
+@pytest.mark.parametrize("H,G,N,Dv", [(2, 1, 64, 64), (4, 2, 128, 64), (40, 8, 128, 128)])
+def test_ssd_walk(steps, H, G, N, Dv):
+    from kv_cache_optimization_for_llm_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(H + N + len(steps))
+    rn = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    T = sum(n for *_, n in steps)
+    xbc, dt = rn(T, H * Dv + 2 * G * N).bfloat16(), rn(T, H).bfloat16()
+    bias, a_log, d = rn(H) - 2.0, rn(H) * 1.5, rn(H)
+    state = rn(12, H * Dv * N + 24)[:, 8:]
+    slots = {r: (3 * r + 1) % 11 for r, *_ in steps}
+    batch = _batch(steps, slots)
+    was, before = state.clone(), ops.choices["ssd_walk"]
+    y = ops.ssd_scan(xbc, (dt, 0), bias, a_log, d, state, batch, H, G, N, Dv)
+    assert ops.choices["ssd_walk"] == before + 1
+    old_state, old = was.clone(), ops.WALK_MIN_RUN
+    ops.WALK_MIN_RUN = 0
+    y_old = ops.ssd_scan(xbc, (dt, 0), bias, a_log, d, old_state, batch, H, G, N, Dv)
+    ops.WALK_MIN_RUN = old
+    order = [e for e in steps if e[2] == 1] + [e for e in steps if e[2] != 1]
+    t = 0
+    for r, start, n in order:
+        s0 = was[slots[r]][:H * Dv * N].double().view(H, Dv, N).transpose(1, 2) * (1.0 if start else 0.0)
+        ref, last = _ssd_plain(xbc[t:t + n], dt[t:t + n], bias, a_log, d, s0, H, G, N, Dv)
+        got = state[slots[r]][:H * Dv * N].view(H, Dv, N).transpose(1, 2)
+        # float32 sums of exactly held operands: 1e-6 relative, and no further off than token by token
+        for mine, other, want in ((y[t:t + n], y_old[t:t + n], ref),
+                                  (got, old_state[slots[r]][:H * Dv * N].view(H, Dv, N).transpose(1, 2), last)):
+            assert _rel(mine, want) < 2e-6 and _rel(mine, want) < 2.0 * _rel(other, want) + 2e-7, (r, _rel(mine, want), _rel(other, want))
+        t += n
+    untouched = [s for s in range(12) if s not in slots.values()]
+    assert torch.equal(state[untouched], was[untouched]) and torch.equal(state[:, H * Dv * N:], was[:, H * Dv * N:])
+
+
+def _mlstm_plain(p, gates, bi, bf, cap, scale, C, n, m, H, N, Dv):
+    T = p.shape[0]
+    q, k, v = p.double().split([H * N, H * N, H * Dv], 1)
+    q, k, v = q.view(T, H, N) * scale, k.view(T, H, N), v.view(T, H, Dv)
+    gi = cap * torch.tanh((gates[:, :H].double() + bi.double()) / cap)
+    gf = torch.nn.functional.logsigmoid(cap * torch.tanh((gates[:, H:2 * H].double() + bf.double()) / cap))
+    y, cond = (torch.empty((T, H, Dv), dtype=torch.float64, device=p.device) for _ in range(2))
+    Ca, na = C.abs(), n.abs()       # the same sums over magnitudes: what the float32 sums' errors go by
+    for t in range(T):
+        top = torch.maximum(gf[t] + m, gi[t])
+        keep, take = torch.exp(gf[t] + m - top)[:, None], torch.exp(gi[t] - top)[:, None]
+        C = C * keep[..., None] + (take * k[t])[:, :, None] * v[t][:, None]
+        Ca = Ca * keep[..., None] + (take * k[t]).abs()[:, :, None] * v[t].abs()[:, None]
+        n, m = n * keep + take * k[t], top
+        na = na * keep + (take * k[t]).abs()
+        den = (torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+        y[t] = torch.einsum("hkv,hk->hv", C, q[t]) / den
+        cond[t] = (torch.einsum("hkv,hk->hv", Ca, q[t].abs()) + y[t].abs() * (na * q[t].abs()).sum(-1, keepdim=True)) / den
+    return y.reshape(T, -1), C, n, m, cond.reshape(T, -1)
+
+
+@pytest.mark.parametrize("steps", STEPS)
+@pytest.mark.parametrize("H,N,Dv", [(2, 64, 64), (3, 128, 128), (64, 64, 128)])
+def test_mlstm_walk(steps, H, N, Dv):
+    from kv_cache_optimization_for_llm_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(H + N + len(steps))
+    rn = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    T, per, sp = sum(n for *_, n in steps), H * Dv * N, Dv // 64
+    p = rn(T, H * (2 * N + Dv) + 8).bfloat16()
+    gates, bi, bf = rn(T, 2 * H) * 4.0, rn(H), rn(H) + 3.0
+    state = rn(12, ops.mlstm_state_floats(H, N, Dv))
+    state[:, per:per + H * sp * N] = rn(12, H, 1, N).expand(-1, -1, sp, -1).reshape(12, -1)       # n and m: the same for every block of columns
+    state[:, per + H * sp * N:] = rn(12, H, 1).expand(-1, -1, sp).reshape(12, -1)
+    slots = {r: (3 * r + 1) % 11 for r, *_ in steps}
+    batch = _batch(steps, slots)
+    args = (p[:, :H * (2 * N + Dv)], 0, H * N, 2 * H * N, gates, bi, bf, 15.0, N ** -0.5)
+    was, before = state.clone(), ops.choices["mlstm_walk"]
+    y = ops.mlstm_scan(*args, state, batch, H, N, Dv)
+    assert ops.choices["mlstm_walk"] == before + 1
+    old_state, old = was.clone(), ops.WALK_MIN_RUN
+    ops.WALK_MIN_RUN = 0
+    y_old = ops.mlstm_scan(*args, old_state, batch, H, N, Dv)
+    ops.WALK_MIN_RUN = old
+    t = 0
+    for r, start, n in [e for e in steps if e[2] == 1] + [e for e in steps if e[2] != 1]:
+        s0, live = was[slots[r]].double(), 1.0 if start else 0.0
+        view = lambda s: (s[:per].view(H, Dv, N).transpose(1, 2), s[per:per + H * sp * N].view(H, sp, N), s[per + H * sp * N:].view(H, sp))
+        C0, n0, m0 = view(s0 * live)
+        ref = _mlstm_plain(args[0][t:t + n], gates[t:t + n], bi, bf, 15.0, N ** -0.5, C0, n0[:, 0], m0[:, 0], H, N, Dv)
+        got, other = view(state[slots[r]]), view(old_state[slots[r]])
+        pairs = [(y[t:t + n], y_old[t:t + n], ref[0]), (got[0], other[0], ref[1])]
+        pairs += [(got[1][:, b], other[1][:, b], ref[2]) for b in range(sp)] + [(got[2][:, b], other[2][:, b], ref[3]) for b in range(sp)]
+        # the read-out divides by n . q, which may be a small difference of large terms: its error is measured against the sums of
+        # magnitudes (float32: 2^-24 times a few tens of roundings)
+        off, off_old = (((o[t:t + n].double() - ref[0]).abs() / (ref[4] + 1e-30)) for o in (y, y_old))
+        assert float(off.max()) < 3e-6 and float(off.norm()) < 2.0 * float(off_old.norm()) + 1e-7 * off.numel() ** 0.5
+        for mine, oth, want in pairs[1:]:
+            assert _rel(mine, want) < 2e-6 and _rel(mine, want) < 2.0 * _rel(oth, want) + 2e-7, (r, _rel(mine, want), _rel(oth, want))
+        t += n
+    untouched = [s for s in range(12) if s not in slots.values()]
+    assert torch.equal(state[untouched], was[untouched])
