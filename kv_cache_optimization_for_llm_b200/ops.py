@@ -1380,8 +1380,10 @@ def _chunk_rows(batch, chunk: int):
     return batch.num_reqs - first + batch.num_tokens // chunk + 1, first
 
 
-# bfloat16 steps with a run of at least this many tokens walk their runs in pieces of 64 tokens on tensor cores where the sizes
-# allow (the matrix states with one decay per head and token).  Measured at 32 heads of 64 x 64: WALK_MIN_MEASURED.
+# bfloat16 steps whose runs bring at least this many tokens each, on average, walk them in pieces of 64 tokens on tensor cores where
+# the sizes allow (the matrix states with one decay per head and token).  A piece costs the same however few tokens it holds.
+# Measured, token by token / the walk, 64 heads of 128 x 64 (ssd): one run of 16 tokens 22 / 22 us (the host's share), of 32 37 / 22,
+# of 64 71 / 18; sixteen runs of 8 45 / 58, of 16 71 / 58, of 64 230 / 60; 32 heads of 64 x 64 (mlstm), sixteen of 8 20 / 27, of 16 30 / 27.
 WALK_MIN_RUN = int(os.environ.get('KVB200_WALK_MIN_RUN', '16'))
 
 
@@ -1389,8 +1391,8 @@ def _walks(batch, n: int, dv: int, x: torch.Tensor, *columns: int) -> bool:
     """Whether a step's runs go to the walk on tensor cores: bfloat16, a state of 64 or 128 rows, whole blocks of 64 value columns,
     every segment of ``x``'s rows (from ``columns``) on a 16-byte boundary."""
     return (x.dtype == torch.bfloat16 and n in (64, 128) and dv >= 64 and dv % 64 == 0 and x.stride(0) % 8 == 0
-            and all(_at(x, c) % 16 == 0 for c in columns)
-            and 0 < WALK_MIN_RUN <= int(getattr(batch, "max_q_len", 0) or 0))
+            and all(_at(x, c) % 16 == 0 for c in columns) and not batch.decode_only and WALK_MIN_RUN > 0
+            and batch.num_tokens - batch.num_single >= WALK_MIN_RUN * (batch.num_reqs - batch.num_single))
 
 
 class _DiagArgs(ctypes.Structure):
@@ -1445,7 +1447,7 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
     step:  ``dt = softplus(dt_raw + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + dt B x^T``, ``y = S^T C + D x``.
     ``xbc`` [T, heads dv + 2 groups n]: x | B | C (head h reads group ``h // (heads / groups)``); ``dt``: (tensor, first
     column) of the raw step sizes [T, heads].  ``state``: float32 [slots, >= heads * dv * n], zero for a request
-    that starts at position 0.  Returns float32 y [T, heads * dv].  bfloat16 steps with runs of ``WALK_MIN_RUN`` tokens go to
+    that starts at position 0.  Returns float32 y [T, heads * dv].  bfloat16 steps with runs of ``WALK_MIN_RUN`` tokens and more go to
     the walk on tensor cores where the sizes allow (:func:`_walks`); otherwise a step with a run of ``SCAN_CHUNK_MIN_RUN``
     tokens or more walks chunks of its runs side by side (64 tokens a chunk, 128 from runs of 1024 on)."""
     _need_cuda(xbc, state)
@@ -1460,7 +1462,7 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
     chunk = first = local = carry = decay = 0
     if _walks(batch, n, dv, xbc, 0, heads * dv, heads * dv + groups * n):
         # single tokens beside the runs (the step's first requests) go token by token
-        singles = int(getattr(batch, "num_single", 0) or 0)
+        singles = int(batch.num_single)
         p = _SsdArgs(xbc.data_ptr(), xbc.stride(0), _at(dtt, dcol), dtt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(),
                      d_skip.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), batch.q_start.data_ptr(),
                      batch.req_start.data_ptr(), batch.slots.data_ptr(), heads, groups, n, dv, 0, 0, 0, 0, 0, 0)
@@ -1578,7 +1580,7 @@ def mlstm_scan(p: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch
     chunk = first = local = carry = fsum = 0
     if _walks(batch, n, dv, p, q_off, k_off, v_off):
         # single tokens beside the runs (the step's first requests) go token by token
-        singles = int(getattr(batch, "num_single", 0) or 0)
+        singles = int(batch.num_single)
         a = _MlstmArgs(p.data_ptr(), p.stride(0), q_off, k_off, v_off, gates.data_ptr(), gates.stride(0),
                        0 if bi is None else bi.data_ptr(), 0 if bf is None else bf.data_ptr(), float(cap), float(q_scale),
                        state.data_ptr(), state.stride(0), y.data_ptr(), batch.q_start.data_ptr(), batch.req_start.data_ptr(),
