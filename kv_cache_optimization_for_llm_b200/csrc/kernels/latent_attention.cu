@@ -414,11 +414,13 @@ KVB_EXPORT int kvb_head_rows(const void* in, void* out, int ld_out, const void* 
 // ---------------------------------------------------------------- the rows that long runs see
 // A block fills eight rows, one per warp, of a page of `rows_per_page` rows of out [n_pages * rows_per_page, rank]: info [n_pages, 4] int32 holds the
 // request's row in the batch, the position of the page's first row, and the first position that the run sees; rows
-// in front of that or behind the request's last token are zero.  16-byte pieces.
+// in front of that or behind the request's last token are zero.  16-byte pieces.  What a cached row holds behind its latent
+// (`behind` pieces: the rotated key part that all heads share) goes into every head's row of `rows`, at piece `at` of `width`.
 __global__ void __launch_bounds__(256)
 latent_rows_kernel(const __nv_bfloat16* __restrict__ pages, const int* __restrict__ block_table, int max_pages, int page_size,
                    int num_pages, const int* __restrict__ ctx_len, const int4* __restrict__ info, int rows_per_page,
-                   int vecs, __nv_bfloat16* __restrict__ out, int* status) {
+                   int vecs, __nv_bfloat16* __restrict__ out, int behind, __nv_bfloat16* __restrict__ rows, int heads, int width,
+                   int at, int* status) {
   pdl_trigger();
   pdl_wait();
   const int4 page_info = info[blockIdx.x];
@@ -434,23 +436,66 @@ latent_rows_kernel(const __nv_bfloat16* __restrict__ pages, const int* __restric
       const int lp = pos / page_size;
       const int page = lp < max_pages ? table[lp] : -1;
       if (page < 0 || page >= num_pages) { if (lane == 0) atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE); }
-      else src = reinterpret_cast<const uint4*>(pages) + ((size_t)page * page_size + pos % page_size) * vecs;
+      else src = reinterpret_cast<const uint4*>(pages) + ((size_t)page * page_size + pos % page_size) * (vecs + behind);
     }
-    uint4* dst = reinterpret_cast<uint4*>(out) + ((size_t)blockIdx.x * rows_per_page + r) * vecs;
+    const size_t row = (size_t)blockIdx.x * rows_per_page + r;
+    uint4* dst = reinterpret_cast<uint4*>(out) + row * vecs;
     for (int v = lane; v < vecs; v += 32) dst[v] = src != nullptr ? src[v] : make_uint4(0u, 0u, 0u, 0u);
+    const size_t head = (size_t)gridDim.x * rows_per_page * width;
+    for (int v = lane; v < behind * heads; v += 32) {
+      const int h = v / behind, b = v - h * behind;
+      reinterpret_cast<uint4*>(rows)[h * head + row * width + at + b] = src != nullptr ? src[vecs + b] : make_uint4(0u, 0u, 0u, 0u);
+    }
   }
 }
 
-// bfloat16, rank a multiple of 8, cache rows of rank elements (nothing behind the latent).
+// bfloat16, rank a multiple of 8, cache rows of rank + behind elements; behind > 0: rows [heads, n_pages * rows_per_page, width]
+// gets the part behind the latent at element `at` of every row (behind, width and at multiples of 8).
 KVB_EXPORT int kvb_latent_rows(const void* pages, const int* block_table, int max_pages, int page_size, int num_pages,
                                const int* ctx_len, const int* info, int n_pages, int rows_per_page, int rank, void* out,
-                               int* status, cudaStream_t stream) {
+                               int behind, void* rows, int heads, int width, int at, int* status, cudaStream_t stream) {
   if (n_pages <= 0) return 0;
   if (rank < 8 || rank % 8 != 0 || rows_per_page < 1) return KVB_ERR_BAD_SIZE;
+  if (behind < 0 || (behind > 0 && (behind % 8 || width % 8 || at % 8 || at < 0 || at + behind > width || heads < 1))) return KVB_ERR_BAD_SIZE;
+  if (behind > 0 && (reinterpret_cast<uintptr_t>(rows) & 15)) return KVB_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(pages) | reinterpret_cast<uintptr_t>(info) | reinterpret_cast<uintptr_t>(out)) & 15)
     return KVB_ERR_ALIGN;
   kvb_launch(latent_rows_kernel, dim3(n_pages, (rows_per_page + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)pages, block_table, max_pages,
-             page_size, num_pages, ctx_len, (const int4*)info, rows_per_page, rank / 8, (__nv_bfloat16*)out, status);
+             page_size, num_pages, ctx_len, (const int4*)info, rows_per_page, rank / 8, (__nv_bfloat16*)out, behind / 8,
+             (__nv_bfloat16*)rows, heads, width / 8, at / 8, status);
+  return kvb_launch_result();
+}
+
+// The queries' parts to be rotated, in place: of every token row and head the pairs (2 i, 2 i + 1), i < half, behind the first `dim`
+// of its `per_head` channels turn by the token's position.  A thread per pair; float32, rounded once.
+__global__ void __launch_bounds__(256)
+latent_rotate_kernel(__nv_bfloat16* __restrict__ q, int ld, int per_head, int dim, int half, int pairs, const float* __restrict__ cos_t,
+                     const float* __restrict__ sin_t, int table_len, const int* __restrict__ positions, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const int pos = positions[t];
+  if (pos < 0 || pos >= table_len) {
+    if (threadIdx.x == 0) atomicCAS(status, 0, KVB_STATUS_BAD_POSITION);
+    return;
+  }
+  for (int x = threadIdx.x; x < pairs; x += blockDim.x) {
+    const int h = x / half, i = x - h * half;
+    __nv_bfloat162* at = reinterpret_cast<__nv_bfloat162*>(q + (size_t)t * ld + (size_t)h * per_head + dim) + i;
+    const float2 v = __bfloat1622float2(*at);
+    const float c = cos_t[(size_t)pos * half + i], s = sin_t[(size_t)pos * half + i];
+    *at = __floats2bfloat162_rn(v.x * c - v.y * s, v.y * c + v.x * s);
+  }
+}
+
+// q [T, >= heads * per_head] with row stride ld, all even; the tables [table_len, rdims / 2].
+KVB_EXPORT int kvb_latent_rotate(void* q, int ld, int heads, int per_head, int dim, int rdims, const float* cos_t, const float* sin_t,
+                                 int table_len, const int* positions, int T_, int* status, cudaStream_t stream) {
+  if (T_ <= 0 || rdims <= 0) return 0;
+  if (heads < 1 || rdims % 2 || dim < 0 || dim + rdims > per_head || ((ld | per_head | dim) & 1)) return KVB_ERR_BAD_SIZE;
+  if (reinterpret_cast<uintptr_t>(q) & 3) return KVB_ERR_ALIGN;
+  kvb_launch(latent_rotate_kernel, dim3(T_), dim3(256), 0, stream, (__nv_bfloat16*)q, ld, per_head, dim, rdims / 2, heads * (rdims / 2),
+             cos_t, sin_t, table_len, positions, status);
   return kvb_launch_result();
 }
 

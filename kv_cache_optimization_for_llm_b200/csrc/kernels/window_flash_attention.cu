@@ -13,8 +13,12 @@
 // With two maps per head (ScoreShape::pair) the lower half of a tile's rows are map 1 of its (token, head) pairs and the
 // upper half map 2 of the same ones, so that a warp's sixteen rows all read the same keys; a head's two results meet in
 // shared memory at the end.
-// Key size dk and value size dv are multiples of 8 up to 128; the tiles are padded with zeros to the next of
-// 64 / 128 (keys) and 32 / 64 / 128 (values), which changes no sum.
+// Key size dk and value size dv are multiples of 8 up to 192 and 128; the tiles are padded with zeros to the next of
+// 64 / 96 / 128 / 192 (keys; two maps: 64 / 128) and 32 / 64 / 128 (values), which changes no sum.
+//
+// What bounds it: the warps' dependent steps (ldmatrix, exponentials, shuffles) between products on mma.sync.  So a tile
+// that every row sees whole skips the mask, scores that nothing shapes take one multiplication, and the results so far are
+// rescaled only when some row's maximum moved.
 #include "common.cuh"
 #include "mma_sync.cuh"
 #include "score_shape.cuh"
@@ -169,6 +173,7 @@ window_flash_attention_kernel(RowsArgs p) {
     slope[rr] = p.shape.slopes != nullptr ? p.shape.slopes[head] : 0.f;
   }
   const float cap = p.shape.softcap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
+  const bool plain = PAIR || (cap <= 0.f && p.shape.slopes == nullptr);      // nothing but a factor on the scores
 
   for (int idx = 0; idx < n_walk; ++idx) {
     const int t = tile_at(idx);
@@ -214,15 +219,14 @@ window_flash_attention_kernel(RowsArgs p) {
     // shape, mask and running softmax; from here on the scores are in units of log2
     const int kbase = t * BN + ((lane & 3) << 1);
     float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
-    if constexpr (PAIR) {
-      // no cap, no bias; a tile that every row sees whole needs no mask
-      const float f = p.scale * kLog2e;
-      if ((t + 1) * BN - 1 <= pos_first && t * BN >= lo_last) {
+    if (plain) {
+      const float f[2] = {hs[0] * kLog2e, hs[1] * kLog2e};
+      if ((t + 1) * BN - 1 <= pos_first && t * BN >= lo_last) {      // every row sees the whole tile
 #pragma unroll
         for (int n = 0; n < BN / 8; ++n) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            s[n][e] *= f;
+            s[n][e] *= f[e >> 1];
             mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
           }
         }
@@ -233,7 +237,7 @@ window_flash_attention_kernel(RowsArgs p) {
           for (int e = 0; e < 4; ++e) {
             const int j = kbase + n * 8 + (e & 1);
             const int rr = e >> 1;
-            s[n][e] = j <= pos_r[rr] && j >= lo_r[rr] ? s[n][e] * f : -CUDART_INF_F;
+            s[n][e] = j <= pos_r[rr] && (j >= lo_r[rr] || j < keep) ? s[n][e] * f[rr] : -CUDART_INF_F;
             mx[rr] = fmaxf(mx[rr], s[n][e]);
           }
         }
@@ -265,7 +269,7 @@ window_flash_attention_kernel(RowsArgs p) {
       m_run[rr] = m_new;
       l_run[rr] *= corr[rr];
     }
-    if (!PAIR || __any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
 #pragma unroll
       for (int n = 0; n < DT; ++n) {
         o[n][0] *= corr[0]; o[n][1] *= corr[0]; o[n][2] *= corr[1]; o[n][3] *= corr[1];
@@ -274,14 +278,8 @@ window_flash_attention_kernel(RowsArgs p) {
     unsigned pf[BN / 16][4];
 #pragma unroll
     for (int n = 0; n < BN / 8; ++n) {
-      float p0, p1, p2, p3;
-      if constexpr (PAIR) {
-        p0 = exp2_hw(s[n][0] - m_use[0]); p1 = exp2_hw(s[n][1] - m_use[0]);
-        p2 = exp2_hw(s[n][2] - m_use[1]); p3 = exp2_hw(s[n][3] - m_use[1]);
-      } else {
-        p0 = exp2f(s[n][0] - m_use[0]); p1 = exp2f(s[n][1] - m_use[0]);
-        p2 = exp2f(s[n][2] - m_use[1]); p3 = exp2f(s[n][3] - m_use[1]);
-      }
+      const float p0 = exp2_hw(s[n][0] - m_use[0]), p1 = exp2_hw(s[n][1] - m_use[0]);
+      const float p2 = exp2_hw(s[n][2] - m_use[1]), p3 = exp2_hw(s[n][3] - m_use[1]);
       l_run[0] += p0 + p1;
       l_run[1] += p2 + p3;
       // the accumulator layout of two neighbouring score tiles is the A layout of one k-step
@@ -415,6 +413,12 @@ int launch_dv(const RowsArgs& a, int num_tiles, cudaStream_t stream) {
 template <bool PAIR>
 int launch_any(const RowsArgs& a, int num_tiles, int wide, cudaStream_t stream) {
   if (a.dk <= 64) return wide ? launch_dv<4, 8, PAIR>(a, num_tiles, stream) : launch_dv<4, 4, PAIR>(a, num_tiles, stream);
+  if constexpr (!PAIR) {
+    if (a.dk <= 96) return wide ? launch_dv<6, 8, PAIR>(a, num_tiles, stream) : launch_dv<6, 4, PAIR>(a, num_tiles, stream);
+    if (a.dk > 128) return wide ? launch_dv<12, 8, PAIR>(a, num_tiles, stream) : launch_dv<12, 4, PAIR>(a, num_tiles, stream);
+  } else if (a.dk > 128) {
+    return KVB_ERR_BAD_SIZE;
+  }
   return wide ? launch_dv<8, 8, PAIR>(a, num_tiles, stream) : launch_dv<8, 4, PAIR>(a, num_tiles, stream);
 }
 
@@ -426,10 +430,10 @@ int log2_exact(int x) {
 
 }  // namespace
 
-// 1 when the kernel takes these sizes: key and value sizes that are multiples of 8 up to 128, a group of at most
-// 64 query heads per key/value head, a page size that is a power of two.
+// 1 when the kernel takes these sizes: key and value sizes that are multiples of 8 up to 192 (two maps: 128) and 128, a group of
+// at most 64 query heads per key/value head, a page size that is a power of two.
 KVB_EXPORT int kvb_window_flash_attention_supported(int dk, int dv, int group, int page_size) {
-  return dk >= 8 && dk <= 128 && dk % 8 == 0 && dv >= 8 && dv <= 128 && dv % 8 == 0 && group >= 1 && group <= 64 &&
+  return dk >= 8 && dk <= 192 && dk % 8 == 0 && dv >= 8 && dv <= 128 && dv % 8 == 0 && group >= 1 && group <= 64 &&
          log2_exact(page_size) >= 0;
 }
 

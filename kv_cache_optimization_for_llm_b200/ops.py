@@ -746,13 +746,16 @@ def latent_up_wanted(batch, window: int) -> bool:
     return keys <= LATENT_UP_MAX_KEYS * tokens
 
 
-def latent_step_rows(pages: torch.Tensor, block_table, batch, w_kv: torch.Tensor, window: int) -> StepRows:
+def latent_step_rows(pages: torch.Tensor, block_table, batch, w_kv: torch.Tensor, window: int, dim: int = 0,
+                     rot: int = 0) -> StepRows:
     """The keys and values of every position that a step's runs see, made from the cached latents: ``pages`` [num_pages, 1,
-    page_size, rank], ``w_kv`` [heads, key size + value size, rank] (bfloat16).  One gather and one batched product by the
-    library."""
+    page_size, rank + rot], ``w_kv`` [heads, key size + value size, rank] (bfloat16).  One gather and one batched product by the
+    library.  ``rot`` > 0: the rotated part that a cached row holds behind its latent follows each head's key (whose size ``dim``
+    then names): rows [key | rotated part | value], the gather copies that part, and keys and values are a product each."""
     _need_cuda(pages, w_kv)
     H, width, rank = w_kv.shape
-    assert pages.dtype == torch.bfloat16 and pages.is_contiguous() and pages.shape[1] == 1 and pages.shape[3] == rank
+    assert pages.dtype == torch.bfloat16 and pages.is_contiguous() and pages.shape[1] == 1 and pages.shape[3] == rank + rot
+    width += rot
     P = StepRows.PAGE
     plans = batch.host.setdefault("latent_rows", {})
     plan = plans.get(window)
@@ -776,16 +779,35 @@ def latent_step_rows(pages: torch.Tensor, block_table, batch, w_kv: torch.Tensor
         plans[window] = plan
     info, table, n_pages, _ = plan
     c = new((n_pages * P, rank), pages.dtype, pages.device)
+    data = new((H, n_pages * P, width), pages.dtype, pages.device)
     rc = lib("latent_attention").kvb_latent_rows(_p(pages), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[2]),
                                                  c_int(pages.shape[0]), _p(batch.ctx_len), _p(info), c_int(n_pages), c_int(P),
-                                                 c_int(rank), _p(c), _p(batch.status), _stream())
+                                                 c_int(rank), _p(c), c_int(rot), _p(data), c_int(H), c_int(width), c_int(dim),
+                                                 _p(batch.status), _stream())
     _check(rc, "latent_rows")
-    data = new((H, n_pages * P, width), pages.dtype, pages.device)
-    torch.bmm(c.unsqueeze(0).expand(H, -1, -1), w_kv.transpose(1, 2), out=data)
+    rows = c.unsqueeze(0).expand(H, -1, -1)
+    if rot:
+        torch.bmm(rows, w_kv[:, :dim].transpose(1, 2), out=data[:, :, :dim])
+        torch.bmm(rows, w_kv[:, dim:].transpose(1, 2), out=data[:, :, dim + rot:])
+    else:
+        torch.bmm(rows, w_kv.transpose(1, 2), out=data)
     if _marks is not None:
         _mark("latent_up_library")
     choices["latent_up_library"] += 1
     return StepRows(data, table, batch.num_single)
+
+
+def latent_rotate(q: torch.Tensor, first_row: int, heads: int, per_head: int, dim: int, cos, sin, batch) -> None:
+    """Rotates, in place, the part behind the first ``dim`` of every head's ``per_head`` channels (neighbouring channels in pairs) of
+    the token rows from ``first_row`` on (``q`` bfloat16 [T, >= heads * per_head])."""
+    _need_cuda(q, cos)
+    assert q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.shape[1] >= heads * per_head and cos.dtype == torch.float32
+    assert cos.is_contiguous() and sin.is_contiguous()
+    rc = lib("latent_attention").kvb_latent_rotate(
+        c_void_p(q.data_ptr() + first_row * q.stride(0) * 2), c_int(q.stride(0)), c_int(heads), c_int(per_head), c_int(dim),
+        c_int(2 * cos.shape[1]), _p(cos), _p(sin), c_int(cos.shape[0]),
+        c_void_p(batch.positions.data_ptr() + 4 * first_row), c_int(q.shape[0] - first_row), _p(batch.status), _stream())
+    _check(rc, "latent_rotate")
 
 
 # ------------------------------------------------------------------ attention
@@ -1099,6 +1121,12 @@ def window_flash_attention_supported(dk: int, dv: int, group: int, page_size: in
     of a power of two."""
     return (dtype == torch.bfloat16 and 8 <= dk <= 128 and dk % 8 == 0 and 8 <= dv <= 128 and dv % 8 == 0
             and 1 <= group <= 64 and page_size >= 1 and page_size & (page_size - 1) == 0)
+
+
+def made_rows_attention_supported(dk: int, dv: int) -> bool:
+    """Whether :func:`window_flash_attention` takes rows that were made for one step, a head to itself: bfloat16, sizes that are
+    multiples of 8, keys up to 192 and values up to 128."""
+    return 8 <= dk <= 192 and dk % 8 == 0 and 8 <= dv <= 128 and dv % 8 == 0
 
 
 # Which tiles the tensor-core attention over [key | value] rows of unequal sizes cuts a step into: "" chosen from the

@@ -28,10 +28,10 @@ class LatentAttention(Part):
 
     The key up-projection is applied to the queries instead (q_plain^T W_uk,h c = (W_uk,h^T q_plain)^T c),
     attention runs for all heads over the cached rows, and the value up-projection is applied
-    to the attended latents; the output projection follows.  Long runs of tokens in bfloat16 (no rotated part, no gate,
-    sizes that the prompt kernels for [key | value] rows take) go the other way: the keys and values of all positions that
-    the runs see are made once (``ops.latent_step_rows``), and every head attends to rows of its own, which is a multiple
-    fewer operations per query and key (dim + vdim against twice the latent) on a faster kernel.  With ``split_decode``
+    to the attended latents; the output projection follows.  Long runs of tokens in bfloat16 (sizes that the prompt kernels
+    for [key | value] rows take) go the other way: the keys and values of all positions that
+    the runs see are made once (``ops.latent_step_rows``, the shared rotated part between them), and every head attends to rows of its
+    own, which is a multiple fewer operations per query and key (dim + rot_dim + vdim against twice the latent) on a faster kernel.  With ``split_decode``
     bfloat16 steps of single tokens deal a request's keys over several blocks and make the products per head on tensor cores:
     faster, but a token's result then differs by rounding between a short portion and a step of its own.
     params: hidden_size, heads, dim, rot_dim, vdim, q_rank, kv_rank, scale, window, sink, gate, borrows_latent, split_decode,
@@ -66,12 +66,14 @@ class LatentAttention(Part):
     @staticmethod
     def _up_sizes(params, dtype):
         """Whether long runs may make their keys and values: what the prompt kernels over such rows take."""
-        return (dtype == torch.bfloat16 and not int(params["rot_dim"]) and not params.get("gate") and int(params["kv_rank"]) % 8 == 0
-                and ops.window_flash_attention_supported(int(params["dim"]), int(params["vdim"]), 1, ops.StepRows.PAGE, dtype))
+        d, r, v = int(params["dim"]), int(params["rot_dim"]), int(params["vdim"])
+        return (dtype == torch.bfloat16 and int(params["kv_rank"]) % 8 == 0 and (not r or (d % 8 == 0 and r % 8 == 0))
+                and ops.made_rows_attention_supported(d + r, v))
 
     @staticmethod
     def _one_size(params):
-        return int(params["dim"]) == int(params["vdim"]) and int(params["dim"]) in (64, 128)
+        return (int(params["dim"]) == int(params["vdim"]) and int(params["dim"]) in (64, 128) and not int(params["rot_dim"])
+                and not params.get("gate"))
 
     def __init__(self, params, weights, ctx):
         super().__init__(params, weights, ctx)
@@ -119,7 +121,7 @@ class LatentAttention(Part):
         widths = [self.w_in.shape[0], self.q_rank, H * (self.dim + self.rot), 3 * H * self.rank, 2 * H * self.vdim,
                   self.o.shape[0]]
         if self.ukv is not None:
-            widths.append(ops.LATENT_UP_MAX_KEYS * (H * (self.dim + self.vdim) + self.rank))
+            widths.append(ops.LATENT_UP_MAX_KEYS * (H * (self.dim + self.rot + self.vdim) + self.rank))
         return widths
 
     def query_tile_heights(self):
@@ -134,23 +136,27 @@ class LatentAttention(Part):
                 heights.append(ops.flash_tokens_per_tile(1, True))
         return heights
 
-    def _over_made_rows(self, q, table, batch, cache):
+    def _over_made_rows(self, q, table, batch, cache, cos, sin, rdims, gate):
         """The heads' results [T, heads * vdim] of a step with long runs; ``q`` holds the queries from column 0 on.  Single
         tokens beside the runs attend to the cached rows as in every other step."""
-        rows = ops.latent_step_rows(cache.k, table, batch, self.ukv, self.window or 0)
+        rows = ops.latent_step_rows(cache.k, table, batch, self.ukv, self.window or 0, self.dim, self.rot)
+        n, per_head = batch.num_single, self.dim + self.rot
+        if self.rot:
+            ops.latent_rotate(q, n, self.heads, per_head, self.dim, cos, sin, batch)
         if self._one_size(self.params) and ops.flash_attention_rows_masked_wanted(batch, self.heads, self.heads, self.dim, self.vdim,
                                                                                   rows.PAGE, self.ctx.dtype, q):
             a = ops.flash_attention_rows_masked(q, None, None, batch, self.heads, self.heads, self.dim, self.scale, sinks=self.sink,
                                                 window=self.window or 0, rows=rows)
         else:
-            a = ops.window_flash_attention(q, None, None, batch, self.heads, self.heads, self.dim, self.vdim, self.scale,
-                                           self.window or 0, 0, False, sinks=self.sink, rows=rows)
-        n = batch.num_single
+            a = ops.window_flash_attention(q, None, None, batch, self.heads, self.heads, per_head, self.vdim, self.scale,
+                                           self.window or 0, 0, False, sinks=self.sink, rows=rows, gate=gate)
         if n:
-            q_abs = ops.head_gemm(q[:n], 0, self.dim, self.uk_t, tensor_cores=self.split)
-            lat = ops.latent_attention(q_abs, q[:n], 0, self.dim, None, None, 0, cache.k, table, batch, self.sink, self.scale,
-                                       self.heads, self.rank, self.behind, self.window or 0, singles=True, split=self.split)
-            a[:n].copy_(ops.head_gemm(lat, 0, self.rank, self.uv, tensor_cores=self.split))
+            q_abs = ops.head_gemm(q[:n], 0, per_head, self.uk_t, tensor_cores=self.split)
+            lat = ops.latent_attention(q_abs, q[:n], self.dim if self.rot else 0, per_head, cos, sin, rdims, cache.k, table, batch,
+                                       self.sink, self.scale, self.heads, self.rank, self.behind, self.window or 0, singles=True,
+                                       split=self.split)
+            first = (gate[0][:n], gate[1]) if gate is not None else None
+            a[:n].copy_(ops.head_gemm(lat, 0, self.rank, self.uv, first, tensor_cores=self.split))
         return a
 
     def forward(self, x, batch, cache):
@@ -164,10 +170,10 @@ class LatentAttention(Part):
                                  self.eps, cos, sin, batch, table, cache.k, cache.write and not self.borrows)
         q = ops.linear(cq, self.uq) if self.q_rank else d         # without a latent the queries are the product's first columns
         per_head = self.dim + self.rot
-        if self.ukv is not None and ops.latent_up_wanted(batch, self.window or 0):
-            return ops.linear(self._over_made_rows(q, table, batch, cache), self.o)
+        gate = (d, self.at_g) if self.at_g is not None else None
+        if self.ukv is not None and ops.latent_up_wanted(batch, self.window or 0) and (gate is None or self.at_g % 2 == 0):
+            return ops.linear(self._over_made_rows(q, table, batch, cache, cos, sin, rdims, gate), self.o)
         q_abs = ops.head_gemm(q, 0, per_head, self.uk_t, tensor_cores=self.split)
         lat = ops.latent_attention(q_abs, q, self.dim if self.rot else 0, per_head, cos, sin, rdims, cache.k, table, batch, self.sink,
                                    self.scale, self.heads, self.rank, self.behind, self.window or 0, split=self.split)
-        gate = (d, self.at_g) if self.at_g is not None else None
         return ops.linear(ops.head_gemm(lat, 0, self.rank, self.uv, gate, tensor_cores=self.split), self.o)

@@ -1,0 +1,103 @@
+"""Latent attention over keys and values that were made for a step, with a rotated part behind every head's key and an output
+gate: against float64 and beside the form that attends over the cached latents, in steps with one run, several, runs that
+continue, single tokens beside them."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from part_harness import _ctx, _make, _run_in_steps, _w
+
+pytestmark = pytest.mark.gpu
+
+
+def _plain(x, w, heads, dim, rot, vdim, rank, scale, eps, sink, gate, window):
+    """One whole sequence in float64: x [T, W]."""
+    rms = lambda v, g: v / np.sqrt((v * v).mean(-1, keepdims=True) + eps) * g
+    T = x.shape[0]
+    q = (rms(x @ w["dq"].T, w["dq_norm"]) @ w["uq"].T).reshape(T, heads, dim + rot)
+    kv = x @ w["dkv"].T
+    c, kr = rms(kv[:, :rank], w["dkv_norm"]), kv[:, rank:]
+    if rot:
+        ang = np.arange(T)[:, None] * 10000.0 ** (-np.arange(0, rot, 2) / rot)
+        cos, sin = np.cos(ang), np.sin(ang)
+
+        def turn(v, cs, sn):
+            out = v.copy()
+            out[..., 0::2], out[..., 1::2] = v[..., 0::2] * cs - v[..., 1::2] * sn, v[..., 1::2] * cs + v[..., 0::2] * sn
+            return out
+        q[..., dim:] = turn(q[..., dim:], cos[:, None], sin[:, None])
+        kr = turn(kr, cos, sin)
+    k = np.concatenate([(c @ w["uk"].T).reshape(T, heads, dim), np.repeat(kr[:, None], heads, 1)], -1)
+    v = (c @ w["uv"].T).reshape(T, heads, vdim)
+    i, j = np.arange(T)[:, None], np.arange(T)[None]
+    seen = (j <= i) & ((i - j < window) if window else True)
+    out = np.zeros((T, heads, vdim))
+    for h in range(heads):
+        s = np.where(seen, q[:, h] @ k[:, h].T * scale, -np.inf)
+        m = s.max(1, keepdims=True)
+        e = np.exp(s - m)
+        out[:, h] = e @ v[:, h] / (e.sum(1, keepdims=True) + (np.exp(w["sink"][h] - m) if sink else 0.0))
+    out = out.reshape(T, heads * vdim)
+    if gate:
+        out = out / (1.0 + np.exp(-(x @ w["g"].T)))
+    return out @ w["o"].T
+
+
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank,sink,gate,window", [
+    (4, 128, 64, 128, 128, True, False, None), (2, 64, 32, 64, 64, False, True, None), (3, 24, 8, 40, 72, True, True, 100),
+    (2, 96, 96, 16, 64, False, False, 64), (2, 120, 8, 128, 64, True, True, None)])
+def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, window):
+    from kv_cache_optimization_for_llm_b200 import ops
+    from kv_cache_optimization_for_llm_b200.models.spec import PartSpec
+    rng = np.random.default_rng(dim + rot)
+    W, qr = 64, 48
+    ctx = _ctx("bfloat16")
+    shapes = {"dq": (qr, W), "uq": (heads * (dim + rot), qr), "dkv": (rank + rot, W), "uk": (heads * dim, rank),
+              "uv": (heads * vdim, rank), "o": (W, heads * vdim), "dq_norm": (qr,), "dkv_norm": (rank,)}
+    if sink:
+        shapes["sink"] = (heads,)
+    if gate:
+        shapes["g"] = (heads * vdim, W)
+    wt, w64 = {}, {}
+    for n, s in shapes.items():
+        wt[n], w64[n] = _w(rng, s, 0.1, 1.0) if n.endswith("norm") else _w(rng, s, 1.0 / math.sqrt(s[-1]) if len(s) > 1 else 0.5)
+    params = {"hidden_size": W, "heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": qr, "kv_rank": rank,
+              "scale": (dim + rot) ** -0.5, "eps": 1e-6, "sink": sink, "gate": gate, "window": window,
+              "position": PartSpec("rope_interleaved", {"dims": rot, "base": 10000.0})}
+    mixer = _make("mixer", "latent_attention", params, wt, ctx)
+    assert mixer.ukv is not None
+    xs, refs = {}, {}
+    for r, T in enumerate((400, 330, 5)):
+        x, x64 = _w(rng, (T, W), 1.0)
+        xs[r] = x.cuda()
+        refs[r] = _plain(x64, w64, heads, dim, rot, vdim, rank, params["scale"], 1e-6, sink, gate, window)
+    steps = [[(0, 300), (2, 1)], [(2, 1), (0, 100), (1, 290)], [(2, 3)], [(1, 40)]]
+    before = ops.choices["latent_up_library"]
+    got = _run_in_steps(mixer, ctx, xs, steps, page=16)
+    assert ops.choices["latent_up_library"] >= before + 2
+    old, ops.LATENT_UP_MIN_ROWS = ops.LATENT_UP_MIN_ROWS, 0
+    absorbed = _run_in_steps(mixer, ctx, xs, steps, page=16)
+    ops.LATENT_UP_MIN_ROWS = old
+    rms = lambda a: float(np.sqrt((a ** 2).mean()))
+    for r in xs:
+        off, off_absorbed = (rms(g[r].double().numpy() - refs[r]) / rms(refs[r]) for g in (got, absorbed))
+        # bfloat16 steps between the products: about 2^-8 a piece, and no further off than over the cached latents
+        assert off < 1.5e-2 and off < 1.5 * off_absorbed + 2e-3, (r, off, off_absorbed)
+
+
+def test_rotation_outside_the_table_is_reported():
+    from kv_cache_optimization_for_llm_b200 import ops
+    st = ops.kernel_status("cuda:0")
+    st.zero_()
+
+    class B:
+        positions, status = torch.tensor([0, 7], dtype=torch.int32, device="cuda"), st
+    q = torch.randn(2, 16, device="cuda").bfloat16()
+    want = q.clone()
+    cos, sin = torch.ones(4, 4, device="cuda"), torch.zeros(4, 4, device="cuda")
+    ops.latent_rotate(q, 0, 1, 16, 8, cos, sin, B)
+    assert int(st.item()) == 2 and torch.equal(q, want)
+    st.zero_()
