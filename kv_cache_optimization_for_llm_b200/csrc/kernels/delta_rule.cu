@@ -31,6 +31,8 @@
 // Also here: the short causal convolution with SiLU in front of such a mixer, whose last
 // inputs are part of the request's state.
 #include "common.cuh"
+#include "delta_walk.cuh"
+#include "head_finish.cuh"
 
 enum DeltaMode { MODE_GENERAL = 0, MODE_GATED = 1 };
 
@@ -290,6 +292,14 @@ __global__ void delta_finish_kernel(const DeltaArgs a, int T_) {
   }
 }
 
+template <typename T>
+static void launch_finish(const DeltaArgs& a, int T_, cudaStream_t stream) {
+  if (sizeof(T) == 2 && head_finish_bf16x8(a.o_raw, a.gate, a.ld_gate, a.norm_w, a.norm_per_head, a.out, a.ld_out, T_, a.H, a.Dv, a.eps,
+                                           a.gate_silu, stream)) return;
+  const long long units = (long long)T_ * a.H;
+  kvb_launch(delta_finish_kernel<T>, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, a, T_);
+}
+
 template <typename T, int KPL, int MODE>
 static int launch_scan(const DeltaArgs& a, int R, int T_, int max_run, cudaStream_t stream) {
   const int dv8 = (a.Dv + 7) & ~7;
@@ -323,8 +333,7 @@ static int launch_scan(const DeltaArgs& a, int R, int T_, int max_run, cudaStrea
     if (e != cudaSuccess) return (int)e;
   }
   kvb_launch(delta_scan_kernel<T, KPL, MODE>, dim3(a.H, R, split), dim3(n_scan + n_help), smem, stream, a, n_scan, cols);
-  const long long units = (long long)T_ * a.H;
-  kvb_launch(delta_finish_kernel<T>, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, a, T_);
+  launch_finish<T>(a, T_, stream);
   return kvb_launch_result();
 }
 
@@ -355,6 +364,33 @@ KVB_EXPORT int kvb_delta_scan(const DeltaArgs* args, int mode, int R, int T_, in
     KVB_DISPATCH_DTYPE(dtype, T, return (launch_scan_kpl<T, MODE_GATED>(a, R, T_, max_run, stream)));
   }
   return KVB_ERR_BAD_DTYPE;
+}
+
+// The runs of requests first .. first + R - 1 (token rows row0 .. T_ - 1) walked in pieces of 64 tokens on tensor cores
+// (delta_walk.cuh), then their read-outs' norm and gate: MODE_GATED with one decay per head, bfloat16, Dk 64 or 128, Dv a multiple of
+// 32, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).
+KVB_EXPORT int kvb_delta_walk(const DeltaArgs* args, int first, int R, int row0, int T_, cudaStream_t stream) {
+  DeltaArgs a = *args;
+  if (R <= 0 || T_ <= row0) return 0;
+  if (a.o_raw == nullptr || !a.decay_per_head || a.G < 1 || a.H % a.G) return KVB_ERR_BAD_SIZE;
+  using B = __nv_bfloat16;
+  delta_walk::Args w = {};
+  w.q = static_cast<const B*>(a.r); w.ld_q = a.ld_r;
+  w.k = static_cast<const B*>(a.k); w.ld_k = a.ld_k;
+  w.v = static_cast<const B*>(a.v); w.ld_v = a.ld_v;
+  w.share = a.H / a.G;
+  w.decay = static_cast<const B*>(a.decay); w.ld_decay = a.ld_decay; w.decay_bias = a.decay_bias; w.head_rate = a.head_rate;
+  w.beta = static_cast<const B*>(a.aux); w.ld_beta = a.ld_aux;
+  w.state = a.state; w.slot_stride = a.slot_stride; w.o = a.o_raw;
+  w.q_start = a.q_start; w.req_start = a.req_start; w.slots = a.slots;
+  w.H = a.H; w.Dv = a.Dv; w.first = first;
+  const int rc = delta_walk::launch_any(w, a.Dk, R, stream);
+  if (rc != 0) return rc;
+  a.o_raw += (size_t)row0 * a.H * a.Dv;
+  a.gate = static_cast<const B*>(a.gate) + (size_t)row0 * a.ld_gate;
+  a.out = static_cast<B*>(a.out) + (size_t)row0 * a.ld_out;
+  launch_finish<B>(a, T_ - row0, stream);
+  return kvb_launch_result();
 }
 
 // ---------------------------------------------------------------- short causal convolution + SiLU
@@ -406,31 +442,38 @@ struct AppendArgs {
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {
   static constexpr int N = 4;
-  static __device__ __forceinline__ void load(const float* p, float* x) {
-    const float4 u = *reinterpret_cast<const float4*>(p); x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+  static __device__ __forceinline__ void unpack(uint4 u, float* x) {
+    x[0] = __uint_as_float(u.x); x[1] = __uint_as_float(u.y); x[2] = __uint_as_float(u.z); x[3] = __uint_as_float(u.w);
   }
+  static __device__ __forceinline__ void load(const float* p, float* x) { unpack(*reinterpret_cast<const uint4*>(p), x); }
   static __device__ __forceinline__ void store(float* p, const float* x) {
     *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
   }
 };
 template <> struct Vec16<__nv_bfloat16> {
   static constexpr int N = 8;
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* x) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const unsigned w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { x[2 * e] = __uint_as_float(w[e] << 16); x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
-  }
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* x) {
-    unsigned w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-      w[e] = *reinterpret_cast<unsigned*>(&v);
-    }
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
+  static __device__ __forceinline__ void unpack(uint4 u, float* x) { unpack_bf16x8(u, x); }
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* x) { unpack(*reinterpret_cast<const uint4*>(p), x); }
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* x) { *reinterpret_cast<uint4*>(p) = pack_bf16x8(x); }
 };
+
+// Channels c .. c + VEC - 1 of a token, at or behind k_off, into the request's page.
+template <typename T>
+__device__ __forceinline__ void append_row(const AppendArgs& ap, int c, int r, int pos, const float* acc) {
+  const bool is_v = c >= ap.v_off;
+  const int width = is_v ? ap.Dv : ap.Dk;
+  const int rel = c - (is_v ? ap.v_off : ap.k_off);
+  const int g = rel / width, i = rel - g * width;
+  if (g >= ap.kv_heads) return;
+  const int lp = pos / ap.page_size;
+  const int page = lp < ap.max_pages ? ap.block_table[(size_t)r * ap.max_pages + lp] : -1;
+  if (page < 0 || page >= ap.num_pages) {
+    atomicCAS(ap.status, 0, KVB_STATUS_UNMAPPED_PAGE);
+    return;
+  }
+  T* row = static_cast<T*>(ap.pages) + (((size_t)page * ap.kv_heads + g) * ap.page_size + (pos % ap.page_size)) * (ap.Dk + ap.Dv);
+  Vec16<T>::store(row + (is_v ? ap.Dk : 0) + i, acc);
+}
 
 // TAPS > 0: the number of taps, known when the kernel is built; the thread's VEC x TAPS weights are then fetched with
 // 16-byte loads into registers.  TAPS 0: any number, the weights fetched one by one.
@@ -516,22 +559,82 @@ __global__ void conv_vec_kernel(const T* __restrict__ in, int ld, const float* _
     for (int e = 0; e < VEC; ++e) acc[e] = acc[e] / (1.0f + expf(-acc[e]));
   }
   Vec16<T>::store(out + (size_t)t * C + c, acc);
-  if (ap.pages != nullptr && c >= ap.k_off) {
-    const bool is_v = c >= ap.v_off;
-    const int width = is_v ? ap.Dv : ap.Dk;
-    const int rel = c - (is_v ? ap.v_off : ap.k_off);
-    const int g = rel / width, i = rel - g * width;
-    if (g < ap.kv_heads) {
-      const int lp = pos / ap.page_size;
-      const int page = lp < ap.max_pages ? ap.block_table[(size_t)r * ap.max_pages + lp] : -1;
-      if (page < 0 || page >= ap.num_pages) {
-        atomicCAS(ap.status, 0, KVB_STATUS_UNMAPPED_PAGE);
+  if (ap.pages != nullptr && c >= ap.k_off) append_row<T>(ap, c, r, pos, acc);
+}
+
+// The same for long steps: a thread takes VEC channels of kConvTokens consecutive token rows, so that the weights are fetched once and every
+// input once (the window moves through registers).  What bounds it: bytes (2048 tokens of 6144 channels in bfloat16: 50 MB).  With a
+// token a thread the weights, 16 bytes a channel, came from the caches again for every token, and every input four times: 75 us; now 39
+// (four tokens a thread: 40; eight without the limit to 128 registers: 52; 2048 tokens of 3072 channels 39, now 26).
+constexpr int kConvTokens = 8;
+
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(256, 2)
+conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, const float* __restrict__ tails, long long slot_stride,
+                T* __restrict__ out, int C, int T_, const int* __restrict__ positions, const int* __restrict__ token_req,
+                const int* __restrict__ req_start, const int* __restrict__ slots, int act, AppendArgs ap,
+                const float* __restrict__ in_bias, const float* __restrict__ out_bias) {
+  constexpr int VEC = Vec16<T>::N, BACK = TAPS - 1;
+  pdl_trigger();
+  pdl_wait();
+  const int groups = C / VEC;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int block = (int)(idx / groups), c = (int)(idx - (long long)block * groups) * VEC;
+  const int t0 = block * kConvTokens;
+  if (t0 >= T_) return;
+  uint4 x[kConvTokens + BACK];                 // rows t0 - BACK .. as they lie in memory
+  int req[kConvTokens + BACK];
+#pragma unroll
+  for (int i = 0; i < kConvTokens + BACK; ++i) {
+    const int t = t0 - BACK + i;
+    const bool in_step = t >= 0 && t < T_;
+    x[i] = in_step ? *reinterpret_cast<const uint4*>(in + (size_t)t * ld + c) : make_uint4(0u, 0u, 0u, 0u);
+    req[i] = in_step ? token_req[t] : -1;
+  }
+  float wv[VEC * TAPS], ob[VEC], ib[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC * TAPS; i += 4) {
+    const float4 u = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + i);
+    wv[i] = u.x; wv[i + 1] = u.y; wv[i + 2] = u.z; wv[i + 3] = u.w;
+  }
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    ob[e] = out_bias ? out_bias[c + e] : 0.f;
+    ib[e] = in_bias ? in_bias[c + e] : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < kConvTokens; ++k) {
+    const int t = t0 + k;
+    if (t >= T_) break;
+    const int r = req[k + BACK], pos = positions[t];
+    float acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = ob[e];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {
+      const int back = BACK - j;
+      float v[VEC];
+      if (req[k + j] == r) {                   // a request's tokens of the step are consecutive rows
+        Vec16<T>::unpack(x[k + j], v);
       } else {
-        T* row = static_cast<T*>(ap.pages) +
-                 (((size_t)page * ap.kv_heads + g) * ap.page_size + (pos % ap.page_size)) * (ap.Dk + ap.Dv);
-        Vec16<T>::store(row + (is_v ? ap.Dk : 0) + i, acc);
+        const int sp = pos - back, start = req_start[r];
+        const float* tp = tails + (size_t)slots[r] * slot_stride + (long long)(sp - (start - BACK)) * C + c;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) v[e] = sp < 0 ? 0.f : tp[e];
       }
+      if (pos - back >= 0) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) v[e] += ib[e];
+      }
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wv[e * TAPS + j], v[e], acc[e]);
     }
+    if (act == 0) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = acc[e] / (1.0f + expf(-acc[e]));
+    }
+    Vec16<T>::store(out + (size_t)t * C + c, acc);
+    if (ap.pages != nullptr && c >= ap.k_off) append_row<T>(ap, c, r, pos, acc);
   }
 }
 
@@ -592,8 +695,18 @@ KVB_EXPORT int kvb_conv_silu(const void* in, int ld, const float* w, int taps, f
   kvb_launch(conv_vec_kernel<T, TAPS>, dim3((unsigned)((units + 255) / 256)), dim3(256), 0, stream, (const T*)in, ld, w, \
              taps, (const float*)tails, slot_stride, (T*)out, C, T_, positions, token_req, q_start, req_start, slots, act, ap, \
              in_bias, out_bias)
+    // blocks of tokens from where they still give every SM a block of threads (measured: 1024 tokens of 3072 channels 23 / 19 us,
+    // 600 of 3072 and 300 of 6144 level)
+    const bool runs = w16 && taps >= 2 && taps <= 4 && units / kConvTokens >= 256ll * kvb_sm_count();
+    const long long run_units = (long long)((T_ + kConvTokens - 1) / kConvTokens) * (C / vec);
+#define KVB_CONV_RUN(TAPS)                                                                                              \
+  kvb_launch(conv_run_kernel<T, TAPS>, dim3((unsigned)((run_units + 255) / 256)), dim3(256), 0, stream, (const T*)in, ld, w, \
+             (const float*)tails, slot_stride, (T*)out, C, T_, positions, token_req, req_start, slots, act, ap, in_bias, out_bias)
     KVB_DISPATCH_DTYPE(dtype, T, {
-      if (taps == 2 && w16) KVB_CONV(2);
+      if (runs && taps == 2) KVB_CONV_RUN(2);
+      else if (runs && taps == 3) KVB_CONV_RUN(3);
+      else if (runs) KVB_CONV_RUN(4);
+      else if (taps == 2 && w16) KVB_CONV(2);
       else if (taps == 3 && w16) KVB_CONV(3);
       else if (taps == 4 && w16) KVB_CONV(4);
       else KVB_CONV(0);
@@ -602,6 +715,7 @@ KVB_EXPORT int kvb_conv_silu(const void* in, int ld, const float* w, int taps, f
                    C, q_start, req_start, ctx_len, slots);
     });
 #undef KVB_CONV
+#undef KVB_CONV_RUN
     return kvb_launch_result();
   }
   KVB_DISPATCH_DTYPE(dtype, T, {

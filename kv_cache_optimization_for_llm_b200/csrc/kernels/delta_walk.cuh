@@ -1,0 +1,460 @@
+// The gated delta rule with one decay per head and token, along a request's run of tokens, on tensor cores:
+//
+//   S <- g S;   u = beta (v - S^T k);   S <- S + k u^T;   o = S^T q          (k, q unit vectors, q also times N^-1/2)
+//
+// A block owns DVC value columns of one (request, head) and walks the run in pieces of 64 tokens.  With P_i the product of a
+// piece's decays up to token i and S what the piece begins with, the corrections u of the piece solve
+//
+//   (I + A) U = R,    A_ij = beta_i (P_i / P_j) (k_i . k_j)  for j < i,    R_i = beta_i (v_i - P_i S^T k_i)
+//
+// and  o_i = P_i S^T q_i + sum_{j <= i} (P_i / P_j) (q_i . k_j) u_j,    S <- P_63 S + sum_j (P_63 / P_j) k_j u_j^T.
+//
+// A does not depend on the state: four helper warps make the inverse of I + A for the next piece (its columns by elimination in
+// float32, two lanes a column) and fetch its rows and gates, while four walking warps do this piece's products on mma.sync.  As in
+// chunk_walk.cuh keys and queries go in as they came (their norms are factors per token) and every float32 operand as the
+// sum of three bfloat16 numbers; where both are float32 (inverse and right side, weighed scores and corrections) six of
+// the nine products are made, the others lie below 2^-24.
+//
+// What bounds it: one piece is a chain of three steps of products with a barrier behind each.  Walking token by token in float32 is a chain
+// of 64 steps of two dot products each: 32 heads of 64 x 64, runs of 1548 + 500 tokens 474 us, now DELTA_WALK_US.
+#pragma once
+
+#include "chunk_walk.cuh"
+
+namespace delta_walk {
+
+using namespace walk;
+
+constexpr int kWalkers = 128, kAll = 256;
+
+struct Args {
+  const bf16* q; int ld_q;            // head h reads q and k at (h / share) * N, v at h * Dv
+  const bf16* k; int ld_k;
+  const bf16* v; int ld_v;
+  int share;
+  const bf16* decay; int ld_decay; const float* decay_bias; const float* head_rate;     // [T, H], [H], [H]
+  const bf16* beta; int ld_beta;                                                        // [T, H], before the sigmoid
+  float* state; long long slot_stride;                                                  // slot 0's [H][Dv][N]
+  float* o;                                                                             // [T, H * Dv] float32
+  const int* q_start; const int* req_start; const int* slots;
+  int H, Dv, first;
+};
+
+struct Gates {
+  float hi[kPiece], lo[kPiece];       // log P_i as a pair
+  float from[kPiece];                 // P_i
+  float beta[kPiece], kinv[kPiece], qinv[kPiece];
+  float weigh[kPiece];                // P_63 / P_j / |k_j|
+  float keep, pad[3];
+};
+
+template <int N, int DVC>
+struct Layout {
+  static constexpr int PN = pitch(N), PX = pitch(DVC), PT = pitch(kPiece), AT = 72;      // AT: floats per column of A
+  static constexpr int K = 0;                                     // [2][64] rows of PN
+  static constexpr int Q = K + 2 * kPiece * PN;                   // [2][64] rows of PN
+  static constexpr int V = Q + 2 * kPiece * PN;                   // [2][64] rows of PX
+  static constexpr int S = V + 2 * kPiece * PX;                   // [3][N] rows of PX
+  static constexpr int R = S + 3 * N * PX;                        // [3][64] rows of PX: right sides
+  static constexpr int U = R + 3 * kPiece * PX;                   // [3][64]: corrections
+  static constexpr int W = U + 3 * kPiece * PX;                   // [3][64]: weighed corrections
+  static constexpr int T = W + 3 * kPiece * PX;                   // [2][3][64] rows of PT: the inverse
+  static constexpr int A = T + 2 * 3 * kPiece * PT;               // [64][2][36] floats: column j's even rows, then its odd ones
+  static constexpr int G = A + kPiece * AT * 4;                   // [2] gates
+  static constexpr int bytes = G + 2 * (int)sizeof(Gates);
+};
+
+__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float softplus20(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+template <int ID, int THREADS> __device__ __forceinline__ void bar() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
+
+template <int N, int DVC>
+__global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
+  using L = Layout<N, DVC>;
+  constexpr int MT = N / 64, NX = DVC / 8, KN = N / 16;
+  extern __shared__ __align__(128) unsigned char sm[];
+  Gates* gates = reinterpret_cast<Gates*>(sm + L::G);
+  float* At = reinterpret_cast<float*>(sm + L::A);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+  const int slices = p.Dv / DVC, h = blockIdx.x / slices, col0 = blockIdx.x % slices * DVC, r = p.first + blockIdx.y;
+  pdl_trigger();
+  pdl_wait();
+  const int t0 = p.q_start[r], t1 = p.q_start[r + 1];
+  const int pieces = (t1 - t0 + kPiece - 1) / kPiece;
+  float* slot = p.state + (size_t)p.slots[r] * p.slot_stride;
+
+  if (warp >= 4) {
+    // ------------------------------------------------------------ helpers
+    const int ht = tid - kWalkers, hw = warp - 4;
+    const bf16* q = p.q + (size_t)(h / p.share) * N;
+    const bf16* k = p.k + (size_t)(h / p.share) * N;
+    const bf16* v = p.v + (size_t)h * p.Dv + col0;
+    const float rate = expf(p.head_rate[h]), dbias = p.decay_bias[h], q_scale = rsqrtf((float)N);
+    for (int piece = 0; piece <= pieces; ++piece) {      // round `piece` prepares it while the walkers walk the one before
+      if (piece < pieces) {
+        const int c0 = t0 + piece * kPiece, b = piece & 1;
+        Gates& g = gates[b];
+        unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
+        auto rows = [&](unsigned char* to, int at, const bf16* from, int ld, int cols) {
+          const int chunks = cols / 8;
+          for (int x = ht; x < kPiece * chunks; x += kWalkers) {
+            const int i = x / chunks, c = x - i * chunks;
+            const bool in = c0 + i < t1;
+            copy16(to + i * at + c * 16, from + (size_t)(in ? c0 + i : t0) * ld + c * 8, in);
+          }
+        };
+        rows(Ks, L::PN, k, p.ld_k, N);
+        rows(sm + L::Q + b * kPiece * L::PN, L::PN, q, p.ld_q, N);
+        rows(sm + L::V + b * kPiece * L::PX, L::PX, v, p.ld_v, DVC);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (hw == 0) {
+          double c[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = lane + 32 * u, t = c0 + i;
+            float la = 0.f, be = 0.f;                    // behind the run's end nothing decays
+            if (t < t1) {
+              la = -(rate * softplus20(__bfloat162float(p.decay[(size_t)t * p.ld_decay + h]) + dbias));
+              be = sigmoid(__bfloat162float(p.beta[(size_t)t * p.ld_beta + h]));
+            }
+            g.beta[i] = be;
+            c[u] = scan_sum((double)la, lane);
+          }
+          c[1] += __shfl_sync(0xffffffffu, c[0], 31);
+          const double total = __shfl_sync(0xffffffffu, c[1], 31);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = lane + 32 * u;
+            as_pair(c[u], g.hi[i], g.lo[i]);
+            g.from[i] = expf((float)c[u]);
+            g.weigh[i] = expf((float)(total - c[u]));
+          }
+          if (lane == 0) g.keep = expf((float)total);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        bar<2, kWalkers>();
+        {                                                // a row's norm a thread: keys, then queries
+          const int i = ht & 63;
+          const unsigned char* from = (ht < 64 ? Ks : sm + L::Q + b * kPiece * L::PN) + i * L::PN;
+          float ss = 0.f;
+#pragma unroll
+          for (int c = 0; c < N / 8; ++c) {
+            const uint4 u = *reinterpret_cast<const uint4*>(from + c * 16);
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float x = __uint_as_float(w[e] << 16), y = __uint_as_float(w[e] & 0xffff0000u);
+              ss = fmaf(x, x, ss);
+              ss = fmaf(y, y, ss);
+            }
+          }
+          if (ht < 64) {
+            const float inv = 1.0f / sqrtf(ss + 1e-6f);
+            g.kinv[i] = inv;
+            g.weigh[i] *= inv;
+          } else {
+            g.qinv[i] = q_scale / sqrtf(ss + 1e-6f);
+          }
+        }
+        bar<2, kWalkers>();
+        {                                                // A, column by column in shared memory
+          float G[8][4];
+#pragma unroll
+          for (int x = 0; x < 8; ++x) G[x][0] = G[x][1] = G[x][2] = G[x][3] = 0.f;
+#pragma unroll
+          for (int kk = 0; kk < KN; ++kk) {
+            uint32_t a[4];
+            ldm4(a, Ks + (hw * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
+#pragma unroll
+            for (int jt = 0; jt < 4; ++jt)
+              if (jt <= hw) {
+                uint32_t f[4];
+                ldm4(f, Ks + (jt * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + (kk * 2 + (lane >> 3 & 1)) * 16);
+                mma(G[2 * jt], a, f[0], f[1]);
+                mma(G[2 * jt + 1], a, f[2], f[3]);
+              }
+          }
+          const int row = hw * 16 + gq;
+#pragma unroll
+          for (int x = 0; x < 8; ++x)
+            if (x / 2 <= hw) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int i = row + (e >> 1) * 8, j = x * 8 + 2 * tq + (e & 1);
+                const float d = expf((g.hi[i] - g.hi[j]) + (g.lo[i] - g.lo[j]));
+                At[j * L::AT + (i & 1) * 36 + (i >> 1)] = j < i ? g.beta[i] * g.kinv[i] * g.kinv[j] * d * G[x][e] : 0.f;
+              }
+            }
+        }
+        bar<2, kWalkers>();
+        {                                                // columns of the inverse: lanes 2 m and 2 m + 1 hold column 16 hw + m's even and odd rows
+          const int par = lane & 1, col = hw * 16 + (lane >> 1);
+          float x[32];
+#pragma unroll
+          for (int s = 0; s < 32; ++s) x[s] = 2 * s + par == col ? 1.f : 0.f;
+#pragma unroll
+          for (int j = 0; j < 63; ++j)
+            if (j >= hw * 16) {                          // above their first row a warp's columns are zero
+              const float u = __shfl_sync(0xffffffffu, x[j >> 1], (lane & ~1) | (j & 1));
+              const float4* a4 = reinterpret_cast<const float4*>(At + j * L::AT + par * 36);
+#pragma unroll
+              for (int s = (j >> 1) & ~3; s < 32; s += 4) {      // rows up to j itself are zero in A
+                const float4 a = a4[s >> 2];
+                x[s] = fmaf(-a.x, u, x[s]);
+                x[s + 1] = fmaf(-a.y, u, x[s + 1]);
+                x[s + 2] = fmaf(-a.z, u, x[s + 2]);
+                x[s + 3] = fmaf(-a.w, u, x[s + 3]);
+              }
+            }
+          unsigned char* Ts = sm + L::T + b * 3 * kPiece * L::PT;
+          const int odd = lane >> 1 & 1;                 // of two neighbouring columns the first writes the even s, the second the odd ones
+#pragma unroll
+          for (int s = 0; s < 32; ++s) {
+            const float y = __shfl_xor_sync(0xffffffffu, x[s], 2);
+            if ((s & 1) == odd) {
+              uint32_t part[3];
+              split3(part, odd ? y : x[s], odd ? x[s] : y);
+#pragma unroll
+              for (int w = 0; w < 3; ++w)
+                *reinterpret_cast<uint32_t*>(Ts + (w * kPiece + 2 * s + par) * L::PT + (col & ~1) * 2) = part[w];
+            }
+          }
+        }
+      }
+      bar<0, kAll>();                                    // the walkers are done with the piece before; this one is ready
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------- walkers
+  const bool fresh = p.req_start[r] == 0;
+  float S[MT][NX][4];                                    // rows (warp * MT + mt) * 16 + gq (+ 8), columns 8 nt + 2 tq (+ 1)
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < NX; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int n = (warp * MT + mt) * 16 + gq + (e >> 1) * 8, c = 8 * nt + 2 * tq + (e & 1);
+        S[mt][nt][e] = fresh ? 0.f : slot[((size_t)h * p.Dv + col0 + c) * N + n];
+      }
+  auto put = [&](int at, int rows, int row, int nt, float x, float y) {      // two neighbouring columns of a row, in three parts
+    uint32_t part[3];
+    split3(part, x, y);
+    unsigned char* to = sm + at + row * L::PX + (8 * nt + 2 * tq) * 2;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(to + s * rows * L::PX) = part[s];
+  };
+  auto put_state = [&]() {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NX; ++nt) {
+        put(L::S, N, (warp * MT + mt) * 16 + gq, nt, S[mt][nt][0], S[mt][nt][1]);
+        put(L::S, N, (warp * MT + mt) * 16 + gq + 8, nt, S[mt][nt][2], S[mt][nt][3]);
+      }
+  };
+  // acc += a (three parts, one 16 x 16 tile) * the three parts at `from`, rows jt * 16 ..: the six products that count
+  auto mma6 = [&](float (*acc)[4], const uint32_t (*a)[4], int from, int jt) {
+#pragma unroll
+    for (int nt = 0; nt < NX; nt += 2) {
+      uint32_t f[3][4];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) ldm4t(f[s], sm + from + (s * kPiece + jt * 16 + (lane & 15)) * L::PX + (nt + (lane >> 4)) * 16);
+#pragma unroll
+      for (int o = 2; o >= 0; --o)
+#pragma unroll
+        for (int s = 0; s <= o; ++s) {
+          mma(acc[nt], a[o - s], f[s][0], f[s][1]);
+          mma(acc[nt + 1], a[o - s], f[s][2], f[s][3]);
+        }
+    }
+  };
+  put_state();
+  bar<0, kAll>();                                        // the first piece is ready
+  const int row = warp * 16 + gq;                        // this thread's tokens of a piece: row and row + 8
+  for (int piece = 0; piece < pieces; ++piece) {
+    const int c0 = t0 + piece * kPiece, b = piece & 1;
+    const Gates& g = gates[b];
+    const unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
+    const unsigned char* Qs = sm + L::Q + b * kPiece * L::PN;
+    const unsigned char* Vs = sm + L::V + b * kPiece * L::PX;
+    float G[8][4], accq[NX][4], acck[NX][4];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) G[x][0] = G[x][1] = G[x][2] = G[x][3] = 0.f;
+#pragma unroll
+    for (int x = 0; x < NX; ++x) {
+      accq[x][0] = accq[x][1] = accq[x][2] = accq[x][3] = 0.f;
+      acck[x][0] = acck[x][1] = acck[x][2] = acck[x][3] = 0.f;
+    }
+#pragma unroll
+    for (int kk = 0; kk < KN; ++kk) {
+      uint32_t aq[4], ak[4];
+      ldm4(aq, Qs + (warp * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
+      ldm4(ak, Ks + (warp * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
+#pragma unroll
+      for (int s = 2; s >= 0; --s)
+#pragma unroll
+        for (int nt = 0; nt < NX; nt += 2) {
+          uint32_t f[4];
+          ldm4t(f, sm + L::S + (s * N + kk * 16 + (lane & 15)) * L::PX + (nt + (lane >> 4)) * 16);
+          mma(acck[nt], ak, f[0], f[1]);
+          mma(acck[nt + 1], ak, f[2], f[3]);
+          mma(accq[nt], aq, f[0], f[1]);
+          mma(accq[nt + 1], aq, f[2], f[3]);
+        }
+#pragma unroll
+      for (int jt = 0; jt < 4; ++jt)
+        if (jt <= warp) {
+          uint32_t f[4];
+          ldm4(f, Ks + (jt * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + (kk * 2 + (lane >> 3 & 1)) * 16);
+          mma(G[2 * jt], aq, f[0], f[1]);
+          mma(G[2 * jt + 1], aq, f[2], f[3]);
+        }
+    }
+    const float from0 = g.from[row], from1 = g.from[row + 8];
+    {
+      const float f0 = from0 * g.kinv[row], f1 = from1 * g.kinv[row + 8], b0 = g.beta[row], b1 = g.beta[row + 8];
+#pragma unroll
+      for (int nt = 0; nt < NX; ++nt) {
+        const uint32_t v0 = *reinterpret_cast<const uint32_t*>(Vs + row * L::PX + (8 * nt + 2 * tq) * 2);
+        const uint32_t v1 = *reinterpret_cast<const uint32_t*>(Vs + (row + 8) * L::PX + (8 * nt + 2 * tq) * 2);
+        put(L::R, kPiece, row, nt, b0 * fmaf(-f0, acck[nt][0], __uint_as_float(v0 << 16)),
+            b0 * fmaf(-f0, acck[nt][1], __uint_as_float(v0 & 0xffff0000u)));
+        put(L::R, kPiece, row + 8, nt, b1 * fmaf(-f1, acck[nt][2], __uint_as_float(v1 << 16)),
+            b1 * fmaf(-f1, acck[nt][3], __uint_as_float(v1 & 0xffff0000u)));
+      }
+    }
+    bar<1, kWalkers>();
+
+    // the corrections
+#pragma unroll
+    for (int x = 0; x < NX; ++x) acck[x][0] = acck[x][1] = acck[x][2] = acck[x][3] = 0.f;
+#pragma unroll
+    for (int jt = 0; jt < 4; ++jt)
+      if (jt <= warp) {
+        uint32_t a[3][4];
+#pragma unroll
+        for (int s = 0; s < 3; ++s)
+          ldm4(a[s], sm + L::T + ((b * 3 + s) * kPiece + warp * 16 + (lane & 15)) * L::PT + (jt * 2 + (lane >> 4)) * 16);
+        mma6(acck, a, L::R, jt);
+      }
+    {
+      const float w0 = g.weigh[row], w1 = g.weigh[row + 8];
+#pragma unroll
+      for (int nt = 0; nt < NX; ++nt) {
+        put(L::U, kPiece, row, nt, acck[nt][0], acck[nt][1]);
+        put(L::U, kPiece, row + 8, nt, acck[nt][2], acck[nt][3]);
+        put(L::W, kPiece, row, nt, w0 * acck[nt][0], w0 * acck[nt][1]);
+        put(L::W, kPiece, row + 8, nt, w1 * acck[nt][2], w1 * acck[nt][3]);
+      }
+    }
+    bar<1, kWalkers>();
+
+    // the read-outs
+#pragma unroll
+    for (int x = 0; x < NX; ++x) { accq[x][0] *= from0; accq[x][1] *= from0; accq[x][2] *= from1; accq[x][3] *= from1; }
+    const float h0 = g.hi[row], l0 = g.lo[row], h1 = g.hi[row + 8], l1 = g.lo[row + 8];
+#pragma unroll
+    for (int jt = 0; jt < 4; ++jt)
+      if (jt <= warp) {
+        uint32_t a[3][4];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float* e = G[2 * jt + half];
+          const int j = jt * 16 + half * 8 + 2 * tq;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
+            e[u] = j + u <= row ? e[u] * (expf((h0 - ch) + (l0 - cl)) * w) : 0.f;
+            e[2 + u] = j + u <= row + 8 ? e[2 + u] * (expf((h1 - ch) + (l1 - cl)) * w) : 0.f;
+          }
+          uint32_t up[3], low[3];
+          split3(up, e[0], e[1]);
+          split3(low, e[2], e[3]);
+#pragma unroll
+          for (int s = 0; s < 3; ++s) { a[s][2 * half] = up[s]; a[s][2 * half + 1] = low[s]; }
+        }
+        mma6(accq, a, L::U, jt);
+      }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = row + 8 * half;
+      if (c0 + i < t1) {
+        const float f = g.qinv[i];
+        float* to = p.o + (size_t)(c0 + i) * p.H * p.Dv + (size_t)h * p.Dv + col0 + 2 * tq;
+#pragma unroll
+        for (int nt = 0; nt < NX; ++nt)
+          *reinterpret_cast<float2*>(to + 8 * nt) = make_float2(accq[nt][2 * half] * f, accq[nt][2 * half + 1] * f);
+      }
+    }
+
+    // the state
+    const float keep = g.keep;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NX; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[mt][nt][e] *= keep;
+#pragma unroll
+    for (int jj = 0; jj < kPiece / 16; ++jj) {
+      uint32_t a[MT][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+        ldm4t(a[mt], Ks + (jj * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + ((warp * MT + mt) * 2 + (lane >> 3 & 1)) * 16);
+#pragma unroll
+      for (int s = 2; s >= 0; --s)
+#pragma unroll
+        for (int nt = 0; nt < NX; nt += 2) {
+          uint32_t f[4];
+          ldm4t(f, sm + L::W + (s * kPiece + jj * 16 + (lane & 15)) * L::PX + (nt + (lane >> 4)) * 16);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            mma(S[mt][nt], a[mt], f[0], f[1]);
+            mma(S[mt][nt + 1], a[mt], f[2], f[3]);
+          }
+        }
+    }
+    if (piece + 1 < pieces) put_state();
+    bar<0, kAll>();
+  }
+  if (pieces > 0) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NX; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int n = (warp * MT + mt) * 16 + gq + (e >> 1) * 8, c = 8 * nt + 2 * tq + (e & 1);
+          slot[((size_t)h * p.Dv + col0 + c) * N + n] = S[mt][nt][e];
+        }
+  }
+}
+
+static inline bool takes(const Args& a, int N) {
+  return (N == 64 || N == 128) && a.Dv >= 32 && a.Dv % 32 == 0 && ((a.ld_q | a.ld_k | a.ld_v) & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
+}
+
+template <int N, int DVC>
+static int launch(const Args& a, int R, cudaStream_t stream) {
+  constexpr int smem = Layout<N, DVC>::bytes;
+  static_assert(smem <= 227 * 1024, "one block's shared memory");
+  cudaError_t e = cudaFuncSetAttribute(delta_walk_kernel<N, DVC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  kvb_launch(delta_walk_kernel<N, DVC>, dim3((unsigned)(a.H * (a.Dv / DVC)), (unsigned)R), dim3(kAll), smem, stream, a);
+  return kvb_launch_result();
+}
+
+// 16 value columns a block, 32 where that still gives (nearly) every SM a block: one block fits an SM, and its time is the run's
+// whatever its width.  A state of 128 rows leaves room for 16 only.
+static int launch_any(const Args& a, int N, int R, cudaStream_t stream) {
+  if (R <= 0) return 0;
+  if (R > 65535 || a.H < 1 || !takes(a, N)) return KVB_ERR_BAD_SIZE;
+  if (N == 128) return launch<128, 16>(a, R, stream);
+  if ((long long)a.H * (a.Dv / 32) * R * 8 < (long long)kvb_sm_count() * 7) return launch<64, 16>(a, R, stream);
+  return launch<64, 32>(a, R, stream);
+}
+
+}  // namespace delta_walk

@@ -30,6 +30,7 @@
 // A run of one chunk reads and writes its slot directly.
 #include "chunk_walk.cuh"
 #include "common.cuh"
+#include "head_finish.cuh"
 
 #include <math_constants.h>
 
@@ -389,6 +390,7 @@ KVB_EXPORT int kvb_head_norm_gate(const float* y, const void* gate, int ld_g, co
   if (heads < 1 || Dv < 1) return KVB_ERR_BAD_SIZE;
   const long long total = (long long)T_ * heads;
   if (total > 0x7fffffffLL) return KVB_ERR_BAD_SIZE;
+  if (dtype == KVB_BF16 && head_finish_bf16x8(y, gate, ld_g, weight, 1, out, heads * Dv, T_, heads, Dv, eps, 0, stream)) return kvb_launch_result();
   KVB_DISPATCH_DTYPE(dtype, T, (kvb_launch(head_norm_gate_kernel<T>, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, stream, y,
                                             (const T*)gate, ld_g, weight, (T*)out, (int)total, heads, Dv, eps)));
   return kvb_launch_result();

@@ -14,6 +14,7 @@
 // request was cut into steps, on the batch or on where the pages lie.  Everything is float32
 // but the cached rows and the query as they are stored.
 #include "common.cuh"
+#include "mma_sync.cuh"
 #include "score_shape.cuh"
 
 #include <math_constants.h>
@@ -509,6 +510,205 @@ static int launch_group_gp(int G, const void* q, int q_row_stride, const void* p
 #undef KVB_WG
 }
 
+// ---------------------------------------------------------------- tokens by themselves on tensor cores
+// The bfloat16 form of the kernel above for groups of up to eight heads (one map) with keys and values of 32, 64 or 128 channels: a
+// block per (token, key/value head), its four warps taking the chunks of 32 keys c with c % 4 == warp, each with two
+// buffers of its own that 16-byte asynchronous copies fill while the chunk before is worked on.  The group's queries are the rows of
+// m16n8k16 products (bfloat16 times bfloat16, exact in float32); scores are shaped and exponentiated in float32, and
+// the exponentials go into the second product as the sum of three bfloat16 numbers (float32's 24 bits).  A key that is not
+// seen adds nothing; its value counts as zero.
+//
+// What bounds it: the rows' bytes and the latency of fetching them.  In the kernel above a lane scores a key by itself (two dependent
+// trips to memory a chunk, 8 FMAs a byte): 64 requests over blocks of 1024 positions, 32 heads of 64 over 8, 56 us for 64 MB;
+// this takes WINDOW_MMA_US.
+constexpr int kMmaWarps = 4, kMmaKeys = 32;
+
+__device__ __forceinline__ void split3_bf16(unsigned* p, float x, float y) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    p[i] = *reinterpret_cast<const unsigned*>(&v);
+    x -= __bfloat162float(v.x);
+    y -= __bfloat162float(v.y);
+  }
+}
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(kMmaWarps * 32)
+window_attention_mma_kernel(const __nv_bfloat16* __restrict__ q_base, int q_row_stride, const __nv_bfloat16* __restrict__ pages,
+                            const int* __restrict__ block_table, int max_pages, int page_size, int num_pages,
+                            const int* __restrict__ positions, const int* __restrict__ token_req, __nv_bfloat16* __restrict__ out,
+                            int nq, int nkv, float scale, int window, int keep_first, int one_more, ScoreShape shape, int* status) {
+  constexpr int KS = DK / 16, NV = DV / 8, CK = DK / 8, CV = DV / 8;
+  // bytes from row to row: an odd number of 16-byte chunks, so that eight rows' chunks lie in different banks
+  constexpr int ROW = ((CK + CV) | 1) * 16, BUF = kMmaKeys * ROW;
+  extern __shared__ __align__(16) unsigned char wsm[];
+  __shared__ float m_s[kMmaWarps][8], l_s[kMmaWarps][8];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, hk = blockIdx.y, G = nq / nkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, tq = lane & 3;
+  unsigned char* bufs = wsm + warp * 2 * BUF;
+  const int pos = positions[t];
+  const int* table = block_table + (size_t)token_req[t] * max_pages;
+  constexpr int row_len = DK + DV;
+  const int lo = first_seen_key(pos, window, shape.chunk);
+  const int keep = window > 0 ? keep_first : 0;
+  const int keep_chunks = (keep + 31) / 32, lo_chunk = lo / 32, last_chunk = pos / 32;
+
+  // the warp's next chunk behind c (c itself if it is one) that holds a key that is seen
+  auto chunk_from = [&](int c) {
+    if (c >= keep_chunks && c < lo_chunk) c += (lo_chunk - c + kMmaWarps - 1) / kMmaWarps * kMmaWarps;
+    return c;
+  };
+  auto bring = [&](int c, int b) {                       // a lane looks up a key's row, then all lanes copy
+    const int j = c * kMmaKeys + lane;
+    long long off = -1;
+    if (j <= pos && (j >= lo || j < keep)) {
+      const int lp = j / page_size;
+      const int page = lp < max_pages ? table[lp] : -1;
+      if (page < 0 || page >= num_pages) atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE);
+      else off = (((long long)page * nkv + hk) * page_size + (j % page_size)) * row_len;
+    }
+#pragma unroll
+    for (int x = 0; x < CK + CV; ++x) {
+      const int at = x * 32 + lane, key = at / (CK + CV), piece = at - key * (CK + CV);
+      const long long o = __shfl_sync(0xffffffffu, off, key);
+      kvb_mma::cp_async_16_zfill(bufs + b * BUF + key * ROW + piece * 16, pages + (o >= 0 ? o + piece * 8 : 0), o >= 0);
+    }
+    kvb_mma::cp_async_commit();
+    return __ballot_sync(0xffffffffu, off >= 0);
+  };
+
+  unsigned qf[KS][4];
+#pragma unroll
+  for (int kk = 0; kk < KS; ++kk) {
+    const __nv_bfloat16* q = q_base + (size_t)t * q_row_stride + (size_t)(hk * G + (row < G ? row : 0)) * DK + kk * 16 + 2 * tq;
+    qf[kk][0] = row < G ? *reinterpret_cast<const unsigned*>(q) : 0u;
+    qf[kk][2] = row < G ? *reinterpret_cast<const unsigned*>(q + 8) : 0u;
+    qf[kk][1] = qf[kk][3] = 0u;                          // rows 8 .. 15 hold nothing
+  }
+  float m = -CUDART_INF_F, l = 0.f, acc[NV][4];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+
+  int c = chunk_from(warp), b = 0;
+  unsigned seen = c <= last_chunk ? bring(c, 0) : 0u;
+  while (c <= last_chunk) {
+    const int next = chunk_from(c + kMmaWarps);
+    unsigned next_seen = 0u;
+    if (next <= last_chunk) {
+      next_seen = bring(next, b ^ 1);
+      kvb_mma::cp_async_wait<1>();
+    } else {
+      kvb_mma::cp_async_wait<0>();
+    }
+    __syncwarp();
+    const unsigned char* kv = bufs + b * BUF;
+    float s[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk)
+#pragma unroll
+      for (int n = 0; n < 4; n += 2) {
+        unsigned f0, f1, f2, f3;
+        kvb_mma::ldmatrix_x4(f0, f1, f2, f3, kv + (n * 8 + (lane & 7) + (lane >> 4) * 8) * ROW + (kk * 2 + (lane >> 3 & 1)) * 16);
+        kvb_mma::mma_bf16(s[n], qf[kk], f0, f1);
+        kvb_mma::mma_bf16(s[n + 1], qf[kk], f2, f3);
+      }
+    // row `row` of the group, keys 8 n + 2 tq (+ 1)
+    float top = -CUDART_INF_F;
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int kk = n * 8 + 2 * tq + u;
+        s[n][u] = seen >> kk & 1 ? shape_score(s[n][u] * scale, shape, hk * G + (row < G ? row : 0), pos - (c * kMmaKeys + kk)) : -CUDART_INF_F;
+        top = fmaxf(top, s[n][u]);
+      }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    const float m_new = fmaxf(m, top);
+    const float corr = m == -CUDART_INF_F ? 0.f : expf(m - m_new);
+    float sum = 0.f;
+    unsigned pf[3][2][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const float p0 = s[n][0] == -CUDART_INF_F ? 0.f : expf(s[n][0] - m_new), p1 = s[n][1] == -CUDART_INF_F ? 0.f : expf(s[n][1] - m_new);
+      sum += p0 + p1;
+      unsigned part[3];
+      split3_bf16(part, p0, p1);
+#pragma unroll
+      for (int w = 0; w < 3; ++w) { pf[w][n >> 1][(n & 1) * 2] = part[w]; pf[w][n >> 1][(n & 1) * 2 + 1] = 0u; }
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    l = fmaf(l, corr, sum);
+    m = m_new;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) { acc[n][0] *= corr; acc[n][1] *= corr; }
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+      for (int n = 0; n < NV; n += 2) {
+        unsigned f0, f1, f2, f3;
+        kvb_mma::ldmatrix_x4_trans(f0, f1, f2, f3, kv + (kk * 16 + (lane & 15)) * ROW + (CK + n + (lane >> 4)) * 16);
+#pragma unroll
+        for (int w = 2; w >= 0; --w) {
+          kvb_mma::mma_bf16(acc[n], pf[w][kk], f0, f1);
+          kvb_mma::mma_bf16(acc[n + 1], pf[w][kk], f2, f3);
+        }
+      }
+    __syncwarp();                                        // this buffer is filled again by the next round
+    c = next;
+    seen = next_seen;
+    b ^= 1;
+  }
+
+  // merge the warps' sums in their order
+  if (tq == 0) { m_s[warp][row] = m; l_s[warp][row] = l; }
+  __syncthreads();
+  float* acc_s = reinterpret_cast<float*>(wsm);          // [warp][8][DV]: the buffers are used up
+  static_assert(8 * DV * 4 <= 2 * BUF, "a warp's sums fit its buffers");
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+    *reinterpret_cast<float2*>(acc_s + ((size_t)warp * 8 + row) * DV + n * 8 + 2 * tq) = make_float2(acc[n][0], acc[n][1]);
+  __syncthreads();
+  for (int x = threadIdx.x; x < G * DV; x += kMmaWarps * 32) {
+    const int g = x / DV, i = x - g * DV, hq = hk * G + g;
+    const float extra = one_more ? 0.f : (shape.sinks != nullptr ? shape.sinks[hq] : -CUDART_INF_F);
+    float M = extra;
+#pragma unroll
+    for (int w = 0; w < kMmaWarps; ++w) M = fmaxf(M, m_s[w][g]);
+    float L = extra == -CUDART_INF_F ? 0.f : expf(extra - M), a = 0.f;
+#pragma unroll
+    for (int w = 0; w < kMmaWarps; ++w) {
+      const float f = m_s[w][g] == -CUDART_INF_F ? 0.f : expf(m_s[w][g] - M);
+      L = fmaf(l_s[w][g], f, L);
+      a = fmaf(acc_s[((size_t)w * 8 + g) * DV + i], f, a);
+    }
+    a = L > 0.f ? a / L * shape.out_scale : 0.f;
+    if (shape.gate != nullptr)
+      a *= 1.0f / (1.0f + expf(-__bfloat162float(static_cast<const __nv_bfloat16*>(shape.gate)[(size_t)t * shape.gate_ld + (size_t)hq * DV + i])));
+    out[((size_t)t * nq + hq) * DV + i] = __float2bfloat16_rn(a);
+  }
+}
+
+template <int DK, int DV>
+static int launch_mma(const void* q, int q_row_stride, const void* pages, const int* block_table, int max_pages, int page_size,
+                      int num_pages, const int* positions, const int* token_req, void* out, int T_, int nq, int nkv, float scale,
+                      int window, int keep_first, int one_more, ScoreShape shape, int* status, cudaStream_t stream) {
+  constexpr int smem = kMmaWarps * 2 * kMmaKeys * ((DK / 8 + DV / 8) | 1) * 16;
+  cudaError_t e = cudaFuncSetAttribute(window_attention_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  using B = __nv_bfloat16;
+  kvb_launch(window_attention_mma_kernel<DK, DV>, dim3(T_, nkv), dim3(kMmaWarps * 32), smem, stream, (const B*)q, q_row_stride,
+             (const B*)pages, block_table, max_pages, page_size, num_pages, positions, token_req, (B*)out, nq, nkv, scale, window,
+             keep_first, one_more, shape, status);
+  return kvb_launch_result();
+}
+
 // q points at the first query head of token 0; consecutive tokens are q_row_stride elements apart.
 // pages: [num_pages, nkv, page_size, Dk + Dv].  out is [T, nq * Dv], dense.
 // Refuses: Dk or Dv above 256, nq not a multiple of nkv, a negative window or keep_first.
@@ -529,6 +729,15 @@ static int window_attention_any(const void* q, int q_row_stride, const void* pag
   // groups of up to 8 heads (4 with two maps) with values of 32, 64 or 128 channels: a block per key/value head, the
   // rows read once
   const int G = nq / nkv * maps;
+  // on tensor cores where the sizes are theirs: queries read in pairs of channels, rows in 16 bytes
+  if (dtype == KVB_BF16 && !shape.pair && G <= 8 && vec && q_row_stride % 2 == 0 && ((uintptr_t)q % 4) == 0) {
+#define KVB_WM(DK, DV)                                                                                                 \
+  if (Dk == DK && Dv == DV)                                                                                            \
+  return launch_mma<DK, DV>(q, q_row_stride, pages, block_table, max_pages, page_size, num_pages, positions, token_req, out, T_, nq, nkv, \
+                            scale, window, keep_first, one_more, shape, status, stream)
+    KVB_WM(32, 32); KVB_WM(64, 64); KVB_WM(128, 64); KVB_WM(128, 128);
+#undef KVB_WM
+  }
   if (G <= kMaxGroup && (Dv == 32 || Dv == 64 || Dv == 128) && vec) {
 #define KVB_WP(VPL, PAIR)                                                                                              \
   KVB_DISPATCH_DTYPE(dtype, T, return (launch_group_gp<T, VPL, PAIR>(G, q, q_row_stride, pages, block_table, max_pages, \

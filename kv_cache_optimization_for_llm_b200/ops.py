@@ -449,6 +449,7 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
     matrix states.  ``mode``: "general" or "gated" (see csrc/kernels/delta_rule.cu).
     ``decay_per_head`` ("gated"): ``decay`` is [T, heads] and ``decay_bias`` [heads], one decay for all key
     channels of a head.  ``gate_act``: "sigmoid" or "silu", the function applied to the output gate.
+    bfloat16 steps with runs of ``WALK_MIN_RUN`` tokens and more and one decay per head go to the walk on tensor cores where the sizes allow.
     Returns the gated, normed read-out [T, heads * dv]."""
     x0 = r[0]
     _need_cuda(x0, state)
@@ -471,11 +472,26 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
     a.o_raw = new((T, heads * dv), torch.float32, x0.device).data_ptr()
     a.decay_per_head = 1 if decay_per_head else 0
     a.gate_silu = {"sigmoid": 0, "silu": 1}[gate_act]
+    global launch_count
+    if (mode == "gated" and decay_per_head and dv % 32 == 0 and k[0].stride(0) % 8 == 0 and v[0].stride(0) % 8 == 0
+            and _at(*k) % 16 == 0 and _at(*v) % 16 == 0 and _walks(batch, dk, 64, x0, r[1])):
+        # single tokens beside the runs (the step's first requests and rows) go token by token
+        singles = int(batch.num_single)
+        if singles:
+            _check(lib("delta_rule").kvb_delta_scan(ctypes.byref(a), c_int(1), c_int(singles), c_int(singles), c_int(1),
+                                                    c_int(dtype_code(x0.dtype)), _stream()), "delta_scan")
+            launch_count += 1
+        rc = lib("delta_rule").kvb_delta_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(singles),
+                                              c_int(T), _stream())
+        _check(rc, "delta_scan")
+        launch_count += 1
+        choices["delta_scan_" + mode] += 1
+        choices["delta_walk"] += 1
+        return out
     rc = lib("delta_rule").kvb_delta_scan(ctypes.byref(a), c_int({"general": 0, "gated": 1}[mode]),
                                           c_int(batch.num_reqs), c_int(T), c_int(int(getattr(batch, "max_q_len", 0) or 0)),
                                           c_int(dtype_code(x0.dtype)), _stream())
     _check(rc, "delta_scan")
-    global launch_count
     launch_count += 1       # the scan and the read-outs' norm
     choices["delta_scan_" + mode] += 1
     return out
@@ -724,6 +740,14 @@ class StepRows:
 # see more than LATENT_UP_MAX_KEYS positions per token they bring.
 LATENT_UP_MIN_ROWS = int(os.environ.get('KVB200_LATENT_UP_MIN_ROWS', '256'))
 LATENT_UP_MAX_KEYS = 3
+# With a rotated part behind the keys, or a gated result, the line is the positions that a run sees: over the cached latents a tile of
+# queries walks its request's rows one tile after the other (0.17 us a row at 16 heads and a latent of 512), making keys and values
+# costs a few launches whatever the length.  Measured (the mixer; cached / made): 64 tokens behind 500 positions 178 / 162 us, behind
+# 2000 420 / 174, behind 7000 1218 / 346; 512 tokens from the start 149 / 162; 8 heads and a latent of 256: 64 behind 500 136 / 159, 512
+# behind 500 187 / 162.  LATENT_UP_KEYS bounds the rows that such a step makes.
+LATENT_UP_MIN_CONTEXT = int(os.environ.get('KVB200_LATENT_UP_MIN_CONTEXT', '768'))
+LATENT_UP_FEW_ROWS = 16
+LATENT_UP_KEYS = 32768
 
 
 def _runs_seen(batch, window: int):
@@ -736,13 +760,17 @@ def _runs_seen(batch, window: int):
     return out
 
 
-def latent_up_wanted(batch, window: int) -> bool:
-    """Whether a step's runs are long enough for keys and values to be worth making: what the captured graphs replay never
-    is (its launches are sized before the positions are known)."""
+def latent_up_wanted(batch, window: int, extra: bool = False) -> bool:
+    """Whether a step's runs are long enough, or see far enough, for keys and values to be worth making: what the captured graphs
+    replay never is (its launches are sized before the positions are known).  ``extra``: rows with a rotated part, or a gated result."""
     tokens = batch.num_tokens - batch.num_single
-    if batch.decode_only or not LATENT_UP_MIN_ROWS or tokens < LATENT_UP_MIN_ROWS or _capturing():
+    if batch.decode_only or not LATENT_UP_MIN_ROWS or tokens < (LATENT_UP_FEW_ROWS if extra else LATENT_UP_MIN_ROWS) or _capturing():
         return False
-    keys = sum(-(-(end - first) // StepRows.PAGE) * StepRows.PAGE for _, first, _, end in _runs_seen(batch, window))
+    seen = _runs_seen(batch, window)
+    keys = sum(-(-(end - first) // StepRows.PAGE) * StepRows.PAGE for _, first, _, end in seen)
+    if extra:
+        return (max(end - lowest for _, _, lowest, end in seen) >= LATENT_UP_MIN_CONTEXT
+                and keys <= max(LATENT_UP_KEYS, LATENT_UP_MAX_KEYS * tokens))
     return keys <= LATENT_UP_MAX_KEYS * tokens
 
 

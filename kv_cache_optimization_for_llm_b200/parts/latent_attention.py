@@ -171,7 +171,8 @@ class LatentAttention(Part):
         q = ops.linear(cq, self.uq) if self.q_rank else d         # without a latent the queries are the product's first columns
         per_head = self.dim + self.rot
         gate = (d, self.at_g) if self.at_g is not None else None
-        if self.ukv is not None and ops.latent_up_wanted(batch, self.window or 0) and (gate is None or self.at_g % 2 == 0):
+        if self.ukv is not None and ops.latent_up_wanted(batch, self.window or 0, bool(self.rot or gate)) and (
+                gate is None or self.at_g % 2 == 0):
             return ops.linear(self._over_made_rows(q, table, batch, cache, cos, sin, rdims, gate), self.o)
         q_abs = ops.head_gemm(q, 0, per_head, self.uk_t, tensor_cores=self.split)
         lat = ops.latent_attention(q_abs, q, self.dim if self.rot else 0, per_head, cos, sin, rdims, cache.k, table, batch, self.sink,

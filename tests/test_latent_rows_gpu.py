@@ -75,9 +75,11 @@ def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, 
         xs[r] = x.cuda()
         refs[r] = _plain(x64, w64, heads, dim, rot, vdim, rank, params["scale"], 1e-6, sink, gate, window)
     steps = [[(0, 300), (2, 1)], [(2, 1), (0, 100), (1, 290)], [(2, 3)], [(1, 40)]]
-    before = ops.choices["latent_up_library"]
+    before, line = ops.choices["latent_up_library"], ops.LATENT_UP_MIN_CONTEXT
+    ops.LATENT_UP_MIN_CONTEXT = 64      # here short contexts go this way as well
     got = _run_in_steps(mixer, ctx, xs, steps, page=16)
-    assert ops.choices["latent_up_library"] >= before + 2
+    ops.LATENT_UP_MIN_CONTEXT = line
+    assert ops.choices["latent_up_library"] == before + 3       # the steps with runs of 16 tokens and more
     old, ops.LATENT_UP_MIN_ROWS = ops.LATENT_UP_MIN_ROWS, 0
     absorbed = _run_in_steps(mixer, ctx, xs, steps, page=16)
     ops.LATENT_UP_MIN_ROWS = old

@@ -139,3 +139,65 @@ def test_mlstm_walk(steps, H, N, Dv):
         t += n
     untouched = [s for s in range(12) if s not in slots.values()]
     assert torch.equal(state[untouched], was[untouched])
+
+
+def _delta_plain(q, k, v, zd, zb, bias, rate, S, H, G, N, Dv):
+    T = q.shape[0]
+    unit = lambda m: m / torch.sqrt(m.square().sum(-1, keepdim=True) + 1e-6)
+    q, k = (unit(m.double().view(T, G, N)).repeat_interleave(H // G, 1) for m in (q, k))
+    q, v, beta = q * N ** -0.5, v.double().view(T, H, Dv), torch.sigmoid(zb.double())
+    g = torch.exp(-rate.double().exp() * torch.nn.functional.softplus(zd.double() + bias.double()))
+    o = torch.empty((T, H, Dv), dtype=torch.float64, device=q.device)
+    for t in range(T):
+        S = S * g[t, :, None, None]
+        u = beta[t, :, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S = S + k[t, :, :, None] * u[:, None]
+        o[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return o, S
+
+
+@pytest.mark.parametrize("alike", [False, True])       # alike: keys that are nearly the same, so that the corrections depend on one another most
+@pytest.mark.parametrize("steps", STEPS)
+@pytest.mark.parametrize("H,G,N,Dv", [(2, 1, 64, 32), (4, 4, 64, 64), (3, 1, 128, 32), (64, 16, 64, 64)])
+def test_delta_walk(steps, H, G, N, Dv, alike):
+    from kv_cache_optimization_for_llm_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(H + N + len(steps))
+    rn = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    T = sum(n for *_, n in steps)
+    c = rn(T, 2 * G * N + H * Dv)
+    if alike:
+        c[:, G * N:2 * G * N] = 0.2 * c[:, G * N:2 * G * N] + rn(1, G * N)
+    c, small, gate = c.bfloat16(), rn(T, 2 * H).bfloat16(), rn(T, H * Dv).bfloat16()
+    if alike:
+        small[:, H:] += 3.0
+    bias, rate, norm = rn(H) - 3.0, rn(H), rn(Dv)
+    state = rn(12, H * Dv * N + 24)[:, 8:]
+    slots = {r: (3 * r + 1) % 11 for r, *_ in steps}
+    batch = _batch(steps, slots)
+    was = state.clone()
+
+    def scan(st):
+        return ops.delta_scan("gated", batch, st, (c, 0), (c, G * N), (c, 2 * G * N), (gate, 0), (small, 0), (small, H), bias, None,
+                              rate, norm, False, H, G, N, Dv, 1e-5, decay_per_head=True, gate_act="silu")
+    before = ops.choices["delta_walk"]
+    y = scan(state)
+    assert ops.choices["delta_walk"] == before + 1
+    old_state, old = was.clone(), ops.WALK_MIN_RUN
+    ops.WALK_MIN_RUN = 0
+    y_old = scan(old_state)
+    ops.WALK_MIN_RUN = old
+    t = 0
+    for r, start, n in [e for e in steps if e[2] == 1] + [e for e in steps if e[2] != 1]:
+        s0 = was[slots[r]][:H * Dv * N].double().view(H, Dv, N).transpose(1, 2) * (1.0 if start else 0.0)
+        cols = c[t:t + n].split([G * N, G * N, H * Dv], 1)
+        o, last = _delta_plain(*cols, small[t:t + n, :H], small[t:t + n, H:], bias, rate, s0, H, G, N, Dv)
+        ref = (o / torch.sqrt(o.square().mean(-1, keepdim=True) + 1e-5) * norm.double()).reshape(n, -1)
+        ref = ref * torch.nn.functional.silu(gate[t:t + n].double())
+        view = lambda s: s[slots[r]][:H * Dv * N].view(H, Dv, N).transpose(1, 2)
+        # the state is float32 sums; the results are rounded to bfloat16 (2^-8 at most, about 2^-9.5 in the mean)
+        assert _rel(view(state), last) < 5e-6 and _rel(view(state), last) < 2.0 * _rel(view(old_state), last) + 2e-7, \
+            (r, _rel(view(state), last), _rel(view(old_state), last))
+        assert _rel(y[t:t + n], ref) < 2.5e-3 and _rel(y[t:t + n], ref) < 1.05 * _rel(y_old[t:t + n], ref) + 1e-6
+        t += n
+    untouched = [s for s in range(12) if s not in slots.values()]
+    assert torch.equal(state[untouched], was[untouched]) and torch.equal(state[:, H * Dv * N:], was[:, H * Dv * N:])
