@@ -29,7 +29,7 @@ namespace walk {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kPiece = 64, kThreads = 128;
+constexpr int kPiece = 64, kThreads = 128, kGateWarp = kThreads / 32, kBlock = kThreads + 32;      // a fifth warp makes the next piece's gates
 
 enum Rule { SSD = 0, MLSTM = 1 };
 
@@ -105,6 +105,9 @@ struct Gates {
   float keep, m, pad[2];
 };
 static_assert(sizeof(Gates) == (8 * kPiece + 4) * 4, "as laid out");
+
+__device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 0, %0;" ::"n"(kBlock) : "memory"); }
+__device__ __forceinline__ void walkers_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
 
 __device__ __forceinline__ void as_pair(double x, float& hi, float& lo) {
   hi = (float)x;
@@ -206,7 +209,7 @@ __device__ __forceinline__ void make_gates(const Args& p, int h, int nt, int lan
 }
 
 template <int RULE, int N, int DVC>
-__global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
+__global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
   using L = Layout<RULE, N, DVC>;
   constexpr int MT = N / 64, NT = L::COLS / 8, NX = DVC / 8, KN = N / 16;      // MT: 16-row tiles of the state per warp
   extern __shared__ __align__(128) unsigned char sm[];
@@ -238,10 +241,32 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  // the state: rows (warp * MT + mt) * 16 + gq (+ 8), columns 8 nt + 2 tq (+ 1)
-  float S[MT][NT][4];
+  const int pieces = (t1 - t0 + kPiece - 1) / kPiece;
   const size_t splits = (size_t)(p.Dv / 64), at_n = (size_t)p.H * p.Dv * N + ((size_t)h * splits + col0 / 64) * N;
   const size_t at_m = (size_t)p.H * p.Dv * N + (size_t)p.H * splits * N + (size_t)h * splits + col0 / 64;
+  if (warp == kGateWarp) {
+    const float m0 = RULE == MLSTM && !fresh ? slot[at_m] : 0.f;
+    if (RULE == MLSTM) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    float raw[4], m = m0;
+    if (pieces > 0) raw_gates<RULE>(p, h, t0, t1, lane, raw);
+    for (int piece = 0; piece < pieces; ++piece) {       // a piece's gates are made while the other warps walk the one before
+      Gates& g = gates[piece & 1];
+      const int c0 = t0 + piece * kPiece;
+      make_gates<RULE>(p, h, min(kPiece, t1 - c0), lane, raw, m, g);
+      if (piece + 1 < pieces) raw_gates<RULE>(p, h, c0 + kPiece, t1, lane, raw);
+      __syncwarp();
+      if (RULE == MLSTM) m = g.m;
+      block_barrier();
+    }
+    if (RULE == MLSTM) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (pieces > 0 && lane == 0 && col0 % 64 == 0) slot[at_m] = m;
+    }
+    return;
+  }
+
+  // the state: rows (warp * MT + mt) * 16 + gq (+ 8), columns 8 nt + 2 tq (+ 1)
+  float S[MT][NT][4];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -256,7 +281,6 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
         }
         S[mt][nt][e] = x;
       }
-  const float m0 = RULE == MLSTM && !fresh ? slot[at_m] : 0.f;
   // MLSTM: the blocks of 64 value columns share n and m in the slot; nobody writes them before all have read
   if (RULE == MLSTM) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   auto put_state = [&]() {
@@ -274,14 +298,8 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
         }
   };
 
-  const int pieces = (t1 - t0 + kPiece - 1) / kPiece;
   if (pieces > 0) bring(0);
   put_state();
-  float raw[4];
-  if (warp == 0 && pieces > 0) {
-    raw_gates<RULE>(p, h, t0, t1, lane, raw);
-    make_gates<RULE>(p, h, min(kPiece, t1 - t0), lane, raw, m0, gates[0]);
-  }
   const int row = warp * 16 + gq;                        // this thread's tokens of a piece: row and row + 8
   for (int piece = 0; piece < pieces; ++piece) {
     const int c0 = t0 + piece * kPiece, b = piece & 1;
@@ -289,8 +307,7 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
     const unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
     const unsigned char* Xs = sm + L::X + b * kPiece * L::PX;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    if (warp == 0 && piece + 1 < pieces) raw_gates<RULE>(p, h, c0 + kPiece, t1, lane, raw);
+    block_barrier();                                     // rows, gates and the state's parts are there, the buffers before them free
 
     // weighed values, three parts each
     for (int x = tid; x < kPiece * NX; x += kThreads) {
@@ -352,7 +369,7 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
         }
       }
     }
-    __syncthreads();                                     // the weighed values are there; q and the state's parts are free
+    walkers_barrier();                                   // the weighed values are there; q and the state's parts are free
     if (piece + 1 < pieces) bring(piece + 1);
 
     // the scores' weights, then their product with the values
@@ -461,10 +478,7 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
         }
       }
     }
-    if (piece + 1 < pieces) {
-      put_state();
-      if (warp == 0) make_gates<RULE>(p, h, min(kPiece, t1 - c0 - kPiece), lane, raw, g.m, gates[b ^ 1]);
-    }
+    if (piece + 1 < pieces) put_state();
   }
   if (RULE == MLSTM) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (pieces > 0) {
@@ -478,7 +492,6 @@ __global__ void __launch_bounds__(kThreads) walk_kernel(const Args p) {
           if (c < DVC) slot[((size_t)h * p.Dv + col0 + c) * N + n] = S[mt][nt][e];
           else if (c == DVC && col0 % 64 == 0) slot[at_n + n] = S[mt][nt][e];
         }
-    if (RULE == MLSTM && tid == 0 && col0 % 64 == 0) slot[at_m] = gates[(pieces - 1) & 1].m;
   }
 }
 
@@ -495,7 +508,7 @@ static int launch(const Args& a, int R, cudaStream_t stream) {
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.H * (a.Dv / DVC)), (unsigned)R);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(kBlock);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];

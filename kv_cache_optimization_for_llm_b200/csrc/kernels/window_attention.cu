@@ -929,6 +929,128 @@ __global__ void __launch_bounds__(256) qk_rot_append_kernel(QkRotArgs a) {
   }
 }
 
+// The same in bfloat16 where every segment and head is whole 16-byte pieces: a thread takes U pieces of eight channels and requests all
+// it needs (rows, biases, weights, angles) before it waits for any of it; only a rotation that pairs channels half a head
+// apart goes through shared memory.  What bounds it: latency (a token is a few KB).  The form above goes to memory five times one
+// behind the other, two bytes at a time: 64 tokens of 32 + 8 + 8 heads of 64 13.3 us; this takes QK_ROT_US.
+template <int U>
+__global__ void __launch_bounds__(256) qk_rot_append_bf16x8_kernel(QkRotArgs a) {
+  extern __shared__ float qk_s[];             // [nQ + nK] normed queries and keys, only for layout 0
+  __shared__ float part[2][8];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kw = a.maps * a.Dk, nQ = a.nq * a.Dk, nK = a.nkv * kw, nV = a.nkv * a.Dv, half = a.rot >> 1;
+  const __nv_bfloat16* row = static_cast<const __nv_bfloat16*>(a.src) + (size_t)t * a.ld;
+  const int pos = a.positions[t];
+  bool turn = a.rot > 0;
+  if (turn && (pos < 0 || pos >= a.table_len)) {
+    if (threadIdx.x == 0) atomicCAS(a.status, 0, KVB_STATUS_BAD_POSITION);
+    turn = false;
+  }
+  int page = -1;
+  if (a.write) {
+    const int lp = pos / a.page_size;
+    page = (pos >= 0 && lp < a.max_pages) ? a.block_table[(size_t)a.token_req[t] * a.max_pages + lp] : -1;
+    if (page < 0 || page >= a.num_pages) {
+      if (threadIdx.x == 0) atomicCAS(a.status, 0, KVB_STATUS_UNMAPPED_PAGE);
+      page = -1;
+    }
+  }
+  float v[U][8], w[U][8], cs[U][8], sn[U][8];
+  float sq = 0.f, sk = 0.f;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int c = (u * 256 + threadIdx.x) * 8;           // queries, then keys, then values
+    if (c >= nQ + nK + nV) continue;
+    const bool is_q = c < nQ, is_k = !is_q && c < nQ + nK;
+    const int at = is_q ? c : (is_k ? c - nQ : c - nQ - nK);
+    const uint4 x = *reinterpret_cast<const uint4*>(row + (is_q ? at : (is_k ? a.k_off + at : a.v_off + at)));
+    const float* bias = is_q ? a.bq : (is_k ? a.bk : a.bv);
+    const float* weight = is_q ? a.qw : (is_k ? a.kw : nullptr);
+    const unsigned xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { v[u][2 * e] = __uint_as_float(xw[e] << 16); v[u][2 * e + 1] = __uint_as_float(xw[e] & 0xffff0000u); }
+    const int d = at % a.Dk;                             // channel of its head (queries and keys)
+    const bool mine = turn && (is_q || is_k) && d < a.rot;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (bias != nullptr) v[u][e] += bias[at + e];
+      w[u][e] = weight != nullptr ? weight[at + e] : 1.f;
+      // the angle of channel d + e: pair d + e or d + e - half with layout 0, (d + e) / 2 with layout 1
+      const int i = !mine ? 0 : (a.layout == 0 ? (d < half ? d + e : d + e - half) : (d + e) >> 1);
+      cs[u][e] = mine ? a.cos_t[(size_t)pos * half + i] : 1.f;
+      sn[u][e] = mine ? a.sin_t[(size_t)pos * half + i] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (is_q) sq = fmaf(v[u][e], v[u][e], sq);
+      else if (is_k) sk = fmaf(v[u][e], v[u][e], sk);
+    }
+  }
+  float rq = 1.f, rk = 1.f;
+  if (a.qw != nullptr || a.kw != nullptr) {
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    if (lane == 0) { part[0][warp] = sq; part[1][warp] = sk; }
+    __syncthreads();
+    float tq = 0.f, tk = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { tq += part[0][i]; tk += part[1][i]; }
+    if (a.qw != nullptr) rq = 1.0f / sqrtf(tq / (float)nQ + a.eps);
+    if (a.kw != nullptr) rk = 1.0f / sqrtf(tk / (float)nK + a.eps);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int c = (u * 256 + threadIdx.x) * 8;
+    if (c >= nQ + nK) continue;
+    const float r = c < nQ ? rq : rk;
+    const bool normed = (c < nQ ? a.qw : a.kw) != nullptr;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (normed) v[u][e] = v[u][e] * r * w[u][e];
+      if (a.layout == 0 && turn) qk_s[c + e] = v[u][e];
+    }
+  }
+  if (a.layout == 0 && turn) __syncthreads();
+  __nv_bfloat16* q_out = static_cast<__nv_bfloat16*>(a.q_out) + (size_t)t * nQ;
+  __nv_bfloat16* pages = static_cast<__nv_bfloat16*>(a.pages);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int c = (u * 256 + threadIdx.x) * 8;
+    if (c >= nQ + nK + nV) continue;
+    const bool is_q = c < nQ, is_k = !is_q && c < nQ + nK;
+    const int at = is_q ? c : (is_k ? c - nQ : c - nQ - nK);
+    if (turn && (is_q || is_k)) {
+      const int d = at % a.Dk;
+      if (d < a.rot) {
+        if (a.layout == 0) {
+          const float* other = qk_s + c + (d < half ? half : -half);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[u][e] = d < half ? v[u][e] * cs[u][e] - other[e] * sn[u][e] : v[u][e] * cs[u][e] + other[e] * sn[u][e];
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            const float x = v[u][e], y = v[u][e + 1];
+            v[u][e] = x * cs[u][e] - y * sn[u][e];
+            v[u][e + 1] = y * cs[u][e] + x * sn[u][e];
+          }
+        }
+      }
+    }
+    unsigned p[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[e] = kvb_mma::pack_bf16(v[u][2 * e], v[u][2 * e + 1]);
+    const uint4 packed = make_uint4(p[0], p[1], p[2], p[3]);
+    if (is_q) {
+      *reinterpret_cast<uint4*>(q_out + at) = packed;
+    } else if (page >= 0) {
+      const int width = is_k ? kw : a.Dv, head = at / width, in = at - head * width + (is_k ? 0 : kw);
+      *reinterpret_cast<uint4*>(pages + (((size_t)page * a.nkv + head) * a.page_size + (pos % a.page_size)) * (kw + a.Dv) + in) = packed;
+    }
+  }
+}
+
 // Refuses: head sizes above 256, rot odd or above Dk, a layout other than 0 or 1, more than 48 K queries and keys a token.
 KVB_EXPORT int kvb_qk_rot_append(const QkRotArgs* args, int T_, int dtype, cudaStream_t stream) {
   if (T_ <= 0) return 0;
@@ -939,6 +1061,15 @@ KVB_EXPORT int kvb_qk_rot_append(const QkRotArgs* args, int T_, int dtype, cudaS
   if (a.rot > 0 && (a.cos_t == nullptr || a.sin_t == nullptr)) return KVB_ERR_BAD_SIZE;
   const size_t smem = (size_t)(a.nq + a.nkv * a.maps) * a.Dk * sizeof(float);
   if (smem > 192 * 1024) return KVB_ERR_BAD_SIZE;
+  const int pieces = ((a.nq + a.nkv * a.maps) * a.Dk + a.nkv * a.Dv) / 8;
+  if (dtype == KVB_BF16 && ((a.Dk | a.Dv | a.ld | a.k_off | a.v_off) & 7) == 0 && a.rot % (a.layout == 0 ? 16 : 8) == 0 && pieces <= 1024 &&
+      smem <= 48 * 1024 && ((reinterpret_cast<uintptr_t>(a.src) | reinterpret_cast<uintptr_t>(a.q_out) | reinterpret_cast<uintptr_t>(a.pages)) & 15) == 0) {
+    const size_t sm = a.layout == 0 && a.rot > 0 ? smem : 0;
+    if (pieces <= 256) kvb_launch(qk_rot_append_bf16x8_kernel<1>, dim3(T_), dim3(256), sm, stream, a);
+    else if (pieces <= 512) kvb_launch(qk_rot_append_bf16x8_kernel<2>, dim3(T_), dim3(256), sm, stream, a);
+    else kvb_launch(qk_rot_append_bf16x8_kernel<4>, dim3(T_), dim3(256), sm, stream, a);
+    return kvb_launch_result();
+  }
   KVB_DISPATCH_DTYPE(dtype, T, {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(qk_rot_append_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

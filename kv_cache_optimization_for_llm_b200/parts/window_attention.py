@@ -308,6 +308,7 @@ class RotaryChunkAttention(Part):
         self.g_off = starts[3] if params.get("gate") else None
         self.q_bias, self.k_bias, self.v_bias = (weights.get(n) for n in ("q_bias", "k_bias", "v_bias"))
         self.o_bias = weights.get("o_bias")
+        self.o_bias_low = None if self.o_bias is None else self.o_bias.to(ctx.dtype)     # for a caller that does not add it itself
         self.q_norm, self.k_norm = weights.get("q_norm"), weights.get("k_norm")
         self.sinks = weights.get("sink")
         self.o = weights["o"]
@@ -364,7 +365,7 @@ class RotaryChunkAttention(Part):
         if bias_out:
             return y, self.o_bias
         if self.o_bias is not None:
-            y = y + self.o_bias.to(y.dtype)
+            y += self.o_bias_low
         return y
 
 
