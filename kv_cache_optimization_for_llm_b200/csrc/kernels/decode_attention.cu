@@ -456,13 +456,6 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // a running max and sum per head (rows lane/4 and lane/4 + 8) and a running output in
   // registers; the slices of a warp are private to it, so the walk needs no block-wide barrier.
   for (int cls = z; cls < C; cls += S) {
-  if (cls != z) {
-    // the new key, if in this class, is in the cache by now
-    my_first = cls;
-    while (my_first < t_first) my_first += C;
-    n_mine = my_first < n_tiles ? (n_tiles - 1 - my_first) / C + 1 : 0;
-    request_first_tiles(false);
-  }
   float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
   float o[DT][4];
 #pragma unroll
@@ -577,6 +570,14 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     if (more && arrived) set_have(stage, request_located(my_first + (i + kStages) * C, stage, next_off));
     else if (more) set_have(stage, 0u);   // (cp.async: the new key, if in that tile, is in the cache by now)
     if constexpr (!kTma) cp_async_commit();
+  }
+  if (cls + S < C) {
+    // the next class's first tiles are under way while this one's partials are merged (this warp is done with its slices; the
+    // new key, if in that class, is in the cache by now)
+    my_first = cls + S;
+    while (my_first < t_first) my_first += C;
+    n_mine = my_first < n_tiles ? (n_tiles - 1 - my_first) / C + 1 : 0;
+    request_first_tiles(false);
   }
 #pragma unroll
   for (int rr = 0; rr < 2; ++rr) {
@@ -799,7 +800,16 @@ KVB_EXPORT int kvb_decode_attention_mma(const void* qkv, int q_row_stride, void*
   // larger batches (every block then walks several classes and pays its fixed cost once)
   int S = cluster;
   // (an SM holds four blocks of head size 64 with one stage, two of head size 128: no second wave)
-  while (S > 1 && (long long)R * nkv * S > (d == 64 ? 4 : 2) * kvb_sm_count()) S >>= 1;
+  const int resident = (d == 64 ? 4 : 2) * kvb_sm_count();
+  while (S > 1 && (long long)R * nkv * S > resident) S >>= 1;
+  // Beyond 2048 positions one block a (request, kv head) walks up to 64 tiles and more, and the longest request is the launch's
+  // time: there up to 2.7 times as many blocks as the GPU holds share the work (the hardware deals the shorter ones out behind
+  // the longer).  Measured, head size 128, 8 kv heads, one block / this rule: 24 requests of 500 to 7900 positions 118 / 85 us, of
+  // 3000 each 67 / 67, of 7000 to 8000 135 / 130; 48 of 500 to 7900 179 / 151, of 3000 138 / 118; 32 of 3000 74 / 80; head size 64: 48 of
+  // 500 to 7900 104 / 78, 64 of 500 to 7900 115 / 101, of 3000 69 / 73.  Where two blocks and more share a request anyway, and below 2048
+  // positions, a second round of blocks cost more than it gave (16 requests of 3000 41 / 46).
+  if (S == 1 && cluster > 4)
+    while (S < cluster && (long long)R * nkv * S * 2 * 10 <= 27ll * resident) S <<= 1;
   // Whole pages by TMA at head size 128 where the pages allow it (at least 8 rows, so that a box fills whole
   // rows of the swizzle pattern; addresses that a tensor map takes); key by key otherwise, at head size 128
   // then in the one-stage form only.  At head size 64 TMA measured level or slower (batch 8 at 4096 tokens
