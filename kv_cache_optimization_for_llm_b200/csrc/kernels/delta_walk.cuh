@@ -187,37 +187,44 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
             }
         }
         bar<2, kWalkers>();
-        {                                                // columns of the inverse: lanes 2 m and 2 m + 1 hold column 16 hw + m's even and odd rows
-          const int par = lane & 1, col = hw * 16 + (lane >> 1);
+        {
+          // Columns of the inverse: lanes 2 m and 2 m + 1 hold column 16 hw + m's even and odd rows, x[s] being row 8 jb + 2 s + par;
+          // above its first row a warp's columns are zero.  Eight rows are finished a turn, then the others move up: the
+          // loop stays a loop (unrolled over all 63 steps its code alone took longer to fetch than the piece's products).
+          const int par = lane & 1, col = hw * 16 + (lane >> 1), odd = lane >> 1 & 1;
+          unsigned char* Ts = sm + L::T + b * 3 * kPiece * L::PT;
           float x[32];
 #pragma unroll
-          for (int s = 0; s < 32; ++s) x[s] = 2 * s + par == col ? 1.f : 0.f;
+          for (int s = 0; s < 32; ++s) x[s] = 2 * s + par == (lane >> 1) ? 1.f : 0.f;
+#pragma unroll 1
+          for (int jb = 2 * hw; jb < 8; ++jb) {
+            const float* column = At + jb * 8 * L::AT + par * 36 + jb * 4;
 #pragma unroll
-          for (int j = 0; j < 63; ++j)
-            if (j >= hw * 16) {                          // above their first row a warp's columns are zero
-              const float u = __shfl_sync(0xffffffffu, x[j >> 1], (lane & ~1) | (j & 1));
-              const float4* a4 = reinterpret_cast<const float4*>(At + j * L::AT + par * 36);
+            for (int jj = 0; jj < 8; ++jj, column += L::AT) {
+              const float u = __shfl_sync(0xffffffffu, x[jj >> 1], (lane & ~1) | (jj & 1));
 #pragma unroll
-              for (int s = (j >> 1) & ~3; s < 32; s += 4) {      // rows up to j itself are zero in A
-                const float4 a = a4[s >> 2];
-                x[s] = fmaf(-a.x, u, x[s]);
-                x[s + 1] = fmaf(-a.y, u, x[s + 1]);
-                x[s + 2] = fmaf(-a.z, u, x[s + 2]);
-                x[s + 3] = fmaf(-a.w, u, x[s + 3]);
+              for (int s = 0; s < 32; s += 4)            // rows up to the column's own are zero in A
+                if (s < 4 * (8 - jb)) {
+                  const float4 a = *reinterpret_cast<const float4*>(column + s);
+                  x[s] = fmaf(-a.x, u, x[s]);
+                  x[s + 1] = fmaf(-a.y, u, x[s + 1]);
+                  x[s + 2] = fmaf(-a.z, u, x[s + 2]);
+                  x[s + 3] = fmaf(-a.w, u, x[s + 3]);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {                // of two neighbouring columns the first writes the even s, the second the odd ones
+              const float y = __shfl_xor_sync(0xffffffffu, x[s], 2);
+              if ((s & 1) == odd) {
+                uint32_t part[3];
+                split3(part, odd ? y : x[s], odd ? x[s] : y);
+#pragma unroll
+                for (int w = 0; w < 3; ++w)
+                  *reinterpret_cast<uint32_t*>(Ts + (w * kPiece + 8 * jb + 2 * s + par) * L::PT + (col & ~1) * 2) = part[w];
               }
             }
-          unsigned char* Ts = sm + L::T + b * 3 * kPiece * L::PT;
-          const int odd = lane >> 1 & 1;                 // of two neighbouring columns the first writes the even s, the second the odd ones
 #pragma unroll
-          for (int s = 0; s < 32; ++s) {
-            const float y = __shfl_xor_sync(0xffffffffu, x[s], 2);
-            if ((s & 1) == odd) {
-              uint32_t part[3];
-              split3(part, odd ? y : x[s], odd ? x[s] : y);
-#pragma unroll
-              for (int w = 0; w < 3; ++w)
-                *reinterpret_cast<uint32_t*>(Ts + (w * kPiece + 2 * s + par) * L::PT + (col & ~1) * 2) = part[w];
-            }
+            for (int s = 0; s < 28; ++s) x[s] = x[s + 4];
           }
         }
       }
@@ -453,7 +460,7 @@ static int launch_any(const Args& a, int N, int R, cudaStream_t stream) {
   if (R <= 0) return 0;
   if (R > 65535 || a.H < 1 || !takes(a, N)) return KVB_ERR_BAD_SIZE;
   if (N == 128) return launch<128, 16>(a, R, stream);
-  if ((long long)a.H * (a.Dv / 32) * R * 8 < (long long)kvb_sm_count() * 7) return launch<64, 16>(a, R, stream);
+  if ((long long)a.H * (a.Dv / 32) * R * 5 < (long long)kvb_sm_count() * 4) return launch<64, 16>(a, R, stream);
   return launch<64, 32>(a, R, stream);
 }
 

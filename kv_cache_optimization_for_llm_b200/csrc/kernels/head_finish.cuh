@@ -5,7 +5,7 @@
 //
 // Dv / 8 neighbouring lanes (a power of two, at most 32) take a head, eight channels each: two 16-byte loads of y, one of the gate
 // and one store a thread, the sum by shuffles.  What bounds it: bytes (2048 tokens of 32 heads of 64: 33 MB).  A warp per head with
-// four-byte and two-byte accesses, y read twice, took 23 to 25 us; this takes HEAD_FINISH_US.
+// four-byte and two-byte accesses, y read twice, took 23 to 25 us; this takes 9.
 #pragma once
 
 #include "common.cuh"

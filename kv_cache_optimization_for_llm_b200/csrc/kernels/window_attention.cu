@@ -520,7 +520,7 @@ static int launch_group_gp(int G, const void* q, int q_row_stride, const void* p
 //
 // What bounds it: the rows' bytes and the latency of fetching them.  In the kernel above a lane scores a key by itself (two dependent
 // trips to memory a chunk, 8 FMAs a byte): 64 requests over blocks of 1024 positions, 32 heads of 64 over 8, 56 us for 64 MB;
-// this takes WINDOW_MMA_US.
+// this takes 27.
 constexpr int kMmaWarps = 4, kMmaKeys = 32;
 
 __device__ __forceinline__ void split3_bf16(unsigned* p, float x, float y) {
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(256) qk_rot_append_kernel(QkRotArgs a) {
 // The same in bfloat16 where every segment and head is whole 16-byte pieces: a thread takes U pieces of eight channels and requests all
 // it needs (rows, biases, weights, angles) before it waits for any of it; only a rotation that pairs channels half a head
 // apart goes through shared memory.  What bounds it: latency (a token is a few KB).  The form above goes to memory five times one
-// behind the other, two bytes at a time: 64 tokens of 32 + 8 + 8 heads of 64 13.3 us; this takes QK_ROT_US.
+// behind the other, two bytes at a time: 64 tokens of 32 + 8 + 8 heads of 64 13.3 us; this takes 6.1.
 template <int U>
 __global__ void __launch_bounds__(256) qk_rot_append_bf16x8_kernel(QkRotArgs a) {
   extern __shared__ float qk_s[];             // [nQ + nK] normed queries and keys, only for layout 0
