@@ -9,14 +9,16 @@
 //
 // and  o_i = P_i S^T q_i + sum_{j <= i} (P_i / P_j) (q_i . k_j) u_j,    S <- P_63 S + sum_j (P_63 / P_j) k_j u_j^T.
 //
-// A does not depend on the state: four helper warps make the inverse of I + A for the next piece (its columns by elimination in
-// float32, two lanes a column) and fetch its rows and gates, while four walking warps do this piece's products on mma.sync.  As in
+// A does not depend on the state: four helper warps fetch the next piece's rows and make the inverse of I + A for it (its diagonal
+// blocks of 16 by elimination in float32, two lanes a column, the blocks below them by products), a ninth warp makes its gates, while
+// four walking warps do this piece's products on mma.sync.  As in
 // chunk_walk.cuh keys and queries go in as they came (their norms are factors per token) and every float32 operand as the
 // sum of three bfloat16 numbers; where both are float32 (inverse and right side, weighed scores and corrections) six of
 // the nine products are made, the others lie below 2^-24.
 //
 // What bounds it: one piece is a chain of three steps of products with a barrier behind each.  Walking token by token in float32 is a chain
-// of 64 steps of two dot products each: 32 heads of 64 x 64, runs of 1548 + 500 tokens 474 us, now DELTA_WALK_US.
+// of 64 steps of two dot products each: 32 heads of 64 x 64, runs of 1548 + 500 tokens 474 us, now 173 (352 and 317 with the
+// whole inverse by elimination).
 #pragma once
 
 #include "chunk_walk.cuh"
@@ -25,7 +27,7 @@ namespace delta_walk {
 
 using namespace walk;
 
-constexpr int kWalkers = 128, kAll = 256;
+constexpr int kWalkers = 128, kAll = 2 * kWalkers + 32;      // walkers, helpers, one warp for the gates
 
 struct Args {
   const bf16* q; int ld_q;            // head h reads q and k at (h / share) * N, v at h * Dv
@@ -50,22 +52,40 @@ struct Gates {
 
 template <int N, int DVC>
 struct Layout {
-  static constexpr int PN = pitch(N), PX = pitch(DVC), PT = pitch(kPiece), AT = 72;      // AT: floats per column of A
-  static constexpr int K = 0;                                     // [2][64] rows of PN
-  static constexpr int Q = K + 2 * kPiece * PN;                   // [2][64] rows of PN
-  static constexpr int V = Q + 2 * kPiece * PN;                   // [2][64] rows of PX
-  static constexpr int S = V + 2 * kPiece * PX;                   // [3][N] rows of PX
+  static constexpr int PN = pitch(N), PX = pitch(DVC), PT = pitch(kPiece);
+  static constexpr int STAGES = N == 64 ? 3 : 2;                  // three where they fit: rows are fetched a round before the helpers need them
+  static constexpr int PD = 20;                                   // floats per column of a diagonal block: eight even rows, eight odd ones
+  static constexpr int K = 0;                                     // [STAGES][64] rows of PN
+  static constexpr int Q = K + STAGES * kPiece * PN;              // [STAGES][64] rows of PN
+  static constexpr int V = Q + STAGES * kPiece * PN;              // [STAGES][64] rows of PX
+  static constexpr int S = V + STAGES * kPiece * PX;              // [3][N] rows of PX
   static constexpr int R = S + 3 * N * PX;                        // [3][64] rows of PX: right sides
   static constexpr int U = R + 3 * kPiece * PX;                   // [3][64]: corrections
   static constexpr int W = U + 3 * kPiece * PX;                   // [3][64]: weighed corrections
   static constexpr int T = W + 3 * kPiece * PX;                   // [2][3][64] rows of PT: the inverse
-  static constexpr int A = T + 2 * 3 * kPiece * PT;               // [64][2][36] floats: column j's even rows, then its odd ones
-  static constexpr int G = A + kPiece * AT * 4;                   // [2] gates
-  static constexpr int bytes = G + 2 * (int)sizeof(Gates);
+  static constexpr int A = T + 2 * 3 * kPiece * PT;               // [3][64] rows of PT: A left of its diagonal blocks
+  static constexpr int D = A + 3 * kPiece * PT;                   // [4][16] columns of PD floats: A's diagonal blocks
+  static constexpr int G = D + 4 * 16 * PD * 4;                   // [3] gates
+  static constexpr int bytes = G + 3 * (int)sizeof(Gates);
 };
 
 __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus20(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+__device__ __forceinline__ void stm4t(const uint32_t* r, void* p) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+               ::"r"(smem_at(p)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+// two 16 x 8 accumulators side by side, times `sign`, as a 16 x 16 left operand in three parts
+__device__ __forceinline__ void left_parts(uint32_t (*to)[4], const float (*d)[4], float sign) {
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t up[3], low[3];
+    split3(up, sign * d[half][0], sign * d[half][1]);
+    split3(low, sign * d[half][2], sign * d[half][3]);
+#pragma unroll
+    for (int s = 0; s < 3; ++s) { to[s][2 * half] = up[s]; to[s][2 * half + 1] = low[s]; }
+  }
+}
 template <int ID, int THREADS> __device__ __forceinline__ void bar() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
 
 template <int N, int DVC>
@@ -74,14 +94,48 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
   constexpr int MT = N / 64, NX = DVC / 8, KN = N / 16;
   extern __shared__ __align__(128) unsigned char sm[];
   Gates* gates = reinterpret_cast<Gates*>(sm + L::G);
-  float* At = reinterpret_cast<float*>(sm + L::A);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
   const int slices = p.Dv / DVC, h = blockIdx.x / slices, col0 = blockIdx.x % slices * DVC, r = p.first + blockIdx.y;
   pdl_trigger();
   pdl_wait();
   const int t0 = p.q_start[r], t1 = p.q_start[r + 1];
-  const int pieces = (t1 - t0 + kPiece - 1) / kPiece;
+  // Round s: the gates of piece s, the rows of piece s (of s - 1 with two stages), the inverse of piece s - 1, the walk over piece s - 2.
+  const int pieces = (t1 - t0 + kPiece - 1) / kPiece, rounds = pieces > 0 ? pieces + 2 : 0;
   float* slot = p.state + (size_t)p.slots[r] * p.slot_stride;
+
+  if (warp == 8) {
+    // ------------------------------------------------------------ gates
+    const float rate = expf(p.head_rate[h]), dbias = p.decay_bias[h];
+    for (int s = 0; s < rounds; ++s) {
+      if (s < pieces) {
+        Gates& g = gates[s % 3];
+        double c[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = lane + 32 * u, t = t0 + s * kPiece + i;
+          float la = 0.f, be = 0.f;                      // behind the run's end nothing decays
+          if (t < t1) {
+            la = -(rate * softplus20(__bfloat162float(p.decay[(size_t)t * p.ld_decay + h]) + dbias));
+            be = sigmoid(__bfloat162float(p.beta[(size_t)t * p.ld_beta + h]));
+          }
+          g.beta[i] = be;
+          c[u] = scan_sum((double)la, lane);
+        }
+        c[1] += __shfl_sync(0xffffffffu, c[0], 31);
+        const double total = __shfl_sync(0xffffffffu, c[1], 31);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = lane + 32 * u;
+          as_pair(c[u], g.hi[i], g.lo[i]);
+          g.from[i] = expf((float)c[u]);
+          g.weigh[i] = expf((float)(total - c[u]));
+        }
+        if (lane == 0) g.keep = expf((float)total);
+      }
+      bar<0, kAll>();
+    }
+    return;
+  }
 
   if (warp >= 4) {
     // ------------------------------------------------------------ helpers
@@ -89,54 +143,51 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
     const bf16* q = p.q + (size_t)(h / p.share) * N;
     const bf16* k = p.k + (size_t)(h / p.share) * N;
     const bf16* v = p.v + (size_t)h * p.Dv + col0;
-    const float rate = expf(p.head_rate[h]), dbias = p.decay_bias[h], q_scale = rsqrtf((float)N);
-    for (int piece = 0; piece <= pieces; ++piece) {      // round `piece` prepares it while the walkers walk the one before
-      if (piece < pieces) {
-        const int c0 = t0 + piece * kPiece, b = piece & 1;
-        Gates& g = gates[b];
-        unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
-        auto rows = [&](unsigned char* to, int at, const bf16* from, int ld, int cols) {
-          const int chunks = cols / 8;
-          for (int x = ht; x < kPiece * chunks; x += kWalkers) {
-            const int i = x / chunks, c = x - i * chunks;
-            const bool in = c0 + i < t1;
-            copy16(to + i * at + c * 16, from + (size_t)(in ? c0 + i : t0) * ld + c * 8, in);
-          }
-        };
-        rows(Ks, L::PN, k, p.ld_k, N);
-        rows(sm + L::Q + b * kPiece * L::PN, L::PN, q, p.ld_q, N);
-        rows(sm + L::V + b * kPiece * L::PX, L::PX, v, p.ld_v, DVC);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (hw == 0) {
-          double c[2];
+    const float q_scale = rsqrtf((float)N);
+    auto rows = [&](unsigned char* to, int at, const bf16* from, int ld, int cols, int c0) {
+      const int chunks = cols / 8;
+      for (int x = ht; x < kPiece * chunks; x += kWalkers) {
+        const int i = x / chunks, c = x - i * chunks;
+        const bool in = c0 + i < t1;
+        copy16(to + i * at + c * 16, from + (size_t)(in ? c0 + i : t0) * ld + c * 8, in);
+      }
+    };
+    auto bring = [&](int piece) {
+      const int c0 = t0 + piece * kPiece, b = piece % L::STAGES;
+      rows(sm + L::K + b * kPiece * L::PN, L::PN, k, p.ld_k, N, c0);
+      rows(sm + L::Q + b * kPiece * L::PN, L::PN, q, p.ld_q, N, c0);
+      rows(sm + L::V + b * kPiece * L::PX, L::PX, v, p.ld_v, DVC, c0);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // acc += left (16 x 16) * the transpose of the 16 x 16 block at `from`, both in three parts: the six products that count
+    auto mma6t = [&](float (*acc)[4], const uint32_t (*left)[4], const unsigned char* from) {
+      uint32_t f[3][4];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int i = lane + 32 * u, t = c0 + i;
-            float la = 0.f, be = 0.f;                    // behind the run's end nothing decays
-            if (t < t1) {
-              la = -(rate * softplus20(__bfloat162float(p.decay[(size_t)t * p.ld_decay + h]) + dbias));
-              be = sigmoid(__bfloat162float(p.beta[(size_t)t * p.ld_beta + h]));
-            }
-            g.beta[i] = be;
-            c[u] = scan_sum((double)la, lane);
-          }
-          c[1] += __shfl_sync(0xffffffffu, c[0], 31);
-          const double total = __shfl_sync(0xffffffffu, c[1], 31);
+      for (int u = 0; u < 3; ++u) ldm4(f[u], from + (u * kPiece + (lane & 7) + (lane >> 4) * 8) * L::PT + (lane >> 3 & 1) * 16);
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int i = lane + 32 * u;
-            as_pair(c[u], g.hi[i], g.lo[i]);
-            g.from[i] = expf((float)c[u]);
-            g.weigh[i] = expf((float)(total - c[u]));
-          }
-          if (lane == 0) g.keep = expf((float)total);
+      for (int o = 2; o >= 0; --o)
+#pragma unroll
+        for (int u = 0; u <= o; ++u) {
+          mma(acc[0], left[o - u], f[u][0], f[u][1]);
+          mma(acc[1], left[o - u], f[u][2], f[u][3]);
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        bar<2, kWalkers>();
+    };
+    for (int s = 0; s < rounds; ++s) {
+      if (L::STAGES == 3 && s < pieces) bring(s);
+      if (s >= 1 && s <= pieces) {
+        const int piece = s - 1, b = piece % L::STAGES;
+        Gates& g = gates[piece % 3];
+        unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
+        unsigned char* Ts = sm + L::T + (piece & 1) * 3 * kPiece * L::PT;
+        if (L::STAGES == 2) {
+          bring(piece);
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+          bar<2, kWalkers>();
+        }
         {                                                // a row's norm a thread: keys, then queries
           const int i = ht & 63;
           const unsigned char* from = (ht < 64 ? Ks : sm + L::Q + b * kPiece * L::PN) + i * L::PN;
-          float ss = 0.f;
+          float ss[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int c = 0; c < N / 8; ++c) {
             const uint4 u = *reinterpret_cast<const uint4*>(from + c * 16);
@@ -144,20 +195,22 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float x = __uint_as_float(w[e] << 16), y = __uint_as_float(w[e] & 0xffff0000u);
-              ss = fmaf(x, x, ss);
-              ss = fmaf(y, y, ss);
+              ss[e] = fmaf(x, x, ss[e]);
+              ss[e] = fmaf(y, y, ss[e]);
             }
           }
+          const float sum = (ss[0] + ss[1]) + (ss[2] + ss[3]);
           if (ht < 64) {
-            const float inv = 1.0f / sqrtf(ss + 1e-6f);
+            const float inv = 1.0f / sqrtf(sum + 1e-6f);
             g.kinv[i] = inv;
             g.weigh[i] *= inv;
           } else {
-            g.qinv[i] = q_scale / sqrtf(ss + 1e-6f);
+            g.qinv[i] = q_scale / sqrtf(sum + 1e-6f);
           }
         }
         bar<2, kWalkers>();
-        {                                                // A, column by column in shared memory
+        float* Dg = reinterpret_cast<float*>(sm + L::D) + hw * 16 * L::PD;
+        {                                                // rows 16 hw .. of A: bfloat16 parts left of the diagonal block, the block itself as floats
           float G[8][4];
 #pragma unroll
           for (int x = 0; x < 8; ++x) G[x][0] = G[x][1] = G[x][2] = G[x][3] = 0.f;
@@ -175,59 +228,95 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
               }
           }
           const int row = hw * 16 + gq;
+          const float h0 = g.hi[row], l0 = g.lo[row], h1 = g.hi[row + 8], l1 = g.lo[row + 8];
+          const float w0 = g.beta[row] * g.kinv[row], w1 = g.beta[row + 8] * g.kinv[row + 8];
 #pragma unroll
           for (int x = 0; x < 8; ++x)
             if (x / 2 <= hw) {
+              const int j = x * 8 + 2 * tq;
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int i = row + (e >> 1) * 8, j = x * 8 + 2 * tq + (e & 1);
-                const float d = expf((g.hi[i] - g.hi[j]) + (g.lo[i] - g.lo[j]));
-                At[j * L::AT + (i & 1) * 36 + (i >> 1)] = j < i ? g.beta[i] * g.kinv[i] * g.kinv[j] * d * G[x][e] : 0.f;
+              for (int u = 0; u < 2; ++u) {
+                const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
+                G[x][u] *= w0 * w * expf((h0 - ch) + (l0 - cl));
+                G[x][2 + u] *= w1 * w * expf((h1 - ch) + (l1 - cl));
+              }
+              if (x / 2 < hw) {
+                uint32_t up[3], low[3];
+                split3(up, G[x][0], G[x][1]);
+                split3(low, G[x][2], G[x][3]);
+                unsigned char* to = sm + L::A + row * L::PT + j * 2;
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                  *reinterpret_cast<uint32_t*>(to + u * kPiece * L::PT) = up[u];
+                  *reinterpret_cast<uint32_t*>(to + (u * kPiece + 8) * L::PT) = low[u];
+                }
+              } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int i = gq + (e >> 1) * 8, c = (j & 15) + (e & 1);
+                  Dg[c * L::PD + (i & 1) * 8 + (i >> 1)] = c < i ? G[x][e] : 0.f;
+                }
               }
             }
         }
-        bar<2, kWalkers>();
-        {
-          // Columns of the inverse: lanes 2 m and 2 m + 1 hold column 16 hw + m's even and odd rows, x[s] being row 8 jb + 2 s + par;
-          // above its first row a warp's columns are zero.  Eight rows are finished a turn, then the others move up: the
-          // loop stays a loop (unrolled over all 63 steps its code alone took longer to fetch than the piece's products).
-          const int par = lane & 1, col = hw * 16 + (lane >> 1), odd = lane >> 1 & 1;
-          unsigned char* Ts = sm + L::T + b * 3 * kPiece * L::PT;
-          float x[32];
+        __syncwarp();
+        {                                                // the diagonal block's inverse: lanes 2 m and 2 m + 1 hold column m's even and odd rows
+          const int par = lane & 1, odd = lane >> 1 & 1;
+          float x[8];
 #pragma unroll
-          for (int s = 0; s < 32; ++s) x[s] = 2 * s + par == (lane >> 1) ? 1.f : 0.f;
-#pragma unroll 1
-          for (int jb = 2 * hw; jb < 8; ++jb) {
-            const float* column = At + jb * 8 * L::AT + par * 36 + jb * 4;
+          for (int e = 0; e < 8; ++e) x[e] = 2 * e + par == (lane >> 1) ? 1.f : 0.f;
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj, column += L::AT) {
-              const float u = __shfl_sync(0xffffffffu, x[jj >> 1], (lane & ~1) | (jj & 1));
+          for (int j = 0; j < 15; ++j) {
+            const float u = __shfl_sync(0xffffffffu, x[j >> 1], (lane & ~1) | (j & 1));
+            const float4* column = reinterpret_cast<const float4*>(Dg + j * L::PD + par * 8);
 #pragma unroll
-              for (int s = 0; s < 32; s += 4)            // rows up to the column's own are zero in A
-                if (s < 4 * (8 - jb)) {
-                  const float4 a = *reinterpret_cast<const float4*>(column + s);
-                  x[s] = fmaf(-a.x, u, x[s]);
-                  x[s + 1] = fmaf(-a.y, u, x[s + 1]);
-                  x[s + 2] = fmaf(-a.z, u, x[s + 2]);
-                  x[s + 3] = fmaf(-a.w, u, x[s + 3]);
-                }
+            for (int e = (j >> 1) & ~3; e < 8; e += 4) { // rows up to j itself are zero in A
+              const float4 a = column[e >> 2];
+              x[e] = fmaf(-a.x, u, x[e]);
+              x[e + 1] = fmaf(-a.y, u, x[e + 1]);
+              x[e + 2] = fmaf(-a.z, u, x[e + 2]);
+              x[e + 3] = fmaf(-a.w, u, x[e + 3]);
             }
+          }
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {                // of two neighbouring columns the first writes the even s, the second the odd ones
-              const float y = __shfl_xor_sync(0xffffffffu, x[s], 2);
-              if ((s & 1) == odd) {
-                uint32_t part[3];
-                split3(part, odd ? y : x[s], odd ? x[s] : y);
+          for (int e = 0; e < 8; e += 2) {               // of two neighbouring columns the first writes the even e, the second the odd ones
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? x[e] : x[e + 1], 2);
+            const float mine = odd ? x[e + 1] : x[e];
+            uint32_t part[3];
+            split3(part, odd ? other : mine, odd ? mine : other);
 #pragma unroll
-                for (int w = 0; w < 3; ++w)
-                  *reinterpret_cast<uint32_t*>(Ts + (w * kPiece + 8 * jb + 2 * s + par) * L::PT + (col & ~1) * 2) = part[w];
-              }
-            }
-#pragma unroll
-            for (int s = 0; s < 28; ++s) x[s] = x[s + 4];
+            for (int u = 0; u < 3; ++u)
+              *reinterpret_cast<uint32_t*>(Ts + (u * kPiece + hw * 16 + 2 * (e + odd) + par) * L::PT + (hw * 16 + (lane >> 1 & ~1)) * 2) = part[u];
           }
         }
+        bar<2, kWalkers>();
+        // The blocks below it, T_IJ = -T_II (sum over K from J to I - 1 of A_IK T_KJ) for J = hw, transposed: every product's result is
+        // the next one's left operand as it lies in the registers.
+        uint32_t left[3][3][4];                          // T_KJ^T, K = hw + the first index
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          ldm4t(left[0][u], Ts + (u * kPiece + hw * 16 + (lane & 7) + (lane >> 4) * 8) * L::PT + (hw * 2 + (lane >> 3 & 1)) * 16);
+#pragma unroll
+        for (int d = 1; d < 4; ++d)
+          if (hw + d < 4) {
+            const int I = hw + d;
+            float X[2][4] = {}, Y[2][4] = {};
+#pragma unroll
+            for (int e = 0; e < d; ++e) mma6t(X, left[e], sm + L::A + I * 16 * L::PT + (hw + e) * 32);
+            uint32_t x[3][4], y[3][4];
+            left_parts(x, X, 1.f);
+            mma6t(Y, x, Ts + I * 16 * L::PT + I * 32);
+            left_parts(y, Y, -1.f);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+              stm4t(y[u], Ts + (u * kPiece + I * 16 + (lane & 7) + (lane >> 4) * 8) * L::PT + (hw * 2 + (lane >> 3 & 1)) * 16);
+              if (d < 3)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) left[d][u][e] = y[u][e];
+            }
+          }
       }
+      if (L::STAGES == 3) asm volatile("cp.async.wait_group 0;" ::: "memory");
       bar<0, kAll>();                                    // the walkers are done with the piece before; this one is ready
     }
     return;
@@ -277,12 +366,15 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
         }
     }
   };
-  put_state();
-  bar<0, kAll>();                                        // the first piece is ready
+  if (pieces > 0) {
+    put_state();
+    bar<0, kAll>();
+    bar<0, kAll>();                                      // the first piece is ready
+  }
   const int row = warp * 16 + gq;                        // this thread's tokens of a piece: row and row + 8
   for (int piece = 0; piece < pieces; ++piece) {
-    const int c0 = t0 + piece * kPiece, b = piece & 1;
-    const Gates& g = gates[b];
+    const int c0 = t0 + piece * kPiece, b = piece % L::STAGES;
+    const Gates& g = gates[piece % 3];
     const unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
     const unsigned char* Qs = sm + L::Q + b * kPiece * L::PN;
     const unsigned char* Vs = sm + L::V + b * kPiece * L::PX;
@@ -343,7 +435,7 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
         uint32_t a[3][4];
 #pragma unroll
         for (int s = 0; s < 3; ++s)
-          ldm4(a[s], sm + L::T + ((b * 3 + s) * kPiece + warp * 16 + (lane & 15)) * L::PT + (jt * 2 + (lane >> 4)) * 16);
+          ldm4(a[s], sm + L::T + (((piece & 1) * 3 + s) * kPiece + warp * 16 + (lane & 15)) * L::PT + (jt * 2 + (lane >> 4)) * 16);
         mma6(acck, a, L::R, jt);
       }
     {
