@@ -29,7 +29,8 @@ namespace walk {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kPiece = 64, kThreads = 128, kGateWarp = kThreads / 32, kBlock = kThreads + 32;      // a fifth warp makes the next piece's gates
+// four walking warps, eight that make what does not depend on the state, two for the gates
+constexpr int kPiece = 64, kThreads = 128, kHelpers = 256, kGateWarp = (kThreads + kHelpers) / 32, kBlock = kThreads + kHelpers + 64;
 
 enum Rule { SSD = 0, MLSTM = 1 };
 
@@ -85,26 +86,33 @@ __device__ __forceinline__ void split3(uint32_t* p, float x, float y) {
 // bytes from row to row: an odd number of 16-byte chunks, so that eight rows' chunks lie in different banks
 __host__ __device__ constexpr int pitch(int cols) { return (cols * 2 / 16 | 1) * 16; }
 
+constexpr int kGateFloats = 8 * kPiece + 100;
+
 template <int RULE, int N, int DVC>
 struct Layout {
   static constexpr int COLS = DVC + (RULE == MLSTM ? 8 : 0);     // MLSTM: the vector n is one more value column, of ones
-  static constexpr int PN = pitch(N), PX = pitch(DVC), PC = pitch(COLS);
-  static constexpr int K = 0;                                     // [2][64] rows of PN
-  static constexpr int Q = K + 2 * kPiece * PN;                   // [64] rows of PN
-  static constexpr int X = Q + kPiece * PN;                       // [2][64] rows of PX
-  static constexpr int W = X + 2 * kPiece * PX;                   // [3][64] rows of PC: weighed values
-  static constexpr int S = W + 3 * kPiece * PC;                   // [3][N] rows of PC: the state
-  static constexpr int G = S + 3 * N * PC;                        // [2] gates
-  static constexpr int bytes = G + 2 * (8 * kPiece + 4) * 4;
+  static constexpr int PN = pitch(N), PX = pitch(DVC), PC = pitch(COLS), PY = DVC == 16 ? 24 : 40;
+  static constexpr int K = 0;                                     // [3][64] rows of PN
+  static constexpr int Q = K + 3 * kPiece * PN;                   // [3][64] rows of PN
+  static constexpr int X = Q + 3 * kPiece * PN;                   // [2][64] rows of PX
+  static constexpr int W = X + 2 * kPiece * PX;                   // [2][3][64] rows of PC: weighed values
+  static constexpr int S = W + 2 * 3 * kPiece * PC;               // [3][N] rows of PC: the state
+  static constexpr int Y = S + 3 * N * PC;                        // [2][2][64][PY] floats: the piece's own share of the results, in two sums
+  static constexpr int G = Y + 2 * 2 * kPiece * PY * 4;               // [3] gates
+  static constexpr int bytes = G + 3 * kGateFloats * 4;
+  static_assert(COLS <= PY && bytes <= 227 * 1024, "one block's shared memory");
 };
 
 // A piece's gates: column j's and row i's logarithms as pairs, weights of the values, factor on the state's part, and
 //   SSD:   scores' factor take_j;  MLSTM: exp(-m_i)
+// Of scores in 16 x 16 blocks below the diagonal the weight exp(row i + column j) is taken as the product of two factors, by way of
+// the last token before the row's block: rows[i] and cols[16 I (I - 1) / 2 + j], I the row's block.  None of them exceeds one.
 struct Gates {
-  float col_hi[kPiece], col_lo[kPiece], row_hi[kPiece], row_lo[kPiece], weigh[kPiece], from[kPiece], aux[kPiece], unused[kPiece];
+  float col_hi[kPiece], col_lo[kPiece], row_hi[kPiece], row_lo[kPiece], weigh[kPiece], from[kPiece], aux[kPiece], rows[kPiece];
+  float cols[96];
   float keep, m, pad[2];
 };
-static_assert(sizeof(Gates) == (8 * kPiece + 4) * 4, "as laid out");
+static_assert(sizeof(Gates) == kGateFloats * 4, "as laid out");
 
 __device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 0, %0;" ::"n"(kBlock) : "memory"); }
 __device__ __forceinline__ void walkers_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
@@ -151,62 +159,79 @@ __device__ __forceinline__ void raw_gates(const Args& p, int h, int c0, int t1, 
   }
 }
 
-// One warp: from the raw gates to `g`.  m: MLSTM's maximum before the piece.
+// One warp's gates of a piece: sums and maxima from the raw gates, then (MLSTM: with the maximum before the piece, m) the rest to `g`.
 template <int RULE>
-__device__ __forceinline__ void make_gates(const Args& p, int h, int nt, int lane, const float (&raw)[4], float m, Gates& g) {
-  if (RULE == SSD) {
-    const float rate = expf(p.A_log[h]), bias = p.dt_bias[h];
-    float take[2];
-    double c[2];
+struct GateWarp {
+  float take[2];          // SSD: step sizes
+  double c[2], a[2];      // logarithms summed up; MLSTM: the input gates, seen from the piece's start
+  double top[2];          // MLSTM: running maxima of a
+
+  __device__ __forceinline__ void sums(const Args& p, int h, int nt, int lane, const float (&raw)[4]) {
+    if (RULE == SSD) {
+      const float rate = expf(p.A_log[h]), bias = p.dt_bias[h];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const bool in = lane + 32 * u < nt;                        // behind the run's end nothing decays and nothing comes in
-      take[u] = in ? softplus(raw[2 * u] + bias) : 0.f;
-      c[u] = scan_sum(in ? -(double)(rate * take[u]) : 0.0, lane);
-    }
-    c[1] += __shfl_sync(0xffffffffu, c[0], 31);
-    const double total = __shfl_sync(0xffffffffu, c[1], 31);
+      for (int u = 0; u < 2; ++u) {
+        const bool in = lane + 32 * u < nt;                      // behind the run's end nothing decays and nothing comes in
+        take[u] = in ? softplus(raw[2 * u] + bias) : 0.f;
+        const float log_keep = -(rate * take[u]);                // (exp(-200) is zero in float32, and sums of -200 lose nothing)
+        c[u] = scan_sum(in ? (double)(log_keep < -200.f ? -200.f : log_keep) : 0.0, lane);
+      }
+      c[1] += __shfl_sync(0xffffffffu, c[0], 31);
+    } else {
+      const float bi = p.bi ? p.bi[h] : 0.f, bf_ = p.bf ? p.bf[h] : 0.f;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = lane + 32 * u;
-      as_pair(c[u], g.row_hi[i], g.row_lo[i]);
-      g.col_hi[i] = -g.row_hi[i];
-      g.col_lo[i] = -g.row_lo[i];
-      g.weigh[i] = expf((float)(total - c[u])) * take[u];
-      g.from[i] = expf((float)c[u]);
-      g.aux[i] = take[u];
-    }
-    if (lane == 0) g.keep = expf((float)total);
-  } else {
-    const float bi = p.bi ? p.bi[h] : 0.f, bf_ = p.bf ? p.bf[h] : 0.f;
-    double F[2], a[2], mu[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const bool in = lane + 32 * u < nt;
-      const float gi = p.cap * tanhf((raw[2 * u] + bi) / p.cap);
-      const float gf = log_sigmoid(p.cap * tanhf((raw[2 * u + 1] + bf_) / p.cap));
-      F[u] = scan_sum(in ? (double)gf : 0.0, lane);
-      if (u) F[1] += __shfl_sync(0xffffffffu, F[0], 31);
-      a[u] = in ? (double)gi - F[u] : -INFINITY;                 // the input gate, seen from the piece's start
-    }
-    mu[0] = fmax(scan_max(a[0], lane), (double)m);               // the maximum, seen from the piece's start
-    mu[1] = fmax(scan_max(a[1], lane), __shfl_sync(0xffffffffu, mu[0], 31));
-    const double mu_end = __shfl_sync(0xffffffffu, mu[1], 31), F_end = __shfl_sync(0xffffffffu, F[1], 31);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = lane + 32 * u;
-      as_pair(a[u], g.col_hi[i], g.col_lo[i]);
-      as_pair(-mu[u], g.row_hi[i], g.row_lo[i]);
-      g.weigh[i] = expf((float)(a[u] - mu_end));
-      g.from[i] = expf((float)((double)m - mu[u]));
-      g.aux[i] = expf((float)(-(F[u] + mu[u])));
-    }
-    if (lane == 0) {
-      g.keep = expf((float)((double)m - mu_end));
-      g.m = (float)(F_end + mu_end);
+      for (int u = 0; u < 2; ++u) {
+        const bool in = lane + 32 * u < nt;
+        const float gi = p.cap * tanhf((raw[2 * u] + bi) / p.cap);
+        const float gf = log_sigmoid(p.cap * tanhf((raw[2 * u + 1] + bf_) / p.cap));
+        c[u] = scan_sum(in ? (double)gf : 0.0, lane);
+        if (u) c[1] += __shfl_sync(0xffffffffu, c[0], 31);
+        a[u] = in ? (double)gi - c[u] : -INFINITY;
+      }
+      top[0] = scan_max(a[0], lane);
+      top[1] = fmax(scan_max(a[1], lane), __shfl_sync(0xffffffffu, top[0], 31));
     }
   }
-}
+
+  __device__ __forceinline__ void put(int lane, float m, Gates& g) const {
+    double row[2], col[2];                                       // a score's weight is exp(row + col)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      row[u] = RULE == SSD ? c[u] : -fmax(top[u], (double)m);
+      col[u] = RULE == SSD ? -c[u] : a[u];
+    }
+    const double row15 = __shfl_sync(0xffffffffu, row[0], 15), row31 = __shfl_sync(0xffffffffu, row[0], 31);
+    const double row47 = __shfl_sync(0xffffffffu, row[1], 15), row63 = __shfl_sync(0xffffffffu, row[1], 31);
+    const double c63 = __shfl_sync(0xffffffffu, c[1], 31);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = lane + 32 * u;
+      as_pair(row[u], g.row_hi[i], g.row_lo[i]);
+      as_pair(col[u], g.col_hi[i], g.col_lo[i]);
+      g.rows[i] = expf((float)(row[u] - (u ? (lane < 16 ? row31 : row47) : row15)));             // (unused in the first block)
+      if (RULE == SSD) {
+        g.weigh[i] = expf((float)(c63 - c[u])) * take[u];
+        g.from[i] = expf((float)c[u]);
+        g.aux[i] = take[u];
+      } else {
+        g.weigh[i] = expf((float)(a[u] + row63));
+        g.from[i] = expf((float)((double)m + row[u]));
+        g.aux[i] = expf((float)(row[u] - c[u]));
+      }
+    }
+    const float t0 = RULE == SSD ? take[0] : 1.f, t1 = RULE == SSD ? take[1] : 1.f;
+    if (lane < 16) {
+      g.cols[lane] = expf((float)(col[0] + row15)) * t0;
+      g.cols[80 + lane] = expf((float)(col[1] + row47)) * t1;
+    }
+    g.cols[16 + lane] = expf((float)(col[0] + row31)) * t0;
+    g.cols[48 + lane] = expf((float)(col[0] + row47)) * t0;
+    if (lane == 0) {
+      g.keep = RULE == SSD ? expf((float)c63) : expf((float)((double)m + row63));
+      if (RULE == MLSTM) g.m = (float)(c63 - row63);
+    }
+  }
+};
 
 template <int RULE, int N, int DVC>
 __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
@@ -225,46 +250,188 @@ __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
   const bf16* k = p.k + (size_t)(h / p.share) * N;
   const bf16* v = p.v + (size_t)h * p.Dv + col0;
 
-  auto bring_rows = [&](unsigned char* to, int at, const bf16* from, int cols, int c0) {
-    const int chunks = cols / 8;
-    for (int x = tid; x < kPiece * chunks; x += kThreads) {
-      const int i = x / chunks, c = x - i * chunks;
-      const bool in = c0 + i < t1;
-      copy16(to + i * at + c * 16, from + (size_t)(in ? c0 + i : t0) * p.ld + c * 8, in);
-    }
-  };
-  auto bring = [&](int piece) {
-    const int c0 = t0 + piece * kPiece;
-    bring_rows(sm + L::K + (piece & 1) * kPiece * L::PN, L::PN, k, N, c0);
-    bring_rows(sm + L::Q, L::PN, q, N, c0);
-    bring_rows(sm + L::X + (piece & 1) * kPiece * L::PX, L::PX, v, DVC, c0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-
-  const int pieces = (t1 - t0 + kPiece - 1) / kPiece;
+  // Round s: the gates of piece s, the state-free half of piece s - 1, the walk over piece s - 2; a barrier behind each.
+  const int pieces = (t1 - t0 + kPiece - 1) / kPiece, rounds = pieces > 0 ? pieces + 2 : 0;
   const size_t splits = (size_t)(p.Dv / 64), at_n = (size_t)p.H * p.Dv * N + ((size_t)h * splits + col0 / 64) * N;
   const size_t at_m = (size_t)p.H * p.Dv * N + (size_t)p.H * splits * N + (size_t)h * splits + col0 / 64;
-  if (warp == kGateWarp) {
+  if (warp >= kGateWarp) {
+    // Two warps take the pieces in turn: the sums of piece s in round s - 1 (the first one's in round 0), the rest in round s.
+    const int mine = warp - kGateWarp;
     const float m0 = RULE == MLSTM && !fresh ? slot[at_m] : 0.f;
     if (RULE == MLSTM) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     float raw[4], m = m0;
-    if (pieces > 0) raw_gates<RULE>(p, h, t0, t1, lane, raw);
-    for (int piece = 0; piece < pieces; ++piece) {       // a piece's gates are made while the other warps walk the one before
-      Gates& g = gates[piece & 1];
-      const int c0 = t0 + piece * kPiece;
-      make_gates<RULE>(p, h, min(kPiece, t1 - c0), lane, raw, m, g);
-      if (piece + 1 < pieces) raw_gates<RULE>(p, h, c0 + kPiece, t1, lane, raw);
-      __syncwarp();
-      if (RULE == MLSTM) m = g.m;
+    GateWarp<RULE> w;
+    if (mine < pieces) raw_gates<RULE>(p, h, t0 + mine * kPiece, t1, lane, raw);
+    if (mine == 0 && pieces > 0) w.sums(p, h, min(kPiece, t1 - t0), lane, raw);
+    for (int s = 0; s < rounds; ++s) {
+      if ((s & 1) == mine) {
+        if (s < pieces) {
+          if (RULE == MLSTM && s > 0) m = gates[(s - 1) % 3].m;
+          w.put(lane, m, gates[s % 3]);
+          if (s + 2 < pieces) raw_gates<RULE>(p, h, t0 + (s + 2) * kPiece, t1, lane, raw);
+        }
+      } else if (s + 1 < pieces) {
+        w.sums(p, h, min(kPiece, t1 - t0 - (s + 1) * kPiece), lane, raw);
+      }
       block_barrier();
     }
     if (RULE == MLSTM) {
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      if (pieces > 0 && lane == 0 && col0 % 64 == 0) slot[at_m] = m;
+      if (pieces > 0 && mine == 0 && lane == 0 && col0 % 64 == 0) slot[at_m] = gates[(pieces - 1) % 3].m;
     }
     return;
   }
 
+  if (warp >= 4) {
+    // ------------------------------------------------------------ what does not depend on the state
+    if (RULE == MLSTM) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // Eight warps, two to a block of 16 rows: of the blocks of 16 keys up to the rows' own, `low` .. `high` - 1 (the first half of
+    // four or three, then the rest; the first block's rows have one key block and the second warp none).
+    const int ht = tid - kThreads, hw = (warp - 4) >> 1, second = (warp - 4) & 1;
+    const int low = second ? (hw + 2) / 2 : 0, high = second ? hw + 1 : (hw + 2) / 2;
+    const int row = hw * 16 + gq;                        // this thread's tokens of a piece: row and row + 8
+    const float skip = RULE == SSD ? p.D[h] : 0.f;
+    auto bring = [&](unsigned char* to, int at, const bf16* from, int cols, int c0) {
+      const int chunks = cols / 8;
+      for (int x = ht; x < kPiece * chunks; x += kHelpers) {
+        const int i = x / chunks, c = x - i * chunks;
+        const bool in = c0 + i < t1;
+        copy16(to + i * at + c * 16, from + (size_t)(in ? c0 + i : t0) * p.ld + c * 8, in);
+      }
+    };
+    for (int s = 0; s < rounds; ++s) {
+      if (s < pieces) {                                  // the next piece's rows
+        const int c0 = t0 + s * kPiece;
+        bring(sm + L::K + s % 3 * kPiece * L::PN, L::PN, k, N, c0);
+        bring(sm + L::Q + s % 3 * kPiece * L::PN, L::PN, q, N, c0);
+        bring(sm + L::X + (s & 1) * kPiece * L::PX, L::PX, v, DVC, c0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+      if (s >= 1 && s <= pieces) {
+        const int piece = s - 1, b = piece & 1;
+        const Gates& g = gates[piece % 3];
+        const unsigned char* Ks = sm + L::K + piece % 3 * kPiece * L::PN;
+        const unsigned char* Qs = sm + L::Q + piece % 3 * kPiece * L::PN;
+        const unsigned char* Xs = sm + L::X + b * kPiece * L::PX;
+        unsigned char* Ws = sm + L::W + b * 3 * kPiece * L::PC;
+
+        // weighed values, three parts each
+        for (int x = ht; x < kPiece * NX; x += kHelpers) {
+          const int j = x / NX, c = x - j * NX;
+          const uint4 in = *reinterpret_cast<const uint4*>(Xs + j * L::PX + c * 16);
+          const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&in);
+          const float wj = g.weigh[j];
+          uint4 out[3];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint32_t part[3];
+            split3(part, __uint_as_float(w2[e] << 16) * wj, __uint_as_float(w2[e] & 0xffff0000u) * wj);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) reinterpret_cast<uint32_t*>(&out[u])[e] = part[u];
+          }
+#pragma unroll
+          for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(Ws + (u * kPiece + j) * L::PC + c * 16) = out[u];
+        }
+        if (RULE == MLSTM && ht < kPiece) {
+          uint32_t part[3];
+          split3(part, g.weigh[ht], 0.f);
+#pragma unroll
+          for (int u = 0; u < 3; ++u)
+            *reinterpret_cast<uint4*>(Ws + (u * kPiece + ht) * L::PC + DVC * 2) = make_uint4(part[u], 0, 0, 0);
+        }
+
+        // q . k for the keys up to the warp's last token
+        float G[4][4], acc[NT][4];                       // (two key blocks at most)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) G[x][0] = G[x][1] = G[x][2] = G[x][3] = 0.f;
+#pragma unroll
+        for (int x = 0; x < NT; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < KN; ++kk) {
+          uint32_t a[4];
+          ldm4(a, Qs + (hw * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj)
+            if (low + jj < high) {
+              uint32_t f[4];
+              ldm4(f, Ks + ((low + jj) * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + (kk * 2 + (lane >> 3 & 1)) * 16);
+              mma(G[2 * jj], a, f[0], f[1]);
+              mma(G[2 * jj + 1], a, f[2], f[3]);
+            }
+        }
+
+        // the scores' weights, then their product with the values
+        const float rh0 = g.row_hi[row], rl0 = g.row_lo[row], rh1 = g.row_hi[row + 8], rl1 = g.row_lo[row + 8];
+        const float r0 = g.rows[row], r1 = g.rows[row + 8];
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj)
+          if (low + jj < high) {
+            const int jt = low + jj;
+            uint32_t part[3][4];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              float* e = G[2 * jj + half];
+              const int j = jt * 16 + half * 8 + 2 * tq;
+              if (jt < hw) {
+                const float2 w = *reinterpret_cast<const float2*>(g.cols + 8 * hw * (hw - 1) + j);
+                e[0] *= r0 * w.x;
+                e[1] *= r0 * w.y;
+                e[2] *= r1 * w.x;
+                e[3] *= r1 * w.y;
+              } else {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                  const float ch = g.col_hi[j + u], cl = g.col_lo[j + u], w = RULE == SSD ? g.aux[j + u] : 1.f;
+                  e[u] = j + u <= row ? e[u] * (expf((rh0 + ch) + (rl0 + cl)) * w) : 0.f;
+                  e[2 + u] = j + u <= row + 8 ? e[2 + u] * (expf((rh1 + ch) + (rl1 + cl)) * w) : 0.f;
+                }
+              }
+              uint32_t up[3], down[3];
+              split3(up, e[0], e[1]);
+              split3(down, e[2], e[3]);
+#pragma unroll
+              for (int u = 0; u < 3; ++u) { part[u][2 * half] = up[u]; part[u][2 * half + 1] = down[u]; }
+            }
+#pragma unroll
+            for (int nt = 0; nt < NX; nt += 2) {
+              uint32_t f[4];
+              ldm4t(f, Xs + (jt * 16 + (lane & 15)) * L::PX + (nt + (lane >> 4)) * 16);
+#pragma unroll
+              for (int u = 2; u >= 0; --u) {
+                mma(acc[nt], part[u], f[0], f[1]);
+                mma(acc[nt + 1], part[u], f[2], f[3]);
+              }
+            }
+            if (RULE == MLSTM) {
+              const uint32_t ones = gq == 0 ? 0x3f803f80u : 0u;  // the column of ones
+#pragma unroll
+              for (int u = 2; u >= 0; --u) mma(acc[NT - 1], part[u], ones, ones);
+            }
+          }
+        float* Ys = reinterpret_cast<float*>(sm + L::Y) + (b * 2 + second) * kPiece * L::PY;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int i = row + 8 * half;
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            float2 o = make_float2(acc[nt][2 * half], acc[nt][2 * half + 1]);
+            if (RULE == SSD && second) {
+              const uint32_t x2 = *reinterpret_cast<const uint32_t*>(Xs + i * L::PX + (8 * nt + 2 * tq) * 2);
+              o.x = fmaf(skip, __uint_as_float(x2 << 16), o.x);
+              o.y = fmaf(skip, __uint_as_float(x2 & 0xffff0000u), o.y);
+            }
+            *reinterpret_cast<float2*>(Ys + i * L::PY + 8 * nt + 2 * tq) = o;
+          }
+        }
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      block_barrier();
+    }
+    if (RULE == MLSTM) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return;
+  }
+
+  // -------------------------------------------------------------- the walk
   // the state: rows (warp * MT + mt) * 16 + gq (+ 8), columns 8 nt + 2 tq (+ 1)
   float S[MT][NT][4];
 #pragma unroll
@@ -298,63 +465,29 @@ __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
         }
   };
 
-  if (pieces > 0) bring(0);
-  put_state();
+  if (pieces > 0) put_state();
   const int row = warp * 16 + gq;                        // this thread's tokens of a piece: row and row + 8
-  for (int piece = 0; piece < pieces; ++piece) {
-    const int c0 = t0 + piece * kPiece, b = piece & 1;
-    const Gates& g = gates[b];
-    const unsigned char* Ks = sm + L::K + b * kPiece * L::PN;
-    const unsigned char* Xs = sm + L::X + b * kPiece * L::PX;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    block_barrier();                                     // rows, gates and the state's parts are there, the buffers before them free
-
-    // weighed values, three parts each
-    for (int x = tid; x < kPiece * NX; x += kThreads) {
-      const int j = x / NX, c = x - j * NX;
-      const uint4 in = *reinterpret_cast<const uint4*>(Xs + j * L::PX + c * 16);
-      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&in);
-      const float wj = g.weigh[j];
-      uint4 out[3];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        uint32_t part[3];
-        split3(part, __uint_as_float(w2[e] << 16) * wj, __uint_as_float(w2[e] & 0xffff0000u) * wj);
-#pragma unroll
-        for (int s = 0; s < 3; ++s) reinterpret_cast<uint32_t*>(&out[s])[e] = part[s];
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(sm + L::W + (s * kPiece + j) * L::PC + c * 16) = out[s];
+  for (int s = 0; s < rounds; ++s) {
+    if (s < 2) {
+      block_barrier();
+      continue;
     }
-    if (RULE == MLSTM && tid < kPiece) {
-      uint32_t part[3];
-      split3(part, g.weigh[tid], 0.f);
-#pragma unroll
-      for (int s = 0; s < 3; ++s)
-        *reinterpret_cast<uint4*>(sm + L::W + (s * kPiece + tid) * L::PC + DVC * 2) = make_uint4(part[s], 0, 0, 0);
-    }
+    const int piece = s - 2, c0 = t0 + piece * kPiece, b = piece & 1;
+    const Gates& g = gates[piece % 3];
+    const unsigned char* Ks = sm + L::K + piece % 3 * kPiece * L::PN;
+    const unsigned char* Qs = sm + L::Q + piece % 3 * kPiece * L::PN;
 
-    // q . k for the keys up to the warp's last token, and S^T q
-    float G[8][4], acc[NT][4];
-#pragma unroll
-    for (int x = 0; x < 8; ++x) G[x][0] = G[x][1] = G[x][2] = G[x][3] = 0.f;
+    // S^T q
+    float acc[NT][4];
 #pragma unroll
     for (int x = 0; x < NT; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < KN; ++kk) {
       uint32_t a[4];
-      ldm4(a, sm + L::Q + (warp * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
+      ldm4(a, Qs + (warp * 16 + (lane & 15)) * L::PN + (kk * 2 + (lane >> 4)) * 16);
 #pragma unroll
-      for (int jt = 0; jt < 4; ++jt)
-        if (jt <= warp) {
-          uint32_t f[4];
-          ldm4(f, Ks + (jt * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + (kk * 2 + (lane >> 3 & 1)) * 16);
-          mma(G[2 * jt], a, f[0], f[1]);
-          mma(G[2 * jt + 1], a, f[2], f[3]);
-        }
-#pragma unroll
-      for (int s = 2; s >= 0; --s) {
-        const unsigned char* Ss = sm + L::S + (s * N + kk * 16 + (lane & 15)) * L::PC;
+      for (int u = 2; u >= 0; --u) {
+        const unsigned char* Ss = sm + L::S + (u * N + kk * 16 + (lane & 15)) * L::PC;
 #pragma unroll
         for (int nt = 0; nt + 1 < NT; nt += 2) {
           uint32_t f[4];
@@ -366,79 +499,6 @@ __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
           uint32_t f[2];
           ldm2t(f, Ss + (NT - 1) * 16);
           mma(acc[NT - 1], a, f[0], f[1]);
-        }
-      }
-    }
-    walkers_barrier();                                   // the weighed values are there; q and the state's parts are free
-    if (piece + 1 < pieces) bring(piece + 1);
-
-    // the scores' weights, then their product with the values
-    const float rh0 = g.row_hi[row], rl0 = g.row_lo[row], rh1 = g.row_hi[row + 8], rl1 = g.row_lo[row + 8];
-    const float f0 = g.from[row], f1 = g.from[row + 8];
-#pragma unroll
-    for (int x = 0; x < NT; ++x) { acc[x][0] *= f0; acc[x][1] *= f0; acc[x][2] *= f1; acc[x][3] *= f1; }
-#pragma unroll
-    for (int jt = 0; jt < 4; ++jt)
-      if (jt <= warp) {
-        uint32_t part[3][4];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float* e = G[2 * jt + half];
-          const int j = jt * 16 + half * 8 + 2 * tq;
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float ch = g.col_hi[j + u], cl = g.col_lo[j + u], w = RULE == SSD ? g.aux[j + u] : 1.f;
-            e[u] = j + u <= row ? e[u] * (expf((rh0 + ch) + (rl0 + cl)) * w) : 0.f;
-            e[2 + u] = j + u <= row + 8 ? e[2 + u] * (expf((rh1 + ch) + (rl1 + cl)) * w) : 0.f;
-          }
-          uint32_t up[3], low[3];
-          split3(up, e[0], e[1]);
-          split3(low, e[2], e[3]);
-#pragma unroll
-          for (int s = 0; s < 3; ++s) { part[s][2 * half] = up[s]; part[s][2 * half + 1] = low[s]; }
-        }
-#pragma unroll
-        for (int nt = 0; nt < NX; nt += 2) {
-          uint32_t f[4];
-          ldm4t(f, Xs + (jt * 16 + (lane & 15)) * L::PX + (nt + (lane >> 4)) * 16);
-#pragma unroll
-          for (int s = 2; s >= 0; --s) {
-            mma(acc[nt], part[s], f[0], f[1]);
-            mma(acc[nt + 1], part[s], f[2], f[3]);
-          }
-        }
-        if (RULE == MLSTM) {
-          const uint32_t ones = gq == 0 ? 0x3f803f80u : 0u;      // the column of ones
-#pragma unroll
-          for (int s = 2; s >= 0; --s) mma(acc[NT - 1], part[s], ones, ones);
-        }
-      }
-    float den0 = 0.f, den1 = 0.f;
-    if (RULE == MLSTM) {
-      den0 = __shfl_sync(0xffffffffu, acc[NT - 1][0], lane & ~3);
-      den1 = __shfl_sync(0xffffffffu, acc[NT - 1][2], lane & ~3);
-      den0 = fmaxf(fabsf(den0 * p.q_scale), g.aux[row]) + 1e-6f;
-      den1 = fmaxf(fabsf(den1 * p.q_scale), g.aux[row + 8]) + 1e-6f;
-    }
-    const float skip = RULE == SSD ? p.D[h] : 0.f;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int i = row + 8 * half;
-      if (c0 + i < t1) {
-        float* to = p.y + (size_t)(c0 + i) * p.H * p.Dv + (size_t)h * p.Dv + col0 + 2 * tq;
-#pragma unroll
-        for (int nt = 0; nt < NX; ++nt) {
-          float2 o = make_float2(acc[nt][2 * half], acc[nt][2 * half + 1]);
-          if (RULE == SSD) {
-            const uint32_t x2 = *reinterpret_cast<const uint32_t*>(Xs + i * L::PX + (8 * nt + 2 * tq) * 2);
-            o.x = fmaf(skip, __uint_as_float(x2 << 16), o.x);
-            o.y = fmaf(skip, __uint_as_float(x2 & 0xffff0000u), o.y);
-          } else {
-            const float den = half ? den1 : den0;
-            o.x = o.x * p.q_scale / den;
-            o.y = o.y * p.q_scale / den;
-          }
-          *reinterpret_cast<float2*>(to + 8 * nt) = o;
         }
       }
     }
@@ -458,8 +518,8 @@ __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
       for (int mt = 0; mt < MT; ++mt)
         ldm4t(a[mt], Ks + (jj * 16 + (lane & 7) + (lane >> 4) * 8) * L::PN + ((warp * MT + mt) * 2 + (lane >> 3 & 1)) * 16);
 #pragma unroll
-      for (int s = 2; s >= 0; --s) {
-        const unsigned char* Ws = sm + L::W + (s * kPiece + jj * 16 + (lane & 15)) * L::PC;
+      for (int u = 2; u >= 0; --u) {
+        const unsigned char* Ws = sm + L::W + ((b * 3 + u) * kPiece + jj * 16 + (lane & 15)) * L::PC;
 #pragma unroll
         for (int nt = 0; nt + 1 < NT; nt += 2) {
           uint32_t f[4];
@@ -478,7 +538,38 @@ __global__ void __launch_bounds__(kBlock) walk_kernel(const Args p) {
         }
       }
     }
+    walkers_barrier();                                   // the state's parts are read
     if (piece + 1 < pieces) put_state();
+
+    // the results: the state's share and the piece's own
+    const float* Ys = reinterpret_cast<const float*>(sm + L::Y) + b * 2 * kPiece * L::PY;
+    const float* Zs = Ys + kPiece * L::PY;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = row + 8 * half;
+      const float f = g.from[i];
+      float den = 1.f;
+      if (RULE == MLSTM) {                               // the column of ones' sum is the denominator
+        den = fmaf(f, acc[NT - 1][2 * half], Ys[i * L::PY + DVC + 2 * tq] + Zs[i * L::PY + DVC + 2 * tq]);
+        den = __shfl_sync(0xffffffffu, den, lane & ~3);
+        den = fmaxf(fabsf(den * p.q_scale), g.aux[i]) + 1e-6f;
+      }
+      if (c0 + i < t1) {
+        float* to = p.y + (size_t)(c0 + i) * p.H * p.Dv + (size_t)h * p.Dv + col0 + 2 * tq;
+#pragma unroll
+        for (int nt = 0; nt < NX; ++nt) {
+          const float2 own = *reinterpret_cast<const float2*>(Ys + i * L::PY + 8 * nt + 2 * tq);
+          const float2 too = *reinterpret_cast<const float2*>(Zs + i * L::PY + 8 * nt + 2 * tq);
+          float2 o = make_float2(fmaf(f, acc[nt][2 * half], own.x + too.x), fmaf(f, acc[nt][2 * half + 1], own.y + too.y));
+          if (RULE == MLSTM) {
+            o.x = o.x * p.q_scale / den;
+            o.y = o.y * p.q_scale / den;
+          }
+          *reinterpret_cast<float2*>(to + 8 * nt) = o;
+        }
+      }
+    }
+    block_barrier();
   }
   if (RULE == MLSTM) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (pieces > 0) {

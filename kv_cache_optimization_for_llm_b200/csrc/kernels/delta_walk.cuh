@@ -47,6 +47,8 @@ struct Gates {
   float from[kPiece];                 // P_i
   float beta[kPiece], kinv[kPiece], qinv[kPiece];
   float weigh[kPiece];                // P_63 / P_j / |k_j|
+  float rows[kPiece], cols[96];       // P_i / P_j = rows[i] cols[8 I (I - 1) + j] for i in the I-th 16 tokens and j before them, by way of
+                                      // the last token before these: neither factor exceeds one
   float keep, pad[3];
 };
 
@@ -116,20 +118,29 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
           float la = 0.f, be = 0.f;                      // behind the run's end nothing decays
           if (t < t1) {
             la = -(rate * softplus20(__bfloat162float(p.decay[(size_t)t * p.ld_decay + h]) + dbias));
+            la = la < -200.f ? -200.f : la;              // (exp(-200) is zero in float32, and sums of -200 lose nothing)
             be = sigmoid(__bfloat162float(p.beta[(size_t)t * p.ld_beta + h]));
           }
           g.beta[i] = be;
           c[u] = scan_sum((double)la, lane);
         }
         c[1] += __shfl_sync(0xffffffffu, c[0], 31);
-        const double total = __shfl_sync(0xffffffffu, c[1], 31);
+        const double total = __shfl_sync(0xffffffffu, c[1], 31), c15 = __shfl_sync(0xffffffffu, c[0], 15);
+        const double c31 = __shfl_sync(0xffffffffu, c[0], 31), c47 = __shfl_sync(0xffffffffu, c[1], 15);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int i = lane + 32 * u;
           as_pair(c[u], g.hi[i], g.lo[i]);
           g.from[i] = expf((float)c[u]);
           g.weigh[i] = expf((float)(total - c[u]));
+          g.rows[i] = expf((float)(c[u] - (u ? (lane < 16 ? c31 : c47) : c15)));                 // (unused in the first 16)
         }
+        if (lane < 16) {
+          g.cols[lane] = expf((float)(c15 - c[0]));
+          g.cols[80 + lane] = expf((float)(c47 - c[1]));
+        }
+        g.cols[16 + lane] = expf((float)(c31 - c[0]));
+        g.cols[48 + lane] = expf((float)(c47 - c[0]));
         if (lane == 0) g.keep = expf((float)total);
       }
       bar<0, kAll>();
@@ -230,15 +241,25 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
           const int row = hw * 16 + gq;
           const float h0 = g.hi[row], l0 = g.lo[row], h1 = g.hi[row + 8], l1 = g.lo[row + 8];
           const float w0 = g.beta[row] * g.kinv[row], w1 = g.beta[row + 8] * g.kinv[row + 8];
+          const float r0 = w0 * g.rows[row], r1 = w1 * g.rows[row + 8];
 #pragma unroll
           for (int x = 0; x < 8; ++x)
             if (x / 2 <= hw) {
               const int j = x * 8 + 2 * tq;
+              if (x / 2 < hw) {
+                const float2 f = *reinterpret_cast<const float2*>(g.cols + 8 * hw * (hw - 1) + j);
+                const float c0 = f.x * g.kinv[j], c1 = f.y * g.kinv[j + 1];
+                G[x][0] *= r0 * c0;
+                G[x][1] *= r0 * c1;
+                G[x][2] *= r1 * c0;
+                G[x][3] *= r1 * c1;
+              } else {
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
-                G[x][u] *= w0 * w * expf((h0 - ch) + (l0 - cl));
-                G[x][2 + u] *= w1 * w * expf((h1 - ch) + (l1 - cl));
+                for (int u = 0; u < 2; ++u) {
+                  const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
+                  G[x][u] *= w0 * w * expf((h0 - ch) + (l0 - cl));
+                  G[x][2 + u] *= w1 * w * expf((h1 - ch) + (l1 - cl));
+                }
               }
               if (x / 2 < hw) {
                 uint32_t up[3], low[3];
@@ -453,7 +474,7 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
     // the read-outs
 #pragma unroll
     for (int x = 0; x < NX; ++x) { accq[x][0] *= from0; accq[x][1] *= from0; accq[x][2] *= from1; accq[x][3] *= from1; }
-    const float h0 = g.hi[row], l0 = g.lo[row], h1 = g.hi[row + 8], l1 = g.lo[row + 8];
+    const float h0 = g.hi[row], l0 = g.lo[row], h1 = g.hi[row + 8], l1 = g.lo[row + 8], r0 = g.rows[row], r1 = g.rows[row + 8];
 #pragma unroll
     for (int jt = 0; jt < 4; ++jt)
       if (jt <= warp) {
@@ -462,11 +483,20 @@ __global__ void __launch_bounds__(kAll) delta_walk_kernel(const Args p) {
         for (int half = 0; half < 2; ++half) {
           float* e = G[2 * jt + half];
           const int j = jt * 16 + half * 8 + 2 * tq;
+          if (jt < warp) {
+            const float2 f = *reinterpret_cast<const float2*>(g.cols + 8 * warp * (warp - 1) + j);
+            const float w0 = f.x * g.kinv[j], w1 = f.y * g.kinv[j + 1];
+            e[0] *= r0 * w0;
+            e[1] *= r0 * w1;
+            e[2] *= r1 * w0;
+            e[3] *= r1 * w1;
+          } else {
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
-            e[u] = j + u <= row ? e[u] * (expf((h0 - ch) + (l0 - cl)) * w) : 0.f;
-            e[2 + u] = j + u <= row + 8 ? e[2 + u] * (expf((h1 - ch) + (l1 - cl)) * w) : 0.f;
+            for (int u = 0; u < 2; ++u) {
+              const float ch = g.hi[j + u], cl = g.lo[j + u], w = g.kinv[j + u];
+              e[u] = j + u <= row ? e[u] * (expf((h0 - ch) + (l0 - cl)) * w) : 0.f;
+              e[2 + u] = j + u <= row + 8 ? e[2 + u] * (expf((h1 - ch) + (l1 - cl)) * w) : 0.f;
+            }
           }
           uint32_t up[3], low[3];
           split3(up, e[0], e[1]);
