@@ -14,11 +14,16 @@
 // logarithms summed up in float64 and differences taken from pairs (high, low) of floats: a quotient P_i / P_j of two close
 // tokens does not lose digits to a long run's sum.
 //
-// What bounds it: one piece is a chain of four products and three barriers (about 2 us for a block alone on its SM); a run is as many
-// pieces one behind the other, and the heads' columns are dealt over the SMs.  Walking token by token in float32 instead was bound
+// Only S^T q and the state's update wait for the piece before.  The rest is made a round ahead by eight helper warps (weighed
+// values; scores, their weights and their product with the values, two warps to a block of 16 rows), the gates two rounds ahead by two
+// warps that take the pieces in turn.
+//
+// What bounds it: latency, about 3500 (N = 64) and 6000 (N = 128) cycles a piece and barrier, for walkers and helpers alike; a run is as
+// many pieces one behind the other, and the heads' columns are dealt over the SMs.  Walking token by token in float32 instead was bound
 // by the FMAs and the shared-memory loads that feed them, and took three launches (pieces side by side, a sweep over
-// their states in memory, the pieces again): 64 heads of 128 x 64, runs of 1111 + 700 + 237 tokens about 700 us, now 118; 32 heads of
-// 64 x 64, 2048 tokens about 260 us, now 125.
+// their states in memory, the pieces again): 64 heads of 128 x 64, runs of 1111 + 700 + 237 tokens about 700 us, 118 with one chain of
+// all four products a piece, now 111; 32 heads of 64 x 64, 2048 tokens about 260 us, then 125, now 66.  Warps of their own for the
+// rows' loads, and products interleaved over all columns, gave nothing (70 and 111 us).
 #pragma once
 
 #include "common.cuh"

@@ -16,9 +16,10 @@
 // sum of three bfloat16 numbers; where both are float32 (inverse and right side, weighed scores and corrections) six of
 // the nine products are made, the others lie below 2^-24.
 //
-// What bounds it: one piece is a chain of three steps of products with a barrier behind each.  Walking token by token in float32 is a chain
-// of 64 steps of two dot products each: 32 heads of 64 x 64, runs of 1548 + 500 tokens 474 us, now 173 (352 and 317 with the
-// whole inverse by elimination).
+// What bounds it: latency, about 9500 cycles a piece, for walkers (three steps of products with a barrier behind each) and helpers
+// (rows, norms, A, its inverse) alike.  Walking token by token in float32 is a chain of 64 steps of two dot products each: 32 heads
+// of 64 x 64, runs of 1548 + 500 tokens 474 us, now 173 (352 and 317 with the whole inverse by elimination; 179 with a warp of its own for the
+// rows' loads and products interleaved over all columns).
 #pragma once
 
 #include "chunk_walk.cuh"
