@@ -1437,10 +1437,13 @@ def _chunk_rows(batch, chunk: int):
 
 
 # bfloat16 steps whose runs bring at least this many tokens each, on average, walk them in pieces of 64 tokens on tensor cores where
-# the sizes allow (the matrix states with one decay per head and token).  A piece costs the same however few tokens it holds.
-# Measured, token by token / the walk, 64 heads of 128 x 64 (ssd): one run of 16 tokens 22 / 22 us (the host's share), of 32 37 / 22,
-# of 64 71 / 18; sixteen runs of 8 45 / 58, of 16 71 / 58, of 64 230 / 60; 32 heads of 64 x 64 (mlstm), sixteen of 8 20 / 27, of 16 30 / 27.
-WALK_MIN_RUN = int(os.environ.get('KVB200_WALK_MIN_RUN', '16'))
+# the sizes allow (the matrix states with one decay per head and token); a lone run from WALK_MIN_LONE_RUN tokens on.  A piece costs the
+# same however few tokens it holds, and a block of the walk has its SM to itself.  Measured, token by token / the walk in us: 64 heads
+# of 128 x 64 (ssd), one run of 16 tokens 22 / 11, sixteen of 16 76 / 94, of 32 136 / 101, of 64 252 / 110, 32 of 16 148 / 192, of 32
+# 242 / 194; 32 heads of 64 x 64 (mlstm), one of 16 14 / 7, sixteen of 24 43 / 49, of 32 53 / 49, 32 of 32 85 / 97, of 64 168 / 99; the delta
+# rule, one of 16 17 / 10, four of 32 20 / 23, of 64 34 / 24, sixteen of 32 77 / 76, of 64 135 / 84, 32 of 32 133 / 150, of 64 239 / 162.
+WALK_MIN_RUN = int(os.environ.get('KVB200_WALK_MIN_RUN', '36'))
+WALK_MIN_LONE_RUN = 16
 
 
 def _walks(batch, n: int, dv: int, x: torch.Tensor, *columns: int) -> bool:
@@ -1448,7 +1451,8 @@ def _walks(batch, n: int, dv: int, x: torch.Tensor, *columns: int) -> bool:
     every segment of ``x``'s rows (from ``columns``) on a 16-byte boundary."""
     return (x.dtype == torch.bfloat16 and n in (64, 128) and dv >= 64 and dv % 64 == 0 and x.stride(0) % 8 == 0
             and all(_at(x, c) % 16 == 0 for c in columns) and not batch.decode_only and WALK_MIN_RUN > 0
-            and batch.num_tokens - batch.num_single >= WALK_MIN_RUN * (batch.num_reqs - batch.num_single))
+            and batch.num_tokens - batch.num_single >= WALK_MIN_RUN * (batch.num_reqs - batch.num_single)
+            - (max(0, WALK_MIN_RUN - WALK_MIN_LONE_RUN) if batch.num_reqs - batch.num_single == 1 else 0))
 
 
 class _DiagArgs(ctypes.Structure):

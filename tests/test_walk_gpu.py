@@ -26,7 +26,7 @@ def _rel(a, b):
 
 STEPS = [
     [(0, 0, 64)], [(0, 0, 16), (1, 7, 63)], [(0, 0, 65), (1, 3, 1), (2, 0, 1), (3, 100, 200)], [(0, 5, 128), (1, 0, 129)],
-    [(0, 0, 700)], [(r, 2 * r, 17 + 30 * r) for r in range(9)],
+    [(0, 0, 700)], [(0, 9, 16)], [(r, 2 * r, 17 + 30 * r) for r in range(9)],
 ]
 
 

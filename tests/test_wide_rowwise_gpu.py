@@ -75,3 +75,42 @@ def test_gated_group_norm(T, groups, gs):
     v = (y.double() * torch.nn.functional.silu(z[:, 8:].double())).view(T, groups, gs)
     ref = (v / torch.sqrt(v.square().mean(-1, keepdim=True) + 1e-5)).view(T, W) * w.double()
     assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -7.99 + 1e-30).all())
+
+
+# (head size, requests): grids of one block a (request, kv head) that beyond 2048 positions are cut in 4, 2 and 4 (8 kv heads on 148 SMs)
+@pytest.mark.parametrize("d,R", [(128, 24), (128, 40), (64, 48)])
+@pytest.mark.parametrize("window", [None, 700])
+def test_decode_attention_of_full_grids_beyond_2048(d, R, window):
+    from kv_cache_optimization_for_llm_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(R + d)
+    nkv, G, ps = 8, 4, 16
+    ctxs = [2049 + (r * 977) % 1400 if r % 3 else 1 + (r * 131) % 2048 for r in range(R)]
+    pages = [-(-c // ps) for c in ctxs]
+    perm = torch.randperm(sum(pages) + 1, generator=gen, device="cuda").int()
+    table, at = torch.full((R, max(pages)), -1, dtype=torch.int32, device="cuda"), 0
+    for r, n in enumerate(pages):
+        table[r, :n] = perm[at:at + n]
+        at += n
+    pools = [torch.randn(sum(pages) + 1, nkv, ps, d, generator=gen, device="cuda").bfloat16() for _ in range(2)]
+    qkv = torch.randn(R, (G + 2) * nkv * d, generator=gen, device="cuda").bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(rows):
+        k, v = (p.clone() for p in pools)
+        n = len(rows)
+        out = ops.decode_attention_mma(qkv[rows].contiguous(), k, v, True, table[rows].contiguous(),
+                                       torch.arange(n + 1, dtype=torch.int32, device="cuda"),
+                                       torch.tensor([ctxs[r] for r in rows], dtype=torch.int32, device="cuda"), None, None, 0, G * nkv, nkv, d,
+                                       d ** -0.5, window, status, max_ctx=max(ctxs))
+        return out, k, v
+
+    out, k, v = run(list(range(R)))
+    for r in (0, 1, R // 2, R - 1):
+        assert torch.equal(run([r])[0][0], out[r])           # a token's sums are cut by its positions, whatever blocks make them
+        c, lo = ctxs[r], max(0, ctxs[r] - window) if window else 0
+        kr, vr = (p[table[r, :pages[r]].long()].transpose(1, 2).reshape(-1, nkv, d)[lo:c].float() for p in (k, v))
+        q = qkv[r, :G * nkv * d].float().view(nkv, G, d)
+        want = torch.einsum("hgk,khd->hgd", torch.softmax(torch.einsum("hgd,khd->hgk", q, kr) * d ** -0.5, -1), vr).reshape(-1)
+        # probabilities and results rounded to bfloat16, 2^-8 each at most
+        assert float((out[r].float() - want).norm() / want.norm()) < 2**-7
+    assert int(status.item()) == 0
