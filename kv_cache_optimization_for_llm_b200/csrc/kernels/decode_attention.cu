@@ -805,11 +805,16 @@ KVB_EXPORT int kvb_decode_attention_mma(const void* qkv, int q_row_stride, void*
   // Beyond 2048 positions one block a (request, kv head) walks up to 64 tiles and more, and the longest request is the launch's
   // time: there up to 2.7 times as many blocks as the GPU holds share the work (the hardware deals the shorter ones out behind
   // the longer).  Measured, head size 128, 8 kv heads, one block / this rule: 24 requests of 500 to 7900 positions 118 / 85 us, of
-  // 3000 each 67 / 67, of 7000 to 8000 135 / 130; 48 of 500 to 7900 179 / 151, of 3000 138 / 118; 32 of 3000 74 / 80; head size 64: 48 of
-  // 500 to 7900 104 / 78, 64 of 500 to 7900 115 / 101, of 3000 69 / 73.  Where two blocks and more share a request anyway, and below 2048
-  // positions, a second round of blocks cost more than it gave (16 requests of 3000 41 / 46).
-  if (S == 1 && cluster > 4)
-    while (S < cluster && (long long)R * nkv * S * 2 * 10 <= 27ll * resident) S <<= 1;
+  // 3000 each 67 / 67, of 7000 to 8000 135 / 130; 48 of 500 to 7900 179 / 151, of 3000 138 / 118; head size 64: 48 of 500 to 7900 104 / 78, of
+  // 3000 61 / 61.  Two blocks where one each fit the GPU at once stay out: they help ragged requests (32 of 500 to 7900
+  // 126 / 108) but cost even ones (of 3000 74 / 80, of 7000 to 8000 156 / 162; head size 64, 64 of 3000 69 / 73), and the launch
+  // knows the longest only.  Where two blocks and more share a request anyway, and below 2048 positions, a second round of
+  // blocks cost more than it gave (16 requests of 3000 41 / 46).
+  if (S == 1 && cluster > 4) {
+    const long long one = (long long)R * nkv;
+    while (S < cluster && one * S * 2 * 10 <= 27ll * resident) S <<= 1;
+    if (S == 2 && one <= resident) S = 1;
+  }
   // Whole pages by TMA at head size 128 where the pages allow it (at least 8 rows, so that a box fills whole
   // rows of the swizzle pattern; addresses that a tensor map takes); key by key otherwise, at head size 128
   // then in the one-stage form only.  At head size 64 TMA measured level or slower (batch 8 at 4096 tokens
