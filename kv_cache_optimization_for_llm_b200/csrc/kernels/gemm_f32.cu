@@ -176,3 +176,5 @@ KVB_EXPORT int kvb_sgemm_nt(const float* A, int lda, const float* W, int ldw, fl
                             int M, int N, int K, cudaStream_t stream) {
   return kvb_sgemm_nt_tile(A, lda, W, ldw, C, ldc, M, N, K, -1, stream);
 }
+
+#include "gemm_f32_split.cuh"

@@ -102,6 +102,8 @@ class DecoderModel:
         copies = int(getattr(self.embedding, "stream_copies", 1))      # a residual stream kept as several copies
         copies += (1 if self.keeps_embedding else 0) + 2 * len(self.from_embedding)
         step = 4 * max_tokens * h * copies + max_logit_rows * 4 * (h + v) + (1 << 16)
+        if self.ctx.dtype == torch.float32:
+            step += max_logit_rows * 6 * h                 # the three bfloat16 parts of the picked rows
         per_layer = 0
         entered = 3 * h if self.from_embedding else 0      # the stream's copy and the float32 product at the start of a pass
         for block in self.layers:

@@ -192,6 +192,25 @@ def new(shape, dtype: torch.dtype, device) -> torch.Tensor:
     return torch.empty(tuple(shape), dtype=dtype, device=device)
 
 
+class lent:
+    """A buffer that only the launches inside the ``with`` use: its place in the arena is the next tensor's afterwards (a step's launches
+    run in order on one stream)."""
+
+    def __init__(self, shape, dtype: torch.dtype, device):
+        self.args = (shape, dtype, device)
+
+    def __enter__(self):
+        self.region = _arena.current if _arena is not None and _arena.device == self.args[2] else None
+        if self.region is not None:
+            self.at = (self.region.block, self.region.offset)
+        return new(*self.args)
+
+    def __exit__(self, *exc):
+        if self.region is not None:
+            self.region.block, self.region.offset = self.at
+        return False
+
+
 def arena_tokens() -> Optional[int]:
     """The tokens of the largest step that the running step's arena was made for (None: no arena, or not told)."""
     return None if _arena is None else _arena.tokens
@@ -1960,9 +1979,20 @@ def fused_norm_rows(rows: int, dtype: torch.dtype) -> bool:
     return FUSED_NORM and dtype == torch.bfloat16 and rows <= min(SKINNY_MAX_ROWS, FUSED_EPILOGUE_MAX_ROWS)
 
 
+def float32_split_ok(w: torch.Tensor) -> bool:
+    """Whether float32 products with ``w`` go through bfloat16 parts on the tensor cores (gemm_f32_split.cuh) rather than chains
+    of FMA (gemm_f32.cu).  By W alone, so that a row's result stays the same whatever rows stand beside it.  From 512 k on: the
+    FMA chain takes 15 us for 512 k and 59 us for 2048 k however few its rows are, the parts 8 to 12 us there (SPLITFIGS)."""
+    return (w.shape[1] >= FLOAT32_SPLIT_MIN_K and w.shape[1] % 4 == 0 and w.stride(1) == 1 and w.stride(0) % 4 == 0
+            and w.data_ptr() % 16 == 0)
+
+
+FLOAT32_SPLIT_MIN_K = 512
+
+
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, into: Optional[torch.Tensor] = None):
     """``x . w^T`` with ``w`` [out, in].
-    float32: this package's FMA kernel (true 32-bit).
+    float32: this package's kernels, true 32-bit (long rows of W as three bfloat16 parts on the tensor cores, others by FMA).
     bfloat16, few rows (decode and short portions): this package's tcgen05/TMA
     kernel, which streams the weights.  bfloat16 with more rows (long prompt portions):
     the library product, float32 accumulation, as upstream's cublasGemmEx.
@@ -1992,6 +2022,13 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, into: Op
     if x.dtype == torch.float32:
         assert x.stride(1) == 1 and w.stride(1) == 1
         out = new((M, N), torch.float32, x.device)
+        if M and float32_split_ok(w):
+            with lent((3, M, -(-K // 8) * 8), torch.bfloat16, x.device) as parts:
+                rc = lib("gemm_f32").kvb_sgemm_nt_split(_p(x), c_int(x.stride(0)), _p(w), c_int(w.stride(0)), _p(out), c_int(N),
+                                                        c_int(M), c_int(N), c_int(K), _p(parts), _p(kernel_status(x.device)), _stream())
+            _check(rc, "sgemm_nt")
+            choices["sgemm_nt"] += 1
+            return out
         rc = lib("gemm_f32").kvb_sgemm_nt(_p(x), c_int(x.stride(0)), _p(w), c_int(w.stride(0)), _p(out),
                                           c_int(N), c_int(M), c_int(N), c_int(K), _stream())
         _check(rc, "sgemm_nt")

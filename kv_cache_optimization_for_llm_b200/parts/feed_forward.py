@@ -50,9 +50,10 @@ class SwiGLU(Part):
 
     def activation_widths(self):
         """Elements per token of the tensors one call produces: gate|up (when the activation is a
-        kernel of its own), the activation, and the output (or its bfloat16 copy with sums)."""
+        kernel of its own), the activation, and the output (or its bfloat16 copy with sums; in float32 the
+        parts of the second product's rows beside it)."""
         inter, hidden = self.gate_up.shape[0] // 2, self.down.shape[0]
-        return [2 * inter, inter, 2 * hidden]
+        return [2 * inter, inter, max(2 * hidden, hidden + 3 * inter // 2 if self.ctx.dtype == torch.float32 else 0)]
 
     def forward(self, x, batch, into=None):
         a = ops.linear_swiglu(x, self.gate_up, self.block)

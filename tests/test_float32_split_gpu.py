@@ -1,0 +1,80 @@
+"""The float32 product through three bfloat16 parts on the tensor cores: against 64 bits and the chain of FMA, whatever rows stand
+beside a row, and with values that are not finite."""
+
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(x, w):
+    from kv_cache_optimization_for_llm_b200 import ops
+    out = torch.empty((x.shape[0], w.shape[0]), device="cuda")
+    rc = ops.lib("gemm_f32").kvb_sgemm_nt(ops._p(x), x.stride(0), ops._p(w), w.stride(0), ops._p(out), w.shape[0], x.shape[0], w.shape[0],
+                                          x.shape[1], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    return out
+
+
+def _draw(M, N, K, seed, spread=False):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x, w = (torch.randn(s, generator=g, device="cuda") for s in ((M, K), (N, K)))
+    if spread:      # magnitudes over many binades, all of one sign: rounding errors that do not cancel would show
+        x, w = (t.abs() * torch.exp2(torch.randint(-20, 20, t.shape, generator=g, device="cuda").float()) for t in (x, w))
+    return x, w
+
+
+# rows: 1, the edges of 16, of a block's 192 and of its halves; features: below, at and above 128; k: the tail of 64 and of 8, cut over
+# 1, 2, 4 and 8 blocks
+@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (2, 1, 516), (15, 130, 2048), (16, 2048, 2048), (17, 3072, 2048), (97, 127, 1028),
+                                   (191, 256, 1024), (192, 129, 8192), (193, 2048, 8188), (385, 1000, 512), (33, 19000, 576)])
+@pytest.mark.parametrize("spread", [False, True])
+def test_split_product_is_as_close_as_a_chain_of_fma(M, N, K, spread):
+    from kv_cache_optimization_for_llm_b200 import ops
+    x, w = _draw(M, N, K, M + N + K, spread)
+    assert ops.float32_split_ok(w)
+    out, ref = ops.linear(x, w), x.double() @ w.double().T
+    scale = x.double().abs() @ w.double().abs().T
+    err, chain = ((t.double() - ref).norm() / ref.norm() for t in (out, _chain(x, w)))
+    assert err <= 1.05 * chain + 2.0 ** -25, (float(err), float(chain))
+    # pieces of 64 k are cut to 24 bits at each of 24 products, then added with one rounding each
+    bound = 24 * 2.0 ** -23 + (-(-K // 64) + 8) * 2.0 ** -24
+    assert bool(((out.double() - ref).abs() <= bound * scale).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 2048, 2048), (50, 300, 1024), (33, 16384 + 128, 512)])
+def test_a_row_is_the_same_alone_and_beside_others_and_at_any_alignment(M, N, K):
+    from kv_cache_optimization_for_llm_b200 import ops
+    x, w = _draw(M, N, K, 7)
+    full = ops.linear(x, w)
+    for rows in (slice(0, 1), slice(M - 1, M), slice(3, 20), slice(0, M // 2)):
+        assert torch.equal(ops.linear(x[rows].contiguous(), w), full[rows])
+    odd = torch.cat([x, x[:, :1]], 1)[:, :K]
+    assert odd.stride(0) % 4 and torch.equal(ops.linear(odd, w), full)
+
+
+def test_values_that_are_not_finite_come_out_as_from_the_chain():
+    from kv_cache_optimization_for_llm_b200 import ops
+    x, w = _draw(40, 384, 1024, 3)
+    inf = float("inf")
+    x[3, 5], x[4, 1000], x[5, 0], x[6, 17] = inf, -inf, float("nan"), 3.4e38      # the last rounds to infinity in bfloat16
+    w[17, 900], w[200, 5], w[201, 5], w[300, 17] = inf, 0.0, -inf, 1e-3
+    x[7, 900], x[8, 900] = 0.0, -1.0
+    x[9], w[5] = 1e30, 1e30                                                       # the sum overflows
+    out, ref = ops.linear(x, w), _chain(x, w)
+    bad = ~torch.isfinite(ref)
+    assert int(bad.sum()) > 1000 and torch.equal(torch.isfinite(out), ~bad)
+    assert torch.equal(torch.nan_to_num(out[bad], nan=1.0), torch.nan_to_num(ref[bad], nan=1.0))
+    # finite ones: a chain of K fmaf is off by at most K * 2^-24 of the sum of magnitudes, and the parts by less
+    scale = torch.nan_to_num(x.double().abs() @ w.double().abs().T, nan=float("inf"))
+    assert bool(((out.double() - ref.double()).abs() <= 2 * 1024 * 2.0 ** -24 * scale)[~bad].all())
+
+
+def test_products_that_the_parts_do_not_take_go_to_the_chain():
+    from kv_cache_optimization_for_llm_b200 import ops
+    x, w = _draw(20, 64, 520, 1)
+    for v in (w[:, :510], w[:, 1:517], w[:, :518]):      # short, off 16 bytes, no multiple of four
+        assert not ops.float32_split_ok(v)
+        assert torch.equal(ops.linear(x[:, :v.shape[1]], v), _chain(x[:, :v.shape[1]], v))
