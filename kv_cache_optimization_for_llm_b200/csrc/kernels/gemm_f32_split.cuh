@@ -4,18 +4,24 @@
 // parts before it left over, and what the three leave is below 2^-26 of the value).  Of the nine partial products the six
 // that matter are made on tcgen05 (bfloat16 products are exact in float32): hi hi, hi mid, mid hi, hi lo, lo hi, mid mid; the
 // others are below 2^-26 of the product.  A tensor core's accumulator truncates, so no sum stays in it for
-// longer than 64 k: float32 additions that round to nearest add these pieces up.  Against 64 bits the result is
-// closer than a chain of K fmaf (measured, normal operands, root mean square of the error over that of the result:
-// see the table below).  A result that is not finite is made again by the chain of fmaf from the float32
-// operands, so infinities and NaNs come out as that kernel's; a magnitude above the largest bfloat16 arrives there too.  (Operands
-// below 2^-110 lose the bits that bfloat16 cannot hold there.)
+// longer than 64 k: float32 additions that round to nearest add these pieces up.  Root mean square error over that of the result,
+// normal operands: 3.2e-7 to 3.4e-7 for 1024 to 8192 k, a chain of K fmaf 5.7e-7 (1024), 8.1e-7 (2048), 1.6e-6 (8192).
+// A result that is not finite is made again by the chain of fmaf from the float32 operands, so infinities and NaNs come out as
+// that kernel's; a magnitude above the largest bfloat16 arrives there too.  (Operands below 2^-110 lose the bits that bfloat16
+// cannot hold there.)
 //
-// A block makes 128 features x up to 192 rows of A (the tensor core's M is W's rows: those are many, whatever the step):
-//   warp 0        loads: W as float32 in pieces of 32 k, the parts of A (a small kernel makes them once per call: every block
-//                 of 128 features reads the same ones) in pieces of 64 k, both by TMA with the 128-byte swizzle;
-//   warp 1        issues the products, A operand (W's parts) out of tensor memory, B operand out of shared memory;
-//   warps 2..5    split W: a thread reads 32 k of its row and puts the three parts into tensor memory;
-//   warps 6..13   add the finished pieces of 64 k to their registers.
+// Measured (M x N x K, this kernel with the split of A / the chain of fmaf, us): 1 x 2048 x 2048 21 / 59, 338 x 3072 x 2048 54 / 135,
+// 338 x 16384 x 2048 142 / 585, 338 x 2048 x 8192 75 / 513, 2048 x 2048 x 2048 153 / 402, 1 x 128256 x 2048 291 / 455.
+// What bounds it: with few rows a thread's issue of 24 products a piece (58 cycles each) and the splitting of W; with many the operands'
+// way from L2 (100 KB a piece for 176 rows, about 40 bytes a cycle and SM; the tensor pipe would take 2112 cycles a piece, a piece
+// takes 2400).
+//
+// A block makes 128 features x up to 176 rows of A (the tensor core's M is W's rows: those are many, whatever the step):
+//   warp 0        loads: W as float32 and the parts of A (a small kernel makes them once per call: every block of 128 features
+//                 reads the same ones) in pieces of 64 k, both by TMA with the 128-byte swizzle;
+//   warps 1, 2    issue the products of every other piece, A operand (W's parts) out of tensor memory, B operand out of shared memory;
+//   warps 4..7    split W: a thread reads 64 k of its row and puts the three parts into tensor memory;
+//   warps 8..15   add the finished pieces of 64 k to their registers.
 // W goes through tensor memory because six products read it: out of shared memory, operands and copies would ask for
 // more than the 128 bytes a cycle that it delivers.  K is cut over the blocks of a cluster where N alone would leave SMs
 // idle; by N and K only, and the parts are added in a fixed order, so a row's result depends neither on the other rows nor on
@@ -26,26 +32,40 @@
 
 namespace f32s {
 
-constexpr int kRows = 128, kCols = 192;      // features and rows of A of a block
-constexpr int kSlice = 32, kBlockK = 64;     // k of a piece of W, of a piece of A's parts
-constexpr int kWStages = 4, kWBytes = kRows * kSlice * 4;
+constexpr int kRows = 128, kCols = 176;      // features and rows of A of a block
+constexpr int kBlockK = 64;                  // k of a piece
+constexpr int kMaxWStages = 6, kHalfBytes = kRows * 128, kWBytes = 2 * kHalfBytes;
+constexpr int kRing = 230400;         // bytes of shared memory for both rings
 constexpr int kMaxStages = 4;
-constexpr int kThreads = 14 * 32;
-constexpr unsigned kTmemCols = 512, kSlotCols = 3 * kSlice / 2, kSlots = 2, kAccCols = kCols;
+constexpr int kThreads = 16 * 32;
+constexpr unsigned kTmemCols = 512, kSlotCols = 3 * kBlockK / 4, kMaxSlots = 4;   // a slot: the parts of W's 32 k
+constexpr int kChunks = (kCols / 16 + 1) / 2;   // of 16 columns, of a half of the adding warps
 
 struct Params {
   const float* a; const float* w; float* c;
   int lda, ldw, ldc, M, N, K;
   int nt;                  // rows of A per block, a multiple of 16
-  int m_tiles, splits, k_blocks, stages;
+  int m_tiles, splits, k_blocks;
+  int stages, w_stages, slots;    // of A's parts, of W, of W's parts in tensor memory
   int* status;
 };
 
 struct Bars {
-  unsigned long long w_full[kWStages], w_empty[kWStages], b_full[kMaxStages], b_empty[kMaxStages];
-  unsigned long long a_full[kSlots], a_empty[kSlots], acc_full[2], acc_empty[2];
+  unsigned long long w_full[kMaxWStages], w_empty[kMaxWStages], b_full[kMaxStages], a_full[kMaxSlots], a_empty[kMaxSlots], acc_empty[2];
+  // piece i's products are over (its parts of A are free, its sum is there): ring of four, so that nobody who waits
+  // for a piece can be passed by the piece that uses the barrier next
+  unsigned long long done[4];
   unsigned tmem;
   int abort_flag;
+};
+
+// A place in a ring and the parity of the phase that fills it.
+struct Turn {
+  int at = 0;
+  unsigned parity = 0;
+  __device__ __forceinline__ void next(int places) {
+    if (++at == places) { at = 0; parity ^= 1u; }
+  }
 };
 
 __device__ __forceinline__ unsigned pack2(float x, float y) {
@@ -107,15 +127,16 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int plane_bytes = p.nt * 128, stage_bytes = 3 * plane_bytes;
   unsigned char* w_s = base;
-  unsigned char* b_s = base + kWStages * kWBytes;
+  unsigned char* b_s = base + p.w_stages * kWBytes;
   Bars* bars = reinterpret_cast<Bars*>(b_s + (size_t)p.stages * stage_bytes);
   volatile int* abort_flag = &bars->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int i = 0; i < kWStages; ++i) { mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_empty[i], 4); }
-    for (int i = 0; i < p.stages; ++i) { mbar_init(&bars->b_full[i], 1); mbar_init(&bars->b_empty[i], 1); }
-    for (int i = 0; i < (int)kSlots; ++i) { mbar_init(&bars->a_full[i], 4); mbar_init(&bars->a_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->acc_full[i], 1); mbar_init(&bars->acc_empty[i], 8); }
+    for (int i = 0; i < p.w_stages; ++i) { mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_empty[i], 4); }
+    for (int i = 0; i < p.stages; ++i) mbar_init(&bars->b_full[i], 1);
+    for (int i = 0; i < p.slots; ++i) { mbar_init(&bars->a_full[i], 4); mbar_init(&bars->a_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) mbar_init(&bars->acc_empty[i], 8);
+    for (int i = 0; i < 4; ++i) mbar_init(&bars->done[i], 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -133,97 +154,112 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int kb0 = (int)((long long)p.k_blocks * split / p.splits), kb1 = (int)((long long)p.k_blocks * (split + 1) / p.splits);
   const int blocks = kb1 - kb0;
   bool failed = false;
-  float acc[kCols / 32][16];                 // warps 6..13: columns 32 c + 16 half ..
-  const int half = (warp - 6) & 4 ? 1 : 0;
+  float acc[kChunks][16];                 // warps 8..15: columns 32 c + 16 half ..
+  const int half = warp >= 12;
 
+  // These loops are chains of one thread (or of one warp): as few barriers as the flow needs, and places in the rings and
+  // the parities of their barriers are counted, not divided out.
+  auto wait_done = [&](int i) { return wait_or_abort(&bars->done[i & 3], (unsigned)(i >> 2) & 1u, abort_flag); };
   if (warp == 0) {
     if (lane == 0) {
-      for (int i = 0; i < blocks && !failed; ++i) {
-        const int s = i % p.stages, k = (kb0 + i) * kBlockK;
-        if (i >= p.stages && !wait_or_abort(&bars->b_empty[s], (unsigned)(i / p.stages - 1) & 1u, abort_flag)) { failed = true; break; }
-        mbar_expect_tx(&bars->b_full[s], (unsigned)stage_bytes);
+      Turn bt, wt;
+      int k = kb0 * kBlockK;
+      for (int i = 0; i < blocks; ++i, k += kBlockK, bt.next(p.stages), wt.next(p.w_stages)) {
+        if (i >= p.w_stages && !wait_or_abort(&bars->w_empty[wt.at], wt.parity ^ 1u, abort_flag)) { failed = true; break; }
+        mbar_expect_tx(&bars->w_full[wt.at], kWBytes);
+        tma_load_2d(w_s + wt.at * kWBytes, &map_w, k, n0, &bars->w_full[wt.at]);
+        tma_load_2d(w_s + wt.at * kWBytes + kHalfBytes, &map_w, k + kBlockK / 2, n0, &bars->w_full[wt.at]);
+        if (i >= p.stages && !wait_done(i - p.stages)) { failed = true; break; }
+        mbar_expect_tx(&bars->b_full[bt.at], (unsigned)stage_bytes);
         for (int part = 0; part < 3; ++part)
-          tma_load_2d(b_s + (size_t)s * stage_bytes + part * plane_bytes, &map_a, k, part * p.M + m0, &bars->b_full[s]);
-        for (int j = 0; j < 2; ++j) {
-          const int t = 2 * i + j, ws = t % kWStages;
-          if (t >= kWStages && !wait_or_abort(&bars->w_empty[ws], (unsigned)(t / kWStages - 1) & 1u, abort_flag)) { failed = true; break; }
-          mbar_expect_tx(&bars->w_full[ws], kWBytes);
-          tma_load_2d(w_s + ws * kWBytes, &map_w, k + j * kSlice, n0, &bars->w_full[ws]);
-        }
+          tma_load_2d(b_s + (size_t)bt.at * stage_bytes + part * plane_bytes, &map_a, k, part * p.M + m0, &bars->b_full[bt.at]);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp < 3) {
     if (lane == 0) {
+      // two threads take turns, each with an accumulator of its own: a wait costs 200 cycles even where nothing is waited for, an
+      // issue 58, and a piece's 24 products at 128 rows 1536
       const unsigned idesc = idesc_bf16(kRows, (unsigned)p.nt);
-      for (int i = 0; i < blocks && !failed; ++i) {
-        const int s = i % p.stages, buf = i & 1;
-        if (!wait_or_abort(&bars->b_full[s], (unsigned)(i / p.stages) & 1u, abort_flag) ||
-            (i >= 2 && !wait_or_abort(&bars->acc_empty[buf], (unsigned)(i / 2 - 1) & 1u, abort_flag))) { failed = true; break; }
-        const unsigned d = tmem + buf * kAccCols;
-        unsigned long long bd[3];
-        for (int part = 0; part < 3; ++part) bd[part] = smem_desc_sw128(smem_u32(b_s + (size_t)s * stage_bytes + part * plane_bytes));
-        for (int j = 0; j < 2; ++j) {
-          const int t = 2 * i + j, slot = t & 1;
-          if (!wait_or_abort(&bars->a_full[slot], (unsigned)(t / 2) & 1u, abort_flag)) { failed = true; break; }
+      const unsigned long long b0 = smem_desc_sw128(smem_u32(b_s));
+      const unsigned plane16 = (unsigned)plane_bytes >> 4, stage16 = (unsigned)stage_bytes >> 4;
+      const int which = warp - 1;
+      const unsigned d = tmem + which * p.nt;
+      Turn bt, at;
+      if (which) { bt.next(p.stages); at.next(p.slots); at.next(p.slots); }
+      unsigned parity = 0;
+      for (int i = which; i < blocks && !failed; i += 2, parity ^= 1u) {
+        if (!wait_or_abort(&bars->b_full[bt.at], bt.parity, abort_flag) ||
+            (i >= 2 && !wait_or_abort(&bars->acc_empty[which], parity ^ 1u, abort_flag))) { failed = true; break; }
+        const unsigned long long bd = b0 + bt.at * stage16;
+#pragma unroll
+        for (int j = 0; j < 2; ++j, at.next(p.slots)) {
+          if (!wait_or_abort(&bars->a_full[at.at], at.parity, abort_flag)) { failed = true; break; }
           fence_after();
-          const unsigned at = tmem + 2 * kAccCols + slot * kSlotCols;
+          const unsigned w = tmem + 2 * p.nt + at.at * kSlotCols;
           // the small products first, while the sum is small
           constexpr int pw[6] = {1, 2, 0, 1, 0, 0}, pa[6] = {1, 0, 2, 0, 1, 0};
 #pragma unroll
           for (int x = 0; x < 6; ++x)
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk)
-              umma_ts(d, at + pw[x] * (kSlice / 2) + kk * 8, bd[pa[x]] + 4 * j + 2 * kk, idesc, (j | x | kk) ? 1u : 0u);
-          umma_commit(&bars->a_empty[slot]);
+              umma_ts(d, w + pw[x] * 16 + kk * 8, bd + pa[x] * plane16 + 4 * j + 2 * kk, idesc, (j | x | kk) ? 1u : 0u);
+          umma_commit(&bars->a_empty[at.at]);
         }
         if (failed) break;
-        umma_commit(&bars->b_empty[s]);
-        umma_commit(&bars->acc_full[buf]);
+        umma_commit(&bars->done[i & 3]);
+        bt.next(p.stages);
+        bt.next(p.stages);
+        at.next(p.slots);
+        at.next(p.slots);
       }
     }
-  } else if (warp < 6) {
+  } else if (warp >= 4 && warp < 8) {
     const int r = (warp & 3) * 32 + lane;
-    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + 2 * kAccCols;
-    for (int t = 0; t < 2 * blocks; ++t) {
-      const int ws = t % kWStages, slot = t & 1;
-      if (!wait_or_abort(&bars->w_full[ws], (unsigned)(t / kWStages) & 1u, abort_flag)) { failed = true; break; }
-      const unsigned char* row = w_s + ws * kWBytes + r * 128;
-      unsigned h[16], m[16], l[16];
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + 2 * p.nt;
+    Turn wt, at;
+    for (int i = 0; i < blocks && !failed; ++i, wt.next(p.w_stages)) {
+      if (!wait_or_abort(&bars->w_full[wt.at], wt.parity, abort_flag)) { failed = true; break; }
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j, at.next(p.slots)) {
+        const unsigned char* row = w_s + wt.at * kWBytes + j * kHalfBytes + r * 128;
+        unsigned h[16], m[16], l[16];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 v = *reinterpret_cast<const float4*>(row + ((c ^ (r & 7)) << 4));
-        split2(v.x, v.y, h[2 * c], m[2 * c], l[2 * c]);
-        split2(v.z, v.w, h[2 * c + 1], m[2 * c + 1], l[2 * c + 1]);
+        for (int c = 0; c < 8; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(row + ((c ^ (r & 7)) << 4));
+          split2(v.x, v.y, h[2 * c], m[2 * c], l[2 * c]);
+          split2(v.z, v.w, h[2 * c + 1], m[2 * c + 1], l[2 * c + 1]);
+        }
+        if (2 * i + j >= p.slots && !wait_or_abort(&bars->a_empty[at.at], at.parity ^ 1u, abort_flag)) { failed = true; break; }
+        fence_after();
+        const unsigned to = lanes + at.at * kSlotCols;
+        tmem_st16(to, h);
+        tmem_st16(to + 16, m);
+        tmem_st16(to + 32, l);
+        wait_st();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&bars->a_full[at.at]);
+          if (j) mbar_arrive(&bars->w_empty[wt.at]);
+        }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->w_empty[ws]);
-      if (t >= (int)kSlots && !wait_or_abort(&bars->a_empty[slot], (unsigned)(t / 2 - 1) & 1u, abort_flag)) { failed = true; break; }
-      fence_after();
-      const unsigned at = lanes + slot * kSlotCols;
-      tmem_st16(at, h);
-      tmem_st16(at + kSlice / 2, m);
-      tmem_st16(at + kSlice, l);
-      wait_st();
-      fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->a_full[slot]);
     }
-  } else {
+  } else if (warp >= 8) {
     const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16);
 #pragma unroll
-    for (int c = 0; c < kCols / 32; ++c)
+    for (int c = 0; c < kChunks; ++c)
 #pragma unroll
       for (int j = 0; j < 16; ++j) acc[c][j] = 0.f;
-    for (int i = 0; i < blocks; ++i) {
-      const int buf = i & 1;
-      if (!wait_or_abort(&bars->acc_full[buf], (unsigned)(i / 2) & 1u, abort_flag)) { failed = true; break; }
+    Turn ct;
+    for (int i = 0; i < blocks; ++i, ct.next(2)) {
+      if (!wait_done(i)) { failed = true; break; }
       fence_after();
 #pragma unroll
-      for (int c = 0; c < kCols / 32; ++c) {
+      for (int c = 0; c < kChunks; ++c) {
         const int col = 32 * c + 16 * half;
         if (col < p.nt) {
           unsigned v[16];
-          tmem_ld16(lanes + buf * kAccCols + col, v);
+          tmem_ld16(lanes + ct.at * p.nt + col, v);
           wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) acc[c][j] += __uint_as_float(v[j]);
@@ -231,16 +267,16 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);
+      if (lane == 0) mbar_arrive(&bars->acc_empty[ct.at]);
     }
   }
   if (failed) *abort_flag = 1;
   __syncwarp();
   const int n_row = (warp & 3) * 32 + lane;
   if (p.splits == 1) {
-    if (warp >= 6) {
+    if (warp >= 8) {
 #pragma unroll
-      for (int c = 0; c < kCols / 32; ++c)
+      for (int c = 0; c < kChunks; ++c)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int col = 32 * c + 16 * half + j;
@@ -252,9 +288,9 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // add up a share of the rows each, the lowest k first
     __syncthreads();
     float* mine = reinterpret_cast<float*>(b_s);
-    if (warp >= 6) {
+    if (warp >= 8) {
 #pragma unroll
-      for (int c = 0; c < kCols / 32; ++c)
+      for (int c = 0; c < kChunks; ++c)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int col = 32 * c + 16 * half + j;
@@ -297,7 +333,7 @@ KVB_EXPORT long long kvb_sgemm_nt_split_scratch(int M, int K) { return 3ll * M *
 static int kvb_split_blocks(int N, int K) {
   const int tiles = (N + f32s::kRows - 1) / f32s::kRows, k_blocks = (K + f32s::kBlockK - 1) / f32s::kBlockK;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= 148 && k_blocks / (s * 2) >= 8) s *= 2;
+  while (s < 4 && tiles * s * 2 <= 148 && k_blocks / (s * 2) >= 8) s *= 2;
   return s;
 }
 
@@ -318,8 +354,13 @@ KVB_EXPORT int kvb_sgemm_nt_split(const float* A, int lda, const float* W, int l
   p.nt = ((M + p.m_tiles - 1) / p.m_tiles + 15) / 16 * 16;
   p.splits = kvb_split_blocks(N, K);
   p.k_blocks = (K + kBlockK - 1) / kBlockK;
-  p.stages = 147456 / (3 * 128 * p.nt);
+  p.slots = ((int)kTmemCols - 2 * p.nt) / (int)kSlotCols;
+  if (p.slots > kMaxSlots) p.slots = kMaxSlots;
+  p.stages = 110592 / (3 * 128 * p.nt);
   if (p.stages > kMaxStages) p.stages = kMaxStages;
+  if (p.stages < 2) p.stages = 2;
+  p.w_stages = (kRing - p.stages * 3 * 128 * p.nt) / kWBytes;
+  if (p.w_stages > kMaxWStages) p.w_stages = kMaxWStages;
   p.status = status;
   const long long grid = (long long)p.m_tiles * ((N + kRows - 1) / kRows) * p.splits;
   if (grid > 0x7fffffffll) return KVB_ERR_BAD_SIZE;
@@ -332,7 +373,8 @@ KVB_EXPORT int kvb_sgemm_nt_split(const float* A, int lda, const float* W, int l
   cudaError_t ce = kvb_launch(split_rows_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, stream, A, lda, M, K, Kp,
                               reinterpret_cast<__nv_bfloat16*>(parts), wide);
   if (ce != cudaSuccess) return (int)ce;
-  constexpr int kSmem = 1024 + kWStages * kWBytes + 147456 + (int)sizeof(Bars);
+  constexpr int kSmem = 1024 + kRing + (int)sizeof(Bars);
+  static_assert(kSmem <= 232448, "shared memory of a block");
   ce = cudaFuncSetAttribute(split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (ce != cudaSuccess) return (int)ce;
   cudaLaunchConfig_t cfg = {};

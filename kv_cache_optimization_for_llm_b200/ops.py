@@ -1981,13 +1981,14 @@ def fused_norm_rows(rows: int, dtype: torch.dtype) -> bool:
 
 def float32_split_ok(w: torch.Tensor) -> bool:
     """Whether float32 products with ``w`` go through bfloat16 parts on the tensor cores (gemm_f32_split.cuh) rather than chains
-    of FMA (gemm_f32.cu).  By W alone, so that a row's result stays the same whatever rows stand beside it.  From 512 k on: the
-    FMA chain takes 15 us for 512 k and 59 us for 2048 k however few its rows are, the parts 8 to 12 us there (SPLITFIGS)."""
+    of FMA (gemm_f32.cu).  By W alone, so that a row's result stays the same whatever rows stand beside it.  From 1024 k on the parts
+    are faster for every number of rows and features that was measured (1024 k, 1 to 338 rows: 20 to 36 us against 33 for 64 features, 24 to
+    58 against 37 to 172 for 8192) and closer to 64 bits; for 512 and 768 k and few rows the chain is (20 against 26 us, 27 against 28)."""
     return (w.shape[1] >= FLOAT32_SPLIT_MIN_K and w.shape[1] % 4 == 0 and w.stride(1) == 1 and w.stride(0) % 4 == 0
             and w.data_ptr() % 16 == 0)
 
 
-FLOAT32_SPLIT_MIN_K = 512
+FLOAT32_SPLIT_MIN_K = 1024
 
 
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, into: Optional[torch.Tensor] = None):

@@ -26,10 +26,10 @@ def _draw(M, N, K, seed, spread=False):
     return x, w
 
 
-# rows: 1, the edges of 16, of a block's 192 and of its halves; features: below, at and above 128; k: the tail of 64 and of 8, cut over
-# 1, 2, 4 and 8 blocks
-@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (2, 1, 516), (15, 130, 2048), (16, 2048, 2048), (17, 3072, 2048), (97, 127, 1028),
-                                   (191, 256, 1024), (192, 129, 8192), (193, 2048, 8188), (385, 1000, 512), (33, 19000, 576)])
+# rows: 1, the edges of 16, of a block's 176 and of its halves; features: below, at and above 128; k: the tail of 64 and of 8, cut over
+# 1, 2 and 4 blocks
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1024), (2, 1, 1028), (15, 130, 2048), (16, 2048, 2048), (17, 3072, 2048), (97, 127, 1028),
+                                   (175, 256, 1024), (176, 129, 8192), (177, 2048, 8188), (353, 1000, 1088), (33, 19000, 1152)])
 @pytest.mark.parametrize("spread", [False, True])
 def test_split_product_is_as_close_as_a_chain_of_fma(M, N, K, spread):
     from kv_cache_optimization_for_llm_b200 import ops
@@ -44,7 +44,7 @@ def test_split_product_is_as_close_as_a_chain_of_fma(M, N, K, spread):
     assert bool(((out.double() - ref).abs() <= bound * scale).all())
 
 
-@pytest.mark.parametrize("M,N,K", [(200, 2048, 2048), (50, 300, 1024), (33, 16384 + 128, 512)])
+@pytest.mark.parametrize("M,N,K", [(200, 2048, 2048), (50, 300, 1024), (33, 16384 + 128, 1024)])
 def test_a_row_is_the_same_alone_and_beside_others_and_at_any_alignment(M, N, K):
     from kv_cache_optimization_for_llm_b200 import ops
     x, w = _draw(M, N, K, 7)
@@ -74,7 +74,7 @@ def test_values_that_are_not_finite_come_out_as_from_the_chain():
 
 def test_products_that_the_parts_do_not_take_go_to_the_chain():
     from kv_cache_optimization_for_llm_b200 import ops
-    x, w = _draw(20, 64, 520, 1)
-    for v in (w[:, :510], w[:, 1:517], w[:, :518]):      # short, off 16 bytes, no multiple of four
+    x, w = _draw(20, 64, 1032, 1)
+    for v in (w[:, :1020], w[:, 1:1029], w[:, :1030]):      # short, off 16 bytes, no multiple of four
         assert not ops.float32_split_ok(v)
         assert torch.equal(ops.linear(x[:, :v.shape[1]], v), _chain(x[:, :v.shape[1]], v))
