@@ -18,6 +18,7 @@
 // Every sum is taken in an order that depends on the sizes only, so a token's result does not
 // depend on its neighbours in the step.
 #include "common.cuh"
+#include "limited_act.cuh"
 
 #include <math_constants.h>
 
@@ -330,12 +331,6 @@ __global__ void limited_act_kernel(const T* __restrict__ p, int ld_p, const floa
 
 // bfloat16 rows whose experts are multiples of 8 features wide: eight results per thread from two 16-byte loads, one
 // look at the token's weight for the expert, and no load at all for an expert that was not chosen.
-__device__ __forceinline__ float limited_one(float g, float u, float w, float limit, float alpha, float offset) {
-  g = fminf(w * g, limit);
-  u = fminf(fmaxf(w * u, -limit), limit);
-  return g / (1.0f + expf(-alpha * g)) * (u + offset);
-}
-
 __global__ void limited_act_bf16x8_kernel(const __nv_bfloat16* __restrict__ p, int ld_p, const float* __restrict__ gate,
                                           int ld_gate, const float* __restrict__ shared_logit, int ld_s,
                                           __nv_bfloat16* __restrict__ out, int E, int F, int S, int width, float limit,

@@ -1852,6 +1852,51 @@ def limited_act(p: torch.Tensor, gate: Optional[torch.Tensor], shared_logit: Opt
     return out
 
 
+# From this much dense work (tokens x width x experts x features of each) on, each expert's matrices are multiplied with the tokens that chose
+# it.  32 experts of which a token uses 4, width 2048, 256 features (us a call, grouped / dense): 640 tokens 101 / 93, 1024 tokens 111 / 117, 2048
+# tokens 157 / 234; width 1024, 128 features, 2048 tokens 96 / 84 (five launches more, each of which the host pays for as well).
+GROUPED_MIN_WORK = 15_000_000_000
+
+
+def experts_grouped_ok(x: torch.Tensor, first: torch.Tensor, down: torch.Tensor, experts: int, ff: int, shared_ff: int, top: int) -> bool:
+    """Whether :func:`experts_grouped` takes this step: bfloat16, many tokens, every token uses a quarter of the experts at most (or all
+    tokens' rows would be no less work than every expert's product), sizes that its tiles divide."""
+    return (x.dtype == torch.bfloat16 and x.shape[0] * x.shape[1] * experts * ff >= GROUPED_MIN_WORK and 4 * top <= experts <= 256 and top <= 16 and ff % 128 == 0
+            and ff > 0 and shared_ff % 128 == 0 and shared_ff > 0 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+            and first.is_contiguous() and down.is_contiguous() and down.shape[1] % 8 == 0
+            and (x.data_ptr() | first.data_ptr() | down.data_ptr()) % 16 == 0)
+
+
+def experts_grouped_widths(hidden: int, experts: int, ff: int, shared_ff: int, top: int) -> int:
+    """Elements of the compute type a token of such a step needs beside its output."""
+    return top * ff + shared_ff + (3 * top + 2) * hidden + 4 * experts + 2 * top + 64
+
+
+def experts_grouped(x: torch.Tensor, first: torch.Tensor, down: torch.Tensor, gate: torch.Tensor, shared_logit: Optional[torch.Tensor],
+                    experts: int, ff: int, shared_ff: int, top: int, limit: float, shared_limit: float, alpha: float,
+                    weigh_output: bool = False, offset: float = 1.0) -> torch.Tensor:
+    """``linear(limited_act(linear(x, first), ...), down)`` with each expert's products over the tokens that chose it only (``gate``
+    [T, >= experts] float32, 0 where not chosen, at most ``top`` others a token).  Sums and activations are float32 up to the activations' and the
+    result's one rounding each."""
+    _need_cuda(x, first, down, gate)
+    T, H = x.shape
+    out = new((T, H), x.dtype, x.device)
+    lists, rows_of = new((experts + 2 * experts * T,), torch.int32, x.device), new((T, top), torch.int32, x.device)
+    xg, act = new((T * top, H), x.dtype, x.device), new((T * top, ff), x.dtype, x.device)
+    shared_act, rows = new((T, shared_ff), x.dtype, x.device), new((T * top, H), torch.float32, x.device)
+    rc = lib("experts_grouped").kvb_experts_grouped(
+        _p(x), c_int(x.stride(0)), _p(first), _p(down), c_int(down.stride(0)), _p(gate), c_int(gate.stride(0)), _p(shared_logit),
+        c_int(0 if shared_logit is None else shared_logit.stride(0)), c_int(T), c_int(H), c_int(experts), c_int(ff), c_int(shared_ff),
+        c_int(top), c_float(limit), c_float(shared_limit), c_float(alpha), c_float(offset), c_int(1 if weigh_output else 0), _p(lists),
+        _p(xg), _p(act), _p(shared_act), _p(rows), _p(rows_of), _p(kernel_status(x.device)), _stream())
+    _check(rc, "experts_grouped")
+    shared = _library_product(shared_act, down[:, experts * ff:experts * ff + shared_ff], torch.float32)
+    rc = lib("experts_grouped").kvb_experts_join(_p(shared), _p(rows), _p(rows_of), _p(out), c_int(T), c_int(H), c_int(top), _stream())
+    _check(rc, "experts_join")
+    choices["experts_grouped"] += 1
+    return out
+
+
 def token_gate(p: torch.Tensor, table: torch.Tensor, first: int, batch, width: int) -> torch.Tensor:
     """``gelu_tanh(p[t, j]) * table[token[t], first + j]`` for every column j of ``p``; the result is ``width`` columns
     wide, those behind ``p``'s zero.  Tokens that are still on the device are found as in :func:`embed_gather`."""

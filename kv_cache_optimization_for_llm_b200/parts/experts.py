@@ -120,8 +120,9 @@ class LimitedExperts(Part):
     the activation behind the limits, which a last matrix without bias hands through), and writes 0
     for an expert that was not chosen; the second product's float32 sums then add up exactly the chosen experts.  The
     shared expert's gate multiplies its activation, which for a last matrix without bias is the same as multiplying its
-    output.  The router's rows and the shared gate's row are one small product with float32 results.  Every expert is
-    computed for every token (see :class:`RoutedExperts` for what that costs).
+    output.  The router's rows and the shared gate's row are one small product with float32 results.  Short steps compute every
+    expert for every token (they read every expert's matrices anyway); long bfloat16 steps each expert for the tokens that chose it
+    (:func:`..ops.experts_grouped`).
     params: hidden_size, experts, top, expert_ff, limit, shared_ff, shared_limit, alpha, offset, score, weigh, correction,
     groups, keep_groups."""
 
@@ -142,7 +143,7 @@ class LimitedExperts(Part):
 
     @classmethod
     def kernel_modules(cls, params, dtype):
-        return ("experts",) + (("gemm_f32",) if dtype == torch.float32 else ("gemm_bf16", "gemm_bf16_wide"))
+        return ("experts",) + (("gemm_f32",) if dtype == torch.float32 else ("experts_grouped", "gemm_bf16", "gemm_bf16_wide"))
 
     def __init__(self, params, weights, ctx):
         super().__init__(params, weights, ctx)
@@ -187,7 +188,8 @@ class LimitedExperts(Part):
 
     def activation_widths(self):
         inner = self.E * self.F + self.S
-        return [2 * inner, inner + self.pad, 4 * (self.E + 1) + 2 * self.small.shape[0], self.hidden]
+        dense, grouped = 3 * inner + self.pad, ops.experts_grouped_widths(self.hidden, self.E, self.F, self.S, self.top)
+        return [max(dense, grouped), 4 * (self.E + 1) + 2 * self.small.shape[0], self.hidden]
 
     def forward(self, x, batch):
         logits = ops.linear(x, self.small, out_dtype=torch.float32)
@@ -196,7 +198,11 @@ class LimitedExperts(Part):
         gate, _ = ops.route(x, None, self.correction, self.E, 0, self.top, 1.0, logits,
                             score="softmax" if chosen_only else "sigmoid", renormalize=chosen_only, groups=self.groups,
                             keep_groups=self.keep_groups)
+        shared = logits[:, self.E] if self.S else None
+        if ops.experts_grouped_ok(x, self.first, self.down, self.E, self.F, self.S, self.top):
+            return ops.experts_grouped(x, self.first, self.down, gate, shared, self.E, self.F, self.S, self.top, self.limit,
+                                       self.shared_limit, self.alpha, weigh_output=self.weigh == "output", offset=self.offset)
         p = ops.linear(x, self.first)
-        a = ops.limited_act(p, gate, logits[:, self.E] if self.S else None, self.E, self.F, self.S, self.pad, self.limit,
+        a = ops.limited_act(p, gate, shared, self.E, self.F, self.S, self.pad, self.limit,
                             self.shared_limit, self.alpha, weigh_output=self.weigh == "output", offset=self.offset)
         return ops.linear(a, self.down)
