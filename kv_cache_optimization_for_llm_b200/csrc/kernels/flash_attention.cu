@@ -771,6 +771,9 @@ constexpr int kWsThreads = 224;
 constexpr int kStages = 3;
 constexpr unsigned kWsTmemCols = 256;
 
+constexpr int ws_key_stages(int dk) { return dk == 64 ? 3 : dk == 192 ? 1 : 2; }
+constexpr int ws_value_stages(int dk) { return dk == 64 ? 3 : dk == 96 ? 2 : 1; }
+
 struct WsBars {
   unsigned long long q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
   unsigned long long s_full[2], s_free[2], p_full[2], o_done[2];
@@ -807,13 +810,15 @@ __device__ __forceinline__ bool wait_or_abort(void* bar, unsigned parity, volati
   return false;
 }
 
-// DH: the head size, 64 or 128.  Operands wider than 64 elements lie in shared memory as sub-tiles of
-// 64 columns side by side (a row of the 128-byte swizzle holds 64 bfloat16): Q, K and V have DH / 64
-// of them.  The scores take DH / 16 products of 16 along the head, the output DH / 64 times 4
-// products of 64 columns each; tensor memory holds the output in columns 128 .. 128 + DH.
+// DK, DV: the sizes of a key and of a value: 64 | 64, 128 | 128, and, for rows that a latent attention makes for one step, 192 | 128 and
+// 96 | 64 (16 heads, runs of 1400 and 648 behind 600: 76 us where the kernel on mma.sync with 255 registers a thread and one block
+// an SM takes 166, launches with events between them).  Operands wider than 64 elements lie in shared memory as sub-tiles of
+// 64 columns side by side (a row of the 128-byte swizzle holds 64 bfloat16), the last one half empty at 96.  The scores take
+// DK / 16 products of 16 along the head, the output DV / 64 times 4
+// products of 64 columns each; tensor memory holds the output in columns 128 .. 128 + DV.
 // EXT: kept first keys (their tiles come first in the walk) and the one more in the denominator, see MaskExt; the
 // stride between cached rows is the tensor maps' business.
-template <int DH, bool EXT>
+template <int DK, int DV, bool EXT>
 __global__ void __launch_bounds__(kWsThreads, 2)
 paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                 int box_rows, const __nv_bfloat16* __restrict__ q_base, int q_row_stride,
@@ -823,18 +828,18 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
                                 float scale_log2, int window, int* status, MaskExt ext) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kSub = DH / 64;                        // sub-tiles of 64 columns in Q, K and V
+  constexpr int kSub = (DK + 63) / 64, kVSub = DV / 64;   // sub-tiles of 64 columns in Q and K, in V
   constexpr int kQSub = BM * 128, kKVSub = BNK * 128;  // bytes of one sub-tile: rows x 128 bytes
-  constexpr int kQB = kSub * kQSub, kKVB = kSub * kKVSub;
+  constexpr int kQB = kSub * kQSub, kKB = kSub * kKVSub, kVB = kVSub * kKVSub;
   // Stages of keys and of values and buffers of probabilities: 3, 3 and 2 at head size 64; 2, 1 and 1
   // at head size 128, where a block then takes 96 KB and two of them fit an SM (eight softmax warps
-  // instead of four).  One value stage is enough: V(i) is requested when P V(i - 1) is over, at the
+  // instead of four); 1, 1 and 1 (104 KB) at 192 | 128 and 2, 2 and 1 at 96 | 64 for the same reason.  One value stage is enough: V(i) is requested when P V(i - 1) is over, at the
   // start of the softmax of tile i, and is needed at its end.
-  constexpr int kKSt = DH == 64 ? 3 : 2, kVSt = DH == 64 ? 3 : 1, kPB = DH == 64 ? 2 : 1;
-  unsigned char* q_s = base;                           // [DH/64][128 rows][64]
-  unsigned char* k_s = q_s + kQB;                      // [kKSt][DH/64][64 keys][64]
-  unsigned char* v_s = k_s + kKSt * kKVB;              // [kVSt][DH/64][64 keys][64]
-  unsigned char* p_s = v_s + kVSt * kKVB;              // [kPB][128 rows][64 keys]
+  constexpr int kKSt = ws_key_stages(DK), kVSt = ws_value_stages(DK), kPB = DK == 64 ? 2 : 1;
+  unsigned char* q_s = base;                           // [kSub][128 rows][64]
+  unsigned char* k_s = q_s + kQB;                      // [kKSt][kSub][64 keys][64]
+  unsigned char* v_s = k_s + kKSt * kKB;               // [kVSt][kVSub][64 keys][64]
+  unsigned char* p_s = v_s + kVSt * kVB;               // [kPB][128 rows][64 keys]
   WsBars* bars = reinterpret_cast<WsBars*>(p_s + kPB * kPBytes);
   unsigned* tmem_holder = reinterpret_cast<unsigned*>(bars + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
@@ -905,8 +910,8 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
       const int lp = (int)(((long long)box * box_rows) >> page_shift);
       return lp < max_pages ? __ldg(table + lp) : -1;
     };
-    auto request = [&](int i, int pg, unsigned char* dst, const CUtensorMap* map, void* bar) {
-      if (lane == 0) mbar_expect_tx(bar, kKVB);
+    auto request = [&](int i, int pg, unsigned char* dst, const CUtensorMap* map, void* bar, int subs) {
+      if (lane == 0) mbar_expect_tx(bar, subs * kKVSub);
       __syncwarp();                                              // the bytes are expected before any copy can report
       const int page = __shfl_sync(0xffffffffu, pg, (i * n_box + lane) & 31);
       if (lane < n_box) {                                        // lane c requests box c of the tile
@@ -919,8 +924,8 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
           atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE);        // keys that a row reads
         }
 #pragma unroll
-        for (int sub = 0; sub < kSub; ++sub)                     // columns 64 sub .. 64 sub + 63 of the box's rows
-          tma_load_2d(dst + sub * kKVSub + lane * box_rows * 128, map, 64 * sub, row, bar);
+        for (int sub = 0; sub < (kSub > kVSub ? kSub : kVSub); ++sub)   // columns 64 sub .. 64 sub + 63 of the box's rows
+          if (sub < subs) tma_load_2d(dst + sub * kKVSub + lane * box_rows * 128, map, 64 * sub, row, bar);
       }
     };
     int pg_k = -1, pg_v = -1, chunk_k = -1, chunk_v = -1;
@@ -934,7 +939,7 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
           failed = true;
         failed = __shfl_sync(0xffffffffu, (int)failed, 0) != 0;
         if (failed) break;
-        request(kt, pg_k, k_s + (kt % kKSt) * kKVB, &map_k, &bars->k_full[kt % kKSt]);
+        request(kt, pg_k, k_s + (kt % kKSt) * kKB, &map_k, &bars->k_full[kt % kKSt], kSub);
       }
       if (vt >= 0) {
         const int chunk = (vt * n_box) >> 5;
@@ -944,7 +949,7 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
           failed = true;
         failed = __shfl_sync(0xffffffffu, (int)failed, 0) != 0;
         if (failed) break;
-        request(vt, pg_v, v_s + (vt % kVSt) * kKVB, &map_v, &bars->v_full[vt % kVSt]);
+        request(vt, pg_v, v_s + (vt % kVSt) * kVB, &map_v, &bars->v_full[vt % kVSt], kVSub);
       }
     }
   } else if (warp <= 2) {
@@ -962,9 +967,9 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
         if (i >= 2 && !wait_or_abort(&bars->s_free[i & 1], (unsigned)((i - 2) >> 1) & 1u, abort_flag)) { failed = true; break; }
         tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {   // 16 of the head per step: sub-tile kk / 4, 32 bytes further along its rows
+        for (int kk = 0; kk < DK / 16; ++kk) {   // 16 of the head per step: sub-tile kk / 4, 32 bytes further along its rows
           const unsigned long long qd = smem_desc_sw128(smem_u32(q_s + (kk >> 2) * kQSub));
-          const unsigned long long kd = smem_desc_sw128(smem_u32(k_s + (i % kKSt) * kKVB + (kk >> 2) * kKVSub));
+          const unsigned long long kd = smem_desc_sw128(smem_u32(k_s + (i % kKSt) * kKB + (kk >> 2) * kKVSub));
           umma_bf16(tmem + 64 * (i & 1), qd + 2 * (kk & 3), kd + 2 * (kk & 3), idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars->k_empty[i % kKSt]);
@@ -978,8 +983,8 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
         tc_fence_after();
         const unsigned long long pd = smem_desc_sw128(smem_u32(p_s + (j % kPB) * kPBytes));
 #pragma unroll
-        for (int sub = 0; sub < kSub; ++sub) {    // output columns 64 sub .. 64 sub + 63 from V's sub-tile
-          const unsigned long long vd = smem_desc_sw128(smem_u32(v_s + (j % kVSt) * kKVB + sub * kKVSub));
+        for (int sub = 0; sub < kVSub; ++sub) {    // output columns 64 sub .. 64 sub + 63 from V's sub-tile
+          const unsigned long long vd = smem_desc_sw128(smem_u32(v_s + (j % kVSt) * kVB + sub * kKVSub));
 #pragma unroll
           for (int kk = 0; kk < BNK / 16; ++kk)   // 16 keys per step: 32 bytes along a row of P, 16 rows of V
             umma_bf16(tmem + 128 + 64 * sub, pd + 2 * kk, vd + 128 * kk, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
@@ -1003,9 +1008,9 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
     const float cap_out = (EXT && ext.softcap > 0.f) ? ext.softcap * 1.4426950408889634f / scale_log2 : 0.f;
     {
       const __nv_bfloat16* src = q_base + (size_t)(tile.t0 + (row_ok ? ti : 0)) * q_row_stride +
-                                 (size_t)(hk * G + (row_ok ? hi : 0)) * DH;
+                                 (size_t)(hk * G + (row_ok ? hi : 0)) * DK;
 #pragma unroll
-      for (int i = 0; i < DH / 8; ++i) cp_async_16_zfill(q_s + (i >> 3) * kQSub + swz<64>(r, i & 7), src + i * 8, row_ok);
+      for (int i = 0; i < DK / 8; ++i) cp_async_16_zfill(q_s + (i >> 3) * kQSub + swz<64>(r, i & 7), src + i * 8, row_ok);
       cp_async_commit();
       cp_async_wait<0>();
       fence_async_smem();
@@ -1069,7 +1074,7 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
           if (!wait_or_abort(&bars->o_done[(i - 1) & 1], (unsigned)((i - 1) >> 1) & 1u, abort_flag)) { failed = true; break; }
           tc_fence_after();
 #pragma unroll
-          for (int part = 0; part < DH / 16; ++part) {
+          for (int part = 0; part < DV / 16; ++part) {
             float ov[16];
             tmem_ld16(o_cols + 16 * part, ov);
 #pragma unroll
@@ -1120,11 +1125,11 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
         else l_run += ex2(sink - m_ref);
       }
       const float inv = (l_run > 0.f && l_run < CUDART_INF_F) ? 1.0f / l_run : 0.f;
-      __nv_bfloat16* dst = out + ((size_t)(tile.t0 + ti) * nq + hk * G + hi) * DH;
+      __nv_bfloat16* dst = out + ((size_t)(tile.t0 + ti) * nq + hk * G + hi) * DV;
       const __nv_bfloat16* gate = (EXT && ext.gate != nullptr && row_ok)
-          ? ext.gate + (size_t)(tile.t0 + ti) * ext.gate_ld + (size_t)(hk * G + hi) * DH : nullptr;
+          ? ext.gate + (size_t)(tile.t0 + ti) * ext.gate_ld + (size_t)(hk * G + hi) * DV : nullptr;
 #pragma unroll
-      for (int half = 0; half < DH / 32; ++half) {
+      for (int half = 0; half < DV / 32; ++half) {
         float o[32];
         tmem_ld32(o_cols + 32 * half, o);
         if (EXT && gate != nullptr) {
@@ -1163,35 +1168,37 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
 
 using kvb_page_maps::pages_map;
 
-template <int DH, bool EXT = false>
+template <int DK, int DV, bool EXT = false>
 int launch_ws(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, const int* block_table,
               int max_pages, int page_shift, int num_pages, const int* positions, const void* tiles, int num_tiles,
               void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status,
-              cudaStream_t stream, MaskExt ext = MaskExt{DH, 0, 0}) {
+              cudaStream_t stream, MaskExt ext = MaskExt{DK, 0, 0}) {
   const int page_size = 1 << page_shift;
   const int box_rows = page_size < BNK ? page_size : BNK;
   const long long rows = ext.head_rows > 0 ? (long long)ext.head_rows * nkv : (long long)num_pages * nkv * page_size;
   if (rows >= (1ll << 31)) return KVB_ERR_BAD_SIZE;
   CUtensorMap mk, mv;
-  int e = pages_map(&mk, k_pages, rows, box_rows, DH, ext.kv_row_stride);
+  int e = pages_map(&mk, k_pages, rows, box_rows, DK, ext.kv_row_stride);
   if (e) return e;
-  e = pages_map(&mv, v_pages, rows, box_rows, DH, ext.kv_row_stride);
+  e = pages_map(&mv, v_pages, rows, box_rows, DV, ext.kv_row_stride);
   if (e) return e;
-  constexpr int kKSt = DH == 64 ? 3 : 2, kVSt = DH == 64 ? 3 : 1, kPB = DH == 64 ? 2 : 1;   // as in the kernel
-  const size_t smem = 1024 + (size_t)BM * DH * 2 + (kKSt + kVSt) * (size_t)BNK * DH * 2 + kPB * kPBytes + sizeof(WsBars) + 64;
+  constexpr int kSub = (DK + 63) / 64, kVSub = DV / 64, kPB = DK == 64 ? 2 : 1;   // as in the kernel
+  constexpr size_t smem = 1024 + (size_t)kSub * BM * 128 + (size_t)(ws_key_stages(DK) * kSub + ws_value_stages(DK) * kVSub) * BNK * 128 +
+                          kPB * kPBytes + sizeof(WsBars) + 64;
+  static_assert(2 * smem + 2048 <= 228 * 1024, "two blocks an SM");
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DH, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DK, DV, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem);
     if (ce != cudaSuccess) return (int)ce;
     // two blocks per SM need the largest shared-memory configuration
-    ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DH, EXT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DK, DV, EXT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                               (int)cudaSharedmemCarveoutMaxShared);
     if (ce != cudaSuccess) return (int)ce;
     attr_set = true;
   }
   dim3 grid(num_tiles, nkv);
-  kvb_launch(paged_flash_attention_ws_kernel<DH, EXT>, grid, dim3(kWsThreads), smem, stream, mk, mv, box_rows,
+  kvb_launch(paged_flash_attention_ws_kernel<DK, DV, EXT>, grid, dim3(kWsThreads), smem, stream, mk, mv, box_rows,
              (const __nv_bfloat16*)q, q_row_stride, block_table, max_pages, page_shift,
              num_pages, positions, (const TileDesc*)tiles, (__nv_bfloat16*)out, nq, nkv, G, gp_shift,
              scale * 1.4426950408889634f, window, status, ext);
@@ -1268,9 +1275,9 @@ KVB_EXPORT int kvb_paged_flash_attention(const void* q, int q_row_stride, const 
         (reinterpret_cast<uintptr_t>(k_pages) & 15) || (reinterpret_cast<uintptr_t>(v_pages) & 15))
       return KVB_ERR_BAD_SIZE;
     if (d == 64)
-      return tc5::launch_ws<64>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
+      return tc5::launch_ws<64, 64>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
                                 positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream);
-    return tc5::launch_ws<128>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
+    return tc5::launch_ws<128, 128>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
                                positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream);
   }
   if (wide == 2) {   // tcgen05 form
@@ -1312,9 +1319,9 @@ KVB_EXPORT int kvb_paged_flash_attention_rows(const void* q, int q_row_stride, c
   if (wide == 3) {   // the tcgen05 form with roles: 128-row tiles, pages of at least 8 rows
     if (page_size < 8) return KVB_ERR_BAD_SIZE;
     if (d == 64)
-      return tc5::launch_ws<64, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
+      return tc5::launch_ws<64, 64, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
                                       positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
-    return tc5::launch_ws<128, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
+    return tc5::launch_ws<128, 128, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
                                      positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
   }
 #define KVB_FA_EXT(D, NW)                                                                                              \
@@ -1329,12 +1336,13 @@ KVB_EXPORT int kvb_paged_flash_attention_rows(const void* q, int q_row_stride, c
 // that mask by blocks of positions, count a learned score per head into the denominator, cap their scores or gate
 // their result (see MaskExt): query i sees key j <= i when i / chunk == j / chunk (chunk 0: every key up to i), or,
 // without a chunk, when i - j < window (window 0: every key up to i).  head_rows: see MaskExt.
-// sinks float32 [nq] or null; softcap 0 for none; gate bfloat16 [T, >= nq * d], 16-byte aligned, gate_ld a multiple
+// Key and value size are 64 or 128 both, or, for rows made for one step, 192 | 128 and 96 | 64.
+// sinks float32 [nq] or null; softcap 0 for none; gate bfloat16 [T, >= nq * dv], 16-byte aligned, gate_ld a multiple
 // of 8, or null.
 KVB_EXPORT int kvb_paged_flash_attention_rows_masked(const void* q, int q_row_stride, const void* pages,
                                                      const int* block_table, int max_pages, int page_size, int num_pages,
                                                      const int* positions, const void* tiles, int num_tiles, void* out,
-                                                     int nq, int nkv, int d, float scale, int window, int chunk, const float* sinks,
+                                                     int nq, int nkv, int dk, int dv, float scale, int window, int chunk, const float* sinks,
                                                      float softcap, const void* gate, int gate_ld, int head_rows,
                                                      int* status, cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
@@ -1342,7 +1350,10 @@ KVB_EXPORT int kvb_paged_flash_attention_rows_masked(const void* q, int q_row_st
       (head_rows > 0 && (long long)head_rows < (long long)num_pages * page_size)) return KVB_ERR_BAD_SIZE;
   if (nkv < 1 || nq % nkv || chunk < 0 || softcap < 0.f || !(scale > 0.f)) return KVB_ERR_BAD_SIZE;
   const int G = nq / nkv;
-  if (!kvb_flash_attention_supported(d, G, page_size) || nkv > 65535 || page_size < 8) return KVB_ERR_BAD_SIZE;
+  // a key wider than its value: rows made for one step only
+  const bool wider = (dk == 192 && dv == 128) || (dk == 96 && dv == 64);
+  if (!kvb_flash_attention_supported(dv, G, page_size) || nkv > 65535 || page_size < 8 || !(dk == dv || (wider && head_rows > 0)))
+    return KVB_ERR_BAD_SIZE;
   if ((reinterpret_cast<uintptr_t>(q) & 15) || (q_row_stride & 7) || (reinterpret_cast<uintptr_t>(pages) & 15) ||
       (reinterpret_cast<uintptr_t>(gate) & 15) || (gate != nullptr && (gate_ld & 7)))
     return KVB_ERR_ALIGN;
@@ -1350,11 +1361,16 @@ KVB_EXPORT int kvb_paged_flash_attention_rows_masked(const void* q, int q_row_st
   while ((1 << gp_shift) < G) ++gp_shift;
   if ((128 >> gp_shift) < 1) return KVB_ERR_BAD_SIZE;
   const int page_shift = log2_exact(page_size);
-  const MaskExt ext{2 * d, 0, 0, chunk, sinks, softcap, static_cast<const __nv_bfloat16*>(gate), gate_ld, head_rows};
-  const void* values = static_cast<const __nv_bfloat16*>(pages) + d;
-  if (d == 64)
-    return tc5::launch_ws<64, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
-                                    positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
-  return tc5::launch_ws<128, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
-                                   positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
+  const MaskExt ext{dk + dv, 0, 0, chunk, sinks, softcap, static_cast<const __nv_bfloat16*>(gate), gate_ld, head_rows};
+  const void* values = static_cast<const __nv_bfloat16*>(pages) + dk;
+#define KVB_WS(DK, DV)                                                                                                  \
+  return (tc5::launch_ws<DK, DV, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages, positions, tiles, \
+                                       num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext))
+  if (wider) {
+    if (dk == 192) KVB_WS(192, 128);
+    KVB_WS(96, 64);
+  }
+  if (dk == 64) KVB_WS(64, 64);
+  KVB_WS(128, 128);
+#undef KVB_WS
 }

@@ -60,7 +60,7 @@ class LatentAttention(Part):
             return ("latent_attention", "gemm_f32")
         up = ()
         if cls._up_sizes(params, dtype):
-            up = ("window_flash_attention",) + (("flash_attention",) if cls._one_size(params) else ())
+            up = ("window_flash_attention",) + (("flash_attention",) if cls._tcgen05_sizes(params) else ())
         return ("latent_attention",) + up + ("gemm_bf16", "gemm_bf16_wide")
 
     @staticmethod
@@ -71,9 +71,10 @@ class LatentAttention(Part):
                 and ops.made_rows_attention_supported(d + r, v))
 
     @staticmethod
-    def _one_size(params):
-        return (int(params["dim"]) == int(params["vdim"]) and int(params["dim"]) in (64, 128) and not int(params["rot_dim"])
-                and not params.get("gate"))
+    def _tcgen05_sizes(params):
+        """Whether the made rows' sizes are those of the prompt attention on tcgen05 (whose gate, of one number a channel, is another)."""
+        dk, dv = int(params["dim"]) + int(params["rot_dim"]), int(params["vdim"])
+        return ((dk == dv and dk in (64, 128)) or (dk, dv) in ops.MADE_WIDER) and not params.get("gate")
 
     def __init__(self, params, weights, ctx):
         super().__init__(params, weights, ctx)
@@ -143,7 +144,7 @@ class LatentAttention(Part):
             heights.append(ops.latent_tokens_per_tile(self.heads))
         if self.ukv is not None:
             heights += [ops.rows_tokens_per_tile(1, False), ops.rows_tokens_per_tile(1, True)]
-            if self._one_size(self.params):
+            if self._tcgen05_sizes(self.params):
                 heights.append(ops.flash_tokens_per_tile(1, True))
         return heights
 
@@ -154,10 +155,10 @@ class LatentAttention(Part):
         n, per_head = batch.num_single, self.dim + self.rot
         if rdims:        # (without a position the part behind the latent is cached, and compared, as it is)
             ops.latent_rotate(q, n, self.heads, per_head, self.dim, cos, sin, batch)
-        if self._one_size(self.params) and ops.flash_attention_rows_masked_wanted(batch, self.heads, self.heads, self.dim, self.vdim,
-                                                                                  rows.PAGE, self.ctx.dtype, q):
-            a = ops.flash_attention_rows_masked(q, None, None, batch, self.heads, self.heads, self.dim, self.scale, sinks=self.sink,
-                                                window=self.window or 0, rows=rows)
+        if self._tcgen05_sizes(self.params) and ops.flash_attention_rows_masked_wanted(batch, self.heads, self.heads, per_head, self.vdim,
+                                                                                       rows.PAGE, self.ctx.dtype, q, made=True):
+            a = ops.flash_attention_rows_masked(q, None, None, batch, self.heads, self.heads, per_head, self.scale, sinks=self.sink,
+                                                window=self.window or 0, rows=rows, dv=self.vdim)
         else:
             a = ops.window_flash_attention(q, None, None, batch, self.heads, self.heads, per_head, self.vdim, self.scale,
                                            self.window or 0, 0, False, sinks=self.sink, rows=rows, gate=gate)

@@ -91,6 +91,16 @@ def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, 
         assert off < 1.5e-2 and off < 1.5 * off_absorbed + 2e-3, (r, off, off_absorbed)
 
 
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank,sink,window", [
+    (2, 64, 32, 64, 64, False, None), (3, 64, 32, 64, 72, True, None), (2, 64, 32, 64, 64, True, 100), (2, 128, 64, 128, 64, False, 70),
+    (1, 160, 32, 128, 64, True, None)])
+def test_made_rows_with_keys_wider_than_values_on_tcgen05(heads, dim, rot, vdim, rank, sink, window):
+    from kv_cache_optimization_for_llm_b200 import ops
+    before = ops.choices["flash_attention_rows_masked"]
+    test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, False, window)
+    assert ops.choices["flash_attention_rows_masked"] > before
+
+
 @pytest.mark.parametrize("dims", [0, 8, 24])       # of 24 channels behind the key: none (the layer has no position), some, all
 @pytest.mark.parametrize("gate", [False, True])
 def test_made_rows_whose_shared_part_turns_in_part_or_not_at_all(dims, gate):
