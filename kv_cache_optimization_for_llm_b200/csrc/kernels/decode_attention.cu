@@ -136,6 +136,13 @@ template <int D> __device__ __forceinline__ int swz(int row, int chunk) {
 // 16 beyond (32 tiles of 128 keys per class at most up to 65536 positions).
 __host__ __device__ __forceinline__ int classes_at(int pos) { return pos < 2048 ? 4 : (pos < 8192 ? 8 : 16); }
 
+// Classes whose four warps' partials wait in shared memory for one merge: every merge is two barriers of the whole block, which short
+// contexts (a tile or two a class) feel more than their keys.  As many as leave the blocks per SM as they are (head size 64 has room for
+// one); four classes of more than two tiles each merge one by one, beside other blocks' loads.  Measured, head size 128, 8 kv heads, one a
+// time / this rule: 48 requests of 100 to 200 positions 20.2 / 19.1 us, of 70 to 900 36.5 / 34.7, 24 of 500 to 2000 37.0 / 35.9, of 500 to
+// 7900 80.5 / 79.8; 64 of 1500 to 2000 81.2 (one a time) against 83.2 (four).
+constexpr int held_classes(int d, int gp, int classes) { return d == 64 || gp > 4 ? 1 : classes == 4 ? 4 : classes == 8 ? 2 : 1; }
+
 // GP: the group of query heads padded to 4, 8 or 16 (rows that are kept).  kClasses: classes
 // of tiles per (request, kv head); gridDim.z = cluster size = blocks that share them.  kStages: tiles in shared memory at a time, 2 when the whole grid
 // is resident at once anyway (small batches: the second tile is under way before the
@@ -168,11 +175,11 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   unsigned char* k_s = smem;                                   // [kStages][4][32][D] bf16, swizzled
   unsigned char* v_s = k_s + kStages * kTileBytes;             // [kStages][4][32][D]
   float* q_s = reinterpret_cast<float*>(v_s + kStages * kTileBytes); // [GP][D] rotated, scaled queries
-  float* run = q_s + GP * D;                                   // [GP][PW] this block's partial so far
-  float* recv = run + GP * PW;                                 // [kClasses][GP][PW], used in block 0 only
-  float* wpart = recv + kClasses * GP * PW;                    // [4][GP][PW] the four warps' partials of a class
+  constexpr int kHeld = held_classes(D, GP, kClasses);
+  float* recv = q_s + GP * D;                                  // [kClasses][GP][PW], used in block 0 only
+  float* wpart = recv + kClasses * GP * PW;                    // [kHeld][4][GP][PW] the four warps' partials of the last classes
   // kTma only:
-  unsigned long long* full_b = reinterpret_cast<unsigned long long*>(wpart + 4 * GP * PW);   // [kStages][4] bytes of a slice
+  unsigned long long* full_b = reinterpret_cast<unsigned long long*>(wpart + kHeld * 4 * GP * PW);   // [kStages][4] bytes of a slice
   __nv_bfloat16* newkv_s = reinterpret_cast<__nv_bfloat16*>(full_b + kStages * 4);           // [2][D] the new key and value
   int* abort_flag = reinterpret_cast<int*>(newkv_s + 2 * D);                                 // a wait ran out
 
@@ -201,8 +208,6 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // Classes of tiles for this token: a function of its own position only (and of the kernel's
   // capacity kClasses, which the launcher takes from the longest context of the step).
   const int C = min(kClasses, classes_at(pos));
-
-  for (int i = tid; i < GP * PW; i += kThreads) run[i] = ((i % PW) == D) ? -CUDART_INF_F : 0.f;
 
   // Requests this warp's 32 keys and values of tile t into a stage and returns the mask of this warp's
   // keys that are there.  In two steps, so that the look-up in the block table (a load whose answer the
@@ -455,6 +460,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // Class after class.  Each warp walks its 32-key slices of the class's tiles on its own, with
   // a running max and sum per head (rows lane/4 and lane/4 + 8) and a running output in
   // registers; the slices of a warp are private to it, so the walk needs no block-wide barrier.
+  int held = 0;
   for (int cls = z; cls < C; cls += S) {
   float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
   float o[DT][4];
@@ -591,36 +597,38 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     for (int rr = 0; rr < 2; ++rr) {
       const int rowi = r0 + rr * 8;
       if (rowi < GP) {
-        float* dst = wpart + ((size_t)warp * GP + rowi) * PW;
+        float* dst = wpart + ((size_t)(held * 4 + warp) * GP + rowi) * PW;
+        if (m_run[rr] != -CUDART_INF_F) {       // (a warp without a key of this class: the merge leaves its output alone)
 #pragma unroll
-        for (int n = 0; n < DT; ++n) { dst[n * 8 + c0] = o[n][rr * 2]; dst[n * 8 + c0 + 1] = o[n][rr * 2 + 1]; }
+          for (int n = 0; n < DT; ++n) { dst[n * 8 + c0] = o[n][rr * 2]; dst[n * 8 + c0 + 1] = o[n][rr * 2 + 1]; }
+        }
         if ((lane & 3) == 0) { dst[D] = m_run[rr]; dst[D + 1] = l_run[rr]; }
       }
     }
   }
+  if (++held < (kHeld > 2 && n_tiles > 8 ? 1 : kHeld) && cls + S < C) continue;
   __syncthreads();
-  // the four warps' partials, merged in warp order, are this block's partial
-  for (int i = tid; i < GP * PW; i += kThreads) {
-    const int g = i / PW, dd = i % PW;
+  // the four warps' partials of a class, merged in warp order, are the block's partial of it, which goes to block 0 of the cluster
+  for (int i = tid; i < held * GP * PW; i += kThreads) {
+    const int k = i / (GP * PW), e = i - k * (GP * PW), g = e / PW, dd = e % PW;
+    const float* part = wpart + (size_t)k * 4 * GP * PW;
     float M = -CUDART_INF_F;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, wpart[((size_t)w * GP + g) * PW + D]);
+    for (int w = 0; w < 4; ++w) M = fmaxf(M, part[((size_t)w * GP + g) * PW + D]);
     float a = 0.f;
     if (dd == D) a = M;
     else if (M != -CUDART_INF_F) {
       const int col = dd == D + 1 ? D + 1 : dd;   // the sum merges like an output dim
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        const float mw = wpart[((size_t)w * GP + g) * PW + D];
-        if (mw != -CUDART_INF_F) a += wpart[((size_t)w * GP + g) * PW + col] * exp2f(mw - M);
+        const float mw = part[((size_t)w * GP + g) * PW + D];
+        if (mw != -CUDART_INF_F) a += part[((size_t)w * GP + g) * PW + col] * exp2f(mw - M);
       }
     }
-    run[i] = a;
+    st_peer_f32(recv + (size_t)(cls - (held - 1 - k) * S) * GP * PW + e, 0u, a);
   }
-  __syncthreads();
-
-  // ---- the class's partial goes to block 0 of the cluster
-  for (int i = tid; i < GP * PW; i += kThreads) st_peer_f32(recv + (size_t)cls * GP * PW + i, 0u, run[i]);
+  held = 0;
+  if (cls + S < C) __syncthreads();      // the partials are read; the next classes' may overwrite them
   }   // classes
   stamp(4);   // the block's partials are complete
   if constexpr (kTma) {
@@ -685,8 +693,8 @@ int log2_exact(int x) {
 template <int D, int GP, int kClasses, int kStages, bool kTma>
 constexpr size_t smem_bytes() {
   constexpr int PW = D + 2;
-  return (size_t)kStages * 2 * 4 * 32 * D * 2 + (size_t)GP * D * 4 + (size_t)GP * PW * 4 +
-         (size_t)kClasses * GP * PW * 4 + (size_t)4 * GP * PW * 4 +
+  return (size_t)kStages * 2 * 4 * 32 * D * 2 + (size_t)GP * D * 4 +
+         (size_t)kClasses * GP * PW * 4 + (size_t)held_classes(D, GP, kClasses) * 4 * GP * PW * 4 +
          (kTma ? 1024 + (size_t)kStages * 4 * 8 + 2 * D * 2 + 16 : 0);   // alignment, barriers, new key and value, flag
 }
 
