@@ -35,7 +35,7 @@
 // Also here: the short causal convolution with SiLU in front of such a mixer, whose last
 // inputs are part of the request's state.
 #include "common.cuh"
-#include "delta_walk.cuh"
+#include "delta_pieces.cuh"
 #include "head_finish.cuh"
 
 enum DeltaMode { MODE_GENERAL = 0, MODE_GATED = 1 };
@@ -370,10 +370,17 @@ KVB_EXPORT int kvb_delta_scan(const DeltaArgs* args, int mode, int R, int T_, in
   return KVB_ERR_BAD_DTYPE;
 }
 
+// Bytes of scratch with which kvb_delta_walk takes the form in three launches (delta_pieces.cuh) for `tokens` tokens in R runs, 0
+// where the sizes are not its own.
+KVB_EXPORT long long kvb_delta_walk_scratch(long long tokens, int R, int H, int Dk, int Dv) {
+  return Dk == delta_pieces::kN && Dv % 32 == 0 && Dv >= 32 && Dv <= 256 ? delta_pieces::scratch_bytes(tokens, R, H, Dv) : 0;
+}
+
 // The runs of requests first .. first + R - 1 (token rows row0 .. T_ - 1) walked in pieces of 64 tokens on tensor cores
 // (delta_walk.cuh), then their read-outs' norm and gate: MODE_GATED with one decay per head, bfloat16, Dk 64 or 128, Dv a multiple of
-// 32, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).
-KVB_EXPORT int kvb_delta_walk(const DeltaArgs* args, int first, int R, int row0, int T_, cudaStream_t stream) {
+// 32, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).  scratch: null for the walk in one launch,
+// or kvb_delta_walk_scratch bytes on a 16-byte boundary.
+KVB_EXPORT int kvb_delta_walk(const DeltaArgs* args, int first, int R, int row0, int T_, void* scratch, cudaStream_t stream) {
   DeltaArgs a = *args;
   if (R <= 0 || T_ <= row0) return 0;
   if (a.o_raw == nullptr || !a.decay_per_head || a.G < 1 || a.H % a.G) return KVB_ERR_BAD_SIZE;
@@ -388,7 +395,8 @@ KVB_EXPORT int kvb_delta_walk(const DeltaArgs* args, int first, int R, int row0,
   w.state = a.state; w.slot_stride = a.slot_stride; w.o = a.o_raw;
   w.q_start = a.q_start; w.req_start = a.req_start; w.slots = a.slots;
   w.H = a.H; w.Dv = a.Dv; w.first = first;
-  const int rc = delta_walk::launch_any(w, a.Dk, R, stream);
+  const int rc = scratch != nullptr && delta_pieces::takes_pieces(w, a.Dk) ? delta_pieces::launch(w, R, T_ - row0, scratch, stream)
+                                                                    : delta_walk::launch_any(w, a.Dk, R, stream);
   if (rc != 0) return rc;
   a.o_raw += (size_t)row0 * a.H * a.Dv;
   a.gate = static_cast<const B*>(a.gate) + (size_t)row0 * a.ld_gate;

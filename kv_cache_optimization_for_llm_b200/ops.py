@@ -462,6 +462,33 @@ def _at(t: torch.Tensor, col: int) -> int:
     return t.data_ptr() + col * t.element_size()
 
 
+# Longest run of a step, in tokens, from which on the walk's products that do not wait for the state are made for all pieces at once
+# (delta_pieces.cuh; keys of 64).
+DELTA_PIECES_MIN_RUN = 128
+
+
+def delta_pieces_width(heads: int, dk: int, dv: int) -> int:
+    """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs."""
+    if dk != 64 or dv % 32 or not 32 <= dv <= 256:
+        return 0
+    fn = lib("delta_rule").kvb_delta_walk_scratch
+    fn.restype = c_longlong
+    return -(-int(fn(c_longlong(64 * 64), c_int(0), c_int(heads), c_int(dk), c_int(dv))) // (2 * 64 * 64))
+
+
+def _delta_pieces_bytes(batch, tokens: int, heads: int, dk: int, dv: int, device) -> int:
+    """Bytes of scratch for the form in three launches, 0 where the runs walk in one (short runs, other sizes, or an arena without the
+    room)."""
+    if dk != 64 or int(getattr(batch, "max_q_len", 0) or 0) < DELTA_PIECES_MIN_RUN:
+        return 0
+    fn = lib("delta_rule").kvb_delta_walk_scratch
+    fn.restype = c_longlong
+    nbytes = int(fn(c_longlong(tokens), c_int(batch.num_reqs - int(batch.num_single)), c_int(heads), c_int(dk), c_int(dv)))
+    if _arena is not None and _arena.device == device and nbytes > _arena.current.capacity:
+        return 0
+    return nbytes
+
+
 def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux, decay_bias, aux_bias, head_rate,
                norm_w, norm_per_head: bool, heads: int, key_heads: int, dk: int, dv: int, eps: float,
                decay_per_head: bool = False, gate_act: str = "sigmoid") -> torch.Tensor:
@@ -473,7 +500,8 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
     matrix states.  ``mode``: "general" or "gated" (see csrc/kernels/delta_rule.cu).
     ``decay_per_head`` ("gated"): ``decay`` is [T, heads] and ``decay_bias`` [heads], one decay for all key
     channels of a head.  ``gate_act``: "sigmoid" or "silu", the function applied to the output gate.
-    bfloat16 steps with runs above :func:`walk_line` and one decay per head go to the walk on tensor cores where the sizes allow.
+    bfloat16 steps with runs above :func:`walk_line` and one decay per head go to the walk on tensor cores where the sizes allow,
+    in three launches from runs of ``DELTA_PIECES_MIN_RUN`` tokens on.
     Returns the gated, normed read-out [T, heads * dv]."""
     x0 = r[0]
     _need_cuda(x0, state)
@@ -505,10 +533,13 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
             _check(lib("delta_rule").kvb_delta_scan(ctypes.byref(a), c_int(1), c_int(singles), c_int(singles), c_int(1),
                                                     c_int(dtype_code(x0.dtype)), _stream()), "delta_scan")
             launch_count += 1
-        rc = lib("delta_rule").kvb_delta_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(singles),
-                                              c_int(T), _stream())
+        nbytes = _delta_pieces_bytes(batch, T - singles, heads, dk, dv, x0.device)
+        with lent((max(nbytes, 16),), torch.uint8, x0.device) as scratch:
+            rc = lib("delta_rule").kvb_delta_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(singles),
+                                                  c_int(T), _p(scratch if nbytes else None), _stream())
         _check(rc, "delta_scan")
-        launch_count += 1
+        launch_count += 3 if nbytes else 1
+        choices["delta_pieces"] += 1 if nbytes else 0
         choices["delta_scan_" + mode] += 1
         choices["delta_walk"] += 1
         return out

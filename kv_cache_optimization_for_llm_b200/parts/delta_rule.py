@@ -222,7 +222,8 @@ class GatedDelta(Part):
 
     def activation_widths(self):
         hv = self.heads * self.vdim
-        return [self.w_in.shape[0], self.channels, hv, 3 * hv, self.o.shape[0]]
+        pieces = ops.delta_pieces_width(self.heads, self.dim, self.vdim) if self.ctx.dtype == torch.bfloat16 else 0
+        return [self.w_in.shape[0], self.channels, hv, 3 * hv, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):
         p = ops.linear(x, self.w_in)
