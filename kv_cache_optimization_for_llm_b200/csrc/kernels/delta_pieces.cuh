@@ -14,8 +14,10 @@
 // block of 16 added up by float32 instructions.  What is not finite is left out of them in the same way (first tokens of a piece whose
 // key, gate or value is not finite are recorded, and results from such a token on, and the state, become NaNs at the end).
 //
-// What bounds it: the chain's products on mma.sync and its two barriers a piece; the other two fill the GPU.
-// MEASURED
+// What bounds it: the chain takes about 4300 cycles a piece of 32 columns (two barriers, and between them every warp's loads from shared
+// memory, then every warp's products); the other two are latency, four blocks an SM.  32 heads of 64 x 64, runs of 1548 + 500 tokens: prepare
+// 46, chain 56, results 31 us, the walk in one launch 206.  (A chain without barriers, a warp for 16 columns of the transposed state as a
+// left operand in registers: 70 us, since one warp issues a product in 18 cycles however many are independent.)
 #pragma once
 
 #include "delta_walk.cuh"
@@ -57,15 +59,20 @@ __device__ __forceinline__ int pieces_before(const Args& p, int r) {
 }
 
 struct PrepareLayout {
-  static constexpr int PN = pitch(kN), PT = pitch(kPiece), PD = 20;
+  // Four blocks an SM: of T and A the 16 x 16 blocks on and below the diagonal only, and the values wait in registers until A is done
+  // with.  A block's rows are 48 bytes apart, so that eight of them lie in different banks.
+  static constexpr int PN = pitch(kN), PT = pitch(kPiece), PB = 48, PD = 20, PV = pitch(64);
+  static constexpr int BLOCK = 16 * PB;
   static constexpr int K = 0;                                     // [64] rows of PN
-  static constexpr int T = K + kPiece * PN;                       // [3][64] rows of PT: the inverse
-  static constexpr int A = T + 3 * kPiece * PT;                   // [3][64] rows of PT: A left of its diagonal blocks, then W
-  static constexpr int D = A + 3 * kPiece * PT;                   // [4][16] columns of PD floats
+  static constexpr int T = K + kPiece * PN;                       // [3][10] blocks: the inverse, block (I, J) at I (I + 1) / 2 + J
+  static constexpr int A = T + 3 * 10 * BLOCK;                    // [3][6] blocks: A below its diagonal blocks, (I, J) at I (I - 1) / 2 + J
+  static constexpr int V = A;                                     // behind A: [64] rows of PV
+  static constexpr int W = T;                                     // behind all of these: [3][64] rows of PT
+  static constexpr int D = A + 3 * 6 * BLOCK;                     // [4][16] columns of PD floats
+  static_assert(kPiece * PV <= 3 * 6 * BLOCK && 3 * kPiece * PT <= 3 * 16 * BLOCK, "what comes later fits what was there");
   static constexpr int G = D + 4 * 16 * PD * 4;
   static constexpr int F = G + (int)sizeof(Gates);                // [1 + Dv]
-  static constexpr int V = (F + (1 + 256) * 4 + 15) / 16 * 16;    // [64] rows of pitch(Dv)
-  static int bytes(int Dv) { return V + kPiece * pitch(Dv); }
+  static constexpr int bytes = F + (1 + 64) * 4;
 };
 
 __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, int R, const Scratch sc) {
@@ -82,7 +89,6 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
   if (!find_piece(p, R, blockIdx.y, r, local)) return;
   const size_t unit = (size_t)blockIdx.y * p.H + h;
   const int c0 = p.q_start[r] + local * kPiece, t1 = p.q_start[r + 1];
-  const int PV = pitch(p.Dv);
   for (int i = tid; i < 1 + p.Dv; i += kWalkers + 32) spoilt[i] = kNoToken;
   unsigned char* Ks = sm + L::K;
   unsigned char* Ts = sm + L::T;
@@ -129,21 +135,25 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
     return;
   }
   const int ht = tid, hw = warp;
+  uint4 values[4];
   {
     const bf16* k = p.k + (size_t)(h / p.share) * kN;
     const bf16* v = p.v + (size_t)h * p.Dv;
-    const int chunks = kN / 8, vchunks = p.Dv / 8;
+    const int chunks = kN / 8;
     for (int x = ht; x < kPiece * chunks; x += kWalkers) {
       const int i = x / chunks, c = x - i * chunks;
       const bool in = c0 + i < t1;
       copy16(Ks + i * L::PN + c * 16, k + (size_t)(in ? c0 + i : c0) * p.ld_k + c * 8, in);
     }
-    for (int x = ht; x < kPiece * vchunks; x += kWalkers) {
-      const int i = x / vchunks, c = x - i * vchunks;
-      const bool in = c0 + i < t1;
-      copy16(sm + L::V + i * PV + c * 16, v + (size_t)(in ? c0 + i : c0) * p.ld_v + c * 8, in);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // two threads a row of values: this one's chunks 4 (ht & 1) ..
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = ht >> 1, at = (ht & 1) * 4 + c;
+      values[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (c0 + i < t1 && at * 8 < p.Dv) values[c] = *reinterpret_cast<const uint4*>(v + (size_t)(c0 + i) * p.ld_v + at * 8);
     }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
   bar<3, kWalkers + 32>();
   // norms of the keys, values that are not finite: two threads a row
@@ -172,15 +182,18 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
     const float inv = 1.0f / sqrtf(sum + 1e-6f);
     g.kinv[ht] = inv;
     g.weigh[ht] *= inv;
-  } else {
-    unsigned char* from = sm + L::V + (ht - 64) * PV;
-    for (int c = 0; c < p.Dv / 2; ++c) {
-      uint32_t* at = reinterpret_cast<uint32_t*>(from) + c;
-      const uint32_t two = *at, bad = not_finite(two);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(values + c);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t bad = not_finite(w[e]);
       if (bad) {
-        if (bad & 0x8000u) atomicMin(spoilt + 1 + 2 * c, ht - 64);
-        if (bad & 0x80000000u) atomicMin(spoilt + 2 + 2 * c, ht - 64);
-        *at = finite_part(two);
+        const int at = 1 + ((ht & 1) * 4 + c) * 8 + 2 * e;
+        if (bad & 0x8000u) atomicMin(spoilt + at, ht >> 1);
+        if (bad & 0x80000000u) atomicMin(spoilt + at + 1, ht >> 1);
+        w[e] = finite_part(w[e]);
       }
     }
   }
@@ -224,11 +237,11 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
           uint32_t up[3], low[3];
           split3(up, G[x][0], G[x][1]);
           split3(low, G[x][2], G[x][3]);
-          unsigned char* to = sm + L::A + row * L::PT + j * 2;
+          unsigned char* to = sm + L::A + (hw * (hw - 1) / 2 + x / 2) * L::BLOCK + gq * L::PB + (j & 15) * 2;
 #pragma unroll
           for (int u = 0; u < 3; ++u) {
-            *reinterpret_cast<uint32_t*>(to + u * kPiece * L::PT) = up[u];
-            *reinterpret_cast<uint32_t*>(to + (u * kPiece + 8) * L::PT) = low[u];
+            *reinterpret_cast<uint32_t*>(to + u * 6 * L::BLOCK) = up[u];
+            *reinterpret_cast<uint32_t*>(to + u * 6 * L::BLOCK + 8 * L::PB) = low[u];
           }
         } else {
 #pragma unroll
@@ -272,15 +285,15 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
       split3(part, odd ? other : mine, odd ? mine : other);
 #pragma unroll
       for (int u = 0; u < 3; ++u)
-        *reinterpret_cast<uint32_t*>(Ts + (u * kPiece + hw * 16 + 2 * (e + odd) + par) * L::PT + (hw * 16 + (lane >> 1 & ~1)) * 2) = part[u];
+        *reinterpret_cast<uint32_t*>(Ts + (u * 10 + hw * (hw + 3) / 2) * L::BLOCK + (2 * (e + odd) + par) * L::PB + (lane >> 1 & ~1) * 2) = part[u];
     }
   }
   bar<2, kWalkers>();
   {                                                // the blocks below it (as in the walk)
-    auto mma6t = [&](float (*acc)[4], const uint32_t (*left)[4], const unsigned char* from) {
+    auto mma6t = [&](float (*acc)[4], const uint32_t (*left)[4], const unsigned char* from, int part) {
       uint32_t f[3][4];
 #pragma unroll
-      for (int u = 0; u < 3; ++u) ldm4(f[u], from + (u * kPiece + (lane & 7) + (lane >> 4) * 8) * L::PT + (lane >> 3 & 1) * 16);
+      for (int u = 0; u < 3; ++u) ldm4(f[u], from + u * part + ((lane & 7) + (lane >> 4) * 8) * L::PB + (lane >> 3 & 1) * 16);
       float t[2][4];
       mma0(t[0], left[2], f[0][0], f[0][1]);
       mma0(t[1], left[2], f[0][2], f[0][3]);
@@ -296,34 +309,37 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
     uint32_t left[3][3][4];
 #pragma unroll
     for (int u = 0; u < 3; ++u)
-      ldm4t(left[0][u], Ts + (u * kPiece + hw * 16 + (lane & 7) + (lane >> 4) * 8) * L::PT + (hw * 2 + (lane >> 3 & 1)) * 16);
+      ldm4t(left[0][u], Ts + (u * 10 + hw * (hw + 3) / 2) * L::BLOCK + ((lane & 7) + (lane >> 4) * 8) * L::PB + (lane >> 3 & 1) * 16);
 #pragma unroll
     for (int d = 1; d < 4; ++d)
       if (hw + d < 4) {
         const int I = hw + d;
         float X[2][4] = {}, Y[2][4] = {};
 #pragma unroll
-        for (int e = 0; e < d; ++e) mma6t(X, left[e], sm + L::A + I * 16 * L::PT + (hw + e) * 32);
+        for (int e = 0; e < d; ++e) mma6t(X, left[e], sm + L::A + (I * (I - 1) / 2 + hw + e) * L::BLOCK, 6 * L::BLOCK);
         uint32_t x[3][4], y[3][4];
         left_parts(x, X, 1.f);
-        mma6t(Y, x, Ts + I * 16 * L::PT + I * 32);
+        mma6t(Y, x, Ts + I * (I + 3) / 2 * L::BLOCK, 10 * L::BLOCK);
         left_parts(y, Y, -1.f);
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
-          stm4t(y[u], Ts + (u * kPiece + I * 16 + (lane & 7) + (lane >> 4) * 8) * L::PT + (hw * 2 + (lane >> 3 & 1)) * 16);
+          stm4t(y[u], Ts + (u * 10 + I * (I + 1) / 2 + hw) * L::BLOCK + ((lane & 7) + (lane >> 4) * 8) * L::PB + (lane >> 3 & 1) * 16);
           if (d < 3)
 #pragma unroll
             for (int e = 0; e < 4; ++e) left[d][u][e] = y[u][e];
         }
       }
   }
-  bar<2, kWalkers>();                              // T is whole, A is free
+  bar<2, kWalkers>();                              // T is whole, A is done with
+#pragma unroll
+  for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sm + L::V + (ht >> 1) * L::PV + ((ht & 1) * 4 + c) * 16) = values[c];
+  bar<2, kWalkers>();
   // Row blocks 0 and 3 hold five blocks of T between them, 1 and 2 as well: warp w takes the rows of block w for the even pairs of
   // columns and of block 3 - w for the odd ones.
   auto scaled = [&](uint32_t (*a)[4], int rb, int jt, bool keys) {      // block (rb, jt) of T, column j times beta_j (and P_j / |k_j|)
     uint32_t b[3][4];
 #pragma unroll
-    for (int u = 0; u < 3; ++u) ldm4(b[u], Ts + (u * kPiece + rb * 16 + (lane & 15)) * L::PT + (jt * 2 + (lane >> 4)) * 16);
+    for (int u = 0; u < 3; ++u) ldm4(b[u], Ts + (u * 10 + rb * (rb + 1) / 2 + jt) * L::BLOCK + (lane & 15) * L::PB + (lane >> 4) * 16);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int j = jt * 16 + (e >> 1) * 8 + 2 * tq;
@@ -337,12 +353,12 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
       for (int u = 0; u < 3; ++u) a[u][e] = part[u];
     }
   };
-  // acc[8 columns 2 np, 2 np + 1] of rows 16 rb .. of (scaled T) * (rows of `from`, bfloat16)
+  float W[2][2][2][4];                             // [turn][pair of 16 columns][8 columns]
 #pragma unroll
   for (int turn = 0; turn < 2; ++turn) {
     const int rb = turn ? 3 - hw : hw;
     const int row = rb * 16 + gq;
-    float acc[2][2][4];
+    float (*acc)[2][4] = W[turn];
 #pragma unroll
     for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -366,59 +382,62 @@ __global__ void __launch_bounds__(kWalkers + 32) prepare_kernel(const Args p, in
         add4(acc[x][1], t[1]);
       }
     }
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int col = (2 * (2 * x + turn) + y) * 8 + 2 * tq;
-        uint32_t up[3], low[3];
-        split3(up, acc[x][y][0], acc[x][y][1]);
-        split3(low, acc[x][y][2], acc[x][y][3]);
-        unsigned char* to = sm + L::A + row * L::PT + col * 2;
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          *reinterpret_cast<uint32_t*>(to + u * kPiece * L::PT) = up[u];
-          *reinterpret_cast<uint32_t*>(to + (u * kPiece + 8) * L::PT) = low[u];
-        }
-      }
-    // U0, two times 16 columns a time
-    for (int np0 = turn; np0 < p.Dv / 16; np0 += 4) {
-      float d[2][2][4] = {};
-      for (int jt = 0; jt <= rb; ++jt) {
-        uint32_t a[3][4];
-        scaled(a, rb, jt, false);
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (np0 + 2 * x < p.Dv / 16) {
-            uint32_t f[4];
-            ldm4t(f, sm + L::V + (jt * 16 + (lane & 15)) * PV + ((np0 + 2 * x) * 2 + (lane >> 4)) * 16);
-            float t[2][4];
-            mma0(t[0], a[2], f[0], f[1]);
-            mma0(t[1], a[2], f[2], f[3]);
-            mma(t[0], a[1], f[0], f[1]);
-            mma(t[1], a[1], f[2], f[3]);
-            mma(t[0], a[0], f[0], f[1]);
-            mma(t[1], a[0], f[2], f[3]);
-            add4(d[x][0], t[0]);
-            add4(d[x][1], t[1]);
-          }
-      }
+    // U0, two times 16 columns
+    float d[2][2][4] = {};
+    for (int jt = 0; jt <= rb; ++jt) {
+      uint32_t a[3][4];
+      scaled(a, rb, jt, false);
 #pragma unroll
       for (int x = 0; x < 2; ++x)
-        if (np0 + 2 * x < p.Dv / 16) {
-          float* to = sc.u + (unit * kPiece + row) * p.Dv + (np0 + 2 * x) * 16 + 2 * tq;
-#pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            *reinterpret_cast<float2*>(to + 8 * y) = make_float2(d[x][y][0], d[x][y][1]);
-            *reinterpret_cast<float2*>(to + (size_t)8 * p.Dv + 8 * y) = make_float2(d[x][y][2], d[x][y][3]);
-          }
+        if (turn + 2 * x < p.Dv / 16) {
+          uint32_t f[4];
+          ldm4t(f, sm + L::V + (jt * 16 + (lane & 15)) * L::PV + ((turn + 2 * x) * 2 + (lane >> 4)) * 16);
+          float t[2][4];
+          mma0(t[0], a[2], f[0], f[1]);
+          mma0(t[1], a[2], f[2], f[3]);
+          mma(t[0], a[1], f[0], f[1]);
+          mma(t[1], a[1], f[2], f[3]);
+          mma(t[0], a[0], f[0], f[1]);
+          mma(t[1], a[0], f[2], f[3]);
+          add4(d[x][0], t[0]);
+          add4(d[x][1], t[1]);
         }
     }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+      if (turn + 2 * x < p.Dv / 16) {
+        float* to = sc.u + (unit * kPiece + row) * p.Dv + (turn + 2 * x) * 16 + 2 * tq;
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          *reinterpret_cast<float2*>(to + 8 * y) = make_float2(d[x][y][0], d[x][y][1]);
+          *reinterpret_cast<float2*>(to + (size_t)8 * p.Dv + 8 * y) = make_float2(d[x][y][2], d[x][y][3]);
+        }
+      }
+  }
+  bar<2, kWalkers>();                              // nobody reads T any more
+#pragma unroll
+  for (int turn = 0; turn < 2; ++turn) {
+    const int row = (turn ? 3 - hw : hw) * 16 + gq;
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int col = (2 * (2 * x + turn) + y) * 8 + 2 * tq;
+          uint32_t up[3], low[3];
+          split3(up, W[turn][x][y][0], W[turn][x][y][1]);
+          split3(low, W[turn][x][y][2], W[turn][x][y][3]);
+          unsigned char* to = sm + L::W + row * L::PT + col * 2;
+#pragma unroll
+          for (int u = 0; u < 3; ++u) {
+            *reinterpret_cast<uint32_t*>(to + u * kPiece * L::PT) = up[u];
+            *reinterpret_cast<uint32_t*>(to + (u * kPiece + 8) * L::PT) = low[u];
+          }
+        }
   }
   bar<2, kWalkers>();
   bf16* wg = sc.w + unit * 3 * kPiece * kN;
   for (int x = ht; x < 3 * kPiece * (kN / 8); x += kWalkers)
-    *reinterpret_cast<uint4*>(wg + x * 8) = *reinterpret_cast<const uint4*>(sm + L::A + (x / 8) * L::PT + (x % 8) * 16);
+    *reinterpret_cast<uint4*>(wg + x * 8) = *reinterpret_cast<const uint4*>(sm + L::W + (x / 8) * L::PT + (x % 8) * 16);
   for (int x = ht; x < (int)sizeof(Gates) / 16; x += kWalkers)
     reinterpret_cast<uint4*>(sc.gates + unit)[x] = reinterpret_cast<const uint4*>(&g)[x];
   for (int x = ht; x < 1 + p.Dv; x += kWalkers) sc.spoilt[unit * (1 + p.Dv) + x] = spoilt[x];
@@ -640,24 +659,21 @@ __global__ void __launch_bounds__(kWalkers) results_kernel(const Args p, int R, 
     asm volatile("cp.async.commit_group;" ::: "memory");
     // the state and the corrections, in parts
     const float* from[2] = {sc.s + unit * kN * p.Dv + col0, sc.u + unit * kPiece * p.Dv + col0};
+    float4 v[8];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      float4 v[4];
+    for (int i = 0; i < 8; ++i) {
+      const int x = tid + (i & 3) * kWalkers;
+      v[i] = *reinterpret_cast<const float4*>(from[i >> 2] + (size_t)(x >> 3) * p.Dv + (x & 7) * 4);
+    }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int x = tid + i * kWalkers;
-        v[i] = *reinterpret_cast<const float4*>(from[m] + (size_t)(x >> 3) * p.Dv + (x & 7) * 4);
-      }
+    for (int i = 0; i < 8; ++i) {
+      const int x = tid + (i & 3) * kWalkers;
+      uint32_t lo[3], hi[3];
+      split3(lo, v[i].x, v[i].y);
+      split3(hi, v[i].z, v[i].w);
+      unsigned char* to = sm + (i >> 2 ? L::U : L::S) + (x >> 3) * L::PX + (x & 7) * 8;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int x = tid + i * kWalkers;
-        uint32_t lo[3], hi[3];
-        split3(lo, v[i].x, v[i].y);
-        split3(hi, v[i].z, v[i].w);
-        unsigned char* to = sm + (m ? L::U : L::S) + (x >> 3) * L::PX + (x & 7) * 8;
-#pragma unroll
-        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(to + s * kPiece * L::PX) = make_uint2(lo[s], hi[s]);
-      }
+      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(to + s * kPiece * L::PX) = make_uint2(lo[s], hi[s]);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
@@ -804,7 +820,7 @@ static long long scratch_bytes(long long tokens, int R, int H, int Dv) {
   return units * (3ll * kPiece * kN * 2 + 2ll * kPiece * Dv * 4 + (long long)sizeof(Gates) + (1 + Dv) * 4) + 64;
 }
 
-static bool takes_pieces(const Args& a, int N) { return N == kN && a.Dv <= 256 && delta_walk::takes(a, N); }
+static bool takes_pieces(const Args& a, int N) { return N == kN && a.Dv <= 64 && delta_walk::takes(a, N); }
 
 static int launch(const Args& a, int R, long long tokens, void* scratch, cudaStream_t stream) {
   const long long pieces = tokens / kPiece + R, units = pieces * a.H;
@@ -817,7 +833,7 @@ static int launch(const Args& a, int R, long long tokens, void* scratch, cudaStr
   sc.s = sc.u + units * kPiece * a.Dv;
   sc.gates = reinterpret_cast<Gates*>(sc.s + units * kPiece * a.Dv);
   sc.spoilt = reinterpret_cast<int*>(sc.gates + units);
-  const int prep = PrepareLayout::bytes(a.Dv);
+  constexpr int prep = PrepareLayout::bytes;
   cudaError_t e = cudaFuncSetAttribute(prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
   if (e == cudaSuccess) e = kvb_launch(prepare_kernel, dim3((unsigned)a.H, (unsigned)pieces), dim3(kWalkers + 32), prep, stream, a, R, sc);
   if (e != cudaSuccess) return (int)e;

@@ -373,7 +373,7 @@ KVB_EXPORT int kvb_delta_scan(const DeltaArgs* args, int mode, int R, int T_, in
 // Bytes of scratch with which kvb_delta_walk takes the form in three launches (delta_pieces.cuh) for `tokens` tokens in R runs, 0
 // where the sizes are not its own.
 KVB_EXPORT long long kvb_delta_walk_scratch(long long tokens, int R, int H, int Dk, int Dv) {
-  return Dk == delta_pieces::kN && Dv % 32 == 0 && Dv >= 32 && Dv <= 256 ? delta_pieces::scratch_bytes(tokens, R, H, Dv) : 0;
+  return Dk == delta_pieces::kN && (Dv == 32 || Dv == 64) ? delta_pieces::scratch_bytes(tokens, R, H, Dv) : 0;
 }
 
 // The runs of requests first .. first + R - 1 (token rows row0 .. T_ - 1) walked in pieces of 64 tokens on tensor cores

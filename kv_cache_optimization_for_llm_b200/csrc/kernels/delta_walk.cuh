@@ -27,7 +27,7 @@
 // What bounds it: latency, about 10500 cycles a piece, for walkers (three steps of products with a barrier behind each) and helpers
 // (rows, norms, A, its inverse) alike.  Walking token by token in float32 is a chain of 64 steps of two dot products each: 32 heads
 // of 64 x 64, runs of 1548 + 500 tokens 474 us, now 197 (176 with all sums in one chain of accumulations; twice that with the whole inverse by
-// elimination).
+// elimination).  Long runs of keys of 64 take three launches instead: delta_pieces.cuh.
 #pragma once
 
 #include "chunk_walk.cuh"

@@ -463,13 +463,14 @@ def _at(t: torch.Tensor, col: int) -> int:
 
 
 # Longest run of a step, in tokens, from which on the walk's products that do not wait for the state are made for all pieces at once
-# (delta_pieces.cuh; keys of 64).
-DELTA_PIECES_MIN_RUN = 128
+# (delta_pieces.cuh; keys of 64, values of 32 or 64).  32 heads, the launches of either form in us (three / one): a run of 64 24 / 12, of 400
+# about 35 / 48, of 1024 79 / 110, 1548 + 500 134 / 206; the host pays for two launches more (7 us a layer), which shows in steps below.
+DELTA_PIECES_MIN_RUN = 512
 
 
 def delta_pieces_width(heads: int, dk: int, dv: int) -> int:
     """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs."""
-    if dk != 64 or dv % 32 or not 32 <= dv <= 256:
+    if dk != 64 or dv not in (32, 64):
         return 0
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong
@@ -479,7 +480,7 @@ def delta_pieces_width(heads: int, dk: int, dv: int) -> int:
 def _delta_pieces_bytes(batch, tokens: int, heads: int, dk: int, dv: int, device) -> int:
     """Bytes of scratch for the form in three launches, 0 where the runs walk in one (short runs, other sizes, or an arena without the
     room)."""
-    if dk != 64 or int(getattr(batch, "max_q_len", 0) or 0) < DELTA_PIECES_MIN_RUN:
+    if dk != 64 or dv not in (32, 64) or int(getattr(batch, "max_q_len", 0) or 0) < DELTA_PIECES_MIN_RUN:
         return 0
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong

@@ -20,7 +20,7 @@ def form(request, monkeypatch):
 
 @pytest.mark.parametrize("alike", [False, True])
 @pytest.mark.parametrize("steps", W.STEPS)
-@pytest.mark.parametrize("H,G,N,Dv", [(2, 1, 64, 32), (4, 4, 64, 64), (3, 3, 64, 96), (64, 16, 64, 64), (2, 1, 64, 256)])
+@pytest.mark.parametrize("H,G,N,Dv", [(2, 1, 64, 32), (4, 4, 64, 64), (3, 3, 64, 32), (64, 16, 64, 64)])
 def test_delta_walk_in_both_forms(form, steps, H, G, N, Dv, alike):
     W.test_delta_walk(steps, H, G, N, Dv, alike)
 
@@ -35,3 +35,12 @@ def test_long_runs_in_both_forms(form, slow):
 @pytest.mark.parametrize("at", [0, 63, 64, 130])
 def test_what_is_not_finite_in_both_forms(form, what, bad, at):
     W.test_what_is_not_finite_stays_behind_its_token("delta", what, bad, at)
+
+
+@pytest.mark.parametrize("N,Dv", [(64, 96), (64, 256), (128, 32)])
+def test_other_sizes_stay_with_the_walk_in_one_launch(N, Dv, monkeypatch):
+    from kv_cache_optimization_for_llm_b200 import ops
+    monkeypatch.setattr(ops, "DELTA_PIECES_MIN_RUN", 1)
+    before = ops.choices["delta_pieces"]
+    W.test_delta_walk(W.STEPS[2], 2, 1, N, Dv, False)
+    assert ops.choices["delta_pieces"] == before
