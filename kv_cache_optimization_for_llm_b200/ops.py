@@ -2317,7 +2317,7 @@ def tiles_of_height(batch, nt: int) -> torch.Tensor:
 
 def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window,
                     wide: Optional[bool] = None, skip_single: bool = False,
-                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                    out: Optional[torch.Tensor] = None, open_late: bool = False) -> torch.Tensor:
     """Tensor-core attention for steps with runs of query tokens (bfloat16).  ``wide``:
     False: 64 query rows per block (mma.sync); True: 128 rows (mma.sync); 2: 128 rows on
     tcgen05 with the scores in tensor memory (head size 64); 3: the same with roles (a TMA
@@ -2325,7 +2325,8 @@ def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale
     8 rows); None:
     chosen from the step's size, the head size and the page size.  ``skip_single``: the step's
     leading single tokens (``batch.num_single``) are somebody else's: their tiles are left out.
-    ``out``: where the rows go; made here if not given."""
+    ``out``: where the rows go; made here if not given.  ``open_late``: the next launch is a
+    :func:`decode_attention_mma` with ``beside``."""
     _need_cuda(qkv, k_pages)
     skip = int(batch.num_single) if skip_single else 0
     T = qkv.shape[0] - skip
@@ -2342,13 +2343,14 @@ def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale
             elif d == 64:
                 wide = 2
     tiles = flash_tiles(batch, nq // nkv, wide)[skip:]      # a single token is one tile, and they come first
+    assert tiles.shape[0] > 0 or not open_late      # the next launch counts on this one's being there
     if out is None:
         out = new((qkv.shape[0], nq * d), qkv.dtype, qkv.device)
     rc = lib("flash_attention").kvb_paged_flash_attention(
         _p(qkv), c_int(qkv.stride(0)), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]),
         c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), _p(batch.positions), _p(tiles), c_int(tiles.shape[0]),
-        c_int(int(wide)), _p(out), c_int(nq), c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)), _p(batch.status),
-        _stream())
+        c_int(int(wide)), _p(out), c_int(nq), c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)),
+        c_int(1 if open_late else 0), _p(batch.status), _stream())
     _check(rc, "paged_flash_attention")
     choices[f"flash_attention_{int(wide)}"] += 1
     return out
@@ -2406,7 +2408,8 @@ def decode_launch_context(batch) -> int:
 
 def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, ctx_len, cos, sin, rot,
                          nq, nkv, d, scale, window, status, max_ctx: int = 0,
-                         trace: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                         trace: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+                         beside: bool = False) -> torch.Tensor:
     """The attention of a bfloat16 decode step in one launch on tensor cores: rotary
     encoding of query and new key, cache write, attention over 128-key tiles spread over
     a cluster of blocks, merge through distributed shared memory.  No scratch.
@@ -2414,7 +2417,8 @@ def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, 
     size 64), whatever the batch; up to that many blocks share a (request, kv head).
     ``max_ctx``: the longest context of the step if the host knows it (the launch is sized
     for it), 0 otherwise.  ``out``: where the rows go ([tokens, nq d], the rows of the requests'
-    tokens are written); made here if not given."""
+    tokens are written); made here if not given.  ``beside``: the launch in front, with ``open_late``, has
+    none of these requests: the two run side by side."""
     _need_cuda(qkv, k_pages)
     assert qkv.dtype == torch.bfloat16
     R = ctx_len.numel()
@@ -2425,7 +2429,7 @@ def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, 
         c_int(block_table.shape[1]), c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), _p(q_start), _p(ctx_len),
         _p(cos), _p(sin), c_int(0 if cos is None else cos.shape[0]), c_int(rot), _p(out), c_int(R), c_int(nq),
         c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)), c_int(int(max_ctx)),
-        _p(status), _p(trace), _stream())
+        c_int(1 if beside else 0), _p(status), _p(trace), _stream())
     _check(rc, "decode_attention_mma")
     choices["decode_attention_mma"] += 1
     return out
@@ -2468,14 +2472,17 @@ def attention_step(qkv, k_pages, v_pages, write_kv, block_table, batch, nq, nkv,
         # Single tokens beside runs: the single tokens (the step's first rows) go to the kernel of
         # decode steps, which rotates, writes and attends in one launch, the runs to the two kernels
         # for runs.  As a tile of the kernel for runs a single token would fill 4 of 128 rows.
+        # The two kernels share no row, page or output and run side by side, the runs' blocks first: they are
+        # bound by latency and products, the single tokens' by the latency of short walks and by reading the cache (24 heads of
+        # 128, 40 tokens of 100 to 2500 positions beside a run of 701 behind 512: 101 -> 82 us).
         out = new((qkv.shape[0], nq * d), qkv.dtype, qkv.device)
-        decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table[:ns], batch.q_start[:ns + 1], batch.ctx_len[:ns],
-                             cos, sin, rot, nq, nkv, d, scale, window, batch.status,
-                             max_ctx=decode_launch_context(batch), out=out)
         rope_kv_write(qkv[ns:], batch.positions[ns:], batch.token_req[ns:], cos, sin, k_pages if write_kv else None,
                       v_pages if write_kv else None, block_table, page_size, nq, nkv, d, rot, batch.status)
-        return flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window,
-                               skip_single=True, out=out)
+        flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window,
+                        skip_single=True, out=out, open_late=True)
+        return decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table[:ns], batch.q_start[:ns + 1],
+                                    batch.ctx_len[:ns], cos, sin, rot, nq, nkv, d, scale, window, batch.status,
+                                    max_ctx=decode_launch_context(batch), out=out, beside=True)
     rope_kv_write(qkv, batch.positions, batch.token_req, cos, sin, k_pages if write_kv else None,
                   v_pages if write_kv else None, block_table, page_size, nq, nkv, d, rot, batch.status)
     if qkv.dtype == torch.bfloat16 and not batch.decode_only and flash_attention_supported(d, group, page_size):
