@@ -469,22 +469,22 @@ template <> struct Vec16<__nv_bfloat16> {
   static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* x) { *reinterpret_cast<uint4*>(p) = pack_bf16x8(x); }
 };
 
-// Channels c .. c + VEC - 1 of a token, at or behind k_off, into the request's page.
+// Where channel c of a token, at or behind k_off, lies in the request's page; null for a channel or a page that is not there.
 template <typename T>
-__device__ __forceinline__ void append_row(const AppendArgs& ap, int c, int r, int pos, const float* acc) {
+__device__ __forceinline__ T* append_at(const AppendArgs& ap, int c, int r, int pos) {
   const bool is_v = c >= ap.v_off;
   const int width = is_v ? ap.Dv : ap.Dk;
   const int rel = c - (is_v ? ap.v_off : ap.k_off);
   const int g = rel / width, i = rel - g * width;
-  if (g >= ap.kv_heads) return;
+  if (g >= ap.kv_heads) return nullptr;
   const int lp = pos / ap.page_size;
   const int page = lp < ap.max_pages ? ap.block_table[(size_t)r * ap.max_pages + lp] : -1;
   if (page < 0 || page >= ap.num_pages) {
     atomicCAS(ap.status, 0, KVB_STATUS_UNMAPPED_PAGE);
-    return;
+    return nullptr;
   }
   T* row = static_cast<T*>(ap.pages) + (((size_t)page * ap.kv_heads + g) * ap.page_size + (pos % ap.page_size)) * (ap.Dk + ap.Dv);
-  Vec16<T>::store(row + (is_v ? ap.Dk : 0) + i, acc);
+  return row + (is_v ? ap.Dk : 0) + i;
 }
 
 // TAPS > 0: the number of taps, known when the kernel is built; the thread's VEC x TAPS weights are then fetched with
@@ -571,22 +571,48 @@ __global__ void conv_vec_kernel(const T* __restrict__ in, int ld, const float* _
     for (int e = 0; e < VEC; ++e) acc[e] = acc[e] / (1.0f + expf(-acc[e]));
   }
   Vec16<T>::store(out + (size_t)t * C + c, acc);
-  if (ap.pages != nullptr && c >= ap.k_off) append_row<T>(ap, c, r, pos, acc);
+  if (ap.pages != nullptr && c >= ap.k_off) {
+    T* to = append_at<T>(ap, c, r, pos);
+    if (to != nullptr) Vec16<T>::store(to, acc);
+  }
 }
 
-// The same for long steps: a thread takes VEC channels of kConvTokens consecutive token rows, so that the weights are fetched once and every
-// input once (the window moves through registers).  What bounds it: bytes (2048 tokens of 6144 channels in bfloat16: 50 MB).  With a
-// token a thread the weights, 16 bytes a channel, came from the caches again for every token, and every input four times: 75 us; now 39
-// (four tokens a thread: 40; eight without the limit to 128 registers: 52; 2048 tokens of 3072 channels 39, now 26).
+// Four channels of a row as they lie in memory.
+template <typename T> struct Quad;
+template <> struct Quad<float> {
+  using Raw = uint4;
+  static __device__ __forceinline__ void unpack(Raw u, float* x) { Vec16<float>::unpack(u, x); }
+  static __device__ __forceinline__ Raw pack(const float* x) {
+    return make_uint4(__float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+  }
+};
+template <> struct Quad<__nv_bfloat16> {
+  using Raw = uint2;
+  static __device__ __forceinline__ void unpack(Raw u, float* x) {
+    x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
+    x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
+  }
+  static __device__ __forceinline__ Raw pack(const float* x) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(x[0], x[1]), b = __floats2bfloat162_rn(x[2], x[3]);
+    return make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+  }
+};
+
+// The same for long steps: a thread takes four channels of kConvTokens consecutive token rows, so that the weights are fetched once and
+// every input once (the window moves through registers).  What bounds it: bytes (2048 tokens of 6144 channels in bfloat16: 50 MB, 8 us)
+// and, before that, instructions.  Rows whose window lies in one request, nearly all, need no look at requests and positions; four
+// channels a thread (8-byte loads) leave room for twice the threads that eight did.  In a layer 2048 tokens of 6144 channels 39 -> 27 us, of
+// 3072 channels 26 -> 17.  Four blocks an SM (64 registers) would spill.
 constexpr int kConvTokens = 8;
 
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2)
 conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, const float* __restrict__ tails, long long slot_stride,
                 T* __restrict__ out, int C, int T_, const int* __restrict__ positions, const int* __restrict__ token_req,
                 const int* __restrict__ req_start, const int* __restrict__ slots, int act, AppendArgs ap,
                 const float* __restrict__ in_bias, const float* __restrict__ out_bias) {
-  constexpr int VEC = Vec16<T>::N, BACK = TAPS - 1;
+  constexpr int VEC = 4, BACK = TAPS - 1;
+  using Raw = typename Quad<T>::Raw;
   pdl_trigger();
   pdl_wait();
   const int groups = C / VEC;
@@ -594,15 +620,13 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
   const int block = (int)(idx / groups), c = (int)(idx - (long long)block * groups) * VEC;
   const int t0 = block * kConvTokens;
   if (t0 >= T_) return;
-  uint4 x[kConvTokens + BACK];                 // rows t0 - BACK .. as they lie in memory
-  int req[kConvTokens + BACK];
+  const int t_last = min(t0 + kConvTokens, T_) - 1;
+  // rows t0 - BACK .. t0 + kConvTokens - 1 as they lie in memory (rows outside the step: the nearest one, not used)
+  Raw x[kConvTokens + BACK];
 #pragma unroll
-  for (int i = 0; i < kConvTokens + BACK; ++i) {
-    const int t = t0 - BACK + i;
-    const bool in_step = t >= 0 && t < T_;
-    x[i] = in_step ? *reinterpret_cast<const uint4*>(in + (size_t)t * ld + c) : make_uint4(0u, 0u, 0u, 0u);
-    req[i] = in_step ? token_req[t] : -1;
-  }
+  for (int i = 0; i < kConvTokens + BACK; ++i)
+    x[i] = *reinterpret_cast<const Raw*>(in + (size_t)min(max(t0 - BACK + i, 0), t_last) * ld + c);
+  const int first = token_req[max(t0 - BACK, 0)], last = token_req[t_last];
   float wv[VEC * TAPS], ob[VEC], ib[VEC];
 #pragma unroll
   for (int i = 0; i < VEC * TAPS; i += 4) {
@@ -614,11 +638,48 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
     ob[e] = out_bias ? out_bias[c + e] : 0.f;
     ib[e] = in_bias ? in_bias[c + e] : 0.f;
   }
+  auto finish = [&](int t, float* acc) {
+    if (act == 0) {
 #pragma unroll
-  for (int k = 0; k < kConvTokens; ++k) {
-    const int t = t0 + k;
-    if (t >= T_) break;
-    const int r = req[k + BACK], pos = positions[t];
+      for (int e = 0; e < VEC; ++e) acc[e] = acc[e] / (1.0f + expf(-acc[e]));
+    }
+    const Raw y = Quad<T>::pack(acc);
+    *reinterpret_cast<Raw*>(out + (size_t)t * C + c) = y;
+    if (ap.pages != nullptr && c >= ap.k_off) {
+      T* to = append_at<T>(ap, c, token_req[t], positions[t]);
+      if (to != nullptr) *reinterpret_cast<Raw*>(to) = y;
+    }
+  };
+  if (t0 >= BACK && first == last) {           // a request's tokens of the step are consecutive rows: all rows here are its own
+    float f[TAPS][VEC];                        // row t - BACK + j at f[(k + j) % TAPS]
+#pragma unroll
+    for (int j = 0; j < BACK; ++j) {
+      Quad<T>::unpack(x[j], f[j]);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) f[j][e] += ib[e];
+    }
+#pragma unroll
+    for (int k = 0; k < kConvTokens; ++k) {
+      if (t0 + k > t_last) break;
+      float* now = f[(k + BACK) % TAPS];
+      Quad<T>::unpack(x[k + BACK], now);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) now[e] += ib[e];
+      float acc[VEC];
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = ob[e];
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wv[e * TAPS + j], f[(k + j) % TAPS][e], acc[e]);
+      }
+      finish(t0 + k, acc);
+    }
+    return;
+  }
+  // rows of several requests, or a request's first: row by row, from the step's rows or the request's tail
+  for (int t = t0; t <= t_last; ++t) {
+    const int r = token_req[t], pos = positions[t];
     float acc[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; ++e) acc[e] = ob[e];
@@ -626,8 +687,8 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
     for (int j = 0; j < TAPS; ++j) {
       const int back = BACK - j;
       float v[VEC];
-      if (req[k + j] == r) {                   // a request's tokens of the step are consecutive rows
-        Vec16<T>::unpack(x[k + j], v);
+      if (t - back >= 0 && token_req[t - back] == r) {
+        Quad<T>::unpack(*reinterpret_cast<const Raw*>(in + (size_t)(t - back) * ld + c), v);
       } else {
         const int sp = pos - back, start = req_start[r];
         const float* tp = tails + (size_t)slots[r] * slot_stride + (long long)(sp - (start - BACK)) * C + c;
@@ -641,12 +702,7 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
 #pragma unroll
       for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wv[e * TAPS + j], v[e], acc[e]);
     }
-    if (act == 0) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) acc[e] = acc[e] / (1.0f + expf(-acc[e]));
-    }
-    Vec16<T>::store(out + (size_t)t * C + c, acc);
-    if (ap.pages != nullptr && c >= ap.k_off) append_row<T>(ap, c, r, pos, acc);
+    finish(t, acc);
   }
 }
 
@@ -707,10 +763,11 @@ KVB_EXPORT int kvb_conv_silu(const void* in, int ld, const float* w, int taps, f
   kvb_launch(conv_vec_kernel<T, TAPS>, dim3((unsigned)((units + 255) / 256)), dim3(256), 0, stream, (const T*)in, ld, w, \
              taps, (const float*)tails, slot_stride, (T*)out, C, T_, positions, token_req, q_start, req_start, slots, act, ap, \
              in_bias, out_bias)
-    // blocks of tokens from where they still give every SM a block of threads (measured: 1024 tokens of 3072 channels 23 / 19 us,
-    // 600 of 3072 and 300 of 6144 level)
-    const bool runs = w16 && taps >= 2 && taps <= 4 && units / kConvTokens >= 256ll * kvb_sm_count();
-    const long long run_units = (long long)((T_ + kConvTokens - 1) / kConvTokens) * (C / vec);
+    // blocks of tokens from where they give every SM most of a block of threads (measured, with the tails' launch, a token a thread /
+    // blocks: 600 tokens of 1536 channels 11.3 / 11.1 us, 1024 of 1536 13.6 / 11.8, 300 of 3072 10.9 / 11.3, 600 of 3072 16.2 / 11.6, 100 of
+    // 6144 8.4 / 10.1, 200 of 6144 12.4 / 11.7)
+    const long long run_units = (long long)((T_ + kConvTokens - 1) / kConvTokens) * (C / 4);
+    const bool runs = w16 && taps >= 2 && taps <= 4 && run_units >= 224ll * kvb_sm_count();
 #define KVB_CONV_RUN(TAPS)                                                                                              \
   kvb_launch(conv_run_kernel<T, TAPS>, dim3((unsigned)((run_units + 255) / 256)), dim3(256), 0, stream, (const T*)in, ld, w, \
              (const float*)tails, slot_stride, (T*)out, C, T_, positions, token_req, req_start, slots, act, ap, in_bias, out_bias)
