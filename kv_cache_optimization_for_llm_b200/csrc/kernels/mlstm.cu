@@ -28,7 +28,7 @@
 //           (m' = max(F + m, m_c);  C' = exp(F + m - m') C + exp(m_c - m') C_c)
 //   FINAL   every chunk from what it begins with, writing y; the run's last chunk leaves the state in the slot
 // A run of one chunk reads and writes its slot directly.
-#include "chunk_walk.cuh"
+#include "chunk_pieces.cuh"
 #include "common.cuh"
 #include "head_finish.cuh"
 
@@ -342,7 +342,10 @@ KVB_EXPORT int kvb_mlstm_scan(const MlstmArgs* args, int R, int max_run, int dty
 
 // The runs of requests first .. first + R - 1 walked in pieces of 64 tokens on tensor cores (chunk_walk.cuh): bfloat16, N 64 or
 // 128, Dv a multiple of 64, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).  The chunk fields are not read.
-KVB_EXPORT int kvb_mlstm_walk(const MlstmArgs* args, int first, int R, cudaStream_t stream) {
+// tokens: of these runs in all, at most.  scratch: null for the walk in one launch; for the three of chunk_pieces.cuh as many bytes as
+// scratch_bytes there says, on a 16-byte boundary.
+KVB_EXPORT int kvb_mlstm_walk(const MlstmArgs* args, int first, int R, int tokens, void* scratch, long long scratch_bytes,
+                               cudaStream_t stream) {
   const MlstmArgs& p = *args;
   if (R <= 0) return 0;
   if (!(p.cap > 0.f)) return KVB_ERR_BAD_SIZE;
@@ -356,6 +359,7 @@ KVB_EXPORT int kvb_mlstm_walk(const MlstmArgs* args, int first, int R, cudaStrea
   a.state = p.state; a.slot_stride = p.slot_stride; a.y = p.y;
   a.q_start = p.q_start; a.req_start = p.req_start; a.slots = p.slots;
   a.H = p.H; a.Dv = p.Dv; a.first = first;
+  if (scratch != nullptr) return pieces::launch<walk::MLSTM>(a, p.N, R, tokens, scratch, scratch_bytes, stream);
   return walk::launch_any<walk::MLSTM>(a, p.N, R, stream);
 }
 

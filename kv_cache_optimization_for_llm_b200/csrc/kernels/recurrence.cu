@@ -17,7 +17,7 @@
 // steps or on the rest of the batch.  Long runs are the exception: chunks side by side, and in bfloat16 the walk of
 // chunk_walk.cuh, cut a run from its first token on, and which form a step takes goes by its longest run, for the walk by the
 // average one; their float32 sums then differ by rounding.
-#include "chunk_walk.cuh"
+#include "chunk_pieces.cuh"
 #include "common.cuh"
 #include "head_finish.cuh"
 
@@ -529,7 +529,10 @@ KVB_EXPORT int kvb_ssd_scan(const SsdArgs* args, int R, int max_run, int dtype, 
 
 // The runs of requests first .. first + R - 1 walked in pieces of 64 tokens on tensor cores (chunk_walk.cuh): bfloat16, N 64 or
 // 128, Dv a multiple of 64, rows and segments on 16-byte boundaries (KVB_ERR_BAD_SIZE otherwise).  The chunk fields are not read.
-KVB_EXPORT int kvb_ssd_walk(const SsdArgs* args, int first, int R, cudaStream_t stream) {
+// tokens: of these runs in all, at most.  scratch: null for the walk in one launch; for the three of chunk_pieces.cuh as many bytes as
+// scratch_bytes there says, on a 16-byte boundary.
+KVB_EXPORT int kvb_ssd_walk(const SsdArgs* args, int first, int R, int tokens, void* scratch, long long scratch_bytes,
+                             cudaStream_t stream) {
   const SsdArgs& p = *args;
   if (R <= 0) return 0;
   if (p.H < 1 || p.G < 1 || p.H % p.G) return KVB_ERR_BAD_SIZE;
@@ -546,6 +549,7 @@ KVB_EXPORT int kvb_ssd_walk(const SsdArgs* args, int first, int R, cudaStream_t 
   a.state = p.state; a.slot_stride = p.slot_stride; a.y = p.y;
   a.q_start = p.q_start; a.req_start = p.req_start; a.slots = p.slots;
   a.H = p.H; a.Dv = p.Dv; a.first = first;
+  if (scratch != nullptr) return pieces::launch<walk::SSD>(a, p.N, R, tokens, scratch, scratch_bytes, stream);
   return walk::launch_any<walk::SSD>(a, p.N, R, stream);
 }
 

@@ -1572,6 +1572,45 @@ def _walks(rule: str, batch, n: int, dv: int, x: torch.Tensor, *columns: int) ->
             and batch.num_tokens - singles >= walk_line(rule, runs, singles) * runs)
 
 
+# Tokens of a step's runs times heads times blocks of 64 value columns from which on a walk's products are made for all its pieces at
+# once, in three launches (chunk_pieces.cuh), and the longest run there must be.  The launches of either form in us, three / one.  ssd, 64
+# heads of 128 x 64: runs of 300 26 / 34, 512 35 / 51, 1024 57 / 95, 2048 115 / 182, 1111 + 700 + 237 116 / 121, five of 400 128 / 140, eight
+# of 128 68 / 76; 32 heads: 300 24 / 18, 512 26 / 26, 2048 58 / 92, 300 + 300 26 / 34.  mlstm, 32 heads of 64 x 64: 300 20 / 17, 512 21 / 24, 2048 51 / 86,
+# 1111 + 700 + 237 51 / 68, eight of 128 35 / 43; 16 heads: 512 20 / 21, 700 22 / 27, 2048 37 / 70, 300 + 300 20 / 17, eight of 128 24 / 22.
+# On the device they cross at about 12000; but the host pays for two launches more (6 us a layer), which shows until a layer's kernels take
+# longer than the host (about 80 us), hence the line.
+PIECES_MIN_WORK, PIECES_MIN_RUN = 40000, 256
+
+
+def _count_more(launches: int) -> None:
+    global launch_count
+    launch_count += launches
+
+
+def _pieces_unit(rule: str, heads: int, n: int, dv: int) -> int:
+    """Bytes of scratch for a piece of 64 tokens."""
+    per_block, per_head = (4 * n * 65 + 4, 16 + 1536) if rule == "mlstm" else (4 * n * 64 + 4, 16 + 2448)
+    return heads * (dv // 64 * per_block + per_head)
+
+
+def pieces_width(rule: str, heads: int, n: int, dv: int) -> int:
+    """bfloat16 elements per token that :func:`ssd_scan` and :func:`mlstm_scan` want for their scratch in steps of long runs."""
+    if n not in (64, 128) or dv % 64:
+        return 0
+    return -(-_pieces_unit(rule, heads, n, dv) // 128)
+
+
+def _pieces_bytes(rule: str, batch, tokens: int, heads: int, n: int, dv: int, device) -> int:
+    """Bytes of scratch for a walk in three launches, 0 where the runs walk in one (short runs, or an arena without the room)."""
+    if (int(getattr(batch, "max_q_len", 0) or 0) < PIECES_MIN_RUN or tokens * heads * (dv // 64) < PIECES_MIN_WORK):
+        return 0
+    pieces = tokens // 64 + batch.num_reqs - int(batch.num_single)
+    nbytes = pieces * _pieces_unit(rule, heads, n, dv) + 64
+    if pieces > 65535 or (_arena is not None and _arena.device == device and nbytes > _arena.current.capacity):
+        return 0
+    return nbytes
+
+
 class _DiagArgs(ctypes.Structure):
     _fields_ = [("a", c_void_p), ("b", c_void_p), ("y", c_void_p), ("ld_y", c_int), ("y_bias", c_void_p),
                 ("out_scale", c_float), ("out", c_void_p), ("state", c_void_p), ("slot_stride", c_longlong),
@@ -1646,8 +1685,13 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
         if singles:
             _check(lib("recurrence").kvb_ssd_scan(ctypes.byref(p), c_int(singles), c_int(1), c_int(dtype_code(xbc.dtype)), _stream()),
                    "ssd_scan")
-        rc = lib("recurrence").kvb_ssd_walk(ctypes.byref(p), c_int(singles), c_int(batch.num_reqs - singles), _stream())
+        nbytes = _pieces_bytes("ssd", batch, T - singles, heads, n, dv, xbc.device)
+        with lent((max(nbytes, 16),), torch.uint8, xbc.device) as scratch:
+            rc = lib("recurrence").kvb_ssd_walk(ctypes.byref(p), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles),
+                                                _p(scratch if nbytes else None), c_longlong(nbytes), _stream())
         _check(rc, "ssd_scan")
+        _count_more(2 if nbytes else 0)
+        choices["ssd_pieces"] += 1 if nbytes else 0
         choices["ssd_walk"] += 1
         return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():
@@ -1765,8 +1809,13 @@ def mlstm_scan(p: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch
         if singles:
             _check(lib("mlstm").kvb_mlstm_scan(ctypes.byref(a), c_int(singles), c_int(1), c_int(dtype_code(p.dtype)), _stream()),
                    "mlstm_scan")
-        rc = lib("mlstm").kvb_mlstm_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), _stream())
+        nbytes = _pieces_bytes("mlstm", batch, T - singles, heads, n, dv, p.device)
+        with lent((max(nbytes, 16),), torch.uint8, p.device) as scratch:
+            rc = lib("mlstm").kvb_mlstm_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles),
+                                             _p(scratch if nbytes else None), c_longlong(nbytes), _stream())
         _check(rc, "mlstm_scan")
+        _count_more(2 if nbytes else 0)
+        choices["mlstm_pieces"] += 1 if nbytes else 0
         choices["mlstm_walk"] += 1
         return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():

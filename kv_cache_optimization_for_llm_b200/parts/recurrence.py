@@ -143,7 +143,8 @@ class StateSpaceDuality(Part):
         return SlotStateSpec((self.matrix_floats + (self.taps - 1) * self.channels,), torch.float32)
 
     def activation_widths(self):
-        return [self.w_in.shape[0], self.channels, 2 * self.inner, self.inner, self.o.shape[0]]
+        pieces = ops.pieces_width("ssd", self.H, self.N, self.Dv) if self.ctx.dtype == torch.bfloat16 else 0
+        return [self.w_in.shape[0], self.channels, 2 * self.inner, self.inner, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):
         p = ops.linear(x, self.w_in)
@@ -203,7 +204,8 @@ class MatrixLSTM(Part):
 
     def activation_widths(self):
         inner = self.H * self.Dv
-        return [self.w_in.shape[0], 2 * (2 * self.H + 8), 2 * inner, inner, self.o.shape[0]]
+        pieces = ops.pieces_width("mlstm", self.H, self.D, self.Dv) if self.ctx.dtype == torch.bfloat16 else 0
+        return [self.w_in.shape[0], 2 * (2 * self.H + 8), 2 * inner, inner, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):
         p = ops.linear(x, self.w_in)
