@@ -138,22 +138,110 @@ KVB_EXPORT int kvb_paged_attention_generic(const void* q, int q_row_stride, cons
 // The general attention over tiles of query rows (float32 steps with runs of tokens): the same sums as the kernel above, to
 // the bit, so that a token's result does not depend on which of the two its step was given to.
 //
-// A block takes a tile of consecutive tokens of one request with all query heads of one key/value head, up to 8 RT rows (token,
-// head), and brings every chunk of 32 keys and values into shared memory once for the whole tile.  Its four groups of 64 threads
+// A block takes a tile of consecutive tokens of one request with all query heads of one key/value head, up to 16 RT rows (token,
+// head), and brings every chunk of 32 keys and values into shared memory once for the whole tile.  Its four groups of 128 threads
 // are the four warps of the kernel above: group g takes the chunks c with c % 4 == g, with a maximum, a sum and a weighted
-// sum of values of its own, merged at the end in the same order.  Within a group a thread stands at row 8 r + ty (r < RT) and
+// sum of values of its own, merged at the end in the same order.  Within a group a thread stands at row 16 r + ty (r < RT) and
 // keys tx, tx + 8, tx + 16, tx + 24 of the chunk: every score is one chain of fmaf over the head's channels; the 32
 // exponentials are added as warp_sum adds them (partners 16, 8, 4, 2, 1 apart); a value channel is one chain over the keys
 // in order.  A key that a row does not see adds nothing to any of the three.
 //
-// What bounds it: the kernel above reads a key's channels one by one, a lane per key (32 rows a warp and load), and every
-// (token, head) reads them again: 575 us for 333 + 5 tokens of 32 heads of 64 over 8 key/value heads.  Here the loads are 16
-// bytes wide and shared by the tile: 95 us.
-constexpr int kTileThreads = 256;
+// Keys and values of a group's next chunk are on their way (cp.async) while it works on this one, where shared memory has room for two
+// (head sizes up to 64).  Two neighbouring rows' scores, and two channels' sums, go through one `fma.rn.f32x2`, which rounds each half as
+// fmaf does.  The chunk's first keys that all rows of a warp see, most of them, are added up without a look at positions.  The blocks
+// that start first are the ones with the latest positions of their run, which have the most keys.
+//
+// What bounds it: one block of sixteen warps an SM (its registers), whose loads from shared memory are 224 of 16 bytes a thread and chunk of
+// 64 rows (four cycles a warp and load, 7 us of a turn's 9).  The kernel above reads a key's channels one by one, a lane per key (32 rows a warp and load), and every (token, head) reads
+// them again: 575 us for 333 + 5 tokens of 32 heads of 64 over 8 key/value heads.
+// Here, us: those 338 tokens 114 -> 50, the 333 alone 112 -> 36, 1024 tokens 497 -> 181, 16 tokens behind 3000 545 -> 239, twenty single tokens
+// behind 3000 beside a run of two 525 -> 231; 24 heads of 128, 333 tokens 152 -> 54 (before: loads one after the other behind a look at
+// the block table each, branches around every key's sums, groups of 64 threads with eight rows each; with eight warps 56, 50, 246, 304, 215).
+constexpr int kTileRows = 16;                          // TY: rows of threads in a group, eight threads a row
+constexpr int kTileThreads = kWarps * 8 * kTileRows, kGroupThreads = 8 * kTileRows;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void copy_16(float* to, const float* from, bool inside) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+               "r"(inside ? 16 : 0) : "memory");
+}
 
 // floats of a group's chunk of keys, in whose place its exponentials are kept
 __host__ __device__ constexpr int tile_key_floats(int dmax, int rt) {
-  return 32 * (dmax + 4) > 8 * rt * 36 ? 32 * (dmax + 4) : 8 * rt * 36;
+  return 32 * (dmax + 4) > kTileRows * rt * 36 ? 32 * (dmax + 4) : kTileRows * rt * 36;
+}
+// chunks of keys and values that a group has room for
+__host__ __device__ constexpr int tile_stages(int dmax) { return dmax <= 64 ? 2 : 1; }
+// floats between the rows of a pair of queries: the pair's channels side by side, eight more for the banks
+__host__ __device__ constexpr int tile_pair_floats(int dmax) { return 2 * dmax + 8; }
+
+// Scores of RP pairs of rows (of a thread: rows 16 r + ty) with four keys.
+template <int RP, int LD, int LDQ>
+__device__ __forceinline__ void tile_scores(f32x2 (&s)[RP][4], const float* q_s, const float* k_s, int d, int tx, int ty) {
+#pragma unroll
+  for (int r = 0; r < RP; ++r)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[r][u] = 0ull;
+#pragma unroll 2
+  for (int i = 0; i < d; i += 4) {
+    float4 kv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) kv[u] = *reinterpret_cast<const float4*>(k_s + (tx + 8 * u) * LD + i);
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(q_s + (kTileRows * r + ty) * LDQ + 2 * i);
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(q_s + (kTileRows * r + ty) * LDQ + 2 * i + 4);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        s[r][u] = fma2(a.x, pack2(kv[u].x, kv[u].x), s[r][u]);
+        s[r][u] = fma2(a.y, pack2(kv[u].y, kv[u].y), s[r][u]);
+        s[r][u] = fma2(b.x, pack2(kv[u].z, kv[u].z), s[r][u]);
+        s[r][u] = fma2(b.y, pack2(kv[u].w, kv[u].w), s[r][u]);
+      }
+    }
+  }
+}
+
+// Keys 0 .. n - 1 of the chunk (n a multiple of four), seen by all of the first R rows of the thread.
+template <int R, int RT, int DT, int LD, int LDP>
+__device__ __forceinline__ void tile_values(f32x2 (&acc)[RT][2 * DT], const float* p_s, const float* v_s, int n, int tx, int ty) {
+#pragma unroll 1
+  for (int jj = 0; jj < n; jj += 4) {
+    float4 pv[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) pv[r] = *reinterpret_cast<const float4*>(p_s + (kTileRows * r + ty) * LDP + jj);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      ulonglong2 vv[DT];
+#pragma unroll
+      for (int x = 0; x < DT; ++x) vv[x] = *reinterpret_cast<const ulonglong2*>(v_s + (jj + u) * LD + 32 * x + 4 * tx);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float pj = u == 0 ? pv[r].x : u == 1 ? pv[r].y : u == 2 ? pv[r].z : pv[r].w;
+        const f32x2 p2 = pack2(pj, pj);
+#pragma unroll
+        for (int x = 0; x < DT; ++x) {
+          acc[r][2 * x] = fma2(p2, vv[x].x, acc[r][2 * x]);
+          acc[r][2 * x + 1] = fma2(p2, vv[x].y, acc[r][2 * x + 1]);
+        }
+      }
+    }
+  }
 }
 
 template <int DMAX, int RT>
@@ -162,19 +250,20 @@ paged_attention_tiles_kernel(const float* __restrict__ q_base, int q_row_stride,
                              const float* __restrict__ v_pages, const int* __restrict__ block_table, int max_pages,
                              int page_size, int num_pages, const int* __restrict__ positions, const int4* __restrict__ tiles,
                              float* __restrict__ out, int nq, int nkv, int d, float scale, int window, int* status) {
-  constexpr int ROWS = 8 * RT, LD = DMAX + 4, LDP = 36, DT = DMAX / 32;      // DT: groups of four channels a thread owns
-  constexpr int KREG = tile_key_floats(DMAX, RT), PER_GROUP = KREG + 32 * LD;
+  constexpr int ROWS = kTileRows * RT, LD = DMAX + 4, LDP = 36, DT = DMAX / 32;      // DT: groups of four channels a thread owns
+  constexpr int RP = RT / 2, LDQ = tile_pair_floats(DMAX), STAGES = tile_stages(DMAX);
+  constexpr int KREG = tile_key_floats(DMAX, RT), PER_CHUNK = KREG + 32 * LD, PER_GROUP = STAGES * PER_CHUNK;
   extern __shared__ __align__(16) float tsm[];
-  float* q_s = tsm;                                    // [ROWS][LD]
-  const int tid = threadIdx.x, g = tid >> 6, gt = tid & 63, tx = gt & 7, ty = gt >> 3;
-  float* k_s = q_s + ROWS * LD + g * PER_GROUP;        // [32][LD]
-  float* v_s = k_s + KREG;                             // [32][LD]
-  float* p_s = k_s;                                    // [ROWS][LDP], once the scores are made
+  float* q_s = tsm;                                    // [RP * 16 pairs of rows][LDQ]: rows 32 r + ty and 32 r + 16 + ty
+  const int tid = threadIdx.x, g = tid / kGroupThreads, gt = tid % kGroupThreads, tx = gt & 7, ty = gt >> 3;
+  float* mine_s = q_s + RP * kTileRows * LDQ + g * PER_GROUP;  // [STAGES]{[32][LD] keys, [32][LD] values}
   __shared__ float m_s[kWarps][ROWS], l_s[kWarps][ROWS];
   pdl_trigger();
   pdl_wait();
-  const int4 tile = tiles[blockIdx.x];
-  const int hk = blockIdx.y, group = nq / nkv, rows = tile.z * group, nr = (rows + 7) / 8;     // r < nr: rows that exist
+  // the tiles come in the order of their tokens: the last ones first, for all key/value heads
+  const int lin = blockIdx.y * gridDim.x + blockIdx.x;
+  const int4 tile = tiles[gridDim.x - 1 - lin / nkv];
+  const int hk = lin % nkv, group = nq / nkv, rows = tile.z * group, nr = (rows + kTileRows - 1) / kTileRows;     // r < nr: rows that exist
   const int* table = block_table + (size_t)tile.x * max_pages;
   int pos_lo = 0x7fffffff, pos_hi = -1;                // of the tile's tokens
   for (int t = 0; t < tile.z; ++t) {
@@ -182,158 +271,180 @@ paged_attention_tiles_kernel(const float* __restrict__ q_base, int q_row_stride,
     pos_lo = min(pos_lo, p);
     pos_hi = max(pos_hi, p);
   }
+  // This group's part of a chunk, on its way to a stage; bit k of the answer: key k lies in a page (the same word in every thread
+  // of the warp).  A lane looks one key's page up for the others.
   const int d4 = d >> 2;
+  auto request = [&](int c, int stage) -> unsigned {
+    const int j = c * 32 + (tid & 31);
+    const int lp = j / page_size;
+    const int page = j <= pos_hi && lp < max_pages ? table[lp] : -1;
+    const bool there = page >= 0 && page < num_pages;
+    if (!there && j <= pos_hi && (window <= 0 || j > pos_lo - window)) atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE);
+    const long long off = there ? (((long long)page * nkv + hk) * page_size + (j - lp * page_size)) * d : -1;
+    float* to = mine_s + stage * PER_CHUNK;
+    for (int x = gt; x < 32 * d4; x += kGroupThreads) {      // (whole warps take part: 32 d4 is a multiple of 32)
+      const int kk = x / d4, i = (x - kk * d4) * 4;
+      const long long of = __shfl_sync(0xffffffffu, off, kk);
+      copy_16(to + kk * LD + i, k_pages + (of >= 0 ? of + i : 0), of >= 0);
+      copy_16(to + KREG + kk * LD + i, v_pages + (of >= 0 ? of + i : 0), of >= 0);
+    }
+    return __ballot_sync(0xffffffffu, there);
+  };
+  const int first = (window > 0 ? max(0, pos_lo - window + 1) : 0) / 32;
+  int c = first + ((g - first) % kWarps + kWarps) % kWarps, stage = 0;
+  unsigned mapped = c * 32 <= pos_hi ? request(c, 0) : 0u;
+  asm volatile("cp.async.commit_group;" ::: "memory");
   for (int x = tid; x < ROWS * d4; x += kTileThreads) {
     const int row = x / d4, i = (x - row * d4) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < rows)
       v = *reinterpret_cast<const float4*>(q_base + (size_t)(tile.y + row / group) * q_row_stride + (size_t)(hk * group + row % group) * d + i);
-    *reinterpret_cast<float4*>(q_s + row * LD + i) = v;
+    float* to = q_s + (row / (2 * kTileRows) * kTileRows + row % kTileRows) * LDQ + 2 * i + row / kTileRows % 2;
+    to[0] = v.x; to[2] = v.y; to[4] = v.z; to[6] = v.w;
   }
   int pos[RT];
 #pragma unroll
-  for (int r = 0; r < RT; ++r) pos[r] = 8 * r + ty < rows ? positions[tile.y + (8 * r + ty) / group] : -1;
+  for (int r = 0; r < RT; ++r) pos[r] = kTileRows * r + ty < rows ? positions[tile.y + (kTileRows * r + ty) / group] : -1;
   __syncthreads();
 
-  float m[RT], l[RT], acc[RT][4 * DT];
+  float m[RT], l[RT];
+  f32x2 acc[RT][2 * DT];
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
     m[r] = -CUDART_INF_F;
     l[r] = 0.f;
 #pragma unroll
-    for (int x = 0; x < 4 * DT; ++x) acc[r][x] = 0.f;
+    for (int x = 0; x < 2 * DT; ++x) acc[r][x] = 0ull;
   }
-  const int first = (window > 0 ? max(0, pos_lo - window + 1) : 0) / 32;
-  for (int c = first + ((g - first) % kWarps + kWarps) % kWarps; c * 32 <= pos_hi; c += kWarps) {
-    // bit k of `mapped`: key k of the chunk lies in a page (the same word in every thread of the warp)
-    bool mine = false;
-    {
-      const int j = c * 32 + (tid & 31);
-      const int lp = j / page_size;
-      const int page = j <= pos_hi && lp < max_pages ? table[lp] : -1;
-      mine = page >= 0 && page < num_pages;
-      if (!mine && j <= pos_hi && (window <= 0 || j > pos_lo - window)) atomicCAS(status, 0, KVB_STATUS_UNMAPPED_PAGE);
+  const bool busy = (ty & ~3) < rows;                    // this warp has rows that exist; a single token's heads leave most without
+  for (; c * 32 <= pos_hi; c += kWarps) {
+    unsigned next = 0u;
+    if (STAGES == 2) {
+      if ((c + kWarps) * 32 <= pos_hi) next = request(c + kWarps, stage ^ 1);
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    const unsigned mapped = __ballot_sync(0xffffffffu, mine);
-    for (int x = gt; x < 32 * d4; x += 64) {
-      const int kk = x / d4, i = (x - kk * d4) * 4, j = c * 32 + kk;
-      float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-      if (mapped >> kk & 1) {
-        const long long off = (((long long)table[j / page_size] * nkv + hk) * page_size + (j % page_size)) * d + i;
-        kv = *reinterpret_cast<const float4*>(k_pages + off);
-        vv = *reinterpret_cast<const float4*>(v_pages + off);
-      }
-      *reinterpret_cast<float4*>(k_s + kk * LD + i) = kv;
-      *reinterpret_cast<float4*>(v_s + kk * LD + i) = vv;
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroupThreads) : "memory");
+    float* k_s = mine_s + stage * PER_CHUNK;             // [32][LD]
+    const float* v_s = k_s + KREG;                       // [32][LD]
+    float* p_s = k_s;                                    // [ROWS][LDP], once the scores are made
+    f32x2 s2[RP][4];
+    if (!busy) {
+#pragma unroll
+      for (int r = 0; r < RP; ++r) s2[r][0] = s2[r][1] = s2[r][2] = s2[r][3] = 0ull;
+    } else if (nr <= 2 && RP > 1) {
+      f32x2 few[1][4];
+      tile_scores<1, LD, LDQ>(few, q_s, k_s, d, tx, ty);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s2[0][u] = few[0][u];
+#pragma unroll
+      for (int r = 1; r < RP; ++r) s2[r][0] = s2[r][1] = s2[r][2] = s2[r][3] = 0ull;
+    } else {
+      tile_scores<RP, LD, LDQ>(s2, q_s, k_s, d, tx, ty);
     }
-    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
-    float s[RT][4];
-#pragma unroll
-    for (int r = 0; r < RT; ++r)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) s[r][u] = 0.f;
-    for (int i = 0; i < d; i += 4) {
-      float4 kv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) kv[u] = *reinterpret_cast<const float4*>(k_s + (tx + 8 * u) * LD + i);
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroupThreads) : "memory");
+    if (busy) {
+      int every = mapped == 0xffffffffu ? 32 : 0;        // keys 0 .. every - 1: seen by all of this thread's rows
+      unsigned skipped = 0;                              // bit r: row 16 r + ty takes nothing of the chunk
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         if (r >= nr) break;
-        const float4 qv = *reinterpret_cast<const float4*>(q_s + (8 * r + ty) * LD + i);
+        float s[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          s[r][u] = fmaf(qv.x, kv[u].x, s[r][u]);
-          s[r][u] = fmaf(qv.y, kv[u].y, s[r][u]);
-          s[r][u] = fmaf(qv.z, kv[u].z, s[r][u]);
-          s[r][u] = fmaf(qv.w, kv[u].w, s[r][u]);
+          const float2 two = unpack2(s2[r >> 1][u]);
+          s[u] = r & 1 ? two.y : two.x;
+        }
+        unsigned seen = 0;                               // bit u: key tx + 8 u
+        float cm;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int kk = tx + 8 * u, j = c * 32 + kk;
+          const bool on = j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> kk & 1);
+          s[u] = on ? s[u] * scale : -CUDART_INF_F;
+          seen |= (on ? 1u : 0u) << u;
+          cm = u == 0 ? s[0] : fmaxf(cm, s[u]);          // (a NaN only if all 32 scores are, as warp_max has it)
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+        const float m_new = fmaxf(m[r], cm);
+        const float corr = m[r] == -CUDART_INF_F ? 0.f : expf(m[r] - m_new);
+        const bool skip = cm == -CUDART_INF_F;           // nothing seen, or no score above the lowest: the row stays as it is
+        if (kTileRows * r + ty < rows) every = skip || (window > 0 && c * 32 <= pos[r] - window) ? 0 : min(every, pos[r] - c * 32 + 1);
+        skipped |= (skip ? 1u : 0u) << r;
+        float p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          p[u] = seen >> u & 1 && !skip ? expf(s[u] - m_new) : 0.f;
+          p_s[(kTileRows * r + ty) * LDP + tx + 8 * u] = p[u];
+        }
+        float sum = (p[0] + p[2]) + (p[1] + p[3]);       // keys 16 apart, then 8 apart
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (!skip) {
+          l[r] = fmaf(l[r], corr, sum);
+#pragma unroll
+          for (int x = 0; x < 2 * DT; ++x) {
+            const float2 two = unpack2(acc[r][x]);
+            acc[r][x] = pack2(two.x * corr, two.y * corr);
+          }
+          m[r] = m_new;
         }
       }
-    }
-    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
-    bool whole = mapped == 0xffffffffu;                // every row of this thread sees every key of the chunk
-    unsigned skipped = 0;                              // bit r: row 8 r + ty takes nothing of the chunk
+      // (rows that do not exist hold a probability of zero, or what lay there, and are never stored)
+      every = __reduce_min_sync(0xffffffffu, every) & ~3;
+      __syncwarp();
+      if (nr <= 1) tile_values<1, RT, DT, LD, LDP>(acc, p_s, v_s, every, tx, ty);
+      else tile_values<RT, RT, DT, LD, LDP>(acc, p_s, v_s, every, tx, ty);
+      const int last = min(32, pos_hi - c * 32 + 1);
+      for (int jj = every; jj < last; ++jj) {
+        ulonglong2 vv[DT];
 #pragma unroll
-    for (int r = 0; r < RT; ++r) {
-      if (r >= nr) break;
-      unsigned seen = 0;                               // bit u: key tx + 8 u
-      float cm;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int kk = tx + 8 * u, j = c * 32 + kk;
-        const bool on = j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> kk & 1);
-        s[r][u] = on ? s[r][u] * scale : -CUDART_INF_F;
-        seen |= (on ? 1u : 0u) << u;
-        cm = u == 0 ? s[r][0] : fmaxf(cm, s[r][u]);    // (a NaN only if all 32 scores are, as warp_max has it)
-      }
-      whole = whole && c * 32 + 31 <= pos[r] && (window <= 0 || c * 32 > pos[r] - window);
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-      const float m_new = fmaxf(m[r], cm);
-      const float corr = m[r] == -CUDART_INF_F ? 0.f : expf(m[r] - m_new);
-      const bool skip = cm == -CUDART_INF_F;           // nothing seen, or no score above the lowest: the row stays as it is
-      whole = whole && !skip;
-      skipped |= (skip ? 1u : 0u) << r;
-      float p[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        p[u] = seen >> u & 1 && !skip ? expf(s[r][u] - m_new) : 0.f;
-        p_s[(8 * r + ty) * LDP + tx + 8 * u] = p[u];
-      }
-      float sum = (p[0] + p[2]) + (p[1] + p[3]);       // keys 16 apart, then 8 apart
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (!skip) {
-        l[r] = fmaf(l[r], corr, sum);
-#pragma unroll
-        for (int x = 0; x < 4 * DT; ++x) acc[r][x] *= corr;
-        m[r] = m_new;
-      }
-    }
-    __syncwarp();
-    for (int jj = 0; jj < 32; jj += 4) {
-      float4 pv[RT];
-#pragma unroll
-      for (int r = 0; r < RT; ++r) pv[r] = *reinterpret_cast<const float4*>(p_s + (8 * r + ty) * LDP + jj);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float4 vv[DT];
-#pragma unroll
-        for (int x = 0; x < DT; ++x) vv[x] = *reinterpret_cast<const float4*>(v_s + (jj + u) * LD + 32 * x + 4 * tx);
-        const int j = c * 32 + jj + u;
+        for (int x = 0; x < DT; ++x) vv[x] = *reinterpret_cast<const ulonglong2*>(v_s + jj * LD + 32 * x + 4 * tx);
+        const int j = c * 32 + jj;
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
           if (r >= nr) break;
-          const float pj = u == 0 ? pv[r].x : u == 1 ? pv[r].y : u == 2 ? pv[r].z : pv[r].w;
           // a value that the row does not see is left out, whatever it holds
-          if (whole || (!(skipped >> r & 1) && j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> (jj + u) & 1))) {
+          if (!(skipped >> r & 1) && j <= pos[r] && (window <= 0 || j > pos[r] - window) && (mapped >> jj & 1)) {
+            const float pj = p_s[(kTileRows * r + ty) * LDP + jj];
+            const f32x2 p2 = pack2(pj, pj);
 #pragma unroll
             for (int x = 0; x < DT; ++x) {
-              acc[r][4 * x + 0] = fmaf(pj, vv[x].x, acc[r][4 * x + 0]);
-              acc[r][4 * x + 1] = fmaf(pj, vv[x].y, acc[r][4 * x + 1]);
-              acc[r][4 * x + 2] = fmaf(pj, vv[x].z, acc[r][4 * x + 2]);
-              acc[r][4 * x + 3] = fmaf(pj, vv[x].w, acc[r][4 * x + 3]);
+              acc[r][2 * x] = fma2(p2, vv[x].x, acc[r][2 * x]);
+              acc[r][2 * x + 1] = fma2(p2, vv[x].y, acc[r][2 * x + 1]);
             }
           }
         }
       }
     }
-    asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroupThreads) : "memory");
+    if (STAGES == 2) {
+      stage ^= 1;
+      mapped = next;
+    } else {
+      if ((c + kWarps) * 32 <= pos_hi) mapped = request(c + kWarps, 0);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
   }
 
   // merge: every group leaves its weighted sums where its chunks of keys and values lay
-  float* acc_s = k_s;                                  // [ROWS][LD]
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  float* acc_s = mine_s;                               // [ROWS][LD]
   static_assert(ROWS * LD <= PER_GROUP, "the weighted sums take the room of both chunks");
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
-    const int row = 8 * r + ty;
+    const int row = kTileRows * r + ty;
 #pragma unroll
-    for (int x = 0; x < DT; ++x)
-      *reinterpret_cast<float4*>(acc_s + row * LD + 32 * x + 4 * tx) =
-          make_float4(acc[r][4 * x], acc[r][4 * x + 1], acc[r][4 * x + 2], acc[r][4 * x + 3]);
+    for (int x = 0; x < DT; ++x) {
+      const float2 a = unpack2(acc[r][2 * x]), b = unpack2(acc[r][2 * x + 1]);
+      *reinterpret_cast<float4*>(acc_s + row * LD + 32 * x + 4 * tx) = make_float4(a.x, a.y, b.x, b.y);
+    }
     if (tx == 0) { m_s[g][row] = m[r]; l_s[g][row] = l[r]; }
   }
   __syncthreads();
-  const float* acc0 = q_s + ROWS * LD;
+  const float* acc0 = q_s + RP * kTileRows * LDQ;
   for (int x = tid; x < rows * d; x += kTileThreads) {
     const int row = x / d, i = x - row * d;
     float M = m_s[0][row];
@@ -366,7 +477,8 @@ KVB_EXPORT int kvb_paged_attention_tiles(const float* q, int q_row_stride, const
                             reinterpret_cast<uintptr_t>(v_pages) | reinterpret_cast<uintptr_t>(tiles)) & 15)) return KVB_ERR_ALIGN;
 #define KVB_TILES(DMAX, RT)                                                                                            \
   {                                                                                                                    \
-    constexpr int smem = (8 * RT * (DMAX + 4) + kWarps * (tile_key_floats(DMAX, RT) + 32 * (DMAX + 4))) * (int)sizeof(float); \
+    constexpr int smem = (kTileRows * RT / 2 * tile_pair_floats(DMAX) +                                                            \
+                          kWarps * tile_stages(DMAX) * (tile_key_floats(DMAX, RT) + 32 * (DMAX + 4))) * (int)sizeof(float); \
     cudaError_t e = cudaFuncSetAttribute(paged_attention_tiles_kernel<DMAX, RT>,                                       \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                           \
     if (e != cudaSuccess) return (int)e;                                                                               \
@@ -374,7 +486,7 @@ KVB_EXPORT int kvb_paged_attention_tiles(const float* q, int q_row_stride, const
                q_row_stride, k_pages, v_pages, block_table, max_pages, page_size, num_pages, positions,                \
                reinterpret_cast<const int4*>(tiles), out, nq, nkv, d, scale, window, status);                          \
   }
-  if (d <= 64) KVB_TILES(64, 8) else KVB_TILES(128, 4)
+  if (d <= 64) KVB_TILES(64, 4) else KVB_TILES(128, 2)
 #undef KVB_TILES
   return kvb_launch_result();
 }

@@ -940,7 +940,8 @@ def paged_attention_tiles_wanted(req_start, ctx_len, nq: int, nkv: int, d: int, 
     fits to 190 measured steps (2 to 1024 tokens, 2 to 64 heads of 32 to 128).  Without it steps of a few short
     prompts, and grids of few blocks, took up to 2.5 times as long over tiles (two prompts of 9 tokens, 8 heads over one: 27 us against 11; 16
     tokens behind 3000 positions, 4 heads over one: 361 against 253); with it none of the 190 is slower than a
-    (token, head) a block."""
+    (token, head) a block.  The tiles have become about twice as fast since (two prompts of 9 tokens, 8 heads over one: 12 us against 7; 40
+    single tokens at 100 beside a run of 40: 15 against 39), so the line lies on the safe side of where they cross."""
     group, f = nq // nkv, d / 64.0
     tokens = paged_attention_tile_tokens(d, group)
     first, each_first, turn, each = 6.0 + 0.1 * d, 0.9 + 0.0195 * d, 2.2 + 0.07 * d, 0.9 + 0.0135 * d
