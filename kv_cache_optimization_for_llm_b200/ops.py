@@ -468,6 +468,14 @@ def _at(t: torch.Tensor, col: int) -> int:
 DELTA_PIECES_MIN_RUN = 512
 
 
+def _with_scratch(nbytes: int, device, call):
+    """``call`` with a buffer of ``nbytes`` that is given back behind its launches, or with None where it wants none."""
+    if not nbytes:
+        return call(None)
+    with lent((nbytes,), torch.uint8, device) as scratch:
+        return call(scratch)
+
+
 def delta_pieces_width(heads: int, dk: int, dv: int) -> int:
     """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs."""
     if dk != 64 or dv not in (32, 64):
@@ -535,9 +543,8 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
                                                     c_int(dtype_code(x0.dtype)), _stream()), "delta_scan")
             launch_count += 1
         nbytes = _delta_pieces_bytes(batch, T - singles, heads, dk, dv, x0.device)
-        with lent((max(nbytes, 16),), torch.uint8, x0.device) as scratch:
-            rc = lib("delta_rule").kvb_delta_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(singles),
-                                                  c_int(T), _p(scratch if nbytes else None), _stream())
+        rc = _with_scratch(nbytes, x0.device, lambda scratch: lib("delta_rule").kvb_delta_walk(
+            ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(singles), c_int(T), _p(scratch), _stream()))
         _check(rc, "delta_scan")
         launch_count += 3 if nbytes else 1
         choices["delta_pieces"] += 1 if nbytes else 0
@@ -1687,12 +1694,13 @@ def ssd_scan(xbc: torch.Tensor, dt, dt_bias: torch.Tensor, a_log: torch.Tensor, 
             _check(lib("recurrence").kvb_ssd_scan(ctypes.byref(p), c_int(singles), c_int(1), c_int(dtype_code(xbc.dtype)), _stream()),
                    "ssd_scan")
         nbytes = _pieces_bytes("ssd", batch, T - singles, heads, n, dv, xbc.device)
-        with lent((max(nbytes, 16),), torch.uint8, xbc.device) as scratch:
-            rc = lib("recurrence").kvb_ssd_walk(ctypes.byref(p), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles),
-                                                _p(scratch if nbytes else None), c_longlong(nbytes), _stream())
+        rc = _with_scratch(nbytes, xbc.device, lambda scratch: lib("recurrence").kvb_ssd_walk(
+            ctypes.byref(p), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles), _p(scratch), c_longlong(nbytes),
+            _stream()))
         _check(rc, "ssd_scan")
-        _count_more(2 if nbytes else 0)
-        choices["ssd_pieces"] += 1 if nbytes else 0
+        if nbytes:
+            _count_more(2)
+            choices["ssd_pieces"] += 1
         choices["ssd_walk"] += 1
         return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():
@@ -1811,12 +1819,13 @@ def mlstm_scan(p: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch
             _check(lib("mlstm").kvb_mlstm_scan(ctypes.byref(a), c_int(singles), c_int(1), c_int(dtype_code(p.dtype)), _stream()),
                    "mlstm_scan")
         nbytes = _pieces_bytes("mlstm", batch, T - singles, heads, n, dv, p.device)
-        with lent((max(nbytes, 16),), torch.uint8, p.device) as scratch:
-            rc = lib("mlstm").kvb_mlstm_walk(ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles),
-                                             _p(scratch if nbytes else None), c_longlong(nbytes), _stream())
+        rc = _with_scratch(nbytes, p.device, lambda scratch: lib("mlstm").kvb_mlstm_walk(
+            ctypes.byref(a), c_int(singles), c_int(batch.num_reqs - singles), c_int(T - singles), _p(scratch), c_longlong(nbytes),
+            _stream()))
         _check(rc, "mlstm_scan")
-        _count_more(2 if nbytes else 0)
-        choices["mlstm_pieces"] += 1 if nbytes else 0
+        if nbytes:
+            _count_more(2)
+            choices["mlstm_pieces"] += 1
         choices["mlstm_walk"] += 1
         return y
     if max_run >= SCAN_CHUNK_MIN_RUN and not _capturing():
