@@ -58,17 +58,6 @@ __device__ __forceinline__ float warp_max(float v) {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Two kernels that touch nothing of each other's, side by side.  The first passes `late` = 1 here: it lets the second be set up only after
-// its own wait, so that by the second's first instruction everything in front of the FIRST has finished and lies in memory.  The second
-// then begins with pdl_beside_begin() instead of pdl_wait() (the fence drops what this SM's cache holds from before), and one block of
-// it ends with pdl_wait(): the second cannot finish before the first, so what comes behind the second finds both complete.
-__device__ __forceinline__ void pdl_open_and_wait(int late) {
-  if (!late) pdl_trigger();
-  pdl_wait();
-  if (late) pdl_trigger();
-}
-__device__ __forceinline__ void pdl_beside_begin() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
 #include <cstdlib>
 #include <utility>
 

@@ -161,7 +161,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                             const int* __restrict__ q_start, const int* __restrict__ ctx_len,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int table_len, int rot,
                             __nv_bfloat16* __restrict__ out, int nq, int nkv, int G, float scale_log2, int window,
-                            int beside, int* status, unsigned long long* trace) {
+                            int* status, unsigned long long* trace) {
   constexpr int CPK = D / 8;      // 16-byte chunks per row
   constexpr int KSTEPS = D / 16;
   constexpr int DT = D / 8;       // n-tiles of the output
@@ -368,8 +368,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     rot_s = sin_t[(size_t)pos * half + j];
   }
 
-  if (beside) pdl_beside_begin();      // the kernel in front is no concern of this one, and what is in front of that has finished
-  else pdl_wait();
+  pdl_wait();
   stamp(1);   // the projection in front has finished
   if (own_key_from_this_step) request_first_tiles(false);
   const __nv_bfloat16* row = qkv + q_row * q_row_stride;
@@ -639,7 +638,6 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // ---- block 0 merges the classes in class order
   cluster_sync_all();
   stamp(5);   // the cluster has met
-  if (beside && blockIdx.x + blockIdx.y + blockIdx.z == 0) pdl_wait();   // this grid ends behind the one in front
   if (z != 0 || bad) {
     if (bad && z == 0 && tid == 0) atomicCAS(status, 0, KVB_STATUS_BAD_POSITION);
     return;
@@ -736,7 +734,7 @@ template <int D, int GP, int kClasses, int kStages, bool kTma>
 int launch(const CUtensorMap& map_k, const CUtensorMap& map_v, const void* qkv, int q_row_stride, void* k_pages, void* v_pages, int write_kv, const int* block_table,
            int max_pages, int page_shift, int num_pages, const int* q_start, const int* ctx_len, const float* cos_t,
            const float* sin_t, int table_len, int rot, void* out, int R, int nq, int nkv, float scale, int window,
-           int blocks_per_cluster, int beside, int* status, unsigned long long* trace, cudaStream_t stream) {
+           int blocks_per_cluster, int* status, unsigned long long* trace, cudaStream_t stream) {
   const size_t smem = smem_bytes<D, GP, kClasses, kStages, kTma>();
   static bool attr_set = false;
   if (!attr_set) {
@@ -769,7 +767,7 @@ int launch(const CUtensorMap& map_k, const CUtensorMap& map_v, const void* qkv, 
   cudaError_t le = cudaLaunchKernelEx(
       &cfg, decode_attention_mma_kernel<D, GP, kClasses, kStages, kTma>, map_k, map_v, (const __nv_bfloat16*)qkv, q_row_stride, (__nv_bfloat16*)k_pages,
       (__nv_bfloat16*)v_pages, write_kv, block_table, max_pages, page_shift, num_pages, q_start, ctx_len, cos_t, sin_t,
-      table_len, rot, (__nv_bfloat16*)out, nq, nkv, nq / nkv, scale * 1.4426950408889634f, window, beside, status, trace);
+      table_len, rot, (__nv_bfloat16*)out, nq, nkv, nq / nkv, scale * 1.4426950408889634f, window, status, trace);
   if (le != cudaSuccess) return (int)le;
   return kvb_launch_result();
 }
@@ -789,14 +787,12 @@ KVB_EXPORT int kvb_decode_attention_mma_supported(int d, int group, int page_siz
 // many classes the kernel has room for and how many blocks share a (request, kv head), not
 // the sums, which are cut by each token's own position.
 // trace: nullptr, or [R * nkv * cluster, 8] uint64 for the phase stamps of every block (profiling only).
-// beside: the kernel in front touches none of these rows, pages and outputs, and lets this one start only when everything in front of
-// IT has finished (pdl_open_and_wait): the two run side by side.
 // Uses no memory beyond its operands.  R <= 65535.
 KVB_EXPORT int kvb_decode_attention_mma(const void* qkv, int q_row_stride, void* k_pages, void* v_pages, int write_kv,
                                         const int* block_table, int max_pages, int page_size, int num_pages,
                                         const int* q_start, const int* ctx_len, const float* cos_t,
                                         const float* sin_t, int table_len, int rot, void* out, int R, int nq, int nkv,
-                                        int d, float scale, int window, int max_ctx, int beside, int* status,
+                                        int d, float scale, int window, int max_ctx, int* status,
                                         unsigned long long* trace, cudaStream_t stream) {
   if (R <= 0) return 0;
   // the kernel is built for as many classes as the longest context of the step needs
@@ -850,7 +846,7 @@ KVB_EXPORT int kvb_decode_attention_mma(const void* qkv, int q_row_stride, void*
   // stages measured well only with one block per SM (head size 64, 64 000 tokens: two requests 97 us with two
   // stages, 61 us with one; four requests 130 to 150 us against 111 us), small clusters also with two.
 #define KVB_DM_ARGS mk, mv, qkv, q_row_stride, k_pages, v_pages, write_kv, block_table, max_pages, ps, num_pages, q_start, \
-                    ctx_len, cos_t, sin_t, table_len, rot, out, R, nq, nkv, scale, window, S, beside, status, trace, stream
+                    ctx_len, cos_t, sin_t, table_len, rot, out, R, nq, nkv, scale, window, S, status, trace, stream
 #define KVB_FITS(D, GP, CL, ST, TMA, SS) (clusters_at_once<D, GP, CL, ST, TMA>(SS) >= R * nkv)
 #define KVB_PICK(D, GP, CL, TMA)                                                                          \
   do {                                                                                                    \
@@ -881,3 +877,5 @@ KVB_EXPORT int kvb_decode_wait_selftest(unsigned polls, int* status, int* flags_
   decode_wait_selftest_kernel<<<1, 64, 0, stream>>>(polls, status, flags_out);
   return kvb_launch_result();
 }
+
+#include "side_stream.cuh"

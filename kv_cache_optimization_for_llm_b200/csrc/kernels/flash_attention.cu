@@ -64,7 +64,7 @@ paged_flash_attention_kernel(const __nv_bfloat16* __restrict__ q_base, int q_row
                              const int* __restrict__ block_table, int max_pages, int page_shift, int num_pages,
                              const int* __restrict__ positions, const TileDesc* __restrict__ tiles,
                              __nv_bfloat16* __restrict__ out, int nq, int nkv, int G, int gp_shift,
-                             float scale_log2, int window, int* status, int open_late, MaskExt ext) {
+                             float scale_log2, int window, int* status, MaskExt ext) {
   constexpr int BM = NW * 16;       // query rows of this block
   constexpr int kThreads = NW * 32;
   constexpr int CPK = D / 8;        // 16-byte chunks per row
@@ -76,7 +76,8 @@ paged_flash_attention_kernel(const __nv_bfloat16* __restrict__ q_base, int q_row
   unsigned char* v_s = k_s + 2 * BN * D * 2;         // [2][BN][D]
   int* row_pos = reinterpret_cast<int*>(v_s + 2 * BN * D * 2);  // [BM] position of each row's token, -1 if none
 
-  pdl_open_and_wait(open_late);
+  pdl_trigger();
+  pdl_wait();
   // the last tiles of a request read the most keys: they start first, so that the grid's
   // last blocks to start are short ones
   const TileDesc tile = tiles[gridDim.x - 1 - blockIdx.x];
@@ -483,7 +484,7 @@ paged_flash_attention_tc_kernel(const __nv_bfloat16* __restrict__ q_base, int q_
                                 const int* __restrict__ block_table, int max_pages, int page_shift, int num_pages,
                                 const int* __restrict__ positions, const TileDesc* __restrict__ tiles,
                                 __nv_bfloat16* __restrict__ out, int nq, int nkv, int G, int gp_shift,
-                                float scale_log2, int window, int* status, int open_late) {
+                                float scale_log2, int window, int* status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* q_s = base;                       // [128 rows][64]
@@ -513,7 +514,8 @@ paged_flash_attention_tc_kernel(const __nv_bfloat16* __restrict__ q_base, int q_
   const unsigned tmem = *tmem_holder;
   // only now may the kernel behind this one start: its resident, waiting blocks must not be
   // able to take tensor memory that a block of this grid still needs
-  pdl_open_and_wait(open_late);
+  pdl_trigger();
+  pdl_wait();
 
   // the last tiles of a request read the most keys: they start first, so that the grid's
   // last blocks to start are short ones
@@ -724,7 +726,7 @@ paged_flash_attention_tc_kernel(const __nv_bfloat16* __restrict__ q_base, int q_
 
 int launch(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, const int* block_table,
            int max_pages, int page_shift, int num_pages, const int* positions, const void* tiles, int num_tiles,
-           void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status, int open_late,
+           void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status,
            cudaStream_t stream) {
   const size_t smem = 1024 + (size_t)kQBytes + 4 * (size_t)kKVBytes + kPBytes + 2 * BM * 4 + 64;
   static bool attr_set = false;
@@ -738,7 +740,7 @@ int launch(const void* q, int q_row_stride, const void* k_pages, const void* v_p
   kvb_launch(paged_flash_attention_tc_kernel, grid, dim3(kThreads), smem, stream, (const __nv_bfloat16*)q, q_row_stride,
              (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, max_pages, page_shift,
              num_pages, positions, (const TileDesc*)tiles, (__nv_bfloat16*)out, nq, nkv, G, gp_shift,
-             scale * 1.4426950408889634f, window, status, open_late);
+             scale * 1.4426950408889634f, window, status);
   return kvb_launch_result();
 }
 
@@ -823,7 +825,7 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
                                 const int* __restrict__ block_table, int max_pages, int page_shift, int num_pages,
                                 const int* __restrict__ positions, const TileDesc* __restrict__ tiles,
                                 __nv_bfloat16* __restrict__ out, int nq, int nkv, int G, int gp_shift,
-                                float scale_log2, int window, int* status, int open_late, MaskExt ext) {
+                                float scale_log2, int window, int* status, MaskExt ext) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kSub = (DK + 63) / 64, kVSub = DV / 64;   // sub-tiles of 64 columns in Q and K, in V
@@ -864,7 +866,8 @@ paged_flash_attention_ws_kernel(const __grid_constant__ CUtensorMap map_k, const
   const unsigned tmem = *tmem_holder;
   // only now may the kernel behind this one start: its resident, waiting blocks must not be
   // able to take tensor memory that a block of this grid still needs
-  pdl_open_and_wait(open_late);
+  pdl_trigger();
+  pdl_wait();
 
   // Blocks start in the order of their linear index.  The last tiles of a request read the most
   // keys: they come first, for every key/value head, so that the blocks that start last are
@@ -1169,7 +1172,7 @@ template <int DK, int DV, bool EXT = false>
 int launch_ws(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, const int* block_table,
               int max_pages, int page_shift, int num_pages, const int* positions, const void* tiles, int num_tiles,
               void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status,
-              cudaStream_t stream, int open_late = 0, MaskExt ext = MaskExt{DK, 0, 0}) {
+              cudaStream_t stream, MaskExt ext = MaskExt{DK, 0, 0}) {
   const int page_size = 1 << page_shift;
   const int box_rows = page_size < BNK ? page_size : BNK;
   const long long rows = ext.head_rows > 0 ? (long long)ext.head_rows * nkv : (long long)num_pages * nkv * page_size;
@@ -1198,7 +1201,7 @@ int launch_ws(const void* q, int q_row_stride, const void* k_pages, const void* 
   kvb_launch(paged_flash_attention_ws_kernel<DK, DV, EXT>, grid, dim3(kWsThreads), smem, stream, mk, mv, box_rows,
              (const __nv_bfloat16*)q, q_row_stride, block_table, max_pages, page_shift,
              num_pages, positions, (const TileDesc*)tiles, (__nv_bfloat16*)out, nq, nkv, G, gp_shift,
-             scale * 1.4426950408889634f, window, status, open_late, ext);
+             scale * 1.4426950408889634f, window, status, ext);
   return kvb_launch_result();
 }
 
@@ -1208,7 +1211,7 @@ template <int D, int NW, bool EXT = false>
 int launch(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, const int* block_table,
            int max_pages, int page_shift, int num_pages, const int* positions, const void* tiles, int num_tiles,
            void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status,
-           cudaStream_t stream, int open_late = 0, MaskExt ext = MaskExt{D, 0, 0}) {
+           cudaStream_t stream, MaskExt ext = MaskExt{D, 0, 0}) {
   constexpr int BM = NW * 16;
   const size_t smem = (size_t)BM * D * 2 + 4 * (size_t)BN * D * 2 + BM * sizeof(int);
   if (smem > 48 * 1024) {
@@ -1220,7 +1223,7 @@ int launch(const void* q, int q_row_stride, const void* k_pages, const void* v_p
   kvb_launch(paged_flash_attention_kernel<D, NW, EXT>, grid, dim3(NW * 32), smem, stream, (const __nv_bfloat16*)q,
              q_row_stride, (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, max_pages,
              page_shift, num_pages, positions, (const TileDesc*)tiles, (__nv_bfloat16*)out, nq, nkv, G, gp_shift,
-             scale * 1.4426950408889634f, window, status, open_late, ext);
+             scale * 1.4426950408889634f, window, status, ext);
   return kvb_launch_result();
 }
 
@@ -1253,13 +1256,12 @@ KVB_EXPORT int kvb_flash_attention_tokens_per_tile(int group, int wide) {
 // wide: 0: the tiles were cut for 64 query rows per block; 1: for 128; 2: for 128, and the
 // kernel is the tcgen05 form (head size 64 only); 3: for 128, the tcgen05 form with roles
 // (head size 64 or 128, pages of at least 8 rows, page pools aligned to 16 bytes).
-// open_late: the kernel behind works beside this one (see pdl_open_and_wait).
 // bfloat16 only.  out is [T, nq*d].
 KVB_EXPORT int kvb_paged_flash_attention(const void* q, int q_row_stride, const void* k_pages, const void* v_pages,
                                          const int* block_table, int max_pages, int page_size, int num_pages,
                                          const int* positions, const void* tiles, int num_tiles, int wide, void* out,
-                                         int nq, int nkv, int d, float scale, int window, int open_late,
-                                         int* status, cudaStream_t stream) {
+                                         int nq, int nkv, int d, float scale, int window, int* status,
+                                         cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
   if (nkv < 1 || nq % nkv) return KVB_ERR_BAD_SIZE;
   const int G = nq / nkv;
@@ -1274,18 +1276,18 @@ KVB_EXPORT int kvb_paged_flash_attention(const void* q, int q_row_stride, const 
       return KVB_ERR_BAD_SIZE;
     if (d == 64)
       return tc5::launch_ws<64, 64>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
-                                positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, open_late);
+                                positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream);
     return tc5::launch_ws<128, 128>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages,
-                               positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, open_late);
+                               positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream);
   }
   if (wide == 2) {   // tcgen05 form
     if (d != 64 || (reinterpret_cast<uintptr_t>(q) & 15) || (q_row_stride & 7)) return KVB_ERR_BAD_SIZE;
     return tc5::launch(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages, positions,
-                       tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, open_late, stream);
+                       tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream);
   }
 #define KVB_FA(D, NW)                                                                                           \
   return launch<D, NW>(q, q_row_stride, k_pages, v_pages, block_table, max_pages, page_shift, num_pages, positions, \
-                       tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, open_late)
+                       tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream)
   if (d == 64) { if (wide) KVB_FA(64, 8); KVB_FA(64, 4); }
   if (wide) KVB_FA(128, 8);
   KVB_FA(128, 4);
@@ -1318,13 +1320,13 @@ KVB_EXPORT int kvb_paged_flash_attention_rows(const void* q, int q_row_stride, c
     if (page_size < 8) return KVB_ERR_BAD_SIZE;
     if (d == 64)
       return tc5::launch_ws<64, 64, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
-                                      positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, 0, ext);
+                                      positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
     return tc5::launch_ws<128, 128, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages,
-                                     positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, 0, ext);
+                                     positions, tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext);
   }
 #define KVB_FA_EXT(D, NW)                                                                                              \
   return (launch<D, NW, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages, positions, \
-                              tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, 0, ext))
+                              tiles, num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext))
   if (d == 64) { if (wide) KVB_FA_EXT(64, 8); KVB_FA_EXT(64, 4); }
   if (wide) KVB_FA_EXT(128, 8);
   KVB_FA_EXT(128, 4);
@@ -1363,7 +1365,7 @@ KVB_EXPORT int kvb_paged_flash_attention_rows_masked(const void* q, int q_row_st
   const void* values = static_cast<const __nv_bfloat16*>(pages) + dk;
 #define KVB_WS(DK, DV)                                                                                                  \
   return (tc5::launch_ws<DK, DV, true>(q, q_row_stride, pages, values, block_table, max_pages, page_shift, num_pages, positions, tiles, \
-                                       num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, 0, ext))
+                                       num_tiles, out, nq, nkv, G, gp_shift, scale, window, status, stream, ext))
   if (wider) {
     if (dk == 192) KVB_WS(192, 128);
     KVB_WS(96, 64);

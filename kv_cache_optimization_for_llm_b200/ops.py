@@ -13,6 +13,7 @@ every matrix product of the float32 path, is a kernel of this package.
 from __future__ import annotations
 
 import collections
+import contextlib
 import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_uint, c_void_p
@@ -137,6 +138,27 @@ def _stream() -> c_void_p:
 
 def _capturing() -> bool:
     return _step_capturing if _step_capturing is not None else torch.cuda.is_current_stream_capturing()
+
+
+class side_stream:
+    """A stream beside the caller's (csrc/kernels/side_stream.cuh): launches on it find everything complete that was launched before the
+    ``with``, and what is launched behind the ``with`` finds them complete.  Inside, the launches on either stream touch nothing of the other's.
+    The tensors on it are the caller's stream's own: behind the ``with`` they may be given back as ever."""
+
+    def __enter__(self) -> c_void_p:
+        self.main, beside = _stream(), c_void_p()
+        rc = lib("decode_attention").kvb_side_fork(self.main, ctypes.byref(beside))
+        if rc != 0:
+            raise KernelError(f"side_stream: CUDA error {rc}")
+        return beside
+
+    def __exit__(self, exc_type, exc, tb):
+        rc = lib("decode_attention").kvb_side_join(self.main)
+        if rc != 0 and exc_type is None:
+            raise KernelError(f"side_stream: CUDA error {rc}")
+        if _marks is not None:
+            _mark("side_stream")
+        return False
 
 
 def _p(t: Optional[torch.Tensor]) -> c_void_p:
@@ -2376,7 +2398,7 @@ def tiles_of_height(batch, nt: int) -> torch.Tensor:
 
 def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window,
                     wide: Optional[bool] = None, skip_single: bool = False,
-                    out: Optional[torch.Tensor] = None, open_late: bool = False) -> torch.Tensor:
+                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Tensor-core attention for steps with runs of query tokens (bfloat16).  ``wide``:
     False: 64 query rows per block (mma.sync); True: 128 rows (mma.sync); 2: 128 rows on
     tcgen05 with the scores in tensor memory (head size 64); 3: the same with roles (a TMA
@@ -2384,8 +2406,7 @@ def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale
     8 rows); None:
     chosen from the step's size, the head size and the page size.  ``skip_single``: the step's
     leading single tokens (``batch.num_single``) are somebody else's: their tiles are left out.
-    ``out``: where the rows go; made here if not given.  ``open_late``: the next launch is a
-    :func:`decode_attention_mma` with ``beside``."""
+    ``out``: where the rows go; made here if not given."""
     _need_cuda(qkv, k_pages)
     skip = int(batch.num_single) if skip_single else 0
     T = qkv.shape[0] - skip
@@ -2402,14 +2423,13 @@ def flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale
             elif d == 64:
                 wide = 2
     tiles = flash_tiles(batch, nq // nkv, wide)[skip:]      # a single token is one tile, and they come first
-    assert tiles.shape[0] > 0 or not open_late      # the next launch counts on this one's being there
     if out is None:
         out = new((qkv.shape[0], nq * d), qkv.dtype, qkv.device)
     rc = lib("flash_attention").kvb_paged_flash_attention(
         _p(qkv), c_int(qkv.stride(0)), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]),
         c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), _p(batch.positions), _p(tiles), c_int(tiles.shape[0]),
         c_int(int(wide)), _p(out), c_int(nq), c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)),
-        c_int(1 if open_late else 0), _p(batch.status), _stream())
+        _p(batch.status), _stream())
     _check(rc, "paged_flash_attention")
     choices[f"flash_attention_{int(wide)}"] += 1
     return out
@@ -2468,7 +2488,7 @@ def decode_launch_context(batch) -> int:
 def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, ctx_len, cos, sin, rot,
                          nq, nkv, d, scale, window, status, max_ctx: int = 0,
                          trace: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                         beside: bool = False) -> torch.Tensor:
+                         stream: Optional[c_void_p] = None) -> torch.Tensor:
     """The attention of a bfloat16 decode step in one launch on tensor cores: rotary
     encoding of query and new key, cache write, attention over 128-key tiles spread over
     a cluster of blocks, merge through distributed shared memory.  No scratch.
@@ -2476,8 +2496,7 @@ def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, 
     size 64), whatever the batch; up to that many blocks share a (request, kv head).
     ``max_ctx``: the longest context of the step if the host knows it (the launch is sized
     for it), 0 otherwise.  ``out``: where the rows go ([tokens, nq d], the rows of the requests'
-    tokens are written); made here if not given.  ``beside``: the launch in front, with ``open_late``, has
-    none of these requests: the two run side by side."""
+    tokens are written); made here if not given.  ``stream``: launched there (:class:`side_stream`)."""
     _need_cuda(qkv, k_pages)
     assert qkv.dtype == torch.bfloat16
     R = ctx_len.numel()
@@ -2488,7 +2507,7 @@ def decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table, q_start, 
         c_int(block_table.shape[1]), c_int(k_pages.shape[2]), c_int(k_pages.shape[0]), _p(q_start), _p(ctx_len),
         _p(cos), _p(sin), c_int(0 if cos is None else cos.shape[0]), c_int(rot), _p(out), c_int(R), c_int(nq),
         c_int(nkv), c_int(d), c_float(scale), c_int(int(window or 0)), c_int(int(max_ctx)),
-        c_int(1 if beside else 0), _p(status), _p(trace), _stream())
+        _p(status), _p(trace), _stream() if stream is None else stream)
     _check(rc, "decode_attention_mma")
     choices["decode_attention_mma"] += 1
     return out
@@ -2501,6 +2520,27 @@ def _tiles_wanted(batch, nq: int, nkv: int, d: int, window: int, device) -> bool
     if key not in known:
         known[key] = paged_attention_tiles_wanted(batch.host["req_start"], batch.host["ctx_len"], nq, nkv, d, window, sm_count(device))
     return known[key]
+
+
+# Runs' tokens times the square of the attention's width times (1 + longest run's context / 1500) from which on a step launched by hand
+# has its single tokens' attention beside the runs' (see attention_beside_wanted).
+BESIDE_MIN_WORK = 3.9e9
+
+
+def attention_beside_wanted(batch, width: int) -> bool:
+    """Whether the attention of a step's single tokens runs on a stream beside the runs' attention.  On the GPU that is the faster form nearly
+    always: both are bound by latency and fill only part of it (24 heads of 128, 40 tokens of 100 to 2500 positions beside a run of 701 behind
+    512: the layer 263 us one after the other, 249 side by side; 60 steps of a 1B and a 3B shape replayed from graphs: 1 to 32 us less
+    in 55, level in 5).  But the events between the streams cost the host 5 us, which is what a layer takes longer where the host is the
+    bound (170 us a layer).  Launched by hand, all 34 of those steps below the line were slower side by side (by 4 to
+    6 us) and 25 of the 26 above it were faster; a captured step does not feel the host."""
+    if _capturing():
+        return True
+    ns = int(batch.num_single)
+    longest = batch.host.get("longest_run")
+    if longest is None:
+        longest = batch.host["longest_run"] = int(max(batch.host["ctx_len"][ns:]))
+    return (batch.num_tokens - ns) * float(width) ** 2 * (1.0 + longest / 1500.0) >= BESIDE_MIN_WORK
 
 
 def attention_step(qkv, k_pages, v_pages, write_kv, block_table, batch, nq, nkv, d, scale, window, max_positions,
@@ -2531,17 +2571,16 @@ def attention_step(qkv, k_pages, v_pages, write_kv, block_table, batch, nq, nkv,
         # Single tokens beside runs: the single tokens (the step's first rows) go to the kernel of
         # decode steps, which rotates, writes and attends in one launch, the runs to the two kernels
         # for runs.  As a tile of the kernel for runs a single token would fill 4 of 128 rows.
-        # The two kernels share no row, page or output and run side by side, the runs' blocks first: they are
-        # bound by latency and products, the single tokens' by the latency of short walks and by reading the cache (24 heads of
-        # 128, 40 tokens of 100 to 2500 positions beside a run of 701 behind 512: 101 -> 82 us).
         out = new((qkv.shape[0], nq * d), qkv.dtype, qkv.device)
         rope_kv_write(qkv[ns:], batch.positions[ns:], batch.token_req[ns:], cos, sin, k_pages if write_kv else None,
                       v_pages if write_kv else None, block_table, page_size, nq, nkv, d, rot, batch.status)
-        flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window,
-                        skip_single=True, out=out, open_late=True)
-        return decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table[:ns], batch.q_start[:ns + 1],
-                                    batch.ctx_len[:ns], cos, sin, rot, nq, nkv, d, scale, window, batch.status,
-                                    max_ctx=decode_launch_context(batch), out=out, beside=True)
+        # the two kernels share no row, page or output
+        with side_stream() if attention_beside_wanted(batch, nq * d) else contextlib.nullcontext() as beside:
+            flash_attention(qkv, k_pages, v_pages, block_table, batch, nq, nkv, d, scale, window, skip_single=True, out=out)
+            decode_attention_mma(qkv, k_pages, v_pages, write_kv, block_table[:ns], batch.q_start[:ns + 1], batch.ctx_len[:ns],
+                                 cos, sin, rot, nq, nkv, d, scale, window, batch.status,
+                                 max_ctx=decode_launch_context(batch), out=out, stream=beside)
+        return out
     rope_kv_write(qkv, batch.positions, batch.token_req, cos, sin, k_pages if write_kv else None,
                   v_pages if write_kv else None, block_table, page_size, nq, nkv, d, rot, batch.status)
     if qkv.dtype == torch.bfloat16 and not batch.decode_only and flash_attention_supported(d, group, page_size):
