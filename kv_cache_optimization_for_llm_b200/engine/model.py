@@ -97,14 +97,21 @@ class DecoderModel:
         ``max_tokens`` tokens with up to ``max_logit_rows`` rows of logits: the residual in
         float32 (every copy of it, where the model keeps several), the picked rows and their logits; and per layer the widths its parts declare
         (``activation_widths``; a part that declares none is taken as eight rows of the model's
-        width) in the compute precision, plus a fifth."""
+        width) in the compute precision, plus a fifth, and what its widest product borrows (``borrowed_width``; one product runs
+        at a time, and gives back what it borrowed)."""
         h, v = self.spec.hidden_size, self.spec.vocab_size
         copies = int(getattr(self.embedding, "stream_copies", 1))      # a residual stream kept as several copies
         copies += (1 if self.keeps_embedding else 0) + 2 * len(self.from_embedding)
         step = 4 * max_tokens * h * copies + max_logit_rows * 4 * (h + v) + (1 << 16)
         if self.ctx.dtype == torch.float32:
             step += max_logit_rows * 6 * h                 # the three bfloat16 parts of the picked rows
-        per_layer = 0
+
+        def borrowed(parts):
+            return max((p.borrowed_width() for p in parts if hasattr(p, "borrowed_width")), default=0)
+
+        step += 4 * max_tokens * borrowed(self.from_embedding.values())
+        before = borrowed(b for b in self.before if b is not None)
+        per_layer, lent = 0, 0
         entered = 3 * h if self.from_embedding else 0      # the stream's copy and the float32 product at the start of a pass
         for block in self.layers:
             widths = 0
@@ -112,8 +119,9 @@ class DecoderModel:
                 declared = getattr(part, "activation_widths", None)
                 widths += sum(declared()) if declared is not None else 8 * h
             per_layer = max(per_layer, (widths or 32 * h) + entered)
+            lent = max(lent, before, borrowed(getattr(block, "parts", {}).values()))
         esize = 4 if self.ctx.dtype == torch.float32 else 2
-        layer = int(1.2 * esize * max_tokens * per_layer) + (1 << 16)
+        layer = int(1.2 * esize * max_tokens * per_layer) + esize * max_tokens * lent + (1 << 16)
         return step, layer
 
     def query_tile_heights(self):

@@ -2160,6 +2160,11 @@ def float32_split_ok(w: torch.Tensor) -> bool:
 FLOAT32_SPLIT_MIN_K = 1024
 
 
+def float32_parts_width(w: torch.Tensor) -> int:
+    """Floats a row of A that a float32 product with ``w`` borrows for the bfloat16 parts (:func:`linear`); 0 where it needs none."""
+    return 3 * (-(-w.shape[1] // 8) * 8) // 2 if w.dtype == torch.float32 and float32_split_ok(w) else 0
+
+
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, into: Optional[torch.Tensor] = None):
     """``x . w^T`` with ``w`` [out, in].
     float32: this package's kernels, true 32-bit (long rows of W as three bfloat16 parts on the tensor cores, others by FMA).

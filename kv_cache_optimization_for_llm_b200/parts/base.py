@@ -35,6 +35,7 @@ from typing import Callable, Dict, Mapping, Optional
 
 import torch
 
+from ..ops import float32_parts_width
 from ..weights.loader import WeightSpec
 
 
@@ -65,3 +66,25 @@ class Part:
     def __init__(self, params: Mapping, weights: Mapping[str, torch.Tensor], ctx: BuildContext):
         self.params = dict(params)
         self.ctx = ctx
+
+    def borrowed_width(self) -> int:
+        """Elements of the compute type per token that one of the part's products borrows from the step's memory while it runs, beside
+        the tensors of ``activation_widths``: in float32 the bfloat16 parts of the widest product's rows."""
+        if self.ctx.dtype != torch.float32:
+            return 0
+        return max((float32_parts_width(w) for w in _matrices(vars(self))), default=0)
+
+
+def _matrices(held):
+    """Every matrix among what a part holds, in its lists and mappings and in the parts it holds as well."""
+    if isinstance(held, torch.Tensor):
+        if held.dim() == 2:
+            yield held
+    elif isinstance(held, Part):
+        yield from _matrices(vars(held))
+    elif isinstance(held, Mapping):
+        for value in held.values():
+            yield from _matrices(value)
+    elif isinstance(held, (list, tuple)):
+        for value in held:
+            yield from _matrices(value)

@@ -55,6 +55,9 @@ class SwiGLU(Part):
         inter, hidden = self.gate_up.shape[0] // 2, self.down.shape[0]
         return [2 * inter, inter, max(2 * hidden, hidden + 3 * inter // 2 if self.ctx.dtype == torch.float32 else 0)]
 
+    def borrowed_width(self):
+        return 0                     # among the widths above; the first product's parts find room where its activation will be
+
     def forward(self, x, batch, into=None):
         a = ops.linear_swiglu(x, self.gate_up, self.block)
         return ops.linear(a, self.down, into=into)
