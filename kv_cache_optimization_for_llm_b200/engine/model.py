@@ -117,7 +117,10 @@ class DecoderModel:
             widths = 0
             for part in getattr(block, "parts", {}).values():
                 declared = getattr(part, "activation_widths", None)
-                widths += sum(declared()) if declared is not None else 8 * h
+                if declared is None:
+                    widths += 8 * h
+                else:
+                    widths += sum(declared(max_tokens) if getattr(part, "widths_by_tokens", False) else declared())
             per_layer = max(per_layer, (widths or 32 * h) + entered)
             lent = max(lent, before, borrowed(getattr(block, "parts", {}).values()))
         esize = 4 if self.ctx.dtype == torch.float32 else 2

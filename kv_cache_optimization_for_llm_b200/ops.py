@@ -498,9 +498,10 @@ def _with_scratch(nbytes: int, device, call):
         return call(scratch)
 
 
-def delta_pieces_width(heads: int, dk: int, dv: int) -> int:
-    """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs."""
-    if dk != 64 or dv not in (32, 64):
+def delta_pieces_width(heads: int, dk: int, dv: int, tokens: Optional[int] = None) -> int:
+    """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs; 0 where steps of up to ``tokens``
+    tokens hold no such run."""
+    if dk != 64 or dv not in (32, 64) or (tokens is not None and tokens < DELTA_PIECES_MIN_RUN):
         return 0
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong
@@ -1623,16 +1624,21 @@ def _pieces_unit(rule: str, heads: int, n: int, dv: int) -> int:
     return heads * (dv // 64 * per_block + per_head)
 
 
-def pieces_width(rule: str, heads: int, n: int, dv: int) -> int:
-    """bfloat16 elements per token that :func:`ssd_scan` and :func:`mlstm_scan` want for their scratch in steps of long runs."""
-    if n not in (64, 128) or dv % 64:
+def _pieces_wanted(longest: int, tokens: int, heads: int, dv: int) -> bool:
+    return longest >= PIECES_MIN_RUN and tokens * heads * (dv // 64) >= PIECES_MIN_WORK
+
+
+def pieces_width(rule: str, heads: int, n: int, dv: int, tokens: Optional[int] = None) -> int:
+    """bfloat16 elements per token that :func:`ssd_scan` and :func:`mlstm_scan` want for their scratch in steps of long runs; 0 where no
+    step of up to ``tokens`` tokens is one."""
+    if n not in (64, 128) or dv % 64 or (tokens is not None and not _pieces_wanted(tokens, tokens, heads, dv)):
         return 0
     return -(-_pieces_unit(rule, heads, n, dv) // 128)
 
 
 def _pieces_bytes(rule: str, batch, tokens: int, heads: int, n: int, dv: int, device) -> int:
     """Bytes of scratch for a walk in three launches, 0 where the runs walk in one (short runs, or an arena without the room)."""
-    if (int(getattr(batch, "max_q_len", 0) or 0) < PIECES_MIN_RUN or tokens * heads * (dv // 64) < PIECES_MIN_WORK):
+    if not _pieces_wanted(int(getattr(batch, "max_q_len", 0) or 0), tokens, heads, dv):
         return 0
     pieces = tokens // 64 + batch.num_reqs - int(batch.num_single)
     nbytes = pieces * _pieces_unit(rule, heads, n, dv) + 64

@@ -15,6 +15,8 @@ nothing of the model it sits in.  Interfaces by family:
                  ``forward(residual, delta, batch, cache) -> (residual, delta)``
 * a part that holds further parts (a ``PartSpec`` among its params) builds them with
   ``ctx.make(family, spec)``, which also hands them their tensors
+* a part may tell the widths of the tensors that one call produces (``activation_widths()``, elements per token); with
+  ``widths_by_tokens = True`` it also takes the tokens of the largest step, without which the widths are those of a step of any length
 * a mixer or feed-forward may set ``fuses_residual = True``; it then has
   ``fold_input_scale(vector)``, and its ``forward`` also takes ``into=residual`` and may get
   ``x`` as an ``ops.PendingNorm`` (see the prenorm block)

@@ -220,9 +220,11 @@ class GatedDelta(Part):
     def cache_spec(self):
         return SlotStateSpec((self.matrix_floats + (self.taps - 1) * self.channels,), torch.float32)
 
-    def activation_widths(self):
+    widths_by_tokens = True
+
+    def activation_widths(self, tokens=None):
         hv = self.heads * self.vdim
-        pieces = ops.delta_pieces_width(self.heads, self.dim, self.vdim) if self.ctx.dtype == torch.bfloat16 else 0
+        pieces = ops.delta_pieces_width(self.heads, self.dim, self.vdim, tokens) if self.ctx.dtype == torch.bfloat16 else 0
         return [self.w_in.shape[0], self.channels, hv, 3 * hv, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):

@@ -142,8 +142,10 @@ class StateSpaceDuality(Part):
     def cache_spec(self):
         return SlotStateSpec((self.matrix_floats + (self.taps - 1) * self.channels,), torch.float32)
 
-    def activation_widths(self):
-        pieces = ops.pieces_width("ssd", self.H, self.N, self.Dv) if self.ctx.dtype == torch.bfloat16 else 0
+    widths_by_tokens = True
+
+    def activation_widths(self, tokens=None):
+        pieces = ops.pieces_width("ssd", self.H, self.N, self.Dv, tokens) if self.ctx.dtype == torch.bfloat16 else 0
         return [self.w_in.shape[0], self.channels, 2 * self.inner, self.inner, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):
@@ -202,9 +204,11 @@ class MatrixLSTM(Part):
     def cache_spec(self):
         return SlotStateSpec((self.state_floats,), torch.float32)
 
-    def activation_widths(self):
+    widths_by_tokens = True
+
+    def activation_widths(self, tokens=None):
         inner = self.H * self.Dv
-        pieces = ops.pieces_width("mlstm", self.H, self.D, self.Dv) if self.ctx.dtype == torch.bfloat16 else 0
+        pieces = ops.pieces_width("mlstm", self.H, self.D, self.Dv, tokens) if self.ctx.dtype == torch.bfloat16 else 0
         return [self.w_in.shape[0], 2 * (2 * self.H + 8), 2 * inner, inner, self.o.shape[0], pieces]
 
     def forward(self, x, batch, cache):

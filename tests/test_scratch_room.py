@@ -1,0 +1,28 @@
+"""Room for the scratch of the state memories' launches: declared where a step can be long enough for them, and nowhere else."""
+
+import pytest
+import torch
+
+
+def _part(kind, params):
+    from kv_cache_optimization_for_llm_b200.parts import BuildContext, lookup
+    cls = lookup("mixer", kind)
+    ctx = BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), max_positions=64, status=torch.zeros(1, dtype=torch.int32))
+    weights = {r: torch.zeros(ws.shape, dtype=torch.float32 if ws.kind in ("vector", "bias") else torch.bfloat16)
+               for r, ws in cls.weight_specs(params).items()}
+    return cls(params, weights, ctx)
+
+
+MLSTM = {"hidden_size": 64, "dim": 64, "vdim": 64, "gate_cap": 15.0, "eps": 1e-6}
+SSD = {"hidden_size": 64, "vdim": 64, "state": 128, "groups": 8, "norm_groups": 8, "conv": 4, "eps": 1e-6}
+DELTA = {"hidden_size": 64, "kv_heads": 4, "dim": 64, "vdim": 64, "conv": 4, "eps": 1e-6}
+
+
+@pytest.mark.parametrize("kind,params,heads,tokens,wanted", [
+    ("mlstm", MLSTM, 16, 2048, False), ("mlstm", MLSTM, 16, 4096, True), ("mlstm", MLSTM, 32, 1024, False), ("mlstm", MLSTM, 32, 2048, True),
+    ("state_space_duality", SSD, 64, 512, False), ("state_space_duality", SSD, 64, 2048, True),
+    ("gated_delta", DELTA, 16, 511, False), ("gated_delta", DELTA, 16, 512, True)])
+def test_scratch_is_declared_where_a_step_can_take_it(kind, params, heads, tokens, wanted):
+    part = _part(kind, dict(params, heads=heads))
+    without, any_step, here = sum(part.activation_widths(1)), sum(part.activation_widths()), sum(part.activation_widths(tokens))
+    assert any_step > without and here == (any_step if wanted else without)
