@@ -44,6 +44,10 @@ class _Region:
     def reset(self) -> None:
         self.block, self.offset = 0, self.pads[0]
 
+    def room(self) -> int:
+        """Bytes that the block in use still has: what the next tensor may take without another block."""
+        return self.pads[self.block] + self.capacity - self.offset
+
     def place(self, nbytes: int):
         """Where a run of ``nbytes`` bytes on a 256-byte boundary lies, as (block, offset), or None
         if the request is larger than the region was built for."""
@@ -123,6 +127,9 @@ class StepArena:
             self.bypassed += 1
             return torch.empty(shape, dtype=dtype, device=self.device)
         return t
+
+    def room(self) -> int:
+        return self.current.room()
 
     def bytes_held(self) -> int:
         return sum(b.numel() for r in (self.step, *self.halves) for b in r.blocks)

@@ -490,6 +490,12 @@ def _at(t: torch.Tensor, col: int) -> int:
 DELTA_PIECES_MIN_RUN = 512
 
 
+def _has_room(nbytes: int, device) -> bool:
+    """Whether the running step's arena lends ``nbytes`` without growing (a step of many short runs has more pieces than its tokens alone
+    would make); without an arena the allocator does."""
+    return _arena is None or _arena.device != device or nbytes <= _arena.room()
+
+
 def _with_scratch(nbytes: int, device, call):
     """``call`` with a buffer of ``nbytes`` that is given back behind its launches, or with None where it wants none."""
     if not nbytes:
@@ -516,9 +522,7 @@ def _delta_pieces_bytes(batch, tokens: int, heads: int, dk: int, dv: int, device
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong
     nbytes = int(fn(c_longlong(tokens), c_int(batch.num_reqs - int(batch.num_single)), c_int(heads), c_int(dk), c_int(dv)))
-    if _arena is not None and _arena.device == device and nbytes > _arena.current.capacity:
-        return 0
-    return nbytes
+    return nbytes if _has_room(nbytes, device) else 0
 
 
 def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux, decay_bias, aux_bias, head_rate,
@@ -1642,9 +1646,7 @@ def _pieces_bytes(rule: str, batch, tokens: int, heads: int, n: int, dv: int, de
         return 0
     pieces = tokens // 64 + batch.num_reqs - int(batch.num_single)
     nbytes = pieces * _pieces_unit(rule, heads, n, dv) + 64
-    if pieces > 65535 or (_arena is not None and _arena.device == device and nbytes > _arena.current.capacity):
-        return 0
-    return nbytes
+    return 0 if pieces > 65535 or not _has_room(nbytes, device) else nbytes
 
 
 class _DiagArgs(ctypes.Structure):

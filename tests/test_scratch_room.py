@@ -26,3 +26,28 @@ def test_scratch_is_declared_where_a_step_can_take_it(kind, params, heads, token
     part = _part(kind, dict(params, heads=heads))
     without, any_step, here = sum(part.activation_widths(1)), sum(part.activation_widths()), sum(part.activation_widths(tokens))
     assert any_step > without and here == (any_step if wanted else without)
+
+
+@pytest.mark.parametrize("rule", ["ssd", "delta"])
+@pytest.mark.parametrize("runs", [1, 40])
+@pytest.mark.parametrize("taken", [0.0, 0.9])
+def test_a_step_without_the_room_left_walks_in_one_launch(rule, runs, taken):
+    """A layer's region of which other tensors hold a part, and a step of many short runs beside a long one, whose pieces are more than
+    its tokens'."""
+    from types import SimpleNamespace
+    from kv_cache_optimization_for_llm_b200 import ops
+    from kv_cache_optimization_for_llm_b200.engine.arena import StepArena
+    device, tokens = torch.device("cpu"), 2048
+    batch = SimpleNamespace(max_q_len=1024, num_reqs=runs, num_single=0)
+    width = ops.pieces_width("ssd", 64, 128, 64) if rule == "ssd" else ops.delta_pieces_width(32, 64, 64)
+    arena = StepArena(device, 1 << 16, int(1.2 * 2 * tokens * width))
+    arena.begin_layer()
+    with ops.use_arena(arena):
+        arena.new((int(taken * arena.current.capacity),), torch.uint8)
+        nbytes = (ops._pieces_bytes("ssd", batch, tokens, 64, 128, 64, device) if rule == "ssd"
+                  else ops._delta_pieces_bytes(batch, tokens, 32, 64, 64, device))
+        assert (nbytes > 0) == (runs == 1 and not taken)
+        if nbytes:
+            with ops.lent((nbytes,), torch.uint8, device):
+                pass
+    assert arena.blocks_grown() == 0 and arena.bypassed == 0
