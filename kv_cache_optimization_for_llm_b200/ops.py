@@ -490,6 +490,9 @@ def _at(t: torch.Tensor, col: int) -> int:
 DELTA_PIECES_MIN_RUN = 512
 
 
+GRID_MAX_Y = 65535      # blocks of a grid's second dimension: pieces (and heads) that the walks in three launches can have
+
+
 def _has_room(nbytes: int, device) -> bool:
     """Whether the running step's arena lends ``nbytes`` without growing (a step of many short runs has more pieces than its tokens alone
     would make); without an arena the allocator does."""
@@ -519,9 +522,12 @@ def _delta_pieces_bytes(batch, tokens: int, heads: int, dk: int, dv: int, device
     room)."""
     if dk != 64 or dv not in (32, 64) or int(getattr(batch, "max_q_len", 0) or 0) < DELTA_PIECES_MIN_RUN:
         return 0
+    runs = batch.num_reqs - int(batch.num_single)
+    if tokens // 64 + runs > GRID_MAX_Y:
+        return 0
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong
-    nbytes = int(fn(c_longlong(tokens), c_int(batch.num_reqs - int(batch.num_single)), c_int(heads), c_int(dk), c_int(dv)))
+    nbytes = int(fn(c_longlong(tokens), c_int(runs), c_int(heads), c_int(dk), c_int(dv)))
     return nbytes if _has_room(nbytes, device) else 0
 
 
@@ -1646,7 +1652,7 @@ def _pieces_bytes(rule: str, batch, tokens: int, heads: int, n: int, dv: int, de
         return 0
     pieces = tokens // 64 + batch.num_reqs - int(batch.num_single)
     nbytes = pieces * _pieces_unit(rule, heads, n, dv) + 64
-    return 0 if pieces > 65535 or not _has_room(nbytes, device) else nbytes
+    return 0 if max(pieces, heads * (dv // 64)) > GRID_MAX_Y or not _has_room(nbytes, device) else nbytes
 
 
 class _DiagArgs(ctypes.Structure):

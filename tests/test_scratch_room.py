@@ -51,3 +51,14 @@ def test_a_step_without_the_room_left_walks_in_one_launch(rule, runs, taken):
             with ops.lent((nbytes,), torch.uint8, device):
                 pass
     assert arena.blocks_grown() == 0 and arena.bypassed == 0
+
+
+@pytest.mark.parametrize("tokens,runs,heads,wanted", [(4096, 4, 64, True), (64 * 65000, 600, 64, False), (4096, 65500, 64, False)])
+def test_grids_beyond_the_hardwares_limit_walk_in_one_launch(tokens, runs, heads, wanted):
+    """More pieces than a grid's second dimension holds, which the walk in one launch, a block a run, takes."""
+    from types import SimpleNamespace
+    from kv_cache_optimization_for_llm_b200 import ops
+    batch = SimpleNamespace(max_q_len=1024, num_reqs=runs, num_single=0)
+    assert (ops._delta_pieces_bytes(batch, tokens, heads, 64, 64, torch.device("cpu")) > 0) == wanted
+    assert (ops._pieces_bytes("ssd", batch, tokens, heads, 128, 64, torch.device("cpu")) > 0) == wanted
+    assert ops._pieces_bytes("ssd", batch, 4096, 65536, 128, 64, torch.device("cpu")) == 0
