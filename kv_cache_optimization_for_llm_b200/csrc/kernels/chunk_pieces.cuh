@@ -527,13 +527,12 @@ static int launch_sized(const Args& a, int R, long long tokens, void* scratch, c
   sc.gates = reinterpret_cast<unsigned char*>(sc.sums + count * a.H);
   sc.m = reinterpret_cast<float*>(sc.gates + count * a.H * gate_bytes(RULE));
   const dim3 grid((unsigned)(a.H * splits), (unsigned)count);
-  static bool sized = false;
-  cudaError_t e = cudaSuccess;
-  if (!sized) {
-    e = cudaFuncSetAttribute(changes_kernel<RULE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChangesLayout<RULE, N>::bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(results_kernel<RULE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ResultsLayout<RULE, N>::bytes);
-    sized = e == cudaSuccess;
-  }
+  static OncePerDevice sized;
+  cudaError_t e = sized(kvb_device(), [] {
+    const cudaError_t first = cudaFuncSetAttribute(changes_kernel<RULE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChangesLayout<RULE, N>::bytes);
+    if (first != cudaSuccess) return first;
+    return cudaFuncSetAttribute(results_kernel<RULE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ResultsLayout<RULE, N>::bytes);
+  });
   if (e == cudaSuccess) e = kvb_launch(changes_kernel<RULE, N>, grid, dim3(kAll), ChangesLayout<RULE, N>::bytes, stream, a, R, sc);
   if (e == cudaSuccess)
     e = kvb_launch(states_kernel<RULE, N>, dim3((unsigned)((cols_of(RULE) * N / 4 + 255) / 256), (unsigned)(a.H * splits), (unsigned)R),

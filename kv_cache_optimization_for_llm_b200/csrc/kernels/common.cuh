@@ -58,6 +58,8 @@ __device__ __forceinline__ float warp_max(float v) {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+#include "per_device.h"
+
 #include <cstdlib>
 #include <utility>
 
@@ -83,6 +85,12 @@ static inline cudaError_t kvb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 b
   cfg.attrs = attr;
   cfg.numAttrs = kvb_pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...);
+}
+
+// The current device, -1 if there is none.
+static inline int kvb_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
 
 // SMs of the current device, asked once per device: what launchers size their grids by.

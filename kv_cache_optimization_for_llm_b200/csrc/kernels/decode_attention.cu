@@ -698,10 +698,13 @@ constexpr size_t smem_bytes() {
          (kTma ? 1024 + (size_t)kStages * 4 * 8 + 2 * D * 2 + 16 : 0);   // alignment, barriers, new key and value, flag
 }
 
-// How many clusters of `blocks_per_cluster` blocks of this form the GPU holds at once (0: the query failed).
+// How many clusters of `blocks_per_cluster` blocks of this form the current device holds at once (0: the query failed).
 template <int D, int GP, int kClasses, int kStages, bool kTma>
 int clusters_at_once(int blocks_per_cluster) {
-  static int answer[17] = {};      // by cluster size; 0: not asked yet, -1: the query failed
+  static int answers[64][17] = {};      // by device and cluster size; 0: not asked yet, -1: the query failed
+  const int device = kvb_device();
+  int unkept[17] = {};
+  int* answer = device >= 0 && device < 64 ? answers[device] : unkept;
   if (answer[blocks_per_cluster] == 0) {
     constexpr size_t smem = smem_bytes<D, GP, kClasses, kStages, kTma>();
     auto* fn = decode_attention_mma_kernel<D, GP, kClasses, kStages, kTma>;
@@ -736,20 +739,21 @@ int launch(const CUtensorMap& map_k, const CUtensorMap& map_v, const void* qkv, 
            const float* sin_t, int table_len, int rot, void* out, int R, int nq, int nkv, float scale, int window,
            int blocks_per_cluster, int* status, unsigned long long* trace, cudaStream_t stream) {
   const size_t smem = smem_bytes<D, GP, kClasses, kStages, kTma>();
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice sized;      // one per instantiation
+  const cudaError_t se = sized(kvb_device(), [&]() -> cudaError_t {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(decode_attention_mma_kernel<D, GP, kClasses, kStages, kTma>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return (int)e;
+      if (e != cudaSuccess) return e;
     }
     if (kClasses > 8) {   // clusters of 16 are beyond the portable size
       cudaError_t e = cudaFuncSetAttribute(decode_attention_mma_kernel<D, GP, kClasses, kStages, kTma>,
                                            cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return (int)e;
+      if (e != cudaSuccess) return e;
     }
-    attr_set = true;
-  }
+    return cudaSuccess;
+  });
+  if (se != cudaSuccess) return (int)se;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nkv, R, blocks_per_cluster);
   cfg.blockDim = dim3(kThreads, 1, 1);

@@ -729,13 +729,14 @@ int launch(const void* q, int q_row_stride, const void* k_pages, const void* v_p
            void* out, int nq, int nkv, int G, int gp_shift, float scale, int window, int* status,
            cudaStream_t stream) {
   const size_t smem = 1024 + (size_t)kQBytes + 4 * (size_t)kKVBytes + kPBytes + 2 * BM * 4 + 64;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice sized;      // one per instantiation
+  const cudaError_t se = sized(kvb_device(), [&]() -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(paged_flash_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+    if (e != cudaSuccess) return e;
+    return cudaSuccess;
+  });
+  if (se != cudaSuccess) return (int)se;
   dim3 grid(num_tiles, nkv);
   kvb_launch(paged_flash_attention_tc_kernel, grid, dim3(kThreads), smem, stream, (const __nv_bfloat16*)q, q_row_stride,
              (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, max_pages, page_shift,
@@ -1186,17 +1187,18 @@ int launch_ws(const void* q, int q_row_stride, const void* k_pages, const void* 
   constexpr size_t smem = 1024 + (size_t)kSub * BM * 128 + (size_t)(ws_key_stages(DK) * kSub + ws_value_stages(DK) * kVSub) * BNK * 128 +
                           kPB * kPBytes + sizeof(WsBars) + 64;
   static_assert(2 * smem + 2048 <= 228 * 1024, "two blocks an SM");
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice sized;      // one per instantiation
+  const cudaError_t se = sized(kvb_device(), [&]() -> cudaError_t {
     cudaError_t ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DK, DV, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem);
-    if (ce != cudaSuccess) return (int)ce;
+    if (ce != cudaSuccess) return ce;
     // two blocks per SM need the largest shared-memory configuration
     ce = cudaFuncSetAttribute(paged_flash_attention_ws_kernel<DK, DV, EXT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                               (int)cudaSharedmemCarveoutMaxShared);
-    if (ce != cudaSuccess) return (int)ce;
-    attr_set = true;
-  }
+    if (ce != cudaSuccess) return ce;
+    return cudaSuccess;
+  });
+  if (se != cudaSuccess) return (int)se;
   dim3 grid(num_tiles, nkv);
   kvb_launch(paged_flash_attention_ws_kernel<DK, DV, EXT>, grid, dim3(kWsThreads), smem, stream, mk, mv, box_rows,
              (const __nv_bfloat16*)q, q_row_stride, block_table, max_pages, page_shift,

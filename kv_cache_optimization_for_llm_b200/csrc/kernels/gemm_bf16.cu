@@ -724,14 +724,15 @@ int gemm_skinny_launch(const void* x, int ldx, const void* w, int ldw, void* out
   (void)x_is_static;
   e = cached_map(&mx, x, M, K, ldx, MP);
   if (e) return e;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice sized;      // one per instantiation
+  const cudaError_t se = sized(kvb_device(), [&]() -> cudaError_t {
     cudaError_t ce = cudaFuncSetAttribute(gemm_skinny_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);  // the kernel also has a little static shared memory
-    if (ce != cudaSuccess) return (int)ce;
+    if (ce != cudaSuccess) return ce;
     ce = cudaFuncSetAttribute(gemm_skinny_kernel<0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (ce != cudaSuccess) return (int)ce;
-    attr_set = true;
-  }
+    if (ce != cudaSuccess) return ce;
+    return cudaSuccess;
+  });
+  if (se != cudaSuccess) return (int)se;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, splits, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);

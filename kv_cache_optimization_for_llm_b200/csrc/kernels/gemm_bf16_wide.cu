@@ -649,16 +649,6 @@ int cached_map(CUtensorMap* out, const void* ptr, int rows, int K, int ld, int b
   return 0;
 }
 
-int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
-      n = kvb_sm_count();
-  }
-  return n;
-}
-
 template <int MT, int BN, int EPI>
 int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, Params p, cudaStream_t stream) {
   const size_t stage_bytes = (size_t)(MT * BM + BN) * BK * 2;
@@ -666,14 +656,15 @@ int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, Params p, cudaStre
   if (stages > kMaxStages) stages = kMaxStages;
   p.stages = stages;
   const size_t smem = 1024 + stages * stage_bytes + sizeof(Bars) + 64;
-  static bool attr_set = false;   // one per instantiation
-  if (!attr_set) {
+  static OncePerDevice sized;      // one per instantiation
+  const cudaError_t se = sized(kvb_device(), [&]() -> cudaError_t {
     cudaError_t ce = cudaFuncSetAttribute(gemm_wide_kernel<MT, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (ce != cudaSuccess) return (int)ce;
-    attr_set = true;
-  }
+    if (ce != cudaSuccess) return ce;
+    return cudaSuccess;
+  });
+  if (se != cudaSuccess) return (int)se;
   const int total = p.m_tiles * p.n_tiles;
-  const int blocks = total < sm_count() ? total : sm_count();
+  const int blocks = total < kvb_sm_count() ? total : kvb_sm_count();
   kvb_launch(gemm_wide_kernel<MT, BN, EPI>, dim3(blocks), dim3(64 + 128 * MT), smem, stream, mx, mw, p);
   return kvb_launch_result();
 }
@@ -698,17 +689,20 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, Params p, cudaStre
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  static int max_pairs = 0;
+  static int pairs_of[64] = {};      // by device; 0: not asked yet
+  const int device = kvb_device();
+  int unkept = 0;
+  int& max_pairs = device >= 0 && device < 64 ? pairs_of[device] : unkept;
   if (!max_pairs) {
     cudaError_t ce = cudaFuncSetAttribute(gemm_wide_pair_kernel<PBN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ce != cudaSuccess) return (int)ce;
-    cfg.gridDim = dim3(2 * (sm_count() / 2), 1, 1);
+    cfg.gridDim = dim3(2 * (kvb_sm_count() / 2), 1, 1);
     cfg.numAttrs = 1;
     int n = 0;
     ce = cudaOccupancyMaxActiveClusters(&n, gemm_wide_pair_kernel<PBN, EPI>, &cfg);
     if (ce != cudaSuccess) return (int)ce;
     if (n < 1) return KVB_ERR_BAD_SIZE;
-    max_pairs = n < sm_count() / 2 ? n : sm_count() / 2;
+    max_pairs = n < kvb_sm_count() / 2 ? n : kvb_sm_count() / 2;
   }
   const int total = p.m_tiles * p.n_tiles;
   const int pairs = total < max_pairs ? total : max_pairs;
@@ -728,7 +722,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, Params p, cudaStre
 // time a tile of that shape takes per 64 of K (measured on a B200, microseconds: a single block
 // is bound by the operand bytes it takes in per product, a pair by the tensor pipe).
 KVB_EXPORT int kvb_gemm_wide_tile(int M, int N, int epilogue, int* rows, int* cols, int* pair) {
-  const int sms = sm_count();
+  const int sms = kvb_sm_count();
   double best_cost = 0;
   *rows = 0;
   for (int form = 0; form < 5; ++form) {
