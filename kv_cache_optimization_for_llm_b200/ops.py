@@ -1153,13 +1153,15 @@ MADE_WIDER = ((192, 128), (96, 64))
 
 
 def flash_attention_rows_masked_wanted(batch, heads: int, kv_heads: int, dk: int, dv: int, page_size: int,
-                                       dtype: torch.dtype, q: Optional[torch.Tensor] = None, made: bool = False) -> bool:
+                                       dtype: torch.dtype, q: Optional[torch.Tensor] = None, made: bool = False,
+                                       scale: float = 1.0) -> bool:
     """Whether a step's attention over blocks of positions goes to the tcgen05 kernel with roles: bfloat16, key and value
     size both 64 or both 128 (``made`` rows: 192 and 128 or 96 and 64 as well), pages of at least 8 rows, and 128-row tiles enough to fill
-    the GPU (twice over at head size 64), as for the other designs' prompt portions.  (For keys wider than values it is the faster one at any number of tiles.)"""
+    the GPU (twice over at head size 64), as for the other designs' prompt portions.  (For keys wider than values it is the faster one at any number of tiles.)
+    Its softmax works on scores that are not scaled yet, so ``scale`` has to be above zero; the kernel on mma.sync takes any."""
     wider = made and (dk, dv) in MADE_WIDER
     if not (dtype == torch.bfloat16 and ((dk == dv and dk in (64, 128)) or wider) and page_size >= 8 and FLASH_WIDE and FLASH_TC
-            and FLASH_TC_ROLES and FLASH_ROWS_WIDE in (None, 3)):
+            and FLASH_TC_ROLES and FLASH_ROWS_WIDE in (None, 3) and scale > 0.0):
         return False
     group = heads // kv_heads
     if not flash_attention_supported(dv, group, page_size):

@@ -156,7 +156,7 @@ class LatentAttention(Part):
         if rdims:        # (without a position the part behind the latent is cached, and compared, as it is)
             ops.latent_rotate(q, n, self.heads, per_head, self.dim, cos, sin, batch)
         if self._tcgen05_sizes(self.params) and ops.flash_attention_rows_masked_wanted(batch, self.heads, self.heads, per_head, self.vdim,
-                                                                                       rows.PAGE, self.ctx.dtype, q, made=True):
+                                                                                       rows.PAGE, self.ctx.dtype, q, made=True, scale=self.scale):
             a = ops.flash_attention_rows_masked(q, None, None, batch, self.heads, self.heads, per_head, self.scale, sinks=self.sink,
                                                 window=self.window or 0, rows=rows, dv=self.vdim)
         else:

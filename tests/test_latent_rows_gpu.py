@@ -50,7 +50,7 @@ def _plain(x, w, heads, dim, rot, vdim, rank, scale, eps, sink, gate, window, di
 @pytest.mark.parametrize("heads,dim,rot,vdim,rank,sink,gate,window", [
     (4, 128, 64, 128, 128, True, False, None), (2, 64, 32, 64, 64, False, True, None), (3, 24, 8, 40, 72, True, True, 100),
     (2, 96, 96, 16, 64, False, False, 64), (2, 120, 8, 128, 64, True, True, None)])
-def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, window):
+def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, window, scale=None):
     from kv_cache_optimization_for_llm_b200 import ops
     from kv_cache_optimization_for_llm_b200.models.spec import PartSpec
     rng = np.random.default_rng(dim + rot)
@@ -66,7 +66,7 @@ def test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, gate, 
     for n, s in shapes.items():
         wt[n], w64[n] = _w(rng, s, 0.1, 1.0) if n.endswith("norm") else _w(rng, s, 1.0 / math.sqrt(s[-1]) if len(s) > 1 else 0.5)
     params = {"hidden_size": W, "heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": qr, "kv_rank": rank,
-              "scale": (dim + rot) ** -0.5, "eps": 1e-6, "sink": sink, "gate": gate, "window": window,
+              "scale": (dim + rot) ** -0.5 if scale is None else scale, "eps": 1e-6, "sink": sink, "gate": gate, "window": window,
               "position": PartSpec("rope_interleaved", {"dims": rot, "base": 10000.0})}
     mixer = _make("mixer", "latent_attention", params, wt, ctx)
     assert mixer.ukv is not None
@@ -99,6 +99,14 @@ def test_made_rows_with_keys_wider_than_values_on_tcgen05(heads, dim, rot, vdim,
     before = ops.choices["flash_attention_rows_masked"]
     test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, False, window)
     assert ops.choices["flash_attention_rows_masked"] > before
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.07])
+def test_scales_that_the_tcgen05_kernel_refuses_stay_on_the_other(scale):
+    from kv_cache_optimization_for_llm_b200 import ops
+    before = ops.choices["flash_attention_rows_masked"]
+    test_made_rows_with_a_rotated_part(2, 64, 32, 64, 64, True, False, None, scale)
+    assert ops.choices["flash_attention_rows_masked"] == before
 
 
 @pytest.mark.parametrize("dims", [0, 8, 24])       # of 24 channels behind the key: none (the layer has no position), some, all
