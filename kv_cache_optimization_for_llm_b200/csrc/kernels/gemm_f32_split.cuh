@@ -7,8 +7,9 @@
 // longer than 64 k: float32 additions that round to nearest add these pieces up.  Root mean square error over that of the result,
 // normal operands: 3.2e-7 to 3.4e-7 for 1024 to 8192 k, a chain of K fmaf 5.7e-7 (1024), 8.1e-7 (2048), 1.6e-6 (8192).
 // A result that is not finite is made again by the chain of fmaf from the float32 operands, so infinities and NaNs come out as
-// that kernel's; a magnitude above the largest bfloat16 arrives there too.  (Operands below 2^-110 lose the bits that bfloat16
-// cannot hold there.)
+// that kernel's; a magnitude above the largest bfloat16 arrives there too.  Operands below 2^-110 lose the bits that bfloat16 cannot hold
+// there, 2^-126 each at most; a result below 2^-64, where that could show, is made again in the same way.  (What
+// remains: magnitudes above 2^38 / K beside those, and results that are all of operands below float32's own normal range, which may come out as 0.)
 //
 // Measured (M x N x K, this kernel with the split of A / the chain of fmaf, us): 1 x 2048 x 2048 21 / 59, 338 x 3072 x 2048 54 / 135,
 // 338 x 16384 x 2048 142 / 585, 338 x 2048 x 8192 75 / 513, 2048 x 2048 x 2048 153 / 402, 1 x 128256 x 2048 291 / 455.
@@ -107,8 +108,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
   *reinterpret_cast<uint2*>(parts + 2 * plane + at) = l;
 }
 
-// The element as the chain of fmaf makes it: for results that are not finite.
-__device__ __noinline__ float chain(const Params& p, int m, int n) {
+// The element as the chain of fmaf makes it: for results that are not finite, and for those so small that the parts' lost bits could show.
+__device__ __noinline__ float chain(const Params& p, int m, int n, float v) {
+  if (v == 0.f) return v;
   const float *x = p.a + (size_t)m * p.lda, *w = p.w + (size_t)n * p.ldw;
   float s = 0.f;
   for (int k = 0; k < p.K; ++k) s = fmaf(x[k], w[k], s);
@@ -116,7 +118,8 @@ __device__ __noinline__ float chain(const Params& p, int m, int n) {
 }
 __device__ __forceinline__ void put(const Params& p, int m, int n, float v) {
   if (m >= p.M || n >= p.N) return;
-  if ((__float_as_uint(v) & 0x7f800000u) == 0x7f800000u) v = chain(p, m, n);
+  constexpr unsigned small = 0x1f800000u, infinite = 0x7f800000u;      // 2^-64
+  if ((__float_as_uint(v) & 0x7fffffffu) - small >= infinite - small) v = chain(p, m, n, v);
   p.c[(size_t)m * p.ldc + n] = v;
 }
 

@@ -72,6 +72,27 @@ def test_values_that_are_not_finite_come_out_as_from_the_chain():
     assert bool(((out.double() - ref.double()).abs() <= 2 * 1024 * 2.0 ** -24 * scale)[~bad].all())
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 256, 1024), (50, 200, 2048), (177, 2048, 1028)])
+@pytest.mark.parametrize("binade", [-95, -108, -112, -118, -124])
+@pytest.mark.parametrize("side", ["rows", "weights", "some rows"])
+def test_operands_whose_last_parts_bfloat16_cannot_hold(M, N, K, binade, side):
+    """Below 2^-110 the third part of an operand has fewer than eight bits: results that are made of such operands are as close as the
+    chain's, and rows beside them are what they are without them."""
+    from kv_cache_optimization_for_llm_b200 import ops
+    x, w = _draw(M, N, K, M + N + K)
+    plain = ops.linear(x, w)
+    tiny = torch.zeros(M, dtype=torch.bool, device="cuda")
+    tiny[::2 if side == "some rows" else 1] = True
+    if side == "weights":
+        w = w * 2.0 ** binade
+    else:
+        x = torch.where(tiny[:, None], x * 2.0 ** binade, x)
+    out, ref, by_chain = ops.linear(x, w), x.double() @ w.double().T, _chain(x, w)
+    err, chain = ((t.double() - ref)[tiny].norm() / ref[tiny].norm() for t in (out, by_chain))
+    assert err <= 1.05 * chain + 2.0 ** -25, (float(err), float(chain))
+    assert torch.equal(out[~tiny], plain[~tiny])
+
+
 def test_products_that_the_parts_do_not_take_go_to_the_chain():
     from kv_cache_optimization_for_llm_b200 import ops
     x, w = _draw(20, 64, 1032, 1)
