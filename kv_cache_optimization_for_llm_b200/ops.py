@@ -2030,6 +2030,7 @@ def experts_grouped(x: torch.Tensor, first: torch.Tensor, down: torch.Tensor, ga
         c_int(top), c_float(limit), c_float(shared_limit), c_float(alpha), c_float(offset), c_int(1 if weigh_output else 0), _p(lists),
         _p(xg), _p(act), _p(shared_act), _p(rows), _p(rows_of), _p(kernel_status(x.device)), _stream())
     _check(rc, "experts_grouped")
+    _count_more(3)              # lists, gathered rows, both products
     shared = _library_product(shared_act, down[:, experts * ff:experts * ff + shared_ff], torch.float32)
     rc = lib("experts_grouped").kvb_experts_join(_p(shared), _p(rows), _p(rows_of), _p(out), c_int(T), c_int(H), c_int(top), _stream())
     _check(rc, "experts_join")
@@ -2218,7 +2219,9 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, into: Op
                 rc = lib("gemm_f32").kvb_sgemm_nt_split(_p(x), c_int(x.stride(0)), _p(w), c_int(w.stride(0)), _p(out), c_int(N),
                                                         c_int(M), c_int(N), c_int(K), _p(parts), _p(kernel_status(x.device)), _stream())
             _check(rc, "sgemm_nt")
+            _count_more(1)              # A's parts, the product
             choices["sgemm_nt"] += 1
+            choices["sgemm_nt_split"] += 1
             return out
         rc = lib("gemm_f32").kvb_sgemm_nt(_p(x), c_int(x.stride(0)), _p(w), c_int(w.stride(0)), _p(out),
                                           c_int(N), c_int(M), c_int(N), c_int(K), _stream())

@@ -35,7 +35,9 @@ def test_split_product_is_as_close_as_a_chain_of_fma(M, N, K, spread):
     from kv_cache_optimization_for_llm_b200 import ops
     x, w = _draw(M, N, K, M + N + K, spread)
     assert ops.float32_split_ok(w)
+    before = ops.choices["sgemm_nt_split"]
     out, ref = ops.linear(x, w), x.double() @ w.double().T
+    assert ops.choices["sgemm_nt_split"] == before + 1
     scale = x.double().abs() @ w.double().abs().T
     err, chain = ((t.double() - ref).norm() / ref.norm() for t in (out, _chain(x, w)))
     assert err <= 1.05 * chain + 2.0 ** -25, (float(err), float(chain))
@@ -98,4 +100,6 @@ def test_products_that_the_parts_do_not_take_go_to_the_chain():
     x, w = _draw(20, 64, 1032, 1)
     for v in (w[:, :1020], w[:, 1:1029], w[:, :1030]):      # short, off 16 bytes, no multiple of four
         assert not ops.float32_split_ok(v)
+        before = ops.choices["sgemm_nt_split"]
         assert torch.equal(ops.linear(x[:, :v.shape[1]], v), _chain(x[:, :v.shape[1]], v))
+        assert ops.choices["sgemm_nt_split"] == before
