@@ -101,6 +101,17 @@ def test_made_rows_with_keys_wider_than_values_on_tcgen05(heads, dim, rot, vdim,
     assert ops.choices["flash_attention_rows_masked"] > before
 
 
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank,sink,window", [
+    (2, 96, 32, 128, 64, True, None), (3, 32, 32, 64, 72, False, 100), (2, 64, 64, 128, 64, True, 70)])
+def test_made_rows_of_equal_sizes_with_a_rotated_part_on_tcgen05(heads, dim, rot, vdim, rank, sink, window, monkeypatch):
+    """Steps with tiles enough to fill the GPU take this kernel; here every step does."""
+    from kv_cache_optimization_for_llm_b200 import ops
+    monkeypatch.setattr(ops, "FLASH_ROWS_WIDE", 3)
+    before = ops.choices["flash_attention_rows_masked"]
+    test_made_rows_with_a_rotated_part(heads, dim, rot, vdim, rank, sink, False, window)
+    assert ops.choices["flash_attention_rows_masked"] > before
+
+
 @pytest.mark.parametrize("scale", [0.0, -0.07])
 def test_scales_that_the_tcgen05_kernel_refuses_stay_on_the_other(scale):
     from kv_cache_optimization_for_llm_b200 import ops
