@@ -60,7 +60,7 @@ def test_the_single_tokens_launch_waits_for_all_in_front_and_is_waited_for(monke
 
 
 def test_below_the_line_one_launch_comes_after_the_other(monkeypatch):
-    assert _step(monkeypatch, line=1e30) == [("kvb_rope_kv_write", MAIN), ("kvb_paged_flash_attention", MAIN), ("kvb_decode_attention_mma", MAIN)]
+    assert _step(monkeypatch, line=1e30) == [("kvb_decode_attention_mma", MAIN), ("kvb_rope_kv_write", MAIN), ("kvb_paged_flash_attention", MAIN)]
 
 
 @pytest.mark.parametrize("width,singles,runs,wanted", [     # (start, tokens) of the runs
