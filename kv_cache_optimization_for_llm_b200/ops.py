@@ -13,8 +13,8 @@ every matrix product of the float32 path, is a kernel of this package.
 from __future__ import annotations
 
 import collections
-import contextlib
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_uint, c_void_p
 from typing import Dict, Optional
@@ -1992,19 +1992,44 @@ def limited_act(p: torch.Tensor, gate: Optional[torch.Tensor], shared_logit: Opt
     return out
 
 
-# From this much dense work (tokens x width x experts x features of each) on, each expert's matrices are multiplied with the tokens that chose
-# it.  32 experts of which a token uses 4, width 2048, 256 features (us a call, grouped / dense): 640 tokens 101 / 93, 1024 tokens 111 / 117, 2048
-# tokens 157 / 234; width 1024, 128 features, 2048 tokens 96 / 84 (five launches more, each of which the host pays for as well).
-GROUPED_MIN_WORK = 15_000_000_000
+# A line of tokens x width x experts x features of each from which on experts' products are grouped, instead of what is estimated (None).
+GROUPED_MIN_WORK: Optional[int] = None
+
+
+def experts_grouped_faster(tokens: int, hidden: int, experts: int, ff: int, shared_ff: int, top: int) -> bool:
+    """Whether each expert's matrices are multiplied with the tokens that chose it (:func:`experts_grouped`) rather than with all of them: by
+    estimates of both (us on the GPU) fitted to 130 steps (8 to 256 experts of 128 to 2048 features of which a token uses 1 to 16, a shared
+    one of 128 to 4096, widths of 512 to 4096, 128 to 4096 tokens; 7 and 12 % off).  All tokens: the products, the activation's bytes, the
+    weights.  Grouped: rounds of tiles of 128 rows over the SMs (half a tile is wasted on average an expert), the chosen rows' copies and
+    float32 results, the shared expert's last product, looking for the tokens, the weights.  Only where the estimate is a tenth less: 62 of those steps,
+    one of them slower (9 %), and 3 that would have been faster by more than 5 % are left out.  By dense work alone, as before, 11 of 81 were slower,
+    and 64 experts of 128 features of which a token uses 16, width 2048, took 377 us against 300 (3577 tokens)."""
+    if GROUPED_MIN_WORK is not None:
+        return tokens * hidden * experts * ff >= GROUPED_MIN_WORK
+    return _grouped_estimate(tokens, hidden, experts, ff, shared_ff, top)
+
+
+@functools.lru_cache(maxsize=1024)
+def _grouped_estimate(tokens: int, hidden: int, experts: int, ff: int, shared_ff: int, top: int) -> bool:
+    rows, inner = tokens * top, experts * ff + shared_ff
+    weights = 6e-6 * hidden * inner
+    dense = 24.0 + 0.54 * 6e-9 * tokens * hidden * inner + 1.45e-6 * tokens * inner + 0.089 * weights
+    tiles = rows / 128.0 + min(experts, rows) / 2.0
+    first = max(1.0, (tiles * (ff / 128.0) + -(-tokens // 128) * (shared_ff / 128.0)) / 148.0)
+    second = max(1.0, tiles * -(-hidden // 256) / 148.0)
+    grouped = (57.0 + 0.23 * first * hidden / 64.0 + 0.38 * second * ff / 64.0 + 2e-6 * rows * hidden + 3.5e-9 * tokens * shared_ff * hidden
+               + 6e-5 * experts * tokens + 0.138 * weights)
+    return grouped < 0.9 * dense
 
 
 def experts_grouped_ok(x: torch.Tensor, first: torch.Tensor, down: torch.Tensor, experts: int, ff: int, shared_ff: int, top: int) -> bool:
-    """Whether :func:`experts_grouped` takes this step: bfloat16, many tokens, every token uses a quarter of the experts at most (or all
-    tokens' rows would be no less work than every expert's product), sizes that its tiles divide."""
-    return (x.dtype == torch.bfloat16 and x.shape[0] * x.shape[1] * experts * ff >= GROUPED_MIN_WORK and 4 * top <= experts <= 256 and top <= 16 and ff % 128 == 0
-            and ff > 0 and shared_ff % 128 == 0 and shared_ff > 0 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+    """Whether :func:`experts_grouped` takes this step: bfloat16, tokens enough for it to be the faster form, every token uses a quarter of
+    the experts at most, a shared expert (whose last product the chosen rows join), sizes that its tiles divide."""
+    return (x.dtype == torch.bfloat16 and 4 * top <= experts <= 256 and top <= 16 and ff % 128 == 0 and ff > 0 and shared_ff % 128 == 0
+            and shared_ff > 0 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
             and first.is_contiguous() and down.is_contiguous() and down.shape[1] % 8 == 0
-            and (x.data_ptr() | first.data_ptr() | down.data_ptr()) % 16 == 0)
+            and (x.data_ptr() | first.data_ptr() | down.data_ptr()) % 16 == 0
+            and experts_grouped_faster(x.shape[0], x.shape[1], experts, ff, shared_ff, top))
 
 
 def experts_grouped_widths(hidden: int, experts: int, ff: int, shared_ff: int, top: int) -> int:

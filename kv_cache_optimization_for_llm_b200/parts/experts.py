@@ -186,10 +186,13 @@ class LimitedExperts(Part):
         if ctx.dtype == torch.bfloat16 and self.small.shape[0] % 8:
             self.small = torch.cat([self.small, self.small.new_zeros((-self.small.shape[0] % 8, self.hidden))], dim=0).contiguous()
 
-    def activation_widths(self):
-        inner = self.E * self.F + self.S
-        dense, grouped = 3 * inner + self.pad, ops.experts_grouped_widths(self.hidden, self.E, self.F, self.S, self.top)
-        return [max(dense, grouped), 4 * (self.E + 1) + 2 * self.small.shape[0], self.hidden]
+    widths_by_tokens = True
+
+    def activation_widths(self, tokens=None):
+        inner, grouped = self.E * self.F + self.S, 0
+        if self.ctx.dtype == torch.bfloat16 and (tokens is None or ops.experts_grouped_faster(tokens, self.hidden, self.E, self.F, self.S, self.top)):
+            grouped = ops.experts_grouped_widths(self.hidden, self.E, self.F, self.S, self.top)
+        return [max(3 * inner + self.pad, grouped), 4 * (self.E + 1) + 2 * self.small.shape[0], self.hidden]
 
     def forward(self, x, batch):
         logits = ops.linear(x, self.small, out_dtype=torch.float32)
