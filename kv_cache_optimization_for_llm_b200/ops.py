@@ -484,10 +484,46 @@ def _at(t: torch.Tensor, col: int) -> int:
     return t.data_ptr() + col * t.element_size()
 
 
-# Longest run of a step, in tokens, from which on the walk's products that do not wait for the state are made for all pieces at once
-# (delta_pieces.cuh; keys of 64, values of 32 or 64).  32 heads, the launches of either form in us (three / one): a run of 64 24 / 12, of 400
-# about 35 / 48, of 1024 79 / 110, 1548 + 500 134 / 206; the host pays for two launches more (7 us a layer), which shows in steps below.
-DELTA_PIECES_MIN_RUN = 512
+# The longest run from which on a delta rule's walk goes in three launches, instead of what is estimated (None).
+DELTA_PIECES_MIN_RUN: Optional[int] = None
+
+
+def delta_pieces_faster(runs, heads: int, dv: int, captured: bool) -> bool:
+    """Whether the walk's products that do not wait for the state are made for all pieces at once, in three launches (delta_pieces.cuh; keys of
+    64, values of 32 or 64), for runs of these lengths, the longest of at least 512 tokens: by estimates of both forms (us on the GPU) fitted to 198 steps (4 to 64
+    heads, runs of 60 to 3000 tokens, up to 16 of them; 8 and 7 % off).  In one launch: a run's pieces one after the other, blocks of 16 or 32
+    columns a run and head in rounds over the SMs (with most SMs busy a piece takes longer).  In three: rounds of preparing blocks, the results'
+    bytes, the chain.  Launched by hand, two launches more cost the host 10 us, which shows in layers of less than about 85 us; the
+    layer's products are counted in for that.  Of those steps 94 are taken, 4 of them 2 to 4 % slower; by the longest run alone 29 of 121
+    were slower, by up to 14 % (8 heads of 64, 512 tokens: 98 us against 87).  Captured: 116 taken, one of them 4 % slower."""
+    pieces = [-(-n // 64) for n in runs]
+    longest, blocks32 = max(pieces), heads * (dv // 32) * len(pieces)
+    wide = blocks32 * 5 >= 148 * 4                         # as the launchers choose their blocks' columns
+    blocks = blocks32 if wide else 2 * blocks32
+    total = sum(pieces) * heads
+    work = total * (blocks // (heads * len(pieces))) / 148.0
+    turns = longest if blocks <= 148 else max(longest, work + 0.5 * longest)
+    busy = max(0.0, min(1.0, work / turns) - 0.5)
+    one = 8.8 + turns * ((6.4 if wide else 4.9) + 6.9 * busy)
+    three = 7.6 + 19.0 * max(1.0, total / 592.0) + 7.2 * total * dv / (64.0 * 148.0) + turns * (2.15 if wide else 1.6)
+    if captured:
+        return three < one
+    return three < 0.95 * one and one + 1.4e-5 * sum(runs) * heads * dv >= 77.0
+
+
+def _delta_pieces_wanted(batch, heads: int, dv: int) -> bool:
+    longest = int(getattr(batch, "max_q_len", 0) or 0)
+    if DELTA_PIECES_MIN_RUN is not None:
+        return longest >= DELTA_PIECES_MIN_RUN
+    if longest < 512:
+        return False
+    captured = _capturing()
+    known = batch.host.setdefault("delta_pieces", {})       # asked once a step
+    key = (heads, dv, captured)
+    if key not in known:
+        starts = batch.host["q_start"]
+        known[key] = delta_pieces_faster([int(starts[r + 1] - starts[r]) for r in range(int(batch.num_single), batch.num_reqs)], heads, dv, captured)
+    return known[key]
 
 
 GRID_MAX_Y = 65535      # blocks of a grid's second dimension: pieces (and heads) that the walks in three launches can have
@@ -510,7 +546,7 @@ def _with_scratch(nbytes: int, device, call):
 def delta_pieces_width(heads: int, dk: int, dv: int, tokens: Optional[int] = None) -> int:
     """bfloat16 elements per token that :func:`delta_scan` wants for its scratch in steps of long runs; 0 where steps of up to ``tokens``
     tokens hold no such run."""
-    if dk != 64 or dv not in (32, 64) or (tokens is not None and tokens < DELTA_PIECES_MIN_RUN):
+    if dk != 64 or dv not in (32, 64) or (tokens is not None and tokens < (512 if DELTA_PIECES_MIN_RUN is None else DELTA_PIECES_MIN_RUN)):
         return 0
     fn = lib("delta_rule").kvb_delta_walk_scratch
     fn.restype = c_longlong
@@ -520,7 +556,7 @@ def delta_pieces_width(heads: int, dk: int, dv: int, tokens: Optional[int] = Non
 def _delta_pieces_bytes(batch, tokens: int, heads: int, dk: int, dv: int, device) -> int:
     """Bytes of scratch for the form in three launches, 0 where the runs walk in one (short runs, other sizes, or an arena without the
     room)."""
-    if dk != 64 or dv not in (32, 64) or int(getattr(batch, "max_q_len", 0) or 0) < DELTA_PIECES_MIN_RUN:
+    if dk != 64 or dv not in (32, 64) or not _delta_pieces_wanted(batch, heads, dv):
         return 0
     runs = batch.num_reqs - int(batch.num_single)
     if tokens // 64 + runs > GRID_MAX_Y:
@@ -543,7 +579,7 @@ def delta_scan(mode: str, batch, state: torch.Tensor, r, k, v, gate, decay, aux,
     ``decay_per_head`` ("gated"): ``decay`` is [T, heads] and ``decay_bias`` [heads], one decay for all key
     channels of a head.  ``gate_act``: "sigmoid" or "silu", the function applied to the output gate.
     bfloat16 steps with runs above :func:`walk_line` and one decay per head go to the walk on tensor cores where the sizes allow,
-    in three launches from runs of ``DELTA_PIECES_MIN_RUN`` tokens on.
+    in three launches where that is estimated to be faster (:func:`delta_pieces_faster`).
     Returns the gated, normed read-out [T, heads * dv]."""
     x0 = r[0]
     _need_cuda(x0, state)

@@ -31,13 +31,14 @@ def test_scratch_is_declared_where_a_step_can_take_it(kind, params, heads, token
 @pytest.mark.parametrize("rule", ["ssd", "delta"])
 @pytest.mark.parametrize("runs", [1, 40])
 @pytest.mark.parametrize("taken", [0.0, 0.9])
-def test_a_step_without_the_room_left_walks_in_one_launch(rule, runs, taken):
+def test_a_step_without_the_room_left_walks_in_one_launch(rule, runs, taken, monkeypatch):
     """A layer's region of which other tensors hold a part, and a step of many short runs beside a long one, whose pieces are more than
     its tokens'."""
     from types import SimpleNamespace
     from kv_cache_optimization_for_llm_b200 import ops
     from kv_cache_optimization_for_llm_b200.engine.arena import StepArena
     device, tokens = torch.device("cpu"), 2048
+    monkeypatch.setattr(ops, "DELTA_PIECES_MIN_RUN", 512)
     batch = SimpleNamespace(max_q_len=1024, num_reqs=runs, num_single=0)
     width = ops.pieces_width("ssd", 64, 128, 64) if rule == "ssd" else ops.delta_pieces_width(32, 64, 64)
     arena = StepArena(device, 1 << 16, int(1.2 * 2 * tokens * width))
@@ -54,10 +55,11 @@ def test_a_step_without_the_room_left_walks_in_one_launch(rule, runs, taken):
 
 
 @pytest.mark.parametrize("tokens,runs,heads,wanted", [(4096, 4, 64, True), (64 * 65000, 600, 64, False), (4096, 65500, 64, False)])
-def test_grids_beyond_the_hardwares_limit_walk_in_one_launch(tokens, runs, heads, wanted):
+def test_grids_beyond_the_hardwares_limit_walk_in_one_launch(tokens, runs, heads, wanted, monkeypatch):
     """More pieces than a grid's second dimension holds, which the walk in one launch, a block a run, takes."""
     from types import SimpleNamespace
     from kv_cache_optimization_for_llm_b200 import ops
+    monkeypatch.setattr(ops, "DELTA_PIECES_MIN_RUN", 512)
     batch = SimpleNamespace(max_q_len=1024, num_reqs=runs, num_single=0)
     assert (ops._delta_pieces_bytes(batch, tokens, heads, 64, 64, torch.device("cpu")) > 0) == wanted
     assert (ops._pieces_bytes("ssd", batch, tokens, heads, 128, 64, torch.device("cpu")) > 0) == wanted
