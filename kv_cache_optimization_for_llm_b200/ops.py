@@ -2068,8 +2068,11 @@ def experts_grouped_ok(x: torch.Tensor, first: torch.Tensor, down: torch.Tensor,
             and experts_grouped_faster(x.shape[0], x.shape[1], experts, ff, shared_ff, top))
 
 
-def experts_grouped_widths(hidden: int, experts: int, ff: int, shared_ff: int, top: int) -> int:
-    """Elements of the compute type a token of such a step needs beside its output."""
+def experts_grouped_widths(hidden: int, experts: int, ff: int, shared_ff: int, top: int, tokens: Optional[int] = None) -> int:
+    """Elements of the compute type a token of such a step needs beside its output; 0 where no step of up to ``tokens`` tokens is one
+    (looked at every eighth of a binade: the grouped form can be the faster one in between only)."""
+    if tokens is not None and not any(experts_grouped_faster(int(tokens * 2.0 ** (-i / 8)), hidden, experts, ff, shared_ff, top) for i in range(64)):
+        return 0
     return top * ff + shared_ff + (3 * top + 2) * hidden + 4 * experts + 2 * top + 64
 
 

@@ -190,8 +190,8 @@ class LimitedExperts(Part):
 
     def activation_widths(self, tokens=None):
         inner, grouped = self.E * self.F + self.S, 0
-        if self.ctx.dtype == torch.bfloat16 and (tokens is None or ops.experts_grouped_faster(tokens, self.hidden, self.E, self.F, self.S, self.top)):
-            grouped = ops.experts_grouped_widths(self.hidden, self.E, self.F, self.S, self.top)
+        if self.ctx.dtype == torch.bfloat16:
+            grouped = ops.experts_grouped_widths(self.hidden, self.E, self.F, self.S, self.top, tokens)
         return [max(3 * inner + self.pad, grouped), 4 * (self.E + 1) + 2 * self.small.shape[0], self.hidden]
 
     def forward(self, x, batch):

@@ -14,3 +14,13 @@ def test_the_faster_form(sizes, grouped, dense):
     from kv_cache_optimization_for_llm_b200 import ops
     H, E, top, F, S, T = sizes
     assert ops.experts_grouped_faster(T, H, E, F, S, top) == (grouped < dense)
+
+
+@pytest.mark.parametrize("most", [100, 900, 1430, 4096])
+@pytest.mark.parametrize("sizes", [(2048, 32, 4, 256, 2048), (2048, 64, 16, 128, 512), (1024, 8, 2, 768, 2048), (2048, 8, 2, 512, 128), (4096, 8, 1, 256, 1024),
+                                   (2048, 256, 16, 128, 128), (512, 128, 3, 512, 4096), (3072, 16, 4, 256, 512)])
+def test_room_is_declared_where_some_step_is_grouped(sizes, most):
+    from kv_cache_optimization_for_llm_b200 import ops
+    H, E, top, F, S = sizes
+    grouped = any(ops.experts_grouped_faster(t, H, E, F, S, top) for t in range(1, most + 1))
+    assert (ops.experts_grouped_widths(H, E, F, S, top, most) > 0) == grouped
