@@ -8,7 +8,7 @@
 //   1. prepare   a block per (piece, head): gates, key norms, A, its inverse, W (three bfloat16 parts) and U0;
 //   2. chain     a block per (run, head, 16 or 32 value columns) walks the pieces: U = U0 - W S, S <- P_63 S + sum_j (P_63 / P_j) k_j u_j^T;
 //                it leaves U and the state that every piece begins with;
-//   3. results   a block per (piece, head, 64 columns): o_i = P_i S^T q_i + sum_{j <= i} (P_i / P_j) (q_i . k_j) u_j.
+//   3. results   a block per (piece, head, 32 columns): o_i = P_i S^T q_i + sum_{j <= i} (P_i / P_j) (q_i . k_j) u_j.
 //
 // The products are those of the walk, operand for operand: bfloat16 ones as they came, float32 ones in three parts, sums over more than a
 // block of 16 added up by float32 instructions.  What is not finite is left out of them in the same way (first tokens of a piece whose
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(DVC * 8) chain_kernel(const Args p, const Scra
     }
 }
 
-// A block makes CB columns (a multiple of 16) of one (piece, head): a warp for 16 tokens of 32 (16) of them.
+// A block makes 32 columns of one (piece, head): a warp for 16 tokens.
 struct ResultsLayout {
   static constexpr int PN = pitch(kN);
   static constexpr int K = 0;

@@ -329,9 +329,6 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
 }  // namespace f32s
 
-// bfloat16 elements of the parts that kvb_sgemm_nt_split wants room for
-KVB_EXPORT long long kvb_sgemm_nt_split_scratch(int M, int K) { return 3ll * M * ((K + 7) / 8 * 8); }
-
 // Blocks of a cluster that share K: as many as keep the SMs busy with one tile of rows and leave each at least 512 k.
 static int kvb_split_blocks(int N, int K) {
   const int tiles = (N + f32s::kRows - 1) / f32s::kRows, k_blocks = (K + f32s::kBlockK - 1) / f32s::kBlockK;
@@ -340,8 +337,8 @@ static int kvb_split_blocks(int N, int K) {
   return s;
 }
 
-// C = A . W^T.  W and its rows on 16-byte boundaries, K a multiple of 4; A any alignment; parts: kvb_sgemm_nt_split_scratch(M, K)
-// bfloat16 elements on a 16-byte boundary.
+// C = A . W^T.  W and its rows on 16-byte boundaries, K a multiple of 4; A any alignment; parts: room for 3 M (K rounded up to 8) bfloat16
+// elements on a 16-byte boundary.
 KVB_EXPORT int kvb_sgemm_nt_split(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
                                   void* parts, int* status, cudaStream_t stream) {
   using namespace f32s;

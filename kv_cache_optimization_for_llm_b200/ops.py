@@ -1010,14 +1010,13 @@ def paged_attention_tiles_supported(qkv, k_pages, v_pages, d: int, group: int) -
 
 def paged_attention_tiles_wanted(req_start, ctx_len, nq: int, nkv: int, d: int, window: int, sms: int) -> bool:
     """Whether a float32 step (the positions that its requests start at and end before) is sooner done over tiles of queries than a
-    (token, head) a block.  A tile's chain of 128 keys a turn is long (at head size 64: 15 us for eight rows and the first 128 keys,
-    31 for 64 rows; 8 and 19 for every further turn) and its blocks may be few; a (token, head)'s is short, but all of them
-    read the keys again.  Both are estimated as the longest chain or all work over the SMs, whichever is longer; the numbers are
-    fits to 190 measured steps (2 to 1024 tokens, 2 to 64 heads of 32 to 128).  Without it steps of a few short
-    prompts, and grids of few blocks, took up to 2.5 times as long over tiles (two prompts of 9 tokens, 8 heads over one: 27 us against 11; 16
-    tokens behind 3000 positions, 4 heads over one: 361 against 253); with it none of the 190 is slower than a
-    (token, head) a block.  The tiles have become about twice as fast since (two prompts of 9 tokens, 8 heads over one: 12 us against 7; 40
-    single tokens at 100 beside a run of 40: 15 against 39), so the line lies on the safe side of where they cross."""
+    (token, head) a block.  A tile's chain of 128 keys a turn is long and its blocks may be few; a (token, head)'s is short, but all of them
+    read the keys again.  Both are estimated as the longest chain or all work over the SMs, whichever is longer.  The numbers are
+    fits to 190 steps (2 to 1024 tokens, 2 to 64 heads of 32 to 128) with tiles that took twice as long as they do now, so the line lies on
+    the safe side of where the two cross: of 150 other steps none over tiles is slower than a (token, head) a block, and 22 of those left to that
+    are slower by more than a tenth.  us, tiles / a (token, head) a block, 8 heads of 64 over one: two prompts of 9 tokens 12 / 7 (left to
+    the latter), 40 single tokens at 100 beside a run of 40 16 / 30 and 16 tokens behind 3000 positions 235 / 301 (left to it too); 32 heads over 8
+    there 240 / 696 (tiles)."""
     group, f = nq // nkv, d / 64.0
     tokens = paged_attention_tile_tokens(d, group)
     first, each_first, turn, each = 6.0 + 0.1 * d, 0.9 + 0.0195 * d, 2.2 + 0.07 * d, 0.9 + 0.0135 * d
@@ -1182,7 +1181,8 @@ def flash_attention_rows(q: torch.Tensor, pages: torch.Tensor, block_table, batc
     return out
 
 
-# (key, value) sizes of rows made for a step that the tcgen05 kernel takes beside equal ones.  It is the faster one at every number of
+# (key, value) sizes of rows made for a step that the tcgen05 kernel takes beside equal ones: the sizes that it is built and was measured for;
+# others of whole 16s would each be a form of their own.  It is the faster one at every number of
 # tiles (16 heads of 192 | 128, the attention in us, this / mma.sync: a run of 300 behind 1400 96 / 122, of 1000 70 / 95, of 2048 100 / 211;
 # 16 heads of 96 | 64: 68 / 86, 63 / 63, 73 / 102).
 MADE_WIDER = ((192, 128), (96, 64))
