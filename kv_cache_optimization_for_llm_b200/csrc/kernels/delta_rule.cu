@@ -602,7 +602,9 @@ template <> struct Quad<__nv_bfloat16> {
 // every input once (the window moves through registers).  What bounds it: bytes (2048 tokens of 6144 channels in bfloat16: 50 MB, 8 us)
 // and, before that, instructions.  Rows whose window lies in one request, nearly all, need no look at requests and positions; four
 // channels a thread (8-byte loads) leave room for twice the threads that eight did.  In a layer 2048 tokens of 6144 channels 39 -> 27 us, of
-// 3072 channels 26 -> 17.  Four blocks an SM (64 registers) would spill.
+// 3072 channels 26 -> 17.  Four blocks an SM (64 registers) would spill.  Rows of several requests look at their window as it lies in
+// registers, too; a bit says where one request ends (looking rows up in memory again: 1200 tokens in runs of 5, 6144 channels in
+// float32 52 us, now 45; in bfloat16 43, now 38).
 constexpr int kConvTokens = 8;
 
 template <typename T, int TAPS>
@@ -677,8 +679,17 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
     }
     return;
   }
-  // rows of several requests, or a request's first: row by row, from the step's rows or the request's tail
-  for (int t = t0; t <= t_last; ++t) {
+  // rows of several requests, or a request's first: from the step's rows or the request's tail
+  unsigned cut = 0;                            // bit i: rows i and i + 1 of the window are not both of one request
+#pragma unroll
+  for (int i = 0; i + 1 < kConvTokens + BACK; ++i) {
+    const int t = t0 - BACK + i;
+    if (t < 0 || t >= t_last || token_req[t] != token_req[t + 1]) cut |= 1u << i;
+  }
+#pragma unroll
+  for (int k = 0; k < kConvTokens; ++k) {
+    const int t = t0 + k;
+    if (t > t_last) break;
     const int r = token_req[t], pos = positions[t];
     float acc[VEC];
 #pragma unroll
@@ -687,8 +698,8 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
     for (int j = 0; j < TAPS; ++j) {
       const int back = BACK - j;
       float v[VEC];
-      if (t - back >= 0 && token_req[t - back] == r) {
-        Quad<T>::unpack(*reinterpret_cast<const Raw*>(in + (size_t)(t - back) * ld + c), v);
+      if ((cut >> (k + j) & ((1u << back) - 1u)) == 0u) {
+        Quad<T>::unpack(x[k + j], v);
       } else {
         const int sp = pos - back, start = req_start[r];
         const float* tp = tails + (size_t)slots[r] * slot_stride + (long long)(sp - (start - BACK)) * C + c;
@@ -765,9 +776,9 @@ KVB_EXPORT int kvb_conv_silu(const void* in, int ld, const float* w, int taps, f
              in_bias, out_bias)
     // blocks of tokens from where they give every SM most of a block of threads (measured, with the tails' launch, a token a thread /
     // blocks: 600 tokens of 1536 channels 11.3 / 11.1 us, 1024 of 1536 13.6 / 11.8, 300 of 3072 10.9 / 11.3, 600 of 3072 16.2 / 11.6, 100 of
-    // 6144 8.4 / 10.1, 200 of 6144 12.4 / 11.7)
+    // 6144 8.4 / 10.1, 200 of 6144 12.4 / 11.7; float32: 1152 tokens of 1024 channels 9.1 / 10.5, 1000 of 1536 10.3 level)
     const long long run_units = (long long)((T_ + kConvTokens - 1) / kConvTokens) * (C / 4);
-    const bool runs = w16 && taps >= 2 && taps <= 4 && run_units >= 224ll * kvb_sm_count();
+    const bool runs = w16 && taps >= 2 && taps <= 4 && run_units >= (dtype == KVB_F32 ? 256ll : 224ll) * kvb_sm_count();
 #define KVB_CONV_RUN(TAPS)                                                                                              \
   kvb_launch(conv_run_kernel<T, TAPS>, dim3((unsigned)((run_units + 255) / 256)), dim3(256), 0, stream, (const T*)in, ld, w, \
              (const float*)tails, slot_stride, (T*)out, C, T_, positions, token_req, req_start, slots, act, ap, in_bias, out_bias)
