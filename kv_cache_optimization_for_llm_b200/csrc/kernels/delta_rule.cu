@@ -602,9 +602,10 @@ template <> struct Quad<__nv_bfloat16> {
 // every input once (the window moves through registers).  What bounds it: bytes (2048 tokens of 6144 channels in bfloat16: 50 MB, 8 us)
 // and, before that, instructions.  Rows whose window lies in one request, nearly all, need no look at requests and positions; four
 // channels a thread (8-byte loads) leave room for twice the threads that eight did.  In a layer 2048 tokens of 6144 channels 39 -> 27 us, of
-// 3072 channels 26 -> 17.  Four blocks an SM (64 registers) would spill.  Rows of several requests look at their window as it lies in
-// registers, too; a bit says where one request ends (looking rows up in memory again: 1200 tokens in runs of 5, 6144 channels in
-// float32 52 us, now 45; in bfloat16 43, now 38).
+// 3072 channels 26 -> 17.  Four blocks an SM (64 registers) would spill.  A bit of rows of several requests
+// says where one request ends; float32 takes them from registers, bfloat16 from the caches in a loop that is not unrolled (its steps are
+// short enough for the larger code to show: a delta layer of 2048 tokens 218 us, 219.5 with it).  Looking each row's request up in memory:
+// 1200 tokens in runs of 5, 6144 channels in float32 52 us, now 45.
 constexpr int kConvTokens = 8;
 
 template <typename T, int TAPS>
@@ -686,11 +687,8 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
     const int t = t0 - BACK + i;
     if (t < 0 || t >= t_last || token_req[t] != token_req[t + 1]) cut |= 1u << i;
   }
-#pragma unroll
-  for (int k = 0; k < kConvTokens; ++k) {
-    const int t = t0 + k;
-    if (t > t_last) break;
-    const int r = token_req[t], pos = positions[t];
+  auto row_of_several = [&](int k, auto window) {            // window(i): row t0 - BACK + i
+    const int t = t0 + k, r = token_req[t], pos = positions[t];
     float acc[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; ++e) acc[e] = ob[e];
@@ -699,7 +697,7 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
       const int back = BACK - j;
       float v[VEC];
       if ((cut >> (k + j) & ((1u << back) - 1u)) == 0u) {
-        Quad<T>::unpack(x[k + j], v);
+        Quad<T>::unpack(window(k + j), v);
       } else {
         const int sp = pos - back, start = req_start[r];
         const float* tp = tails + (size_t)slots[r] * slot_stride + (long long)(sp - (start - BACK)) * C + c;
@@ -714,6 +712,17 @@ conv_run_kernel(const T* __restrict__ in, int ld, const float* __restrict__ w, c
       for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wv[e * TAPS + j], v[e], acc[e]);
     }
     finish(t, acc);
+  };
+  if (sizeof(T) == 4) {
+#pragma unroll
+    for (int k = 0; k < kConvTokens; ++k) {
+      if (t0 + k > t_last) break;
+      row_of_several(k, [&](int i) { return x[i]; });
+    }
+  } else {
+#pragma unroll 1
+    for (int k = 0; k <= t_last - t0; ++k)
+      row_of_several(k, [&](int i) { return *reinterpret_cast<const Raw*>(in + (size_t)(t0 - BACK + i) * ld + c); });
   }
 }
 
