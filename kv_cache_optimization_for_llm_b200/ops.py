@@ -1657,7 +1657,8 @@ def _walks(rule: str, batch, n: int, dv: int, x: torch.Tensor, *columns: int) ->
 # of 128 68 / 76; 32 heads: 300 24 / 18, 512 26 / 26, 2048 58 / 92, 300 + 300 26 / 34.  mlstm, 32 heads of 64 x 64: 300 20 / 17, 512 21 / 24, 2048 51 / 86,
 # 1111 + 700 + 237 51 / 68, eight of 128 35 / 43; 16 heads: 512 20 / 21, 700 22 / 27, 2048 37 / 70, 300 + 300 20 / 17, eight of 128 24 / 22.
 # On the device they cross at about 12000; but the host pays for two launches more (6 us a layer), which shows until a layer's kernels take
-# longer than the host (about 80 us), hence the line.
+# longer than the host (about 80 us), hence the line.  Below it, layers of width 1024 launched by hand (replayed from a graph), three / one:
+# 16 heads of 64 x 64, 512 tokens 91 / 81 (37 / 39), 1024 + 1000 93 / 84 (66 / 78), 2048 93 / 110 (68 / 103); 32 heads, 1000 tokens 92 / 85 (65 / 78).
 PIECES_MIN_WORK, PIECES_MIN_RUN = 40000, 256
 
 
